@@ -36,6 +36,8 @@
 // non-finite as the reference's do.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "kernels.cuh"
 
@@ -229,106 +231,214 @@ __device__ __forceinline__ unsigned long long* face_slot(const FaceBufs& f, uint
   return f.fz + ((uint64_t)gx * n + gy) * nt + gz / TB;
 }
 
-__global__ void __launch_bounds__(256) tile_deposit_kernel(
+// A particle's eight corner quanta (corner k at x + (k >> 2 & 1), y + (k >> 1
+// & 1), z + (k & 1)), which sum to exactly `whole`: the reference's products
+// (grid.c:627-650), (x, y) pairs times z (wz0, wz1: times the weight), each
+// rounded, and the remainder added to the first largest.
+__device__ __forceinline__ void corner_quanta(float tx, float ty, float wz0, float wz1,
+                                              float qscale, int whole, uint32_t (&q)[8]) {
+  const float wx0 = fsub(1.0f, tx), wy0 = fsub(1.0f, ty);
+  const float w00 = fmul(wx0, wy0), w01 = fmul(wx0, ty);
+  const float w10 = fmul(tx, wy0), w11 = fmul(tx, ty);
+  const float w[8] = {fmul(w00, wz0), fmul(w00, wz1), fmul(w01, wz0), fmul(w01, wz1),
+                      fmul(w10, wz0), fmul(w10, wz1), fmul(w11, wz0), fmul(w11, wz1)};
+  // w times a power of two is exact in float, so rounding it to an
+  // integer in float is the quantisation itself; GB300's FP64 rate is
+  // no place for it.
+  int sum = 0;
+  int big = 0;
+  float wbig = fabsf(w[0]);
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    const int qk = __float2int_rn(fmul(w[k], qscale));
+    q[k] = (uint32_t)qk;
+    sum += qk;
+    if (fabsf(w[k]) > wbig) {  // the first largest, as a scan from corner 0 finds it
+      wbig = fabsf(w[k]);
+      big = k;
+    }
+  }
+  const int fix = whole - sum;
+#pragma unroll
+  for (int k = 0; k < 8; k++) q[k] = (uint32_t)((int)q[k] + (k == big ? fix : 0));
+}
+
+constexpr int kWhole = 16777216;  // one particle, in quanta of 2^-24
+constexpr int kTileWords = TS * TS * TS;
+constexpr int kDepositT = 256;
+
+__device__ __forceinline__ uint32_t tile_cell(uint32_t local) {
+  return ((local >> 8) * TS + ((local >> 4) & 15u)) * TS + (local & 15u);
+}
+__device__ __forceinline__ uint32_t corner_offset(int k) {
+  return (uint32_t)(((k >> 2) & 1) * TS * TS + ((k >> 1) & 1) * TS + (k & 1));
+}
+
+// One cell of a tile's flush, at (a, b, c) of the 17^3: cells 1..TB-1 of the
+// tile (within the grid) are touched by no other tile and go straight to the
+// grid; the rest are shared with a neighbour.
+struct TileFlush {
+  uint32_t ox, oy, oz, ex, ey, ez;
+  __device__ __forceinline__ TileFlush(uint32_t tile, const CicGeom& g) {
+    const uint32_t nt = g.nt;
+    ox = tile / (nt * nt) * TB;
+    oy = (tile / nt) % nt * TB;
+    oz = tile % nt * TB;
+    ex = min((uint32_t)TB, g.n - ox);
+    ey = min((uint32_t)TB, g.n - oy);
+    ez = min((uint32_t)TB, g.n - oz);
+  }
+  __device__ __forceinline__ void put(uint32_t a, uint32_t b, uint32_t c, unsigned long long v,
+                                      const CicGeom& g, float qinv, float inv_cell_vol,
+                                      float* __restrict__ grid, const FaceBufs& faces) const {
+    if (a > ex || b > ey || c > ez) return;
+    const uint32_t gx = ox + a == g.n ? 0u : ox + a;
+    const uint32_t gy = oy + b == g.n ? 0u : oy + b;
+    const uint32_t gz = oz + c == g.n ? 0u : oz + c;
+    const bool interior = a >= 1 && a < ex && b >= 1 && b < ey && c >= 1 && c < ez;
+    if (interior) {
+      grid[((uint64_t)gx * g.n + gy) * g.n + gz] =
+          fmul(fmul(__ll2float_rn((long long)v), qinv), inv_cell_vol);
+    } else if (v != 0ull) {
+      atomicAdd(face_slot(faces, gx, gy, gz, g), v);
+    }
+  }
+};
+
+// The unweighted deposit, one CTA a tile at a time: the tile's sums as one
+// 32-bit word a cell, one shared atomic a corner. The kernel is bound by
+// those atomics, so the word's wraps are not watched add by add: every
+// quantum is non-negative (the weights are, and the remainder of a few quanta
+// goes to a corner of at least 2^21), so the words of a tile sum to its
+// particles times 2^24 exactly when none of them wrapped, and each wrap takes
+// 2^32 from that sum. A tile whose sum falls short (a cell of 256 particles or
+// more, in an unweighted count) is left to tile_deposit_wide_kernel, through
+// `redo` (redo[0] counts them), as is one with so many particles that one of
+// its cells must have wrapped.
+// (Two words a cell, as the wide kernel keeps, cost a second atomic a corner:
+// the 512^3 deposit 1.57 ms in 39 KB of shared memory a CTA.)
+__global__ void __launch_bounds__(kDepositT, 6) tile_deposit_kernel(
+    const float4* __restrict__ rec, const uint32_t* __restrict__ offsets, CicGeom g,
+    float inv_cell_vol, float* __restrict__ grid, FaceBufs faces, uint32_t* __restrict__ redo) {
+  __shared__ uint32_t acc[kTileWords];
+  __shared__ unsigned long long wsum[kDepositT / 32];
+  const uint32_t n_tiles = g.nt * g.nt * g.nt;
+  constexpr float qscale = (float)kWhole, qinv = 1.0f / (float)kWhole;
+  const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  // Cleared once; each flush leaves the cells it reads cleared for the next tile.
+  for (int i = threadIdx.x; i < kTileWords; i += kDepositT) acc[i] = 0u;
+  __syncthreads();
+  for (uint32_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+    const uint32_t s = offsets[tile], e = offsets[tile + 1];
+    if (e - s >= 256u * kTileWords) {  // a cell must pass 256 particles
+      if (threadIdx.x == 0) redo[1 + atomicAdd(redo, 1u)] = tile;
+      continue;
+    }
+    for (uint32_t p = s + threadIdx.x; p < e; p += kDepositT) {
+      const float4 r = __ldg(rec + p);
+      uint32_t q[8];
+      corner_quanta(r.x, r.y, fsub(1.0f, r.z), r.z, qscale, kWhole, q);
+      uint32_t* cell = acc + tile_cell(__float_as_uint(r.w));
+#pragma unroll
+      for (int k = 0; k < 8; k++) atomicAdd(cell + corner_offset(k), q[k]);
+    }
+    __syncthreads();
+    unsigned long long sum = 0;
+    for (int i = threadIdx.x; i < kTileWords; i += kDepositT) sum += acc[i];
+    // A lane's sum is below 20 * 2^32: in two parts whose warp sums fit.
+    const uint32_t lo = __reduce_add_sync(0xffffffffu, (uint32_t)sum & 0xfffffu);
+    const uint32_t hi = __reduce_add_sync(0xffffffffu, (uint32_t)(sum >> 20));
+    if (lane == 0) wsum[warp] = ((unsigned long long)hi << 20) + lo;
+    __syncthreads();
+    sum = 0;
+#pragma unroll
+    for (int w = 0; w < kDepositT / 32; w++) sum += wsum[w];
+    const bool whole = sum == (unsigned long long)(e - s) << 24;
+    if (!whole && threadIdx.x == 0) redo[1 + atomicAdd(redo, 1u)] = tile;
+
+    // The flush: 16 cells of a z row per half-warp, then the rows' last cells.
+    const TileFlush f(tile, g);
+    const uint32_t c = threadIdx.x & 15u;
+    for (uint32_t row = threadIdx.x >> 4; row < TS * TS; row += kDepositT / 16) {
+      const uint32_t v = acc[row * TS + c];
+      acc[row * TS + c] = 0u;
+      if (whole) f.put(row / TS, row % TS, c, v, g, qinv, inv_cell_vol, grid, faces);
+    }
+    for (uint32_t row = threadIdx.x; row < TS * TS; row += kDepositT) {
+      const uint32_t v = acc[row * TS + TB];
+      acc[row * TS + TB] = 0u;
+      if (whole) f.put(row / TS, row % TS, TB, v, g, qinv, inv_cell_vol, grid, faces);
+    }
+    __syncthreads();
+  }
+}
+
+// The deposit of any sums: weighted particles, and the tiles the kernel above
+// lists in `redo` (NULL: every tile). Two 32-bit words a cell: a 32-bit
+// shared atomic add is one instruction, a 64-bit one a compare-and-swap loop
+// (measured: the 512^3 deposit with one 64-bit add per corner took 3.4 ms,
+// against 1.7). A tile with fewer than 2^16 particles adds each quantum's low
+// 16 bits to the first word and its high bits (arithmetic shift) to the
+// second, neither of which can wrap (a cell takes one add per particle), with
+// adds that return nothing; a denser tile adds the whole quantum to the first
+// word and counts its wraps in the second (each add is below 2^32, so it wraps
+// at most once), which needs the old value back. Either pair is the exact
+// 64-bit sum whatever the order of the adds.
+__global__ void __launch_bounds__(kDepositT) tile_deposit_wide_kernel(
     const float4* __restrict__ rec, const uint32_t* __restrict__ offsets, CicGeom g,
     float inv_cell_vol, float* __restrict__ grid, FaceBufs faces,
-    const float* __restrict__ wrec, const unsigned* __restrict__ wmax) {
-  // The tile's sums as two 32-bit words a cell: a 32-bit shared atomic add is
-  // one instruction, a 64-bit one a compare-and-swap loop (measured: the
-  // 512^3 deposit with one 64-bit add per corner took 3.4 ms, against 1.7). A tile with fewer
-  // than 2^16 particles adds each quantum's low 16 bits to the first word and
-  // its high bits (arithmetic shift) to the second, neither of which can wrap
-  // (a cell takes one add per particle), with adds that return nothing; a
-  // denser tile adds the whole quantum to the first word and counts its wraps
-  // in the second (each add is below 2^32, so it wraps at most once), which
-  // needs the old value back. Either pair is the exact 64-bit sum whatever the
-  // order of the adds.
+    const float* __restrict__ wrec, const unsigned* __restrict__ wmax,
+    const uint32_t* __restrict__ redo) {
   extern __shared__ uint32_t acc_lo[];  // TS^3 words, then TS^3 carries
-  uint32_t* acc_hi = acc_lo + TS * TS * TS;
-  const uint32_t nt = g.nt;
-  const uint32_t n_tiles = nt * nt * nt;
+  uint32_t* acc_hi = acc_lo + kTileWords;
+  const uint32_t n_items = redo ? redo[0] : g.nt * g.nt * g.nt;
+  if (blockIdx.x >= n_items) return;
   // The quantum: 2^-24 of a particle, or of the largest weight's binade.
-  float qscale = 16777216.0f, qinv = 1.0f / 16777216.0f;
+  float qscale = (float)kWhole, qinv = 1.0f / (float)kWhole;
   if (wrec) {
     const int e = weight_scale_exp(wmax);
     qscale = __uint_as_float((uint32_t)(127 + e) << 23);
     qinv = __uint_as_float((uint32_t)(127 - e) << 23);
   }
   // Cleared once; each flush leaves the cells it reads cleared for the next tile.
-  for (int i = threadIdx.x; i < 2 * TS * TS * TS; i += blockDim.x) acc_lo[i] = 0u;
+  for (int i = threadIdx.x; i < 2 * kTileWords; i += kDepositT) acc_lo[i] = 0u;
   __syncthreads();
-  for (uint32_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-    const uint32_t tx = tile / (nt * nt), ty = (tile / nt) % nt, tz = tile % nt;
-    const uint32_t ox = tx * TB, oy = ty * TB, oz = tz * TB;
-
+  for (uint32_t item = blockIdx.x; item < n_items; item += gridDim.x) {
+    const uint32_t tile = redo ? redo[1 + item] : item;
     const uint32_t s = offsets[tile], e = offsets[tile + 1];
     const bool split = e - s < (1u << 16);
-    for (uint32_t base = s; base < e; base += blockDim.x) {
-      const uint32_t p = base + threadIdx.x;
-      const bool valid = p < e;
-      uint32_t cell = 0xffffffffu;
-      uint32_t q[8];
-      if (valid) {
-        const float4 r = __ldg(rec + p);
-        const float tx_ = r.x, ty_ = r.y, tz_ = r.z;
-        const uint32_t local = __float_as_uint(r.w);
-        float wz0 = fsub(1.0f, tz_), wz1 = tz_;
-        float pw = 1.0f;
-        if (wrec) {
-          // A non-finite weight is added afterwards, outside the sums.
-          pw = __ldg(wrec + p);
-          if ((__float_as_uint(pw) & 0x7fffffffu) >= 0x7f800000u) pw = 0.0f;
-          wz0 = fmul(pw, wz0);
-          wz1 = fmul(pw, wz1);
-        }
-        const float wx0 = fsub(1.0f, tx_), wy0 = fsub(1.0f, ty_);
-        // The reference's eight products (grid.c:627-650): (x,y) pairs times
-        // z (times the weight).
-        const float w00 = fmul(wx0, wy0), w01 = fmul(wx0, ty_);
-        const float w10 = fmul(tx_, wy0), w11 = fmul(tx_, ty_);
-        const float w[8] = {fmul(w00, wz0), fmul(w00, wz1), fmul(w01, wz0), fmul(w01, wz1),
-                            fmul(w10, wz0), fmul(w10, wz1), fmul(w11, wz0), fmul(w11, wz1)};
-        // w times a power of two is exact in float, so rounding it to an
-        // integer in float is the quantisation itself; GB300's FP64 rate is
-        // no place for it.
-        int sum = 0;
-        int big = 0;
-        float wbig = fabsf(w[0]);
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-          const int qk = __float2int_rn(fmul(w[k], qscale));
-          q[k] = (uint32_t)qk;
-          sum += qk;
-          if (fabsf(w[k]) > wbig) {  // the first largest, as a scan from corner 0 finds it
-            wbig = fabsf(w[k]);
-            big = k;
-          }
-        }
-        // The eight sum to the particle's own quantised weight.
-        const int fix = (wrec ? __float2int_rn(fmul(pw, qscale)) : 16777216) - sum;
-#pragma unroll
-        for (int k = 0; k < 8; k++) q[k] = (uint32_t)((int)q[k] + (k == big ? fix : 0));
-        cell = ((local >> 8) * TS + ((local >> 4) & 15u)) * TS + (local & 15u);
+    for (uint32_t p = s + threadIdx.x; p < e; p += kDepositT) {
+      const float4 r = __ldg(rec + p);
+      float wz0 = fsub(1.0f, r.z), wz1 = r.z;
+      int whole = kWhole;
+      if (wrec) {
+        // A non-finite weight is added afterwards, outside the sums.
+        float pw = __ldg(wrec + p);
+        if ((__float_as_uint(pw) & 0x7fffffffu) >= 0x7f800000u) pw = 0.0f;
+        wz0 = fmul(pw, wz0);
+        wz1 = fmul(pw, wz1);
+        whole = __float2int_rn(fmul(pw, qscale));  // the particle's own quantised weight
       }
-      // One shared atomic per corner. (Reducing lanes bound for the same cell
-      // first with __reduce_add_sync over each lane group's own mask costs a
-      // serialised pass per distinct group: eight per corner per cell in the
-      // warp, far more than the atomics it saves.)
-      if (valid && split) {
+      uint32_t q[8];
+      corner_quanta(r.x, r.y, wz0, wz1, qscale, whole, q);
+      const uint32_t cell = tile_cell(__float_as_uint(r.w));
+      // One shared atomic per word and corner. (Reducing lanes bound for the
+      // same cell first with __reduce_add_sync over each lane group's own mask
+      // costs a serialised pass per distinct group: eight per corner per cell
+      // in the warp, far more than the atomics it saves.)
+      if (split) {
 #pragma unroll
         for (int k = 0; k < 8; k++) {
-          const uint32_t c =
-              cell + (uint32_t)(((k >> 2) & 1) * TS * TS + ((k >> 1) & 1) * TS + (k & 1));
+          const uint32_t c = cell + corner_offset(k);
           atomicAdd(acc_lo + c, q[k] & 0xffffu);
           const int hi16 = (int)q[k] >> 16;
           if (hi16) atomicAdd(acc_hi + c, (uint32_t)hi16);
         }
-      } else if (valid) {
+      } else {
 #pragma unroll
         for (int k = 0; k < 8; k++) {
           const uint32_t v = q[k];
-          const uint32_t c =
-              cell + (uint32_t)(((k >> 2) & 1) * TS * TS + ((k >> 1) & 1) * TS + (k & 1));
+          const uint32_t c = cell + corner_offset(k);
           const uint32_t old = atomicAdd(acc_lo + c, v);
           // The carry, and for a negative value its sign extension.
           const uint32_t hi = (old + v < old ? 1u : 0u) + ((int)v < 0 ? 0xffffffffu : 0u);
@@ -337,29 +447,14 @@ __global__ void __launch_bounds__(256) tile_deposit_kernel(
       }
     }
     __syncthreads();
-
-    // Flush. Cells 1..TB-1 of this tile (within the grid) are touched by no
-    // other tile; the rest are shared with a neighbour.
-    const uint32_t ex = min((uint32_t)TB, g.n - ox), ey = min((uint32_t)TB, g.n - oy),
-                   ez = min((uint32_t)TB, g.n - oz);
-    for (int i = threadIdx.x; i < TS * TS * TS; i += blockDim.x) {
-      const uint32_t a = i / (TS * TS), b = (i / TS) % TS, c = i % TS;
-      if (a > ex || b > ey || c > ez) continue;
+    const TileFlush f(tile, g);
+    for (int i = threadIdx.x; i < kTileWords; i += kDepositT) {
       const unsigned long long v =
           split ? (unsigned long long)((long long)(int)acc_hi[i] * 65536ll + (long long)acc_lo[i])
                 : ((unsigned long long)acc_hi[i] << 32) | acc_lo[i];
       acc_lo[i] = 0u;
       acc_hi[i] = 0u;
-      const uint32_t gx = ox + a == g.n ? 0u : ox + a;
-      const uint32_t gy = oy + b == g.n ? 0u : oy + b;
-      const uint32_t gz = oz + c == g.n ? 0u : oz + c;
-      const bool interior = a >= 1 && a < ex && b >= 1 && b < ey && c >= 1 && c < ez;
-      if (interior) {
-        grid[((uint64_t)gx * g.n + gy) * g.n + gz] =
-            fmul(fmul(__ll2float_rn((long long)v), qinv), inv_cell_vol);
-      } else if (v != 0ull) {
-        atomicAdd(face_slot(faces, gx, gy, gz, g), v);
-      }
+      f.put(i / (TS * TS), (i / TS) % TS, i % TS, v, g, qinv, inv_cell_vol, grid, faces);
     }
     __syncthreads();
   }
@@ -655,13 +750,18 @@ __global__ void __launch_bounds__(kMeanThreads) mean_partial_kernel<float>(
   if (threadIdx.x == 0) partial[blockIdx.x] = s[0];
 }
 
-__global__ void mean_final_kernel(const double* __restrict__ partial, uint64_t n,
-                                  double* __restrict__ mean_out) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    double t = 0.0;
-    for (int b = 0; b < kMeanBlocks; b++) t += partial[b];
-    mean_out[0] = t / (double)n;
+// The blocks' sums added by pairs, in a fixed order: eleven dependent adds
+// and one load deep. (One thread adding 1,024 of them in a row took 56 us.)
+__global__ void __launch_bounds__(kMeanBlocks / 2) mean_final_kernel(
+    const double* __restrict__ partial, uint64_t n, double* __restrict__ mean_out) {
+  __shared__ double s[kMeanBlocks / 2];
+  s[threadIdx.x] = partial[threadIdx.x] + partial[threadIdx.x + kMeanBlocks / 2];
+  __syncthreads();
+  for (int w = kMeanBlocks / 4; w > 0; w >>= 1) {
+    if ((int)threadIdx.x < w) s[threadIdx.x] += s[threadIdx.x + w];
+    __syncthreads();
   }
+  if (threadIdx.x == 0) mean_out[0] = s[0] / (double)n;
 }
 
 template <class R>
@@ -747,18 +847,24 @@ void cic_deposit(const float* x, const float* y, const float* z, uint64_t n_part
   if (sorted) SIFG_CUDA(cudaEventRecord(sorted, st));
   const float cl = box / (float)n;
   const float inv_cell_vol = 1.0f / (float)(cl * cl * cl);
-  const size_t smem = (size_t)2 * TS * TS * TS * sizeof(uint32_t);
-  thread_local bool attr = false;  // a per-thread flag: the attribute is set once per thread
-  if (!attr) {
-    SIFG_CUDA(cudaFuncSetAttribute(tile_deposit_kernel,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr = true;
-  }
-  const unsigned dgrid = (unsigned)(tiles < 152u * 5u ? tiles : 152u * 5u);
+  const size_t smem = (size_t)2 * kTileWords * sizeof(uint32_t);
+  auto grid_of = [&](unsigned per_sm) { return (unsigned)std::min<uint64_t>(tiles, 152u * per_sm); };
   if (timer) timer->begin(st);
-  tile_deposit_kernel<<<dgrid, 256, smem, st>>>(rec, counts, g, inv_cell_vol, grid, faces,
-                                                 wrec, wmax);
-  SIFG_LAUNCH_CHECK();
+  if (w) {
+    tile_deposit_wide_kernel<<<grid_of(5), kDepositT, smem, st>>>(rec, counts, g, inv_cell_vol, grid,
+                                                                  faces, wrec, wmax, nullptr);
+    SIFG_LAUNCH_CHECK();
+  } else {
+    // The scatter's cursors are free: the list of tiles to do again.
+    uint32_t* redo = cursor;
+    SIFG_CUDA(cudaMemsetAsync(redo, 0, sizeof(uint32_t), st));
+    tile_deposit_kernel<<<grid_of(6), kDepositT, 0, st>>>(rec, counts, g, inv_cell_vol, grid, faces,
+                                                          redo);
+    SIFG_LAUNCH_CHECK();
+    tile_deposit_wide_kernel<<<grid_of(1), kDepositT, smem, st>>>(rec, counts, g, inv_cell_vol, grid,
+                                                                  faces, nullptr, nullptr, redo);
+    SIFG_LAUNCH_CHECK();
+  }
   if (timer) timer->end(st);
   face_fixup_kernel<<<grid_for(3 * face_elems, 256), 256, 0, st>>>(g, inv_cell_vol, grid, faces,
                                                                   wmax);
@@ -775,7 +881,7 @@ void density_contrast(R* v, uint64_t n, double* d_scratch, cudaStream_t st, bool
   // d_scratch: kMeanBlocks + 1 doubles.
   mean_partial_kernel<R><<<kMeanBlocks, kMeanThreads, 0, st>>>(v, n, d_scratch);
   SIFG_LAUNCH_CHECK();
-  mean_final_kernel<<<1, 32, 0, st>>>(d_scratch, n, d_scratch + kMeanBlocks);
+  mean_final_kernel<<<1, kMeanBlocks / 2, 0, st>>>(d_scratch, n, d_scratch + kMeanBlocks);
   SIFG_LAUNCH_CHECK();
   if (!mean_only) apply_contrast(v, n, d_scratch + kMeanBlocks, st);
 }
