@@ -52,6 +52,8 @@ struct CicGeom {
   float box;
   float idx_hi;     // n / box in double, as a pair of floats
   float idx_lo;
+  float margin;     // 2^-21 n: see cic_axis_inner
+  float last;       // n as a float
 };
 
 // A coordinate in cell units, u = fold(v) * n / box, and its base cell and
@@ -82,39 +84,90 @@ __device__ __forceinline__ void cic_axis(float v, const CicGeom& g, uint32_t& ce
   t = f;
 }
 
-__device__ __forceinline__ uint32_t tile_of(float x, float y, float z, const CicGeom& g) {
-  uint32_t cx, cy, cz;
-  float t;
-  cic_axis(x, g, cx, t);
-  cic_axis(y, g, cy, t);
-  cic_axis(z, g, cz, t);
-  return ((cx / TB) * g.nt + cy / TB) * g.nt + cz / TB;
+// The same for a position well inside its cell, without the fold, the carries
+// and the clamp: v in [0, box) folds to itself, and where hi lies further from
+// the integers than |lo| can reach -- lo is at most half an ulp of hi plus x *
+// idx_lo, below 2^-22 n together, for hi <= n -- the floor of hi is u's and
+// hi - floor(hi) + lo needs no carry. False, for the general form to decide,
+// outside that: 2^-21 n of the positions (NaN among them), since every
+// comparison must hold.
+__device__ __forceinline__ bool cic_axis_inner(float v, const CicGeom& g, uint32_t& cell, float& t) {
+  const float hi = fmul(v, g.idx_hi);
+  const float lo = fadd(__fmaf_rn(v, g.idx_hi, -hi), fmul(v, g.idx_lo));
+  const float r = floorf(hi);
+  const float f0 = fsub(hi, r);
+  cell = (uint32_t)(int32_t)r;
+  t = fadd(f0, lo);
+  return v >= 0.0f && v < g.box && hi < g.last && f0 > g.margin && f0 < 1.0f - g.margin;
 }
+
+// A particle's base cell (and fractions): most take the short form, and the
+// two give the same bits where both apply.
+__device__ __forceinline__ void cic_particle(float x, float y, float z, const CicGeom& g,
+                                             uint32_t (&c)[3], float (&t)[3]) {
+  const bool bx = cic_axis_inner(x, g, c[0], t[0]), by = cic_axis_inner(y, g, c[1], t[1]),
+             bz = cic_axis_inner(z, g, c[2], t[2]);
+  if (!(bx && by && bz)) {
+    cic_axis(x, g, c[0], t[0]);
+    cic_axis(y, g, c[1], t[1]);
+    cic_axis(z, g, c[2], t[2]);
+  }
+}
+
+__device__ __forceinline__ uint32_t tile_index(const uint32_t (&c)[3], const CicGeom& g) {
+  return ((c[0] / TB) * g.nt + c[1] / TB) * g.nt + c[2] / TB;
+}
+
+// Both passes of the tile sort were bound by their instructions (a particle's
+// three folds, carries and clamps), not by their traffic: the short form of
+// cic_particle, and kSortUnroll particles' loads, matches and atomics in
+// flight a thread.
+constexpr int kSortT = 256;
+constexpr int kSortUnroll = 4;
 
 // With `outside` set, also counts the particles outside [lo, hi] on any axis
 // (NaN included): the box check, from the same reads.
-__global__ void tile_count_kernel(const float* __restrict__ x, const float* __restrict__ y,
-                                  const float* __restrict__ z, uint64_t n, CicGeom g,
-                                  uint32_t* __restrict__ counts, float lo, float hi,
-                                  unsigned long long* __restrict__ outside) {
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  unsigned long long bad = 0;
-  for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < n; base += stride) {
-    const uint64_t p = base + threadIdx.x;
-    const bool valid = p < n;
-    uint32_t tile = 0xffffffffu;
-    if (valid) {
-      const float px = x[p], py = y[p], pz = z[p];
-      tile = tile_of(px, py, pz, g);
-      bad += (px >= lo && px <= hi && py >= lo && py <= hi && pz >= lo && pz <= hi) ? 0u : 1u;
+__global__ void __launch_bounds__(kSortT) tile_count_kernel(
+    const float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ z, uint64_t n,
+    CicGeom g, uint32_t* __restrict__ counts, float lo, float hi,
+    unsigned long long* __restrict__ outside) {
+  const uint64_t stride = (uint64_t)gridDim.x * kSortT * kSortUnroll;
+  uint32_t bad = 0;
+  for (uint64_t base = (uint64_t)blockIdx.x * kSortT * kSortUnroll; base < n; base += stride) {
+    float px[kSortUnroll], py[kSortUnroll], pz[kSortUnroll];
+    uint32_t tile[kSortUnroll];
+#pragma unroll
+    for (int u = 0; u < kSortUnroll; u++) {
+      const uint64_t p = base + u * kSortT + threadIdx.x;
+      if (p < n) {
+        px[u] = x[p];
+        py[u] = y[p];
+        pz[u] = z[p];
+      }
     }
-    const unsigned peers = __match_any_sync(0xffffffffu, tile);
-    if (valid && (threadIdx.x & 31u) == (unsigned)(__ffs(peers) - 1))
-      atomicAdd(counts + tile, (uint32_t)__popc(peers));
+#pragma unroll
+    for (int u = 0; u < kSortUnroll; u++) {
+      tile[u] = 0xffffffffu;
+      if (base + u * kSortT + threadIdx.x < n) {
+        uint32_t c[3];
+        float t[3];
+        cic_particle(px[u], py[u], pz[u], g, c, t);
+        tile[u] = tile_index(c, g);
+        const float mn = fminf(fminf(px[u], py[u]), pz[u]), mx = fmaxf(fmaxf(px[u], py[u]), pz[u]);
+        // fminf and fmaxf pass over a NaN: the sum of the three keeps it.
+        bad += (mn >= lo && mx <= hi && px[u] + py[u] + pz[u] == px[u] + py[u] + pz[u]) ? 0u : 1u;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kSortUnroll; u++) {
+      const unsigned peers = __match_any_sync(0xffffffffu, tile[u]);
+      if (tile[u] != 0xffffffffu && (threadIdx.x & 31u) == (unsigned)(__ffs(peers) - 1))
+        atomicAdd(counts + tile[u], (uint32_t)__popc(peers));
+    }
   }
   if (outside) {
-    for (int d = 16; d > 0; d >>= 1) bad += __shfl_down_sync(0xffffffffu, bad, d);
-    if ((threadIdx.x & 31u) == 0 && bad) atomicAdd(outside, bad);
+    unsigned long long b = __reduce_add_sync(0xffffffffu, bad);
+    if ((threadIdx.x & 31u) == 0 && b) atomicAdd(outside, b);
   }
 }
 
@@ -122,34 +175,51 @@ __global__ void tile_count_kernel(const float* __restrict__ x, const float* __re
 // fourth word's bits, its base cell within its tile (x << 8 | y << 4 | z).
 static_assert(TB == 16, "4 bits per axis of the cell within its tile");
 
-__global__ void tile_scatter_kernel(const float* __restrict__ x, const float* __restrict__ y,
-                                    const float* __restrict__ z, uint64_t n, CicGeom g,
-                                    uint32_t* __restrict__ cursor, float4* __restrict__ rec,
-                                    const float* __restrict__ w, float* __restrict__ wrec) {
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+__global__ void __launch_bounds__(kSortT) tile_scatter_kernel(
+    const float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ z, uint64_t n,
+    CicGeom g, uint32_t* __restrict__ cursor, float4* __restrict__ rec, const float* __restrict__ w,
+    float* __restrict__ wrec) {
+  const uint64_t stride = (uint64_t)gridDim.x * kSortT * kSortUnroll;
   const unsigned lane = threadIdx.x & 31u;
-  for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < n; base += stride) {
-    const uint64_t p = base + threadIdx.x;
-    const bool valid = p < n;
-    float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
-    uint32_t tile = 0xffffffffu;
-    if (valid) {
-      uint32_t cx, cy, cz;
-      cic_axis(x[p], g, cx, r.x);
-      cic_axis(y[p], g, cy, r.y);
-      cic_axis(z[p], g, cz, r.z);
-      tile = ((cx / TB) * g.nt + cy / TB) * g.nt + cz / TB;
-      r.w = __uint_as_float((cx % TB) << 8 | (cy % TB) << 4 | (cz % TB));
+  for (uint64_t base = (uint64_t)blockIdx.x * kSortT * kSortUnroll; base < n; base += stride) {
+    float px[kSortUnroll], py[kSortUnroll], pz[kSortUnroll];
+    float4 r[kSortUnroll];
+    uint32_t slot[kSortUnroll], tile[kSortUnroll], peers[kSortUnroll];
+#pragma unroll
+    for (int u = 0; u < kSortUnroll; u++) {
+      const uint64_t p = base + u * kSortT + threadIdx.x;
+      if (p < n) {
+        px[u] = x[p];
+        py[u] = y[p];
+        pz[u] = z[p];
+      }
     }
-    const unsigned peers = __match_any_sync(0xffffffffu, tile);
-    const unsigned leader = __ffs(peers) - 1;
-    uint32_t slot0 = 0;
-    if (valid && lane == leader) slot0 = atomicAdd(cursor + tile, (uint32_t)__popc(peers));
-    slot0 = __shfl_sync(0xffffffffu, slot0, leader);
-    if (valid) {
-      const uint32_t slot = slot0 + __popc(peers & ((1u << lane) - 1u));
-      rec[slot] = r;
-      if (w) wrec[slot] = w[p];
+#pragma unroll
+    for (int u = 0; u < kSortUnroll; u++) {
+      tile[u] = 0xffffffffu;
+      if (base + u * kSortT + threadIdx.x < n) {
+        uint32_t c[3];
+        float t[3];
+        cic_particle(px[u], py[u], pz[u], g, c, t);
+        tile[u] = tile_index(c, g);
+        r[u] = make_float4(t[0], t[1], t[2],
+                           __uint_as_float((c[0] % TB) << 8 | (c[1] % TB) << 4 | (c[2] % TB)));
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kSortUnroll; u++) {
+      peers[u] = __match_any_sync(0xffffffffu, tile[u]);
+      if (tile[u] != 0xffffffffu && lane == (unsigned)(__ffs(peers[u]) - 1))
+        slot[u] = atomicAdd(cursor + tile[u], (uint32_t)__popc(peers[u]));
+    }
+#pragma unroll
+    for (int u = 0; u < kSortUnroll; u++) {
+      const uint32_t s = __shfl_sync(0xffffffffu, slot[u], __ffs(peers[u]) - 1) +
+                         __popc(peers[u] & ((1u << lane) - 1u));
+      if (tile[u] != 0xffffffffu) {
+        rec[s] = r[u];
+        if (w) wrec[s] = w[base + u * kSortT + threadIdx.x];
+      }
     }
   }
 }
@@ -274,12 +344,10 @@ __device__ __forceinline__ uint32_t corner_offset(int k) {
   return (uint32_t)(((k >> 2) & 1) * TS * TS + ((k >> 1) & 1) * TS + (k & 1));
 }
 
-// One cell of a tile's flush, at (a, b, c) of the 17^3: cells 1..TB-1 of the
-// tile (within the grid) are touched by no other tile and go straight to the
-// grid; the rest are shared with a neighbour.
-struct TileFlush {
+// A tile's place in the grid: its first node and its extent.
+struct TilePlace {
   uint32_t ox, oy, oz, ex, ey, ez;
-  __device__ __forceinline__ TileFlush(uint32_t tile, const CicGeom& g) {
+  __device__ __forceinline__ TilePlace(uint32_t tile, const CicGeom& g) {
     const uint32_t nt = g.nt;
     ox = tile / (nt * nt) * TB;
     oy = (tile / nt) % nt * TB;
@@ -288,35 +356,30 @@ struct TileFlush {
     ey = min((uint32_t)TB, g.n - oy);
     ez = min((uint32_t)TB, g.n - oz);
   }
-  __device__ __forceinline__ void put(uint32_t a, uint32_t b, uint32_t c, unsigned long long v,
-                                      const CicGeom& g, float qinv, float inv_cell_vol,
-                                      float* __restrict__ grid, const FaceBufs& faces) const {
-    if (a > ex || b > ey || c > ez) return;
-    const uint32_t gx = ox + a == g.n ? 0u : ox + a;
-    const uint32_t gy = oy + b == g.n ? 0u : oy + b;
-    const uint32_t gz = oz + c == g.n ? 0u : oz + c;
-    const bool interior = a >= 1 && a < ex && b >= 1 && b < ey && c >= 1 && c < ez;
-    if (interior) {
-      grid[((uint64_t)gx * g.n + gy) * g.n + gz] =
-          fmul(fmul(__ll2float_rn((long long)v), qinv), inv_cell_vol);
-    } else if (v != 0ull) {
-      atomicAdd(face_slot(faces, gx, gy, gz, g), v);
-    }
-  }
 };
 
 // The unweighted deposit, one CTA a tile at a time: the tile's sums as one
-// 32-bit word a cell, one shared atomic a corner. The kernel is bound by
-// those atomics, so the word's wraps are not watched add by add: every
-// quantum is non-negative (the weights are, and the remainder of a few quanta
-// goes to a corner of at least 2^21), so the words of a tile sum to its
-// particles times 2^24 exactly when none of them wrapped, and each wrap takes
-// 2^32 from that sum. A tile whose sum falls short (a cell of 256 particles or
-// more, in an unweighted count) is left to tile_deposit_wide_kernel, through
-// `redo` (redo[0] counts them), as is one with so many particles that one of
-// its cells must have wrapped.
+// 32-bit word a cell, one shared atomic a corner. The word's wraps are not
+// watched add by add: every quantum is non-negative (the weights are, and the
+// remainder of a few quanta goes to a corner of at least 2^21), so the words
+// of a tile sum to its particles times 2^24 exactly when none of them wrapped,
+// and each wrap takes 2^32 from that sum. A tile whose sum falls short (a cell
+// of 256 particles or more, in an unweighted count) is left to
+// tile_deposit_wide_kernel, through `redo` (redo[0] counts them), as is one
+// with so many particles that one of its cells must have wrapped.
 // (Two words a cell, as the wide kernel keeps, cost a second atomic a corner:
-// the 512^3 deposit 1.57 ms in 39 KB of shared memory a CTA.)
+// the 512^3 deposit 1.57 ms in 39 KB of shared memory a CTA, 1.23 with one.)
+//
+// The kernel is bound by its instructions. A corner's quantum is rounded by
+// adding 2^23 to it (an fma; an integer conversion runs at a quarter of the
+// rate): exact for every weight up to a half. The largest corner's can be
+// more, and whatever its bits then say, the remainder -- what the eight lack
+// of one particle, added modulo 2^32 to the same word by a ninth atomic --
+// makes it the particle's rest: the same quanta as corner_quanta's, without
+// a select per corner to place the remainder. The flush takes the tile's
+// inside and its faces in passes of their own, each cell's place a few
+// instructions (one loop over all 17^3 with a test of each cell's kind was
+// half of the kernel).
 __global__ void __launch_bounds__(kDepositT, 6) tile_deposit_kernel(
     const float4* __restrict__ rec, const uint32_t* __restrict__ offsets, CicGeom g,
     float inv_cell_vol, float* __restrict__ grid, FaceBufs faces, uint32_t* __restrict__ redo) {
@@ -336,11 +399,25 @@ __global__ void __launch_bounds__(kDepositT, 6) tile_deposit_kernel(
     }
     for (uint32_t p = s + threadIdx.x; p < e; p += kDepositT) {
       const float4 r = __ldg(rec + p);
-      uint32_t q[8];
-      corner_quanta(r.x, r.y, fsub(1.0f, r.z), r.z, qscale, kWhole, q);
+      const float wx0 = fsub(1.0f, r.x), wy0 = fsub(1.0f, r.y), wz0 = fsub(1.0f, r.z);
+      const float w00 = fmul(wx0, wy0), w01 = fmul(wx0, r.y);
+      const float w10 = fmul(r.x, wy0), w11 = fmul(r.x, r.y);
+      const float w[8] = {fmul(w00, wz0), fmul(w00, r.z), fmul(w01, wz0), fmul(w01, r.z),
+                          fmul(w10, wz0), fmul(w10, r.z), fmul(w11, wz0), fmul(w11, r.z)};
       uint32_t* cell = acc + tile_cell(__float_as_uint(r.w));
+      uint32_t sum = 0, big = 0;
+      float wbig = w[0];
 #pragma unroll
-      for (int k = 0; k < 8; k++) atomicAdd(cell + corner_offset(k), q[k]);
+      for (int k = 0; k < 8; k++) {
+        const uint32_t q = __float_as_uint(__fmaf_rn(w[k], qscale, 8388608.0f)) - 0x4b000000u;
+        atomicAdd(cell + corner_offset(k), q);
+        sum += q;
+        if (k > 0 && w[k] > wbig) {  // the first largest, as corner_quanta finds it
+          wbig = w[k];
+          big = corner_offset(k);
+        }
+      }
+      atomicAdd(cell + big, (uint32_t)kWhole - sum);
     }
     __syncthreads();
     unsigned long long sum = 0;
@@ -353,21 +430,53 @@ __global__ void __launch_bounds__(kDepositT, 6) tile_deposit_kernel(
     sum = 0;
 #pragma unroll
     for (int w = 0; w < kDepositT / 32; w++) sum += wsum[w];
-    const bool whole = sum == (unsigned long long)(e - s) << 24;
-    if (!whole && threadIdx.x == 0) redo[1 + atomicAdd(redo, 1u)] = tile;
-
-    // The flush: 16 cells of a z row per half-warp, then the rows' last cells.
-    const TileFlush f(tile, g);
-    const uint32_t c = threadIdx.x & 15u;
-    for (uint32_t row = threadIdx.x >> 4; row < TS * TS; row += kDepositT / 16) {
-      const uint32_t v = acc[row * TS + c];
-      acc[row * TS + c] = 0u;
-      if (whole) f.put(row / TS, row % TS, c, v, g, qinv, inv_cell_vol, grid, faces);
+    if (sum != (unsigned long long)(e - s) << 24) {
+      if (threadIdx.x == 0) redo[1 + atomicAdd(redo, 1u)] = tile;
+      for (int i = threadIdx.x; i < kTileWords; i += kDepositT) acc[i] = 0u;
+      __syncthreads();
+      continue;
     }
-    for (uint32_t row = threadIdx.x; row < TS * TS; row += kDepositT) {
-      const uint32_t v = acc[row * TS + TB];
-      acc[row * TS + TB] = 0u;
-      if (whole) f.put(row / TS, row % TS, TB, v, g, qinv, inv_cell_vol, grid, faces);
+
+    // The flush: nodes 1 .. e-1 of the tile on every axis are touched by no
+    // other tile and go straight to the grid, a half-warp a z row; the rest to
+    // the face buffers, each in face_slot's order of precedence. Cells past
+    // the grid's end hold nothing.
+    const TilePlace t(tile, g);
+    const uint32_t n = g.n;
+    for (uint32_t row = threadIdx.x >> 4; row < (TB - 1) * (TB - 1); row += kDepositT / 16) {
+      const uint32_t a = 1 + row / (TB - 1), b = 1 + row % (TB - 1), c = 1 + (threadIdx.x & 15u);
+      if (a < t.ex && b < t.ey && c < t.ez) {
+        uint32_t* src = acc + (a * TS + b) * TS + c;
+        grid[(size_t)((t.ox + a) * n + t.oy + b) * n + t.oz + c] =
+            fmul(fmul(__uint2float_rn(*src), qinv), inv_cell_vol);
+        *src = 0u;
+      }
+    }
+    auto to_face = [&](uint32_t a, uint32_t b, uint32_t c, unsigned long long* slot) {
+      uint32_t* src = acc + (a * TS + b) * TS + c;
+      const uint32_t v = *src;
+      *src = 0u;
+      if (v) atomicAdd(slot, (unsigned long long)v);
+    };
+    auto wrap = [&](uint32_t v) { return v == n ? 0u : v; };
+    for (uint32_t i = threadIdx.x; i < 2 * TS * TS; i += kDepositT) {
+      const uint32_t a = i < TS * TS ? 0u : t.ex, b = i / TS % TS, c = i % TS;
+      if (b <= t.ey && c <= t.ez)
+        to_face(a, b, c,
+                faces.fx + ((size_t)(wrap(t.ox + a) / TB) * n + wrap(t.oy + b)) * n + wrap(t.oz + c));
+    }
+    for (uint32_t i = threadIdx.x; i < 2 * (TB - 1) * TS; i += kDepositT) {
+      const uint32_t b = i < (TB - 1) * TS ? 0u : t.ey, a = 1 + i / TS % (TB - 1), c = i % TS;
+      if (a < t.ex && c <= t.ez)
+        to_face(a, b, c,
+                faces.fy + ((size_t)(t.ox + a) * g.nt + wrap(t.oy + b) / TB) * n + wrap(t.oz + c));
+    }
+    for (uint32_t i = threadIdx.x; i < 2 * (TB - 1) * (TB - 1); i += kDepositT) {
+      const uint32_t c = i < (TB - 1) * (TB - 1) ? 0u : t.ez, a = 1 + i / (TB - 1) % (TB - 1),
+                     b = 1 + i % (TB - 1);
+      if (a < t.ex && b < t.ey)
+        to_face(a, b, c,
+                faces.fz + (size_t)((t.ox + a) * n + t.oy + b) * g.nt + wrap(t.oz + c) / TB);
     }
     __syncthreads();
   }
@@ -447,14 +556,25 @@ __global__ void __launch_bounds__(kDepositT) tile_deposit_wide_kernel(
       }
     }
     __syncthreads();
-    const TileFlush f(tile, g);
+    // Nodes 1 .. e-1 of the tile on every axis are touched by no other tile
+    // and go straight to the grid; the rest are shared with a neighbour.
+    const TilePlace t(tile, g);
     for (int i = threadIdx.x; i < kTileWords; i += kDepositT) {
+      const uint32_t a = i / (TS * TS), b = (i / TS) % TS, c = i % TS;
+      if (a > t.ex || b > t.ey || c > t.ez) continue;
       const unsigned long long v =
           split ? (unsigned long long)((long long)(int)acc_hi[i] * 65536ll + (long long)acc_lo[i])
                 : ((unsigned long long)acc_hi[i] << 32) | acc_lo[i];
       acc_lo[i] = 0u;
       acc_hi[i] = 0u;
-      f.put(i / (TS * TS), (i / TS) % TS, i % TS, v, g, qinv, inv_cell_vol, grid, faces);
+      const uint32_t gx = t.ox + a == g.n ? 0u : t.ox + a;
+      const uint32_t gy = t.oy + b == g.n ? 0u : t.oy + b;
+      const uint32_t gz = t.oz + c == g.n ? 0u : t.oz + c;
+      if (a >= 1 && a < t.ex && b >= 1 && b < t.ey && c >= 1 && c < t.ez)
+        grid[((uint64_t)gx * g.n + gy) * g.n + gz] =
+            fmul(fmul(__ll2float_rn((long long)v), qinv), inv_cell_vol);
+      else if (v != 0ull)
+        atomicAdd(face_slot(faces, gx, gy, gz, g), v);
     }
     __syncthreads();
   }
@@ -788,6 +908,8 @@ static CicGeom make_geom(uint32_t n, float box) {
   const double idx = (double)n / (double)box;
   g.idx_hi = (float)idx;
   g.idx_lo = (float)(idx - (double)g.idx_hi);
+  g.margin = (float)n / 2097152.0f;
+  g.last = (float)n;
   return g;
 }
 
@@ -830,19 +952,20 @@ void cic_deposit(const float* x, const float* y, const float* z, uint64_t n_part
   SIFG_CUDA(cudaMemsetAsync(faces.fz, 0, face_elems * 8, st));
   const unsigned blk = 256;
   const unsigned grd = grid_for(n_particles, blk, 152u * 16u);
+  const unsigned sgrd = grid_for(n_particles, kSortT * kSortUnroll, 152u * 8u);
   if (w) {
     SIFG_CUDA(cudaMemsetAsync(wmax, 0, 2 * sizeof(unsigned), st));
     weight_max_kernel<<<grd, blk, 0, st>>>(w, n_particles, wmax);
     SIFG_LAUNCH_CHECK();
   }
-  tile_count_kernel<<<grd, blk, 0, st>>>(x, y, z, n_particles, g, counts,
+  tile_count_kernel<<<sgrd, kSortT, 0, st>>>(x, y, z, n_particles, g, counts,
                                          bounds ? bounds[0] : 0.f, bounds ? bounds[1] : 0.f,
                                          bounds ? outside : nullptr);
   SIFG_LAUNCH_CHECK();
   exclusive_scan_u32(counts, (uint32_t)(tiles + 1), st);
   SIFG_CUDA(cudaMemcpyAsync(cursor, counts, (tiles + 1) * sizeof(uint32_t),
                             cudaMemcpyDeviceToDevice, st));
-  tile_scatter_kernel<<<grd, blk, 0, st>>>(x, y, z, n_particles, g, cursor, rec, w, wrec);
+  tile_scatter_kernel<<<sgrd, kSortT, 0, st>>>(x, y, z, n_particles, g, cursor, rec, w, wrec);
   SIFG_LAUNCH_CHECK();
   if (sorted) SIFG_CUDA(cudaEventRecord(sorted, st));
   const float cl = box / (float)n;
