@@ -139,6 +139,19 @@ static void box_bounds(double box, double* lo, double* hi) {
   *hi = box + tol;
 }
 
+// The range error for the particles counted outside the box at *d, if any.
+template <class R>
+static int outside_status(const unsigned long long* d, uint64_t n, R box, const char* name,
+                          cudaStream_t st) {
+  unsigned long long h = 0;
+  SIFG_CUDA(cudaMemcpyAsync(&h, d, sizeof h, cudaMemcpyDeviceToHost, st));
+  SIFG_CUDA(cudaStreamSynchronize(st));
+  if (h)
+    return fail(SIF_ERR_RANGE, fmt("%s: %llu of %llu particles outside the box [0, %g)", name, h,
+                                   (unsigned long long)n, (double)box));
+  return SIF_OK;
+}
+
 template <class R>
 static int check_in_box(const R* dx, const R* dy, const R* dz, uint64_t n, R box,
                         const char* name, cudaStream_t st, DevBuf& flag) {
@@ -148,14 +161,30 @@ static int check_in_box(const R* dx, const R* dy, const R* dz, uint64_t n, R box
   box_bounds(box, &lo, &hi);
   box_check_kernel<R><<<grid_for(n, 256), 256, 0, st>>>(dx, dy, dz, n, lo, hi, d);
   SIFG_LAUNCH_CHECK();
-  unsigned long long h[2];
-  SIFG_CUDA(cudaMemcpyAsync(h, d, 16, cudaMemcpyDeviceToHost, st));
-  SIFG_CUDA(cudaStreamSynchronize(st));
-  if (h[0])
-    return fail(SIF_ERR_RANGE,
-                fmt("%s: %llu of %llu particles outside the box [0, %g)", name, h[0],
-                    (unsigned long long)n, (double)box));
-  return SIF_OK;
+  return outside_status(d, n, box, name, st);
+}
+
+// The same check from the reads of a build's own first pass (cic_count,
+// mesh_count), which writes nothing but scratch: a field refused leaves the
+// caller's arrays as they were, and the particles are not read once more.
+static int count_tiles(const float* dx, const float* dy, const float* dz, uint64_t n, uint32_t n_grid,
+                       float box, void* scratch, cudaStream_t st, DevBuf& flag) {
+  unsigned long long* d = (unsigned long long*)flag.ensure(16);
+  float bounds[2];
+  box_bounds(box, &bounds[0], &bounds[1]);
+  cic_count(dx, dy, dz, n, n_grid, box, scratch, st, bounds, d);
+  return outside_status(d, n, box, "field", st);
+}
+
+template <class R>
+static int count_cells(const R* dx, const R* dy, const R* dz, uint64_t n, const DeviceMeshT<R>& m,
+                       void* scratch, cudaStream_t st, DevBuf& flag) {
+  unsigned long long* d = (unsigned long long*)flag.ensure(16);
+  SIFG_CUDA(cudaMemsetAsync(d, 0, 16, st));
+  R bounds[2];
+  box_bounds(m.box_length, &bounds[0], &bounds[1]);
+  mesh_count(dx, dy, dz, n, m, scratch, st, (const R*)bounds, d);
+  return outside_status(d, n, m.box_length, "field", st);
 }
 
 static int check_field(const sif_field_t* field, const char* tag) {
@@ -552,7 +581,9 @@ int sif_grid_assign_cic(sif_grid_t* grid, const sif_field_t* field) {
   cudaStream_t s = e->stream();
   const float* dp[3];
   positions_in(field, s, dp);
-  st = check_in_box(dp[0], dp[1], dp[2], field->n_particles, grid->box_length, "field", s, bufs().bad);
+  e->scratch.ensure(cic_scratch_bytes(field->n_particles, grid->n_cells, field->weights != nullptr));
+  st = count_tiles(dp[0], dp[1], dp[2], field->n_particles, grid->n_cells, grid->box_length,
+                   e->scratch.ptr, s, bufs().bad);
   if (st != SIF_OK) return st;
   const size_t gb = grid->total_cells * sizeof(float);
   bool holds = false;
@@ -561,9 +592,8 @@ int sif_grid_assign_cic(sif_grid_t* grid, const sif_field_t* field) {
   const float* dw = nullptr;
   if (field->weights)
     dw = (const float*)array_in(field->weights, field->n_particles * sizeof(float), bufs().pw, s);
-  e->scratch.ensure(cic_scratch_bytes(field->n_particles, grid->n_cells, dw != nullptr));
   cic_deposit(dp[0], dp[1], dp[2], field->n_particles, grid->n_cells, grid->box_length, dg,
-              e->scratch.ptr, s, nullptr, nullptr, nullptr, nullptr, dw);
+              e->scratch.ptr, s, nullptr, nullptr, nullptr, nullptr, dw, nullptr, true);
   copy_down(grid->values, dg, gb, s);
   SIFG_CUDA(cudaStreamSynchronize(s));
   mirror_commit(grid->values);
@@ -635,8 +665,14 @@ static sif_chain_mesh_t* mesh_alloc(uint32_t n_cells, sif_real box, sif_field_t*
   cudaStream_t s = e->stream();
   const float* dp[3];
   positions_in(field, s, dp);
-  if (check_in_box(dp[0], dp[1], dp[2], n, box, "field", s, bufs().bad) != SIF_OK) return nullptr;
   const uint64_t cells = (uint64_t)n_cells * n_cells * n_cells;
+  DeviceMesh m;
+  m.n_cells = n_cells;
+  m.box_length = box;
+  m.cell_length = box / (float)n_cells;
+  e->scratch.ensure(std::max(mesh_scratch_bytes(n, n_cells),
+                             field->weights ? mesh_weights_scratch_bytes(n_cells) : (size_t)0));
+  if (count_cells(dp[0], dp[1], dp[2], n, m, e->scratch.ptr, s, bufs().bad) != SIF_OK) return nullptr;
   const bool keep_idx = !(opt & SIF_MESH_DROP_INDICES);
   const bool weighted = field->weights != nullptr;
   // The struct and its host arrays first: the device buffers the build
@@ -653,7 +689,7 @@ static sif_chain_mesh_t* mesh_alloc(uint32_t n_cells, sif_real box, sif_field_t*
   mesh->n_cells = n_cells;
   mesh->total_cells = cells;
   mesh->box_length = box;
-  mesh->cell_length = box / (float)n_cells;
+  mesh->cell_length = m.cell_length;
   mesh->n_particles = n;
   mesh->total_weight = (double)n;
   mesh->_position_block = (float*)host_block_get(3 * (n ? n : 1) * sizeof(float));
@@ -672,10 +708,6 @@ static sif_chain_mesh_t* mesh_alloc(uint32_t n_cells, sif_real box, sif_field_t*
   mesh->y = mesh->_position_block + n;
   mesh->z = mesh->_position_block + 2 * n;
 
-  DeviceMesh m;
-  m.n_cells = n_cells;
-  m.box_length = box;
-  m.cell_length = mesh->cell_length;
   bool holds = false;
   m.x = (float*)mirror_acquire(mesh->x, n * 4, n * 4, bufs().mx, &holds);
   m.y = (float*)mirror_acquire(mesh->y, n * 4, n * 4, bufs().my, &holds);
@@ -686,9 +718,7 @@ static sif_chain_mesh_t* mesh_alloc(uint32_t n_cells, sif_real box, sif_field_t*
   // A weighted mesh takes its weights through the source indices, kept on
   // the device whether or not the caller keeps them.
   m.orig = (keep_idx || weighted) ? (uint32_t*)bufs().orig.ensure(n * 4) : nullptr;
-  e->scratch.ensure(std::max(mesh_scratch_bytes(n, n_cells),
-                             weighted ? mesh_weights_scratch_bytes(n_cells) : (size_t)0));
-  mesh_build(dp[0], dp[1], dp[2], n, m, e->scratch.ptr, s, nullptr);
+  mesh_build(dp[0], dp[1], dp[2], n, m, e->scratch.ptr, s, nullptr, nullptr, true, true);
   if (weighted) {
     // chain_mesh.c:800-801, 624-672: the weights in mesh order, each cell's
     // sum, the total.
@@ -1628,14 +1658,16 @@ static int cic_device(const R* x, const R* y, const R* z, uint64_t n, uint32_t n
   if (!e) return SIF_ERR_UNINITIALISED;
   if (n_grid < 4) return fail(SIF_ERR_INVALID, "n_grid: expected at least 4");
   cudaStream_t s = e->stream();
-  const int st = check_in_box(x, y, z, n, box, "field", s, e->io.flag);
-  if (st != SIF_OK) return st;
   RunTimings tm;
   if constexpr (sizeof(R) == 4) {
     e->scratch.ensure(cic_scratch_bytes(n, n_grid, w != nullptr));
+    const int st = count_tiles(x, y, z, n, n_grid, box, e->scratch.ptr, s, e->io.flag);
+    if (st != SIF_OK) return st;
     cic_deposit(x, y, z, n, n_grid, box, grid, e->scratch.ptr, s, &tm.cic, nullptr, nullptr,
-                nullptr, w);
+                nullptr, w, nullptr, true);
   } else {
+    const int st = check_in_box(x, y, z, n, box, "field", s, e->io.flag);
+    if (st != SIF_OK) return st;
     e->scratch.ensure(cic_f64_scratch_bytes(n_grid));
     cic_deposit_f64(x, y, z, n, n_grid, box, grid, e->scratch.ptr, s, &tm.cic, w);
   }
@@ -1669,8 +1701,6 @@ static int mesh_device(const R* x, const R* y, const R* z, uint64_t n, uint32_t 
   if (n_cells > kMaxMeshSide)
     return fail(SIF_ERR_RANGE, fmt("mesh: %u cells a side (at most %u)", n_cells, kMaxMeshSide));
   cudaStream_t s = e->stream();
-  const int st = check_in_box(x, y, z, n, box, "field", s, e->io.flag);
-  if (st != SIF_OK) return st;
   DeviceMeshT<R> m;
   m.n_cells = n_cells;
   m.box_length = box;
@@ -1681,8 +1711,10 @@ static int mesh_device(const R* x, const R* y, const R* z, uint64_t n, uint32_t 
   m.offsets = offsets;
   m.orig = orig;
   e->scratch.ensure(mesh_scratch_bytes(n, n_cells) * sizeof(R) / sizeof(float));
+  const int st = count_cells(x, y, z, n, m, e->scratch.ptr, s, e->io.flag);
+  if (st != SIF_OK) return st;
   RunTimings tm;
-  mesh_build(x, y, z, n, m, e->scratch.ptr, s, &tm.mesh);
+  mesh_build(x, y, z, n, m, e->scratch.ptr, s, &tm.mesh, nullptr, true, true);
   SIFG_CUDA(cudaStreamSynchronize(s));
   drop_pending_timings();
   g_timings.mesh_ms = tm.mesh.total_ms();

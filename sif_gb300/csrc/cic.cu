@@ -580,38 +580,38 @@ __global__ void __launch_bounds__(kDepositT) tile_deposit_wide_kernel(
   }
 }
 
+// The face buffers converted to density: blockIdx.y is a buffer and one of
+// its nt shares of n^2 entries (in x and y, a boundary plane). A plane past the
+// grid's end holds nothing, and a node on an earlier buffer's planes belongs
+// to that buffer.
 __global__ void face_fixup_kernel(CicGeom g, float inv_cell_vol, float* __restrict__ grid,
                                   FaceBufs faces, const unsigned* __restrict__ wmax) {
   float qinv = 1.0f / 16777216.0f;
   if (wmax) qinv = __uint_as_float((uint32_t)(127 - weight_scale_exp(wmax)) << 23);
-  const uint64_t n = g.n, nt = g.nt;
-  const uint64_t nfx = nt * n * n;
-  const uint64_t total = 3 * nfx;
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-    const uint64_t which = i / nfx, j = i % nfx;
-    uint64_t gx, gy, gz;
-    unsigned long long v;
+  const uint32_t n = g.n, nt = g.nt;
+  const uint32_t which = blockIdx.y / nt, k = blockIdx.y % nt;
+  if (which < 2 && k * TB >= n) return;
+  for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n * n; j += gridDim.x * blockDim.x) {
+    const uint32_t u = j / n, v = j % n;
+    uint32_t gx, gy, gz;
+    const unsigned long long* from;
     if (which == 0) {
-      gx = (j / (n * n)) * TB;
-      gy = (j / n) % n;
-      gz = j % n;
-      if (gx >= n) continue;
-      v = faces.fx[j];
+      gx = k * TB, gy = u, gz = v;
+      from = faces.fx + (size_t)k * n * n + j;
     } else if (which == 1) {
-      gx = j / (nt * n);
-      gy = ((j / n) % nt) * TB;
-      gz = j % n;
-      if (gy >= n || gx % TB == 0) continue;
-      v = faces.fy[j];
+      gx = u, gy = k * TB, gz = v;
+      if (gx % TB == 0) continue;
+      from = faces.fy + ((size_t)gx * nt + k) * n + gz;
     } else {
-      gx = j / (n * nt);
-      gy = (j / nt) % n;
-      gz = (j % nt) * TB;
-      if (gz >= n || gx % TB == 0 || gy % TB == 0) continue;
-      v = faces.fz[j];
+      // The buffer's z planes lie next to one another: its k-th n^2 entries.
+      const size_t i = (size_t)k * n * n + j;
+      const size_t line = i < 0xffffffffull ? (uint32_t)i / nt : i / nt;
+      gx = (uint32_t)line / n, gy = (uint32_t)line % n, gz = (uint32_t)(i - line * nt) * TB;
+      if (gx % TB == 0 || gy % TB == 0 || gz >= n) continue;
+      from = faces.fz + i;
     }
-    grid[(gx * n + gy) * n + gz] = fmul(fmul(__ll2float_rn((long long)v), qinv), inv_cell_vol);
+    grid[(size_t)(gx * n + gy) * n + gz] =
+        fmul(fmul(__ll2float_rn((long long)*from), qinv), inv_cell_vol);
   }
 }
 
@@ -884,9 +884,42 @@ __global__ void __launch_bounds__(kMeanBlocks / 2) mean_final_kernel(
   if (threadIdx.x == 0) mean_out[0] = s[0] / (double)n;
 }
 
+// Sixteen bytes a load and store (v is 16-byte aligned), the values past the
+// last whole ones by the last block's first threads. From the end backwards:
+// the mean's pass, just before it, left the end of the grid in L2.
 template <class R>
-__global__ void contrast_kernel(R* __restrict__ v, uint64_t n, const double* __restrict__ mean) {
+__global__ void __launch_bounds__(256) contrast_kernel(R* __restrict__ v, uint64_t n,
+                                                       const double* __restrict__ mean) {
   // The double division once a block (this GPU's FP64 rate is low).
+  __shared__ R inv_s;
+  if (threadIdx.x == 0) inv_s = (R)(1.0 / mean[0]);
+  __syncthreads();
+  const R inv = inv_s;
+  constexpr uint32_t kPer = 16 / sizeof(R);
+  struct alignas(16) Pack {
+    R v[kPer];
+  };
+  Pack* packs = (Pack*)v;
+  const uint64_t np = n / kPer, stride = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < np; i += 2 * stride) {
+    const bool two = i + stride < np;
+    Pack a = packs[np - 1 - i], b{};
+    if (two) b = packs[np - 1 - i - stride];
+#pragma unroll
+    for (uint32_t k = 0; k < kPer; k++) {
+      a.v[k] = fsub(fmul(a.v[k], inv), R(1.0f));
+      b.v[k] = fsub(fmul(b.v[k], inv), R(1.0f));
+    }
+    packs[np - 1 - i] = a;
+    if (two) packs[np - 1 - i - stride] = b;
+  }
+  const uint64_t i = np * kPer + threadIdx.x;
+  if (blockIdx.x == gridDim.x - 1 && i < n) v[i] = fsub(fmul(v[i], inv), R(1.0f));
+}
+
+// The same, one value a thread, where v is not 16-byte aligned.
+template <class R>
+__global__ void contrast_any_kernel(R* __restrict__ v, uint64_t n, const double* __restrict__ mean) {
   __shared__ R inv_s;
   if (threadIdx.x == 0) inv_s = (R)(1.0 / mean[0]);
   __syncthreads();
@@ -921,80 +954,105 @@ size_t cic_scratch_bytes(uint64_t n_particles, uint32_t n, bool weighted) {
          (2 * tiles + 2) * sizeof(uint32_t) + face + 16 * 256 + 512;
 }
 
+// The deposit's scratch, laid out.
+struct CicScratch {
+  float4* rec;
+  uint32_t *counts, *cursor;
+  FaceBufs faces;
+  float* wrec;
+  unsigned* wmax;
+  size_t face_elems;
+  uint64_t tiles;
+  CicScratch(void* scratch, uint64_t n_particles, uint32_t n, const CicGeom& g, bool weighted) {
+    char* p = (char*)scratch;
+    auto take = [&](size_t bytes) {
+      char* r = p;
+      p += (bytes + 255) & ~(size_t)255;
+      return (void*)r;
+    };
+    tiles = (uint64_t)g.nt * g.nt * g.nt;
+    face_elems = (size_t)g.nt * n * n;
+    rec = (float4*)take(n_particles * sizeof(float4));
+    counts = (uint32_t*)take((tiles + 1) * sizeof(uint32_t));
+    cursor = (uint32_t*)take((tiles + 1) * sizeof(uint32_t));
+    faces.fx = (unsigned long long*)take(face_elems * 8);
+    faces.fy = (unsigned long long*)take(face_elems * 8);
+    faces.fz = (unsigned long long*)take(face_elems * 8);
+    wrec = weighted ? (float*)take(n_particles * sizeof(float)) : nullptr;
+    wmax = weighted ? (unsigned*)take(2 * sizeof(unsigned)) : nullptr;
+  }
+};
+
+static void tile_count(const float* x, const float* y, const float* z, uint64_t n_particles,
+                       const CicGeom& g, const CicScratch& b, cudaStream_t st, const float* bounds,
+                       unsigned long long* outside) {
+  SIFG_CUDA(cudaMemsetAsync(b.counts, 0, (b.tiles + 1) * sizeof(uint32_t), st));
+  tile_count_kernel<<<grid_for(n_particles, kSortT * kSortUnroll, 152u * 8u), kSortT, 0, st>>>(
+      x, y, z, n_particles, g, b.counts, bounds ? bounds[0] : 0.f, bounds ? bounds[1] : 0.f,
+      bounds ? outside : nullptr);
+  SIFG_LAUNCH_CHECK();
+}
+
+void cic_count(const float* x, const float* y, const float* z, uint64_t n_particles, uint32_t n,
+               float box, void* scratch, cudaStream_t st, const float* bounds,
+               unsigned long long* outside) {
+  const CicGeom g = make_geom(n, box);
+  SIFG_CUDA(cudaMemsetAsync(outside, 0, sizeof(*outside), st));
+  // The weights' buffers lie after everything this pass touches.
+  tile_count(x, y, z, n_particles, g, CicScratch(scratch, n_particles, n, g, false), st, bounds, outside);
+}
+
 void cic_deposit(const float* x, const float* y, const float* z, uint64_t n_particles,
                  uint32_t n, float box, float* grid, void* scratch, cudaStream_t st,
                  KernelTimer* timer, const float* bounds, unsigned long long* outside,
-                 cudaEvent_t sorted, const float* w, KernelTimer* stage) {
+                 cudaEvent_t sorted, const float* w, KernelTimer* stage, bool counted) {
   const CicGeom g = make_geom(n, box);
-  const uint64_t nt = g.nt, tiles = nt * nt * nt;
-  char* p = (char*)scratch;
-  auto take = [&](size_t bytes) {
-    char* r = p;
-    p += (bytes + 255) & ~(size_t)255;
-    return (void*)r;
-  };
-  float4* rec = (float4*)take(n_particles * sizeof(float4));
-  uint32_t* counts = (uint32_t*)take((tiles + 1) * sizeof(uint32_t));
-  uint32_t* cursor = (uint32_t*)take((tiles + 1) * sizeof(uint32_t));
-  const size_t face_elems = nt * (uint64_t)n * n;
-  FaceBufs faces;
-  faces.fx = (unsigned long long*)take(face_elems * 8);
-  faces.fy = (unsigned long long*)take(face_elems * 8);
-  faces.fz = (unsigned long long*)take(face_elems * 8);
-  float* wrec = w ? (float*)take(n_particles * sizeof(float)) : nullptr;
-  unsigned* wmax = w ? (unsigned*)take(2 * sizeof(unsigned)) : nullptr;
+  const CicScratch b(scratch, n_particles, n, g, w != nullptr);
 
   // The stage: the tile sort, the deposit proper and the faces' fix-up.
   if (stage) stage->begin(st);
-  SIFG_CUDA(cudaMemsetAsync(counts, 0, (tiles + 1) * sizeof(uint32_t), st));
-  SIFG_CUDA(cudaMemsetAsync(faces.fx, 0, face_elems * 8, st));
-  SIFG_CUDA(cudaMemsetAsync(faces.fy, 0, face_elems * 8, st));
-  SIFG_CUDA(cudaMemsetAsync(faces.fz, 0, face_elems * 8, st));
-  const unsigned blk = 256;
-  const unsigned grd = grid_for(n_particles, blk, 152u * 16u);
-  const unsigned sgrd = grid_for(n_particles, kSortT * kSortUnroll, 152u * 8u);
+  SIFG_CUDA(cudaMemsetAsync(b.faces.fx, 0, (char*)(b.faces.fz + b.face_elems) - (char*)b.faces.fx, st));
   if (w) {
-    SIFG_CUDA(cudaMemsetAsync(wmax, 0, 2 * sizeof(unsigned), st));
-    weight_max_kernel<<<grd, blk, 0, st>>>(w, n_particles, wmax);
+    SIFG_CUDA(cudaMemsetAsync(b.wmax, 0, 2 * sizeof(unsigned), st));
+    weight_max_kernel<<<grid_for(n_particles, 256, 152u * 16u), 256, 0, st>>>(w, n_particles, b.wmax);
     SIFG_LAUNCH_CHECK();
   }
-  tile_count_kernel<<<sgrd, kSortT, 0, st>>>(x, y, z, n_particles, g, counts,
-                                         bounds ? bounds[0] : 0.f, bounds ? bounds[1] : 0.f,
-                                         bounds ? outside : nullptr);
-  SIFG_LAUNCH_CHECK();
-  exclusive_scan_u32(counts, (uint32_t)(tiles + 1), st);
-  SIFG_CUDA(cudaMemcpyAsync(cursor, counts, (tiles + 1) * sizeof(uint32_t),
+  if (!counted) tile_count(x, y, z, n_particles, g, b, st, bounds, outside);
+  exclusive_scan_u32(b.counts, (uint32_t)(b.tiles + 1), st);
+  SIFG_CUDA(cudaMemcpyAsync(b.cursor, b.counts, (b.tiles + 1) * sizeof(uint32_t),
                             cudaMemcpyDeviceToDevice, st));
-  tile_scatter_kernel<<<sgrd, kSortT, 0, st>>>(x, y, z, n_particles, g, cursor, rec, w, wrec);
+  tile_scatter_kernel<<<grid_for(n_particles, kSortT * kSortUnroll, 152u * 8u), kSortT, 0, st>>>(
+      x, y, z, n_particles, g, b.cursor, b.rec, w, b.wrec);
   SIFG_LAUNCH_CHECK();
   if (sorted) SIFG_CUDA(cudaEventRecord(sorted, st));
   const float cl = box / (float)n;
   const float inv_cell_vol = 1.0f / (float)(cl * cl * cl);
   const size_t smem = (size_t)2 * kTileWords * sizeof(uint32_t);
-  auto grid_of = [&](unsigned per_sm) { return (unsigned)std::min<uint64_t>(tiles, 152u * per_sm); };
+  auto grid_of = [&](unsigned per_sm) { return (unsigned)std::min<uint64_t>(b.tiles, 152u * per_sm); };
   if (timer) timer->begin(st);
   if (w) {
-    tile_deposit_wide_kernel<<<grid_of(5), kDepositT, smem, st>>>(rec, counts, g, inv_cell_vol, grid,
-                                                                  faces, wrec, wmax, nullptr);
+    tile_deposit_wide_kernel<<<grid_of(5), kDepositT, smem, st>>>(b.rec, b.counts, g, inv_cell_vol,
+                                                                  grid, b.faces, b.wrec, b.wmax, nullptr);
     SIFG_LAUNCH_CHECK();
   } else {
     // The scatter's cursors are free: the list of tiles to do again.
-    uint32_t* redo = cursor;
+    uint32_t* redo = b.cursor;
     SIFG_CUDA(cudaMemsetAsync(redo, 0, sizeof(uint32_t), st));
-    tile_deposit_kernel<<<grid_of(6), kDepositT, 0, st>>>(rec, counts, g, inv_cell_vol, grid, faces,
-                                                          redo);
+    tile_deposit_kernel<<<grid_of(6), kDepositT, 0, st>>>(b.rec, b.counts, g, inv_cell_vol, grid,
+                                                          b.faces, redo);
     SIFG_LAUNCH_CHECK();
-    tile_deposit_wide_kernel<<<grid_of(1), kDepositT, smem, st>>>(rec, counts, g, inv_cell_vol, grid,
-                                                                  faces, nullptr, nullptr, redo);
+    tile_deposit_wide_kernel<<<grid_of(1), kDepositT, smem, st>>>(
+        b.rec, b.counts, g, inv_cell_vol, grid, b.faces, nullptr, nullptr, redo);
     SIFG_LAUNCH_CHECK();
   }
   if (timer) timer->end(st);
-  face_fixup_kernel<<<grid_for(3 * face_elems, 256), 256, 0, st>>>(g, inv_cell_vol, grid, faces,
-                                                                  wmax);
+  face_fixup_kernel<<<dim3(grid_for((uint64_t)n * n, 256, 152u * 16u), 3 * g.nt), 256, 0, st>>>(
+      g, inv_cell_vol, grid, b.faces, b.wmax);
   SIFG_LAUNCH_CHECK();
   if (stage) stage->end(st);
   if (w) {
-    nonfinite_weights_kernel<<<grd, blk, 0, st>>>(x, y, z, w, n_particles, g, wmax, grid);
+    nonfinite_weights_kernel<<<grid_for(n_particles, 256, 152u * 16u), 256, 0, st>>>(
+        x, y, z, w, n_particles, g, b.wmax, grid);
     SIFG_LAUNCH_CHECK();
   }
 }
@@ -1013,7 +1071,10 @@ template void density_contrast<double>(double*, uint64_t, double*, cudaStream_t,
 
 template <class R>
 void apply_contrast(R* v, uint64_t n, const double* mean, cudaStream_t st) {
-  contrast_kernel<R><<<grid_for(n, 256), 256, 0, st>>>(v, n, mean);
+  if ((uintptr_t)v % 16 == 0)
+    contrast_kernel<R><<<grid_for(n * sizeof(R) / 32, 256, 152u * 8u), 256, 0, st>>>(v, n, mean);
+  else
+    contrast_any_kernel<R><<<grid_for(n, 256), 256, 0, st>>>(v, n, mean);
   SIFG_LAUNCH_CHECK();
 }
 template void apply_contrast<float>(float*, uint64_t, const double*, cudaStream_t);

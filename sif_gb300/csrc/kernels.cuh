@@ -101,11 +101,18 @@ size_t cic_scratch_bytes(uint64_t n_particles, uint32_t n, bool weighted = false
 // follows (the deposit proper) is bound by shared-memory atomics, not by HBM.
 // w: per-particle weights (device), or NULL for 1 each; the scratch is then
 // cic_scratch_bytes(n_particles, n, true).
+// cic_count is the deposit's first pass on its own, for a caller that checks
+// the positions before the grid is written: it counts into the scratch (and
+// the particles outside `bounds` into *outside, which it zeroes), and a
+// deposit with `counted` set goes on from there.
+void cic_count(const float* x, const float* y, const float* z, uint64_t n_particles, uint32_t n,
+               float box, void* scratch, cudaStream_t st, const float* bounds,
+               unsigned long long* outside);
 void cic_deposit(const float* x, const float* y, const float* z, uint64_t n_particles,
                  uint32_t n, float box, float* grid, void* scratch, cudaStream_t st,
                  KernelTimer* timer, const float* bounds = nullptr,
                  unsigned long long* outside = nullptr, cudaEvent_t sorted = nullptr,
-                 const float* w = nullptr, KernelTimer* stage = nullptr);
+                 const float* w = nullptr, KernelTimer* stage = nullptr, bool counted = false);
 // The FP64 form's deposit: scratch is cic_f64_scratch_bytes(n).
 size_t cic_f64_scratch_bytes(uint32_t n);
 void cic_deposit_f64(const double* x, const double* y, const double* z, uint64_t n_particles,
@@ -156,10 +163,17 @@ size_t mesh_scratch_bytes(uint64_t n_particles, uint32_t n_cells);
 // placed them (no orig) and, in the float form, the positions go to m.xyzw:
 // the same cells and counts, for a mesh only the sphere growth reads -- a
 // radius depends on which particles a cell holds, not on their order.
+// mesh_count is the build's first pass on its own, for a caller that checks
+// the positions before anything of the mesh is written (bounds, outside: as
+// cic_count's): it counts into the scratch, and a build with `counted` set
+// goes on from there.
+template <class R>
+void mesh_count(const R* x, const R* y, const R* z, uint64_t n_particles, const DeviceMeshT<R>& m,
+                void* scratch, cudaStream_t st, const R* bounds, unsigned long long* outside);
 template <class R>
 void mesh_build(const R* x, const R* y, const R* z, uint64_t n_particles, DeviceMeshT<R>& m,
                 void* scratch, cudaStream_t st, KernelTimer* timer, uint32_t* scan_sums = nullptr,
-                bool canonical = true);
+                bool canonical = true, bool counted = false);
 // A canonical mesh's weight columns from the field's weights (device, source
 // order): m.w (n_particles) and m.cell_w (n_cells^3) written, the total to
 // *d_total (device). scratch: mesh_weights_scratch_bytes(n_cells).

@@ -6,14 +6,13 @@
 // the reference's: (int32)(fold(x) * (1/cell_length)) clamped into the mesh
 // (chain_mesh.c:316-331), so the mesh is the reference's bit for bit.
 //
-//   1. cell_count:  per-cell counts, warp-aggregated atomics;
-//   2. exclusive scan into the cell offsets;
+//   1. cell_count:  per-cell counts, warp-aggregated atomics, in scratch;
+//   2. exclusive scan, copied to the cell offsets;
 //   3. cell_scatter: (source index, x, y, z) into each cell's range, in the
 //      order the atomics hand out slots;
-//   4. cell_canon:  per cell, each entry's rank among the cell's source
-//      indices (a count over the cell, with every lane reading the same
-//      shared word at once), and the entry written to that rank -- the
-//      canonical order, which no atomic race can change.
+//   4. cell_canon:  per entry, its rank among its cell's source indices (a
+//      count over the cell's keys in shared memory), and the entry written
+//      to that rank -- the canonical order, which no atomic race can change.
 #include <cuda_runtime.h>
 
 #include "common.cuh"
@@ -37,174 +36,280 @@ struct alignas(16) MeshRec {
 static_assert(sizeof(MeshRec<float>) == 16, "float records are 16 bytes");
 static_assert(sizeof(MeshRec<double>) == 32, "double records are 32 bytes");
 
+// A particle's cell, its coordinates folded into the box on the way. Nearly
+// every coordinate is in [0, box), where the fold and the clamp at zero do
+// nothing; any that is not (NaN among them) takes all three through them.
 template <class R>
-__device__ __forceinline__ uint32_t mesh_cell(R x, R y, R z, const MeshGeom<R>& g) {
-  int32_t ix = (int32_t)fmul(box_fold(x, g.box), g.inv_l);
-  int32_t iy = (int32_t)fmul(box_fold(y, g.box), g.inv_l);
-  int32_t iz = (int32_t)fmul(box_fold(z, g.box), g.inv_l);
+__device__ __forceinline__ uint32_t mesh_cell(R& x, R& y, R& z, const MeshGeom<R>& g) {
   const int32_t hi = (int32_t)g.n - 1;
-  ix = ix < 0 ? 0 : (ix > hi ? hi : ix);
-  iy = iy < 0 ? 0 : (iy > hi ? hi : iy);
-  iz = iz < 0 ? 0 : (iz > hi ? hi : iz);
-  return ((uint32_t)ix * g.n + (uint32_t)iy) * g.n + (uint32_t)iz;
+  int32_t ix, iy, iz;
+  if (x >= R(0) && x < g.box && y >= R(0) && y < g.box && z >= R(0) && z < g.box) {
+    ix = (int32_t)fmul(x, g.inv_l);
+    iy = (int32_t)fmul(y, g.inv_l);
+    iz = (int32_t)fmul(z, g.inv_l);
+  } else {
+    x = box_fold(x, g.box);
+    y = box_fold(y, g.box);
+    z = box_fold(z, g.box);
+    ix = max((int32_t)fmul(x, g.inv_l), 0);
+    iy = max((int32_t)fmul(y, g.inv_l), 0);
+    iz = max((int32_t)fmul(z, g.inv_l), 0);
+  }
+  return ((uint32_t)min(ix, hi) * g.n + (uint32_t)min(iy, hi)) * g.n + (uint32_t)min(iz, hi);
 }
 
+// The passes over the particles wait on their loads and on the atomics that
+// hand out slots: kMeshUnroll particles a thread in flight. (One at a time,
+// the scatter of 64.5 M particles into 117^3 cells spent 87% of its stalls on
+// them.)
+constexpr int kMeshT = 256;
+constexpr int kMeshUnroll = 4;
+
+// With `outside` set, also counts the particles outside [lo, hi] on any axis
+// (NaN included): the box check, from the same reads.
 template <class R>
-__global__ void cell_count_kernel(const R* __restrict__ x, const R* __restrict__ y,
-                                  const R* __restrict__ z, uint64_t n, MeshGeom<R> g,
-                                  uint32_t* __restrict__ counts) {
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < n; base += stride) {
-    const uint64_t p = base + threadIdx.x;
-    const bool valid = p < n;
-    const uint32_t c = valid ? mesh_cell(x[p], y[p], z[p], g) : 0xffffffffu;
-    const unsigned peers = __match_any_sync(0xffffffffu, c);
-    if (valid && (threadIdx.x & 31u) == (unsigned)(__ffs(peers) - 1))
-      atomicAdd(counts + c, (uint32_t)__popc(peers));
+__global__ void __launch_bounds__(kMeshT) cell_count_kernel(
+    const R* __restrict__ x, const R* __restrict__ y, const R* __restrict__ z, uint64_t n,
+    MeshGeom<R> g, uint32_t* __restrict__ counts, R lo, R hi,
+    unsigned long long* __restrict__ outside) {
+  const uint64_t stride = (uint64_t)gridDim.x * kMeshT * kMeshUnroll;
+  uint32_t bad = 0;
+  for (uint64_t base = (uint64_t)blockIdx.x * kMeshT * kMeshUnroll; base < n; base += stride) {
+    R px[kMeshUnroll], py[kMeshUnroll], pz[kMeshUnroll];
+#pragma unroll
+    for (int u = 0; u < kMeshUnroll; u++) {
+      const uint64_t p = base + u * kMeshT + threadIdx.x;
+      if (p < n) {
+        px[u] = x[p];
+        py[u] = y[p];
+        pz[u] = z[p];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kMeshUnroll; u++) {
+      uint32_t c = 0xffffffffu;
+      if (base + u * kMeshT + threadIdx.x < n) {
+        if (outside)
+          bad += px[u] >= lo && px[u] <= hi && py[u] >= lo && py[u] <= hi && pz[u] >= lo && pz[u] <= hi
+                     ? 0u
+                     : 1u;
+        c = mesh_cell(px[u], py[u], pz[u], g);
+      }
+      const unsigned peers = __match_any_sync(0xffffffffu, c);
+      if (c != 0xffffffffu && (threadIdx.x & 31u) == (unsigned)(__ffs(peers) - 1))
+        atomicAdd(counts + c, (uint32_t)__popc(peers));
+    }
+  }
+  if (outside) {
+    const unsigned long long b = __reduce_add_sync(0xffffffffu, bad);
+    if ((threadIdx.x & 31u) == 0 && b) atomicAdd(outside, b);
   }
 }
 
+// Where a scatter leaves a particle: a record with its source index, for the
+// canonical order; a 16-byte position record (the float form of a build that
+// leaves each cell in scatter order); the mesh's position arrays (its FP64
+// form).
 template <class R>
-__global__ void cell_scatter_kernel(const R* __restrict__ x, const R* __restrict__ y,
-                                    const R* __restrict__ z, uint64_t n, MeshGeom<R> g,
-                                    uint32_t* __restrict__ cursor, MeshRec<R>* __restrict__ tmp) {
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+struct ToRecord {
+  MeshRec<R>* tmp;
+  __device__ __forceinline__ void put(uint32_t slot, uint64_t p, R x, R y, R z) const {
+    MeshRec<R> rec;
+    rec.i = (uint32_t)p;
+    rec.x = x;
+    rec.y = y;
+    rec.z = z;
+    tmp[slot] = rec;
+  }
+};
+struct ToXyzw {
+  float4* out;
+  __device__ __forceinline__ void put(uint32_t slot, uint64_t, float x, float y, float z) const {
+    out[slot] = make_float4(x, y, z, 0.f);
+  }
+};
+template <class R>
+struct ToArrays {
+  R *ox, *oy, *oz;
+  __device__ __forceinline__ void put(uint32_t slot, uint64_t, R x, R y, R z) const {
+    ox[slot] = x;
+    oy[slot] = y;
+    oz[slot] = z;
+  }
+};
+
+template <class R, class To>
+__global__ void __launch_bounds__(kMeshT) cell_scatter_kernel(
+    const R* __restrict__ x, const R* __restrict__ y, const R* __restrict__ z, uint64_t n,
+    MeshGeom<R> g, uint32_t* __restrict__ cursor, To to) {
+  const uint64_t stride = (uint64_t)gridDim.x * kMeshT * kMeshUnroll;
   const unsigned lane = threadIdx.x & 31u;
-  for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < n; base += stride) {
-    const uint64_t p = base + threadIdx.x;
-    const bool valid = p < n;
-    R px = 0, py = 0, pz = 0;
-    uint32_t c = 0xffffffffu;
-    if (valid) {
-      px = box_fold(x[p], g.box);
-      py = box_fold(y[p], g.box);
-      pz = box_fold(z[p], g.box);
-      c = mesh_cell(x[p], y[p], z[p], g);
+  for (uint64_t base = (uint64_t)blockIdx.x * kMeshT * kMeshUnroll; base < n; base += stride) {
+    R px[kMeshUnroll], py[kMeshUnroll], pz[kMeshUnroll];
+    uint32_t slot[kMeshUnroll], peers[kMeshUnroll];
+#pragma unroll
+    for (int u = 0; u < kMeshUnroll; u++) {
+      const uint64_t p = base + u * kMeshT + threadIdx.x;
+      if (p < n) {
+        px[u] = x[p];
+        py[u] = y[p];
+        pz[u] = z[p];
+      }
     }
-    const unsigned peers = __match_any_sync(0xffffffffu, c);
-    const unsigned leader = __ffs(peers) - 1;
-    uint32_t slot0 = 0;
-    if (valid && lane == leader) slot0 = atomicAdd(cursor + c, (uint32_t)__popc(peers));
-    slot0 = __shfl_sync(0xffffffffu, slot0, leader);
-    if (valid) {
-      const uint32_t slot = slot0 + __popc(peers & ((1u << lane) - 1u));
-      MeshRec<R> rec;
-      rec.i = (uint32_t)p;
-      rec.x = px;
-      rec.y = py;
-      rec.z = pz;
-      tmp[slot] = rec;
+#pragma unroll
+    for (int u = 0; u < kMeshUnroll; u++) {
+      const bool valid = base + u * kMeshT + threadIdx.x < n;
+      const uint32_t c = valid ? mesh_cell(px[u], py[u], pz[u], g) : 0xffffffffu;
+      peers[u] = __match_any_sync(0xffffffffu, c);
+      if (valid && lane == (unsigned)(__ffs(peers[u]) - 1))
+        slot[u] = atomicAdd(cursor + c, (uint32_t)__popc(peers[u]));
+    }
+#pragma unroll
+    for (int u = 0; u < kMeshUnroll; u++) {
+      const uint64_t p = base + u * kMeshT + threadIdx.x;
+      const uint32_t s = __shfl_sync(0xffffffffu, slot[u], __ffs(peers[u]) - 1) +
+                         __popc(peers[u] & ((1u << lane) - 1u));
+      if (p < n) to.put(s, p, px[u], py[u], pz[u]);
     }
   }
 }
 
-// The float form's scatter straight into 16-byte position records, for a
-// build that leaves each cell in scatter order.
-__global__ void cell_scatter_xyzw_kernel(const float* __restrict__ x, const float* __restrict__ y,
-                                         const float* __restrict__ z, uint64_t n,
-                                         MeshGeom<float> g, uint32_t* __restrict__ cursor,
-                                         float4* __restrict__ out) {
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+// The canonical order: each entry written at its rank among its cell's source
+// indices. A warp a cell, up to kCanonSort entries: the keys sorted in
+// registers (a bitonic network, 32 K of them for the smallest K that holds the
+// cell), left in shared memory, and each entry's key looked up among them. The
+// kernel is bound by its instructions: counting the smaller keys one by one is
+// two or three a pair, 60 pairs an entry at a mean of 40 a cell. (64.5 M
+// particles in 117^3 cells: 0.98 ms counted by a warp a cell, 0.86 by a thread
+// an entry, 0.66 sorted.) A cell with more entries is ranked by the CTA's warps together,
+// its keys counted as they pass through shared memory.
+constexpr int kCanonT = 256;
+constexpr int kCanonCells = 256;  // cells a CTA takes at a time
+constexpr int kCanonSort = 256;   // entries a warp sorts
+constexpr int kCanonKeys = 1024;  // keys in shared memory while a larger cell is counted
+
+// Ascending sort of 32 K values held by one warp, v[j] at index j * 32 + lane:
+// partners in other lanes through shuffles, in other registers directly.
+template <int K>
+__device__ __forceinline__ void warp_sort_keys(uint32_t (&v)[K]) {
   const unsigned lane = threadIdx.x & 31u;
-  for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < n; base += stride) {
-    const uint64_t p = base + threadIdx.x;
-    const bool valid = p < n;
-    float px = 0, py = 0, pz = 0;
-    uint32_t c = 0xffffffffu;
-    if (valid) {
-      px = x[p];
-      py = y[p];
-      pz = z[p];
-      c = mesh_cell(px, py, pz, g);
+#pragma unroll
+  for (int k = 2; k <= 32 * K; k <<= 1) {
+#pragma unroll
+    for (int d = k >> 1; d > 0; d >>= 1) {
+#pragma unroll
+      for (int j = 0; j < K; j++) {
+        if (d >= 32) {
+          const int dj = d >> 5;
+          if (j & dj) continue;
+          const bool up = ((j << 5) & k) == 0;  // k > 32 here
+          const uint32_t a = v[j], b = v[j | dj];
+          v[j] = up ? min(a, b) : max(a, b);
+          v[j | dj] = up ? max(a, b) : min(a, b);
+        } else {
+          const uint32_t o = __shfl_xor_sync(0xffffffffu, v[j], d);
+          const bool up = (((j << 5) | (int)lane) & k) == 0;
+          const bool lower = (lane & (unsigned)d) == 0;
+          v[j] = lower == up ? min(v[j], o) : max(v[j], o);
+        }
+      }
     }
-    const unsigned peers = __match_any_sync(0xffffffffu, c);
-    const unsigned leader = __ffs(peers) - 1;
-    uint32_t slot0 = 0;
-    if (valid && lane == leader) slot0 = atomicAdd(cursor + c, (uint32_t)__popc(peers));
-    slot0 = __shfl_sync(0xffffffffu, slot0, leader);
-    if (valid)
-      out[slot0 + __popc(peers & ((1u << lane) - 1u))] =
-          make_float4(box_fold(px, g.box), box_fold(py, g.box), box_fold(pz, g.box), 0.f);
   }
 }
 
-// The FP64 form's: straight into the mesh's position arrays.
 template <class R>
-__global__ void cell_scatter_soa_kernel(const R* __restrict__ x, const R* __restrict__ y,
-                                        const R* __restrict__ z, uint64_t n, MeshGeom<R> g,
-                                        uint32_t* __restrict__ cursor, R* __restrict__ ox,
-                                        R* __restrict__ oy, R* __restrict__ oz) {
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+__device__ __forceinline__ void canon_write(const MeshRec<R>& v, uint32_t dst, R* ox, R* oy, R* oz,
+                                            uint32_t* orig) {
+  ox[dst] = v.x;
+  oy[dst] = v.y;
+  oz[dst] = v.z;
+  if (orig) orig[dst] = v.i;
+}
+
+// One warp orders the cell at [s, e), e - s <= 32 K; keys: 32 K words of its own.
+template <int K, class R>
+__device__ __forceinline__ void canon_cell(const MeshRec<R>* __restrict__ tmp, uint32_t s, uint32_t e,
+                                           uint32_t* keys, R* ox, R* oy, R* oz, uint32_t* orig) {
   const unsigned lane = threadIdx.x & 31u;
-  for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < n; base += stride) {
-    const uint64_t p = base + threadIdx.x;
-    const bool valid = p < n;
-    R px = 0, py = 0, pz = 0;
-    uint32_t c = 0xffffffffu;
-    if (valid) {
-      px = x[p];
-      py = y[p];
-      pz = z[p];
-      c = mesh_cell(px, py, pz, g);
-    }
-    const unsigned peers = __match_any_sync(0xffffffffu, c);
-    const unsigned leader = __ffs(peers) - 1;
-    uint32_t slot0 = 0;
-    if (valid && lane == leader) slot0 = atomicAdd(cursor + c, (uint32_t)__popc(peers));
-    slot0 = __shfl_sync(0xffffffffu, slot0, leader);
-    if (valid) {
-      const uint32_t slot = slot0 + __popc(peers & ((1u << lane) - 1u));
-      ox[slot] = box_fold(px, g.box);
-      oy[slot] = box_fold(py, g.box);
-      oz[slot] = box_fold(pz, g.box);
+  uint32_t v[K], mine[K];
+#pragma unroll
+  for (int j = 0; j < K; j++) {
+    const uint32_t p = s + j * 32 + lane;
+    v[j] = mine[j] = p < e ? tmp[p].i : 0xffffffffu;  // above every source index
+  }
+  warp_sort_keys<K>(v);
+#pragma unroll
+  for (int j = 0; j < K; j++) keys[j * 32 + lane] = v[j];
+  __syncwarp();
+#pragma unroll
+  for (int j = 0; j < K; j++) {
+    const uint32_t p = s + j * 32 + lane;
+    if (p < e) {
+      uint32_t rank = 0;
+#pragma unroll
+      for (int step = 16 * K; step > 0; step >>= 1)
+        if (keys[rank + step - 1] < mine[j]) rank += step;
+      canon_write(tmp[p], s + rank, ox, oy, oz, orig);
     }
   }
+  __syncwarp();
 }
 
-constexpr int kCanonThreads = 128;
-constexpr int kCanonSmem = 2048;  // entries a CTA ranks in shared memory
-
-// One warp per cell. A cell of up to kCanonSmem/4 entries per warp is ranked
-// from shared memory; a larger one is ranked straight from global memory.
 template <class R>
-__global__ void __launch_bounds__(kCanonThreads) cell_canon_kernel(
+__global__ void __launch_bounds__(kCanonT) cell_canon_kernel(
     const MeshRec<R>* __restrict__ tmp, const uint32_t* __restrict__ offsets,
     uint32_t n_cells_total, R* __restrict__ ox, R* __restrict__ oy, R* __restrict__ oz,
     uint32_t* __restrict__ orig) {
-  __shared__ uint32_t keys[kCanonSmem];
-  const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-  const unsigned warps = kCanonThreads / 32;
-  const uint32_t per_warp = kCanonSmem / warps;
-  uint32_t* wk = keys + warp * per_warp;
-  for (uint32_t cell = blockIdx.x * warps + warp; cell < n_cells_total;
-       cell += gridDim.x * warps) {
-    const uint32_t s = offsets[cell], e = offsets[cell + 1], cnt = e - s;
-    if (cnt == 0) continue;
-    const bool in_smem = cnt <= per_warp;
-    if (in_smem) {
-      for (uint32_t i = lane; i < cnt; i += 32) wk[i] = tmp[s + i].i;
-      __syncwarp();
+  __shared__ uint32_t keys[kCanonT / 32 * kCanonSort];
+  __shared__ uint32_t offs[kCanonCells + 1];
+  __shared__ uint32_t large[kCanonCells];
+  __shared__ uint32_t n_large;
+  static_assert(kCanonKeys <= kCanonT / 32 * kCanonSort && kCanonCells == kCanonT, "shared layout");
+  const unsigned warp = threadIdx.x >> 5;
+  const uint32_t groups = (n_cells_total + kCanonCells - 1) / kCanonCells;
+  for (uint32_t group = blockIdx.x; group < groups; group += gridDim.x) {
+    const uint32_t c0 = group * kCanonCells, nc = min((uint32_t)kCanonCells, n_cells_total - c0);
+    __syncthreads();
+    if (threadIdx.x < nc) offs[threadIdx.x] = offsets[c0 + threadIdx.x];
+    if (threadIdx.x == 0) {
+      offs[nc] = offsets[c0 + nc];
+      n_large = 0;
     }
-    for (uint32_t i = lane; i < cnt + (32 - cnt % 32) % 32; i += 32) {
-      const bool mine = i < cnt;
-      MeshRec<R> v;
-      v.i = 0;
-      if (mine) v = tmp[s + i];
-      uint32_t rank = 0;
-      if (in_smem) {
-        for (uint32_t j = 0; j < cnt; j++) rank += wk[j] < v.i;
-      } else {
-        for (uint32_t j = 0; j < cnt; j++) rank += tmp[s + j].i < v.i;
-      }
-      if (mine) {
-        const uint32_t dst = s + rank;
-        ox[dst] = v.x;
-        oy[dst] = v.y;
-        oz[dst] = v.z;
-        if (orig) orig[dst] = v.i;
+    __syncthreads();
+    if (threadIdx.x < nc && offs[threadIdx.x + 1] - offs[threadIdx.x] > kCanonSort)
+      large[atomicAdd(&n_large, 1u)] = threadIdx.x;
+    for (uint32_t c = warp; c < nc; c += kCanonT / 32) {
+      const uint32_t s = offs[c], e = offs[c + 1], cnt = e - s;
+      uint32_t* wk = keys + warp * kCanonSort;
+      if (cnt == 0 || cnt > kCanonSort) continue;
+      if (cnt <= 32)
+        canon_cell<1>(tmp, s, e, wk, ox, oy, oz, orig);
+      else if (cnt <= 64)
+        canon_cell<2>(tmp, s, e, wk, ox, oy, oz, orig);
+      else if (cnt <= 128)
+        canon_cell<4>(tmp, s, e, wk, ox, oy, oz, orig);
+      else
+        canon_cell<8>(tmp, s, e, wk, ox, oy, oz, orig);
+    }
+    __syncthreads();
+    for (uint32_t l = 0; l < n_large; l++) {
+      const uint32_t s = offs[large[l]], e = offs[large[l] + 1];
+      for (uint32_t p0 = s; p0 < e; p0 += kCanonT) {
+        const uint32_t p = p0 + threadIdx.x;
+        MeshRec<R> v{};
+        if (p < e) v = tmp[p];
+        uint32_t rank = 0;
+        for (uint32_t k0 = s; k0 < e; k0 += kCanonKeys) {
+          const uint32_t nk = min((uint32_t)kCanonKeys, e - k0);
+          __syncthreads();
+          for (uint32_t k = threadIdx.x; k < nk; k += kCanonT) keys[k] = tmp[k0 + k].i;
+          __syncthreads();
+#pragma unroll 8
+          for (uint32_t k = 0; k < nk; k++) rank += keys[k] < v.i ? 1u : 0u;
+        }
+        if (p < e) canon_write(v, s + rank, ox, oy, oz, orig);
       }
     }
-    __syncwarp();
   }
 }
 
@@ -214,41 +319,55 @@ size_t mesh_scratch_bytes(uint64_t n_particles, uint32_t n_cells) {
 }
 
 template <class R>
+static MeshGeom<R> mesh_geom(const DeviceMeshT<R>& m) {
+  return MeshGeom<R>{m.n_cells, m.box_length, R(1.0f) / m.cell_length};
+}
+
+static uint32_t* mesh_cursor(void* scratch, uint64_t n_particles, size_t record) {
+  return (uint32_t*)((char*)scratch + ((n_particles * record + 255) & ~(size_t)255));
+}
+
+template <class R>
+void mesh_count(const R* x, const R* y, const R* z, uint64_t n_particles, const DeviceMeshT<R>& m,
+                void* scratch, cudaStream_t st, const R* bounds, unsigned long long* outside) {
+  const uint64_t cells = (uint64_t)m.n_cells * m.n_cells * m.n_cells;
+  uint32_t* cursor = mesh_cursor(scratch, n_particles, sizeof(MeshRec<R>));
+  SIFG_CUDA(cudaMemsetAsync(cursor, 0, (cells + 1) * sizeof(uint32_t), st));
+  cell_count_kernel<R><<<grid_for(n_particles, kMeshT * kMeshUnroll, 152u * 8u), kMeshT, 0, st>>>(
+      x, y, z, n_particles, mesh_geom(m), cursor, bounds ? bounds[0] : R(0), bounds ? bounds[1] : R(0),
+      bounds ? outside : nullptr);
+  SIFG_LAUNCH_CHECK();
+}
+
+template <class R>
 void mesh_build(const R* x, const R* y, const R* z, uint64_t n_particles, DeviceMeshT<R>& m,
                 void* scratch, cudaStream_t st, KernelTimer* timer, uint32_t* scan_sums,
-                bool canonical) {
-  MeshGeom<R> g;
-  g.n = m.n_cells;
-  g.box = m.box_length;
-  g.inv_l = R(1.0f) / m.cell_length;
+                bool canonical, bool counted) {
+  const MeshGeom<R> g = mesh_geom(m);
   const uint64_t cells = (uint64_t)m.n_cells * m.n_cells * m.n_cells;
   MeshRec<R>* tmp = (MeshRec<R>*)scratch;
-  uint32_t* cursor = (uint32_t*)((char*)scratch +
-                                 ((n_particles * sizeof(MeshRec<R>) + 255) & ~(size_t)255));
-  SIFG_CUDA(cudaMemsetAsync(m.offsets, 0, (cells + 1) * sizeof(uint32_t), st));
-  const unsigned grd = grid_for(n_particles, 256, 152u * 16u);
+  uint32_t* cursor = mesh_cursor(scratch, n_particles, sizeof(MeshRec<R>));
+  const unsigned grd = grid_for(n_particles, kMeshT * kMeshUnroll, 152u * 8u);
   if (timer) timer->begin(st);
-  cell_count_kernel<R><<<grd, 256, 0, st>>>(x, y, z, n_particles, g, m.offsets);
-  SIFG_LAUNCH_CHECK();
-  exclusive_scan_u32(m.offsets, (uint32_t)(cells + 1), st, scan_sums);
-  SIFG_CUDA(cudaMemcpyAsync(cursor, m.offsets, cells * sizeof(uint32_t),
+  if (!counted) mesh_count(x, y, z, n_particles, m, scratch, st, (const R*)nullptr, nullptr);
+  exclusive_scan_u32(cursor, (uint32_t)(cells + 1), st, scan_sums);
+  SIFG_CUDA(cudaMemcpyAsync(m.offsets, cursor, (cells + 1) * sizeof(uint32_t),
                             cudaMemcpyDeviceToDevice, st));
   if (!canonical) {
     if constexpr (sizeof(R) == 4)
-      cell_scatter_xyzw_kernel<<<grd, 256, 0, st>>>(x, y, z, n_particles, g, cursor, m.xyzw);
+      cell_scatter_kernel<R><<<grd, kMeshT, 0, st>>>(x, y, z, n_particles, g, cursor, ToXyzw{m.xyzw});
     else
-      cell_scatter_soa_kernel<R><<<grd, 256, 0, st>>>(x, y, z, n_particles, g, cursor, m.x, m.y,
-                                                      m.z);
+      cell_scatter_kernel<R><<<grd, kMeshT, 0, st>>>(x, y, z, n_particles, g, cursor,
+                                                     ToArrays<R>{m.x, m.y, m.z});
     SIFG_LAUNCH_CHECK();
     if (timer) timer->end(st);
     m.n_particles = n_particles;
     return;
   }
-  cell_scatter_kernel<R><<<grd, 256, 0, st>>>(x, y, z, n_particles, g, cursor, tmp);
+  cell_scatter_kernel<R><<<grd, kMeshT, 0, st>>>(x, y, z, n_particles, g, cursor, ToRecord<R>{tmp});
   SIFG_LAUNCH_CHECK();
-  const unsigned cgrid = grid_for(cells, kCanonThreads / 32 * 1, 152u * 16u);
-  cell_canon_kernel<R><<<cgrid, kCanonThreads, 0, st>>>(tmp, m.offsets, (uint32_t)cells, m.x, m.y,
-                                                        m.z, m.orig);
+  cell_canon_kernel<R><<<grid_for(cells, kCanonCells, 152u * 8u), kCanonT, 0, st>>>(
+      tmp, m.offsets, (uint32_t)cells, m.x, m.y, m.z, m.orig);
   SIFG_LAUNCH_CHECK();
   if (timer) timer->end(st);
   m.n_particles = n_particles;
@@ -326,9 +445,15 @@ template void mesh_weights<double>(const double*, DeviceMeshT<double>&, void*, d
 
 template void mesh_build<float>(const float*, const float*, const float*, uint64_t,
                                 DeviceMeshT<float>&, void*, cudaStream_t, KernelTimer*, uint32_t*,
-                                bool);
+                                bool, bool);
 template void mesh_build<double>(const double*, const double*, const double*, uint64_t,
                                  DeviceMeshT<double>&, void*, cudaStream_t, KernelTimer*,
-                                 uint32_t*, bool);
+                                 uint32_t*, bool, bool);
+template void mesh_count<float>(const float*, const float*, const float*, uint64_t,
+                                const DeviceMeshT<float>&, void*, cudaStream_t, const float*,
+                                unsigned long long*);
+template void mesh_count<double>(const double*, const double*, const double*, uint64_t,
+                                 const DeviceMeshT<double>&, void*, cudaStream_t, const double*,
+                                 unsigned long long*);
 
 }  // namespace sifg
