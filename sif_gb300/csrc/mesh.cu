@@ -15,6 +15,8 @@
 //      to that rank -- the canonical order, which no atomic race can change.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "kernels.cuh"
 
@@ -181,12 +183,10 @@ __global__ void __launch_bounds__(kMeshT) cell_scatter_kernel(
 // kernel is bound by its instructions: counting the smaller keys one by one is
 // two or three a pair, 60 pairs an entry at a mean of 40 a cell. (64.5 M
 // particles in 117^3 cells: 0.98 ms counted by a warp a cell, 0.86 by a thread
-// an entry, 0.66 sorted.) A cell with more entries is ranked by the CTA's warps together,
-// its keys counted as they pass through shared memory.
+// an entry, 0.66 sorted.)
 constexpr int kCanonT = 256;
-constexpr int kCanonCells = 256;  // cells a CTA takes at a time
-constexpr int kCanonSort = 256;   // entries a warp sorts
-constexpr int kCanonKeys = 1024;  // keys in shared memory while a larger cell is counted
+constexpr int kCanonSort = 256;    // entries a warp sorts in cell_canon_kernel
+constexpr int kCanonLarge = 1024;  // and in cell_canon_large_kernel
 
 // Ascending sort of 32 K values held by one warp, v[j] at index j * 32 + lane:
 // partners in other lanes through shuffles, in other registers directly.
@@ -255,60 +255,80 @@ __device__ __forceinline__ void canon_cell(const MeshRec<R>* __restrict__ tmp, u
   __syncwarp();
 }
 
+// Cells of up to kCanonSort entries, a warp each; the larger ones are listed in
+// `more` (more[0] counts them) for cell_canon_large_kernel, which takes four
+// times the registers.
 template <class R>
 __global__ void __launch_bounds__(kCanonT) cell_canon_kernel(
     const MeshRec<R>* __restrict__ tmp, const uint32_t* __restrict__ offsets,
     uint32_t n_cells_total, R* __restrict__ ox, R* __restrict__ oy, R* __restrict__ oz,
-    uint32_t* __restrict__ orig) {
+    uint32_t* __restrict__ orig, uint32_t* __restrict__ more, uint32_t span) {
   __shared__ uint32_t keys[kCanonT / 32 * kCanonSort];
-  __shared__ uint32_t offs[kCanonCells + 1];
-  __shared__ uint32_t large[kCanonCells];
-  __shared__ uint32_t n_large;
-  static_assert(kCanonKeys <= kCanonT / 32 * kCanonSort && kCanonCells == kCanonT, "shared layout");
-  const unsigned warp = threadIdx.x >> 5;
-  const uint32_t groups = (n_cells_total + kCanonCells - 1) / kCanonCells;
-  for (uint32_t group = blockIdx.x; group < groups; group += gridDim.x) {
-    const uint32_t c0 = group * kCanonCells, nc = min((uint32_t)kCanonCells, n_cells_total - c0);
-    __syncthreads();
-    if (threadIdx.x < nc) offs[threadIdx.x] = offsets[c0 + threadIdx.x];
-    if (threadIdx.x == 0) {
-      offs[nc] = offsets[c0 + nc];
-      n_large = 0;
-    }
-    __syncthreads();
-    if (threadIdx.x < nc && offs[threadIdx.x + 1] - offs[threadIdx.x] > kCanonSort)
-      large[atomicAdd(&n_large, 1u)] = threadIdx.x;
-    for (uint32_t c = warp; c < nc; c += kCanonT / 32) {
-      const uint32_t s = offs[c], e = offs[c + 1], cnt = e - s;
-      uint32_t* wk = keys + warp * kCanonSort;
-      if (cnt == 0 || cnt > kCanonSort) continue;
+  const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+  uint32_t* wk = keys + warp * kCanonSort;
+  const uint32_t warps = gridDim.x * (kCanonT / 32);
+  // `span` (up to 32) neighbouring cells a warp at a time, their offsets read
+  // together.
+  for (uint64_t at = (uint64_t)(blockIdx.x * (kCanonT / 32) + warp) * span; at < n_cells_total;
+       at += (uint64_t)warps * span) {
+    const uint32_t c0 = (uint32_t)at, nc = min(span, n_cells_total - c0);
+    const uint32_t first = lane < nc ? offsets[c0 + lane] : 0u;
+    const uint32_t last = offsets[c0 + nc];
+    for (uint32_t k = 0; k < nc; k++) {
+      const uint32_t s = __shfl_sync(0xffffffffu, first, k);
+      const uint32_t t = __shfl_sync(0xffffffffu, first, (k + 1) & 31u);
+      const uint32_t e = k + 1 < nc ? t : last, cnt = e - s;
+      if (cnt == 0) continue;
       if (cnt <= 32)
         canon_cell<1>(tmp, s, e, wk, ox, oy, oz, orig);
       else if (cnt <= 64)
         canon_cell<2>(tmp, s, e, wk, ox, oy, oz, orig);
       else if (cnt <= 128)
         canon_cell<4>(tmp, s, e, wk, ox, oy, oz, orig);
-      else
+      else if (cnt <= kCanonSort)
         canon_cell<8>(tmp, s, e, wk, ox, oy, oz, orig);
+      else if (lane == 0)
+        more[1 + atomicAdd(more, 1u)] = c0 + k;
     }
-    __syncthreads();
-    for (uint32_t l = 0; l < n_large; l++) {
-      const uint32_t s = offs[large[l]], e = offs[large[l] + 1];
-      for (uint32_t p0 = s; p0 < e; p0 += kCanonT) {
-        const uint32_t p = p0 + threadIdx.x;
-        MeshRec<R> v{};
-        if (p < e) v = tmp[p];
-        uint32_t rank = 0;
-        for (uint32_t k0 = s; k0 < e; k0 += kCanonKeys) {
-          const uint32_t nk = min((uint32_t)kCanonKeys, e - k0);
-          __syncthreads();
-          for (uint32_t k = threadIdx.x; k < nk; k += kCanonT) keys[k] = tmp[k0 + k].i;
-          __syncthreads();
+  }
+}
+
+// The listed cells: a warp each up to kCanonLarge entries, then the others, the
+// CTA's warps together counting each entry's smaller keys as they pass through
+// shared memory.
+template <class R>
+__global__ void __launch_bounds__(kCanonT) cell_canon_large_kernel(
+    const MeshRec<R>* __restrict__ tmp, const uint32_t* __restrict__ offsets,
+    const uint32_t* __restrict__ more, R* __restrict__ ox, R* __restrict__ oy, R* __restrict__ oz,
+    uint32_t* __restrict__ orig) {
+  __shared__ uint32_t keys[kCanonT / 32 * kCanonLarge];
+  const uint32_t n = more[0];
+  const unsigned warp = threadIdx.x >> 5;
+  uint32_t* wk = keys + warp * kCanonLarge;
+  for (uint32_t i = blockIdx.x * (kCanonT / 32) + warp; i < n; i += gridDim.x * (kCanonT / 32)) {
+    const uint32_t s = offsets[more[1 + i]], e = offsets[more[1 + i] + 1];
+    if (e - s <= kCanonLarge / 2)
+      canon_cell<16>(tmp, s, e, wk, ox, oy, oz, orig);
+    else if (e - s <= kCanonLarge)
+      canon_cell<32>(tmp, s, e, wk, ox, oy, oz, orig);
+  }
+  for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
+    const uint32_t s = offsets[more[1 + i]], e = offsets[more[1 + i] + 1];
+    if (e - s <= kCanonLarge) continue;
+    for (uint32_t p0 = s; p0 < e; p0 += kCanonT) {
+      const uint32_t p = p0 + threadIdx.x;
+      MeshRec<R> v{};
+      if (p < e) v = tmp[p];
+      uint32_t rank = 0;
+      for (uint32_t k0 = s; k0 < e; k0 += kCanonT / 32 * kCanonLarge) {
+        const uint32_t nk = min((uint32_t)(kCanonT / 32 * kCanonLarge), e - k0);
+        __syncthreads();
+        for (uint32_t k = threadIdx.x; k < nk; k += kCanonT) keys[k] = tmp[k0 + k].i;
+        __syncthreads();
 #pragma unroll 8
-          for (uint32_t k = 0; k < nk; k++) rank += keys[k] < v.i ? 1u : 0u;
-        }
-        if (p < e) canon_write(v, s + rank, ox, oy, oz, orig);
+        for (uint32_t k = 0; k < nk; k++) rank += keys[k] < v.i ? 1u : 0u;
       }
+      if (p < e) canon_write(v, s + rank, ox, oy, oz, orig);
     }
   }
 }
@@ -366,8 +386,16 @@ void mesh_build(const R* x, const R* y, const R* z, uint64_t n_particles, Device
   }
   cell_scatter_kernel<R><<<grd, kMeshT, 0, st>>>(x, y, z, n_particles, g, cursor, ToRecord<R>{tmp});
   SIFG_LAUNCH_CHECK();
-  cell_canon_kernel<R><<<grid_for(cells, kCanonCells, 152u * 8u), kCanonT, 0, st>>>(
-      tmp, m.offsets, (uint32_t)cells, m.x, m.y, m.z, m.orig);
+  // The scatter's cursors are free: the list of the large cells.
+  uint32_t* more = cursor;
+  SIFG_CUDA(cudaMemsetAsync(more, 0, sizeof(uint32_t), st));
+  // As many neighbours a warp as still leave every SM its warps.
+  const uint32_t span = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(cells / (152u * 64u), 1), 32);
+  cell_canon_kernel<R><<<grid_for(cells, kCanonT / 32 * span, 152u * 8u), kCanonT, 0, st>>>(
+      tmp, m.offsets, (uint32_t)cells, m.x, m.y, m.z, m.orig, more, span);
+  SIFG_LAUNCH_CHECK();
+  cell_canon_large_kernel<R><<<(unsigned)std::min<uint64_t>(cells, 152u * 2u), kCanonT, 0, st>>>(
+      tmp, m.offsets, more, m.x, m.y, m.z, m.orig);
   SIFG_LAUNCH_CHECK();
   if (timer) timer->end(st);
   m.n_particles = n_particles;

@@ -1,5 +1,5 @@
 """The chain mesh's canonical order at the edges of its ranking: cells around
-what a warp sorts in one, two, four and eight registers, cells ranked through
+what a warp sorts in one to thirty-two registers, cells ranked through
 shared memory in parts, empty cells, against a stable sort by cell."""
 import numpy as np
 import pytest
@@ -34,8 +34,8 @@ def _check(dev, pos, n_cells):
         assert np.array_equal(got.cpu().numpy(), a[order])
 
 
-# One cell of `crowd` particles among others: around the 256 entries a warp
-# sorts and the 1,024 keys counted at a time, and several times that.
+# One cell of `crowd` particles among others: around the 1,024 entries a warp
+# sorts, and several times that.
 @pytest.mark.parametrize("dtype", [np.float32, np.float64])
 @pytest.mark.parametrize("crowd", [0, 1, 31, 255, 256, 257, 1023, 1024, 1025, 5000])
 @pytest.mark.parametrize("n_cells", [1, 7, 23])
@@ -49,7 +49,7 @@ def test_order_is_the_stable_sort(dev, crowd, n_cells, dtype):
 
 # Nearly empty meshes, and every size about the sorts' register counts.
 @pytest.mark.parametrize("counts", [[1024] * 5, [1024, 0, 1, 1025, 1023, 2], [3] * 300, [0] * 511 + [4],
-                                    [31, 32, 33, 63, 64, 65, 127, 128, 129, 255, 256, 257] * 3])
+                                    [31, 32, 33, 63, 64, 65, 127, 128, 129, 255, 256, 257, 511, 512, 513] * 3])
 def test_runs_of_cells(dev, counts):
     n_cells = 8
     rng = np.random.default_rng(len(counts))
