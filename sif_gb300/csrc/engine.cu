@@ -986,8 +986,11 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
     if (ext0 == n_ext && n_ext > 0 && ext_reach[n_ext - 1] > r_search) ext0 = n_ext - 1;
 
     // 3. Pre-filter at the rung, against the catalogue as the rung begins.
-    VoidViewT<R> vv{cat_x_.as<R>(), cat_y_.as<R>(), cat_z_.as<R>(), cat_r_.as<R>(),
-                vstart, vids_.as<uint32_t>(), (R)kVoidCells / box, max_r, n_voids};
+    auto void_view = [&] {
+      return VoidViewT<R>{cat_x_.as<R>(), cat_y_.as<R>(), cat_z_.as<R>(), cat_r_.as<R>(),
+                          vstart, vids_.as<uint32_t>(), (R)kVoidCells / box, max_r, n_voids};
+    };
+    VoidViewT<R> vv = void_view();
     uint8_t* alive = grow_to<uint8_t>(alive_, m);
     uint32_t* scand = grow_to<uint32_t>(surv_cand_, m);
     uint32_t* sflat = grow_to<uint32_t>(surv_flat_, m);
@@ -1050,11 +1053,54 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
     uint8_t* sa = nullptr;
     uint8_t* sb = nullptr;
     uint32_t* acc = nullptr;
-    if (!displace) {
-      // Radii reach the top level's reach where the rung enters the extended one.
-      const R r_max = ext0 < n_ext ? std::max(r_search, ext_reach[n_ext - 1]) : r_search;
-      const R reach = 2.0f * scale * r_max + 2.0f * cell;
-      int32_t ng = (int32_t)std::floor(box / reach);
+    const bool small = !displace && commit_is_small(m);
+    SmallCommitT<R> sc{};
+    // Radii reach the top level's reach where the rung enters the extended one.
+    const R r_max = ext0 < n_ext ? std::max(r_search, ext_reach[n_ext - 1]) : r_search;
+    const R reach = 2.0f * scale * r_max + 2.0f * cell;
+    int32_t ng = (int32_t)std::floor(box / reach);
+    if (small) {
+      if (ng < 3) ng = 1;
+      if (ng > 16) ng = 16;
+      // Room for every survivor; a catalogue that moved takes its index anew.
+      const void* was = vids_.ptr;
+      ensure_cat(n_voids + m);
+      if (vids_.ptr != was)
+        build_void_index(cat_x_.as<R>(), cat_y_.as<R>(), cat_z_.as<R>(), n_voids, box, vstart,
+                         vids_.as<uint32_t>(), vcell_.as<uint32_t>(), st_);
+      vv = void_view();
+      sc.ng = ng;
+      sc.cells = (uint32_t)(ng * ng * ng);
+      static_assert(16 * 16 * 16 == kSmallHashCells, "the hash's widest");
+      // Zeroed together: the counters and the hash's counts.
+      sc.counters = grow_to<uint32_t>(small_, kCommitCounters + 2 * (kSmallHashCells + 4) + vcells + 16 +
+                                                  kSmallSurvivors);
+      sc.start = sc.counters + kCommitCounters;
+      sc.cursor = sc.start + kSmallHashCells + 4;
+      sc.vcursor = sc.cursor + kSmallHashCells + 4;
+      sc.vshare = sc.vcursor + vcells;
+      sc.acc_rank = sc.vshare + 16;
+      sc.inv_cell = (R)ng / box;
+      sc.cell_of = grow_to<uint32_t>(sgrid_cellof_, m);
+      sc.ids = grow_to<uint32_t>(sgrid_ids_, m);
+      sc.hrank = grow_to<uint32_t>(sgrid_rank_, m);
+      sc.pack = grow_to<SurvPackT<R>>(sgrid_pack_, m);
+      sc.sa = grow_to<uint8_t>(state_a_, m);
+      sc.sb = grow_to<uint8_t>(state_b_, m);
+      sc.acc = grow_to<uint32_t>(acc_, m);
+      sc.cat_x = cat_x_.as<R>();
+      sc.cat_y = cat_y_.as<R>();
+      sc.cat_z = cat_z_.as<R>();
+      sc.cat_r = cat_r_.as<R>();
+      sc.n_voids = n_voids;
+      sc.vstart = vstart;
+      sc.vids = vids_.as<uint32_t>();
+      sc.vcell = vcell_.as<uint32_t>();
+      sc.void_inv = (R)kVoidCells / box;
+      sc.report = h_counters_;
+      SIFG_CUDA(cudaMemsetAsync(sc.counters, 0, (kCommitCounters + sc.cells + 1) * sizeof(uint32_t), st_));
+      commit_small_init(sv, vv, rc, sc, m, st_);
+    } else if (!displace) {
       if (ng < 3) ng = 1;
       if (ng > 256) ng = 256;
       const uint32_t sg_cells = (uint32_t)(ng * ng * ng);
@@ -1082,7 +1128,7 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
     rs.sort_ms = ms_since(t_sort);
     uint32_t* rank = grow_to<uint32_t>(rank_, m);
     SIFG_CUDA(cudaMemcpyAsync(rank, h_rank_, m * sizeof(uint32_t), cudaMemcpyHostToDevice, st_));
-    if (!displace) survivor_grid_ranks(sv, rank, sg.ids, (uint32_t*)sg.hrank, m, st_);
+    if (!displace && !small) survivor_grid_ranks(sv, rank, sg.ids, (uint32_t*)sg.hrank, m, st_);
 
     // 6. The commit, in rounds; under displacement one survivor at a time.
     const auto t_commit = clk::now();
@@ -1126,6 +1172,35 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
       rs.n_survivors = m;
       rs.n_accepted = n_acc;
       rs.n_displaced = n_removed;
+      rs.rung_ms = ms_since(t_rung);
+      if (stats) stats->push_back(rs);
+      if (const int hs = rung_done(ri + 1, rs.n_mismatched); hs != kOk) return hs;
+      continue;
+    }
+    if (small) {
+      if (tm) tm->commit.begin(st_);
+      commit_small(sv, rank, rc, mask, sc, st_);
+      if (tm) tm->commit.end(st_);
+      if (tm) tm->rung.end(st_);
+      SIFG_CUDA(cudaStreamSynchronize(st_));
+      if (h_counters_[kCommitReport + 2]) {
+        set_error(kErrInvalid, "commit: no progress");
+        return kErrInvalid;
+      }
+      rs.commit_ms = ms_since(t_commit);
+      rs.n_survivors = h_counters_[kCommitReport];
+      rs.n_accepted = h_counters_[0];
+      rs.rounds = h_counters_[kCommitReport + 1];
+      rs.n_rescale_fail = h_counters_[4];
+      rs.n_overflow = h_counters_[5];
+      rs.n_witness = h_counters_[8];
+      rs.n_mismatched = h_counters_[9];
+      if (h_counters_[0]) {
+        R rmax;
+        std::memcpy(&rmax, sizeof(R) == 4 ? (void*)&h_counters_[3] : (void*)&h_counters_[6], sizeof(R));
+        if (rmax > max_r) max_r = rmax;
+        n_voids += h_counters_[0];
+      }
       rs.rung_ms = ms_since(t_rung);
       if (stats) stats->push_back(rs);
       if (const int hs = rung_done(ri + 1, rs.n_mismatched); hs != kOk) return hs;

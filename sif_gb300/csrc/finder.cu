@@ -2867,15 +2867,26 @@ __global__ void commit_round_kernel(SurvivorsT<R> sv, const uint32_t* __restrict
 // is one whose sphere at its rescaled radius overlaps a void of the
 // catalogue as the rung began (the re-check's exact overlap, whose answer no
 // round can change; a warp per survivor); the rest start undecided.
+// With `counts` set (zeroed before), also the survivors' hash cells and their
+// counts, for commit_small's hash of ng cells a side.
 template <class R>
 __global__ void commit_init_kernel(SurvivorsT<R> sv, VoidViewT<R> voids, RungConstsT<R> rc,
-                                   uint8_t* __restrict__ state, uint32_t* __restrict__ counters) {
+                                   uint8_t* __restrict__ state, uint32_t* __restrict__ counters,
+                                   int32_t ng, R inv, uint32_t* __restrict__ counts,
+                                   uint32_t* __restrict__ cell_of) {
   const uint32_t n = *sv.count;
   const unsigned lane = threadIdx.x & 31u;
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
   for (uint32_t i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += warps) {
     const R r = sv.r[i];
     const bool ok = r >= 0.0f;
+    if (counts && lane == 0) {
+      const uint32_t c =
+          (uint32_t)((hash_axis(sv.cx[i], inv, ng) * ng + hash_axis(sv.cy[i], inv, ng)) * ng +
+                     hash_axis(sv.cz[i], inv, ng));
+      cell_of[i] = c;
+      atomicAdd(counts + c, 1u);
+    }
     const bool overlaps =
         ok && overlap_exact_warp(voids, sv.cx[i], sv.cy[i], sv.cz[i], r, rc.f, rc.scale, rc.box);
     if (lane == 0) {
@@ -2891,8 +2902,8 @@ template <class R>
 void commit_init(SurvivorsT<R> s, VoidViewT<R> voids, RungConstsT<R> rc, uint8_t* state,
                  uint32_t* counters, uint32_t max_survivors, cudaStream_t st) {
   if (max_survivors == 0) return;
-  commit_init_kernel<<<grid_for((uint64_t)max_survivors * 32, 256), 256, 0, st>>>(s, voids, rc, state,
-                                                                                counters);
+  commit_init_kernel<<<grid_for((uint64_t)max_survivors * 32, 256), 256, 0, st>>>(
+      s, voids, rc, state, counters, 1, R(0), nullptr, nullptr);
   SIFG_LAUNCH_CHECK();
 }
 
@@ -3190,6 +3201,193 @@ void build_void_index(const R* cx, const R* cy, const R* cz, uint32_t n, R box,
   SIFG_CUDA(cudaMemcpyAsync(cur, start, (cells + 1) * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st));
   scatter_ids_kernel<<<grid_for(n, 256), 256, 0, st>>>(cell_of, nullptr, n, cur, ids);
   SIFG_LAUNCH_CHECK();
+}
+
+// ---------------------------------------------------------------------------
+// A small rung's commit in one launch
+// ---------------------------------------------------------------------------
+// Most rungs have a few hundred survivors, and their commit was a chain of
+// twenty launches and copies -- the hash, the ranks, the rounds, the append,
+// the void index, each a few microseconds of work -- with a read by the host
+// in the middle, and rounds whose two grid barriers each gathered every block
+// through one word of memory. Here one thread-block cluster does all of it
+// between cluster barriers (a hardware barrier, under a microsecond): the hash
+// scanned and filled from the counts commit_init left, the rounds, the
+// accepted voids appended in rank order, and the void index rebuilt, the
+// outcome written straight to pinned host memory. Eight blocks (the portable
+// cluster) hold 2,048 threads, so this is for up to kSmallSurvivors; past that
+// the rounds want the whole GPU. (201^3 particles on 243^3, rungs of 5 to 2,351
+// candidates: see the rule at commit_small.)
+constexpr int kSmallT = 256;
+constexpr int kSmallCtas = 8;
+constexpr uint32_t kVoidIndexCells = kVoidCells * kVoidCells * kVoidCells;
+
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;\n" ::: "memory");
+}
+
+// Exclusive scan of PER consecutive values a thread over the block's
+// kSmallT * PER; *total the sum.
+template <int PER>
+__device__ __forceinline__ void small_scan(uint32_t (&v)[PER], uint32_t* ws, uint32_t* total) {
+  const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  uint32_t sum = 0;
+#pragma unroll
+  for (int k = 0; k < PER; k++) sum += v[k];
+  uint32_t x = sum;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
+    if (lane >= (unsigned)d) x += y;
+  }
+  if (lane == 31) ws[warp] = x;
+  __syncthreads();
+  uint32_t run = x - sum, t = 0;
+#pragma unroll
+  for (int w = 0; w < kSmallT / 32; w++) {
+    const uint32_t q = ws[w];
+    run += (w < (int)warp) ? q : 0u;
+    t += q;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < PER; k++) {
+    const uint32_t c = v[k];
+    v[k] = run;
+    run += c;
+  }
+  *total = t;
+}
+
+template <class R>
+__global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallT)
+    commit_small_kernel(SurvivorsT<R> sv, const uint32_t* __restrict__ rank, RungConstsT<R> rc,
+                        uint32_t* mask, SmallCommitT<R> w) {
+  __shared__ uint32_t ws[kSmallT / 32];
+  __shared__ __align__(16) uint32_t ranks[kSmallSurvivors];
+  const uint32_t n = *sv.count;
+  const uint32_t tid = blockIdx.x * kSmallT + threadIdx.x, threads = kSmallCtas * kSmallT;
+  // The hash's counts to its starts and cursors, by the first block; the
+  // others clear the void index's counts.
+  uint32_t total;
+  if (blockIdx.x == 0) {
+    uint32_t v[kSmallHashCells / kSmallT];
+    const uint32_t c0 = threadIdx.x * (kSmallHashCells / kSmallT);
+#pragma unroll
+    for (int k = 0; k < (int)(kSmallHashCells / kSmallT); k++)
+      v[k] = c0 + k < w.cells ? w.start[c0 + k] : 0u;
+    small_scan(v, ws, &total);
+#pragma unroll
+    for (int k = 0; k < (int)(kSmallHashCells / kSmallT); k++)
+      if (c0 + k < w.cells) {
+        w.start[c0 + k] = v[k];
+        w.cursor[c0 + k] = v[k];
+      }
+    if (threadIdx.x == 0) w.start[w.cells] = total;
+  } else {
+    for (uint32_t c = tid - kSmallT; c < kVoidIndexCells; c += threads - kSmallT) w.vcursor[c] = 0;
+  }
+  cluster_barrier();
+  for (uint32_t i = tid; i < n; i += threads) {
+    const uint32_t k = atomicAdd(w.cursor + w.cell_of[i], 1u);
+    w.ids[k] = i;
+    w.pack[k] = SurvPackT<R>{sv.cx[i], sv.cy[i], sv.cz[i], sv.r[i]};
+    w.hrank[k] = rank[sv.cand[i]];
+  }
+  cluster_barrier();
+  // The rounds. Each decides at least the undecided survivor of lowest rank,
+  // so n rounds are enough; one more is reported as an error.
+  const SurvivorGridT<R> g{w.start, w.ids, w.ng, w.inv_cell, w.pack, w.hrank};
+  uint32_t round = 0, undecided = 0;
+  for (;; round++) {
+    const uint32_t slot = round % kRoundRing;
+    commit_pass(sv, rank, g, VoidViewT<R>{}, mask, rc, (round & 1) ? w.sb : w.sa,
+                (round & 1) ? w.sa : w.sb, w.acc, w.counters, slot);
+    cluster_barrier();
+    undecided = __ldcg(w.counters + kRoundUndecided + slot);
+    if (tid == 0) w.counters[kRoundUndecided + (slot + 1) % kRoundRing] = 0;
+    paint_pass(sv, w.acc, w.counters, slot, mask, rc);
+    cluster_barrier();
+    if (undecided == 0 || round > n) break;
+  }
+  // The accepted voids in rank order: each one's place is the number accepted
+  // at a lower rank.
+  const uint32_t n_acc = __ldcg(w.counters);
+  if (n_acc) {
+    for (uint32_t a = tid; a < n_acc; a += threads) w.acc_rank[a] = rank[sv.cand[__ldcg(w.acc + a)]];
+    cluster_barrier();
+    const uint32_t padded = (n_acc + 3) & ~3u;
+    for (uint32_t a = threadIdx.x; a < padded; a += kSmallT)
+      ranks[a] = a < n_acc ? __ldcg(w.acc_rank + a) : 0xffffffffu;
+    __syncthreads();
+    for (uint32_t a = tid; a < n_acc; a += threads) {
+      const uint32_t mine = ranks[a];
+      uint32_t at = w.n_voids;
+      for (uint32_t q = 0; q < padded / 4; q++) {
+        const uint4 k = reinterpret_cast<const uint4*>(ranks)[q];
+        at += (k.x < mine ? 1u : 0u) + (k.y < mine ? 1u : 0u) + (k.z < mine ? 1u : 0u) +
+              (k.w < mine ? 1u : 0u);
+      }
+      const uint32_t i = __ldcg(w.acc + a);
+      const R cx = sv.cx[i], cy = sv.cy[i], cz = sv.cz[i];
+      w.cat_x[at] = cx;
+      w.cat_y[at] = cy;
+      w.cat_z[at] = cz;
+      w.cat_r[at] = sv.r[i];
+      const uint32_t c = (void_axis(cx, w.void_inv) * kVoidCells + void_axis(cy, w.void_inv)) * kVoidCells +
+                         void_axis(cz, w.void_inv);
+      w.vcell[at] = c;
+      atomicAdd(w.vcursor + c, 1u);
+    }
+    // The void index over all of them (the older voids' cells as they were).
+    const uint32_t n_all = w.n_voids + n_acc;
+    for (uint32_t v = tid; v < w.n_voids; v += threads) atomicAdd(w.vcursor + w.vcell[v], 1u);
+    cluster_barrier();
+    constexpr uint32_t kShare = kVoidIndexCells / kSmallCtas, kPer = kShare / kSmallT;
+    uint32_t v[kPer];
+    const uint32_t c0 = blockIdx.x * kShare + threadIdx.x * kPer;
+#pragma unroll
+    for (uint32_t k = 0; k < kPer; k++) v[k] = __ldcg(w.vcursor + c0 + k);
+    small_scan(v, ws, &total);
+    if (threadIdx.x == 0) w.vshare[blockIdx.x] = total;
+    cluster_barrier();
+    uint32_t base = 0;
+    for (uint32_t b = 0; b < blockIdx.x; b++) base += __ldcg(w.vshare + b);
+#pragma unroll
+    for (uint32_t k = 0; k < kPer; k++) {
+      w.vstart[c0 + k] = base + v[k];
+      w.vcursor[c0 + k] = base + v[k];
+    }
+    if (tid == 0) w.vstart[kVoidIndexCells] = n_all;
+    cluster_barrier();
+    for (uint32_t v2 = tid; v2 < n_all; v2 += threads)
+      w.vids[atomicAdd(w.vcursor + __ldcg(w.vcell + v2), 1u)] = v2;
+  }
+  if (tid < kCommitReport) w.report[tid] = __ldcg(w.counters + tid);
+  if (tid == 0) {
+    w.report[kCommitReport] = n;
+    w.report[kCommitReport + 1] = round + 1;
+    w.report[kCommitReport + 2] = undecided;
+  }
+}
+
+template <class R>
+void commit_small_init(SurvivorsT<R> s, VoidViewT<R> voids, RungConstsT<R> rc, const SmallCommitT<R>& w,
+                       uint32_t max_survivors, cudaStream_t st) {
+  commit_init_kernel<<<grid_for((uint64_t)max_survivors * 32, 256), 256, 0, st>>>(
+      s, voids, rc, w.sa, w.counters, w.ng, w.inv_cell, w.start, w.cell_of);
+  SIFG_LAUNCH_CHECK();
+}
+
+template <class R>
+void commit_small(SurvivorsT<R> s, const uint32_t* rank, RungConstsT<R> rc, uint32_t* mask,
+                  const SmallCommitT<R>& w, cudaStream_t st) {
+  commit_small_kernel<R><<<kSmallCtas, kSmallT, 0, st>>>(s, rank, rc, mask, w);
+  SIFG_LAUNCH_CHECK();
+}
+
+bool commit_is_small(uint32_t max_survivors) {
+  return g_commit_mode == 0 && max_survivors <= kSmallSurvivors;
 }
 
 // ---------------------------------------------------------------------------
@@ -3609,6 +3807,10 @@ void compact_voids(R* cx, R* cy, R* cz, R* r, uint32_t* state, cudaStream_t st) 
                              RungConstsT<R>, uint32_t, cudaStream_t);                              \
   template void paint_voids<R>(const R*, const R*, const R*, const R*, uint32_t, uint32_t*,        \
                                RungConstsT<R>, cudaStream_t);                                      \
+  template void commit_small_init<R>(SurvivorsT<R>, VoidViewT<R>, RungConstsT<R>,                  \
+                                     const SmallCommitT<R>&, uint32_t, cudaStream_t);              \
+  template void commit_small<R>(SurvivorsT<R>, const uint32_t*, RungConstsT<R>, uint32_t*,         \
+                                const SmallCommitT<R>&, cudaStream_t);                             \
   template bool commit_rounds<R>(SurvivorsT<R>, const uint32_t*, SurvivorGridT<R>, VoidViewT<R>,   \
                                  uint32_t*, RungConstsT<R>, uint8_t*, uint8_t*, uint32_t*,         \
                                  uint32_t*, uint32_t, uint32_t, unsigned*, uint32_t, cudaStream_t);\

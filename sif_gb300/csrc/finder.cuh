@@ -368,6 +368,43 @@ bool commit_rounds(SurvivorsT<R> s, const uint32_t* rank, SurvivorGridT<R> g, Vo
 // allows it; 1: a launch per round. The catalogue does not depend on it.
 void set_commit_mode(int mode);
 
+// A small rung's whole commit -- the survivor hash, the rounds, the append and
+// the void index -- in one launch of a thread-block cluster. Whether a rung is
+// small: by its survivors' bound, with the rounds in one launch
+// (set_commit_mode(0)).
+constexpr uint32_t kSmallSurvivors = 4096;
+constexpr uint32_t kSmallHashCells = 4096;  // the hash's cells, at most (16 a side)
+constexpr uint32_t kCommitReport = 10;      // the counters reported
+template <class R>
+struct SmallCommitT {
+  // counters and start (zeroed by the caller before commit_small_init): the
+  // commit's counters; the hash's cells + 1 counts, then starts.
+  uint32_t *counters, *start, *cursor, *cell_of, *ids, *hrank;
+  SurvPackT<R>* pack;
+  uint32_t cells;
+  int32_t ng;
+  R inv_cell;
+  uint8_t *sa, *sb;         // survivor states (sa from commit_small_init)
+  uint32_t *acc, *acc_rank;  // the accepted survivors, their ranks
+  // The catalogue and its index (room for every survivor), n_voids so far.
+  R *cat_x, *cat_y, *cat_z, *cat_r;
+  uint32_t n_voids;
+  uint32_t *vstart, *vids, *vcell, *vcursor, *vshare;
+  R void_inv;
+  // Pinned host memory: counters [0, kCommitReport), then the survivors, the
+  // rounds, and how many the last round left undecided.
+  uint32_t* report;
+};
+bool commit_is_small(uint32_t max_survivors);
+// commit_init and the hash's counts.
+template <class R>
+void commit_small_init(SurvivorsT<R> s, VoidViewT<R> voids, RungConstsT<R> rc, const SmallCommitT<R>& w,
+                       uint32_t max_survivors, cudaStream_t st);
+// Everything else, once rank is on the device.
+template <class R>
+void commit_small(SurvivorsT<R> s, const uint32_t* rank, RungConstsT<R> rc, uint32_t* mask,
+                  const SmallCommitT<R>& w, cudaStream_t st);
+
 // Paints n_voids given voids (a prior catalogue) into the mask at scale * r
 // (rc: scale, cell, gbox, grid_n), as the commit paints the ones it accepts.
 template <class R>
