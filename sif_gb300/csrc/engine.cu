@@ -680,8 +680,11 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
   }
   R* gbuf = grow_to<R>(gbuf_, (size_t)growth_grid() * kGrowCap);
   uint32_t* dcount = grow_to<uint32_t>(dcount_, 16);
-  // The growth and witness kernels' work counters (the survivors' queue).
-  uint32_t* work = grow_to<uint32_t>(work_, 4);
+  // The survivors' count and the growth and witness kernels' work counters
+  // (the survivors' queue), zeroed together.
+  uint32_t* n_surv = dcount;
+  uint32_t* work = dcount + 1;
+  constexpr uint32_t kWork = 3;
   // Gathered particles and visited cells of each rung's sphere growth.
   const size_t n_rungs = radii.size();
   unsigned long long* traffic = (unsigned long long*)grow_to<uint64_t>(traffic_, 2 * n_rungs + 2);
@@ -865,20 +868,20 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
     const BelowList& bl = below[ri % 2];
     rs.from_list = listed ? 1u : 0u;
     if (listed) {
-      below_count_pass(bl.counts, bl.flat, nb_below, kBelowBlock, mask, blocks, dcount, st_);
+      below_count_pass(bl.counts, bl.flat, nb_below, kBelowBlock, mask, blocks, h_counters_, st_);
     } else {
       const uint64_t slots = scan_region_slots(cells);
       region_delta = grow_to<R>(region_delta_, slots);
       region_flat = grow_to<uint32_t>(region_flat_, slots);
       // Refined, the candidates are every cell at or below the threshold
       // (the minima are found on the refinement's field, below).
-      scan_fused_pass(field, mask, cells, threshold, blocks, dcount, region_delta, region_flat, st_,
-                      N, minima && !gaussian);
+      scan_fused_pass(field, mask, cells, threshold, blocks, h_counters_, region_delta, region_flat,
+                      st_, N, minima && !gaussian);
       // The field's last reader: the next rung but one may smooth into it
       // (refined, the placing reads it again: recorded after that).
       if (!gaussian) SIFG_CUDA(cudaEventRecord(ev_scanned_[ri % 2], st_));
     }
-    SIFG_CUDA(cudaMemcpyAsync(h_counters_, dcount, sizeof(uint32_t), cudaMemcpyDeviceToHost, st_));
+    // The total goes straight to pinned host memory.
     const auto t_wait = clk::now();
     SIFG_CUDA(cudaStreamSynchronize(st_));
     rs.count_wait_ms = ms_since(t_wait);
@@ -926,10 +929,13 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
       continue;
     }
 
+    ensure_host(m);
     if (gaussian) {
       // placed above
+      SIFG_CUDA(cudaMemcpyAsync(h_delta_, cdelta, m * sizeof(R), cudaMemcpyDeviceToHost, st_));
     } else if (listed) {
-      cdelta = grow_to<R>(cand_delta_, m);
+      // The depths go straight to the host, where alone they are read.
+      cdelta = (R*)h_delta_;
       cflat = grow_to<uint32_t>(cand_flat_, m);
       if constexpr (sizeof(R) == 4)
         below_write_pass(bl.counts, bl.delta, bl.flat, nb_below, kBelowBlock, mask, blocks, cdelta,
@@ -937,12 +943,10 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
       // The list's last reader: the next rung but one may smooth into it.
       SIFG_CUDA(cudaEventRecord(ev_scanned_[ri % 2], st_));
     } else {
-      cdelta = grow_to<R>(cand_delta_, m);
+      cdelta = (R*)h_delta_;
       cflat = grow_to<uint32_t>(cand_flat_, m);
       scan_compact(blocks, cells, region_delta, region_flat, cdelta, cflat, st_);
     }
-    ensure_host(m);
-    SIFG_CUDA(cudaMemcpyAsync(h_delta_, cdelta, m * sizeof(R), cudaMemcpyDeviceToHost, st_));
     SIFG_CUDA(cudaEventRecord(ev_cand_, st_));
 
     RungConstsT<R> rc0{};
@@ -957,6 +961,27 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
     const RungConstsT<R> rc = shell_consts(rc0, rmin, r_search);
     const R span = rc.rs2 - rc.rc2;
 
+    // 3. Pre-filter at the rung, against the catalogue as the rung begins.
+    auto void_view = [&] {
+      return VoidViewT<R>{cat_x_.as<R>(), cat_y_.as<R>(), cat_z_.as<R>(), cat_r_.as<R>(),
+                          vstart, vids_.as<uint32_t>(), (R)kVoidCells / box, max_r, n_voids};
+    };
+    VoidViewT<R> vv = void_view();
+    uint32_t* scand = grow_to<uint32_t>(surv_cand_, m);
+    uint32_t* sflat = grow_to<uint32_t>(surv_flat_, m);
+    R* scx = grow_to<R>(scx_, m);
+    R* scy = grow_to<R>(scy_, m);
+    R* scz = grow_to<R>(scz_, m);
+    R* sr = grow_to<R>(sr_, m);
+    uint8_t* sreason = grow_to<uint8_t>(sreason_, m);
+    uint32_t* blocks2 = grow_to<uint32_t>(rank_slots_, (size_t)m + 2048);
+    R* soff = coff ? grow_to<R>(soff_, m) : nullptr;
+    SIFG_CUDA(cudaMemsetAsync(n_surv, 0, (1 + kWork) * sizeof(uint32_t), st_));
+    prefilter(cflat, m, mask, vv, rc, scand, sflat, scx, scy, scz, sreason, n_surv, st_, displace,
+              coff, soff);
+    SurvivorsT<R> sv{scand, sflat, scx, scy, scz, sr, sreason, n_surv, soff};
+
+    // The template, built while the GPU takes the pre-filter.
     HostTemplateT<R> ht;
     if (build_template(ht, mesh.n_cells, mesh.cell_length, rmin, r_search) != kOk) {
       set_error(kErrRange, "search sphere of " + std::to_string(r_search) +
@@ -985,26 +1010,6 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
       if (ext_reach[k] >= kExtSlack * r_search) ext0 = k;
     if (ext0 == n_ext && n_ext > 0 && ext_reach[n_ext - 1] > r_search) ext0 = n_ext - 1;
 
-    // 3. Pre-filter at the rung, against the catalogue as the rung begins.
-    auto void_view = [&] {
-      return VoidViewT<R>{cat_x_.as<R>(), cat_y_.as<R>(), cat_z_.as<R>(), cat_r_.as<R>(),
-                          vstart, vids_.as<uint32_t>(), (R)kVoidCells / box, max_r, n_voids};
-    };
-    VoidViewT<R> vv = void_view();
-    uint8_t* alive = grow_to<uint8_t>(alive_, m);
-    uint32_t* scand = grow_to<uint32_t>(surv_cand_, m);
-    uint32_t* sflat = grow_to<uint32_t>(surv_flat_, m);
-    R* scx = grow_to<R>(scx_, m);
-    R* scy = grow_to<R>(scy_, m);
-    R* scz = grow_to<R>(scz_, m);
-    R* sr = grow_to<R>(sr_, m);
-    uint8_t* sreason = grow_to<uint8_t>(sreason_, m);
-    uint32_t* blocks2 = grow_to<uint32_t>(rank_slots_, (size_t)m + 2048);
-    R* soff = coff ? grow_to<R>(soff_, m) : nullptr;
-    prefilter(cflat, m, mask, vv, rc, alive, blocks2, scand, sflat, scx, scy, scz, dcount + 1, st_,
-              displace, coff, soff);
-    SurvivorsT<R> sv{scand, sflat, scx, scy, scz, sr, sreason, dcount + 1, soff};
-
     // 4. Sphere growth of every survivor.
     if (!(span > 0.0f)) {
       // RESCALE_DEGENERATE for every candidate: no annulus.
@@ -1021,10 +1026,11 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
       // displacement every survivor is grown: a void refusing it now may be
       // displaced before its turn.
       // No witness on a weighted mesh either (1865-1868).
-      if (displace || weighted || survey)
-        SIFG_CUDA(cudaMemsetAsync(sreason, kRescaleOk, m, st_));
-      else
+      auto fresh_work = [&] { SIFG_CUDA(cudaMemsetAsync(work, 0, kWork * sizeof(uint32_t), st_)); };
+      if (witness_on() && !(displace || weighted || survey)) {
         witness(mv, tv, rc, sv, vv, m, traffic + 2 * ri, st_, tm ? &tm->witness : nullptr, work);
+        fresh_work();
+      }
       if (survey)
         grow_survey(mv, tv, rmv, rtv, rc, survey_K, sv, m, gbuf, gwbuf, kGrowCap, traffic + 2 * ri,
                     st_, tm ? &tm->growth : nullptr, work);
@@ -1038,6 +1044,7 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
       // still lies past the reach (exodus_finder.c:2060-2072).
       for (uint32_t e = ext0; e < n_ext; e++) {
         const RungConstsT<R> ec = shell_consts(rc, ext_rmin[e], ext_reach[e]);
+        fresh_work();
         if (weighted)
           grow_weighted(mv, ext_tv[e], ec, sv, m, gbuf, gwbuf, kGrowCap, traffic + 2 * ri, st_,
                         tm ? &tm->growth : nullptr, kRescaleBeyondSearch, work);
@@ -1108,7 +1115,7 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
       uint32_t* sg_ids = grow_to<uint32_t>(sgrid_ids_, m);
       uint32_t* sg_cell = grow_to<uint32_t>(sgrid_cellof_, m);
       SurvPackT<R>* sg_pack = grow_to<SurvPackT<R>>(sgrid_pack_, m);
-      build_survivor_grid(scx, scy, scz, (const R*)sr, dcount + 1, m, ng, box, sg_start, sg_ids,
+      build_survivor_grid(scx, scy, scz, (const R*)sr, n_surv, m, ng, box, sg_start, sg_ids,
                           sg_cell, sg_pack, st_);
       sg = SurvivorGridT<R>{sg_start, sg_ids, ng, (R)ng / box, sg_pack,
                             grow_to<uint32_t>(sgrid_rank_, m)};
@@ -1233,7 +1240,7 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
       if (tm) tm->commit.end(st_);
       SIFG_CUDA(cudaMemcpyAsync(h_counters_, counters, kCommitCounters * sizeof(uint32_t),
                                 cudaMemcpyDeviceToHost, st_));
-      SIFG_CUDA(cudaMemcpyAsync(h_count, dcount + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, st_));
+      SIFG_CUDA(cudaMemcpyAsync(h_count, n_surv, sizeof(uint32_t), cudaMemcpyDeviceToHost, st_));
       SIFG_CUDA(cudaStreamSynchronize(st_));
       if (one_launch) {
         if (h_bar[2] || h_bar[3] == 0) {

@@ -187,7 +187,7 @@ class Engine {
  private:
   int device_;
   cudaStream_t st_ = 0;
-  DevBuf field_[2], mask_, cand_delta_, cand_flat_, blocks_, rank_, rank_slots_, alive_;
+  DevBuf field_[2], mask_, cand_delta_, cand_flat_, blocks_, rank_, rank_slots_;
   DevBuf surv_cand_, surv_flat_, scx_, scy_, scz_, sr_, sreason_, state_a_, state_b_, acc_;
   DevBuf commit_bar_;  // the cooperative commit's grid barrier and its report
   DevBuf counters_, dcount_, sgrid_start_, sgrid_ids_, sgrid_cellof_, sgrid_pack_, sgrid_rank_;
@@ -195,7 +195,6 @@ class Engine {
   DevBuf pend_;  // the sphere growth's warp-kernel leftovers
   DevBuf cat_x_, cat_y_, cat_z_, cat_r_, vstart_, vids_, vcell_;
   DevBuf vhead_, vnext_, dlist_;  // displacement: the linked void index, its lists
-  DevBuf work_;  // the sphere growth's and the witness's survivor queues
   DevBuf gwbuf_, wcheck_;  // a weighted mesh: the wide windows' weights, the weight check
   // SIF_FINDER_REFINE_GAUSSIAN: the refinement's fields, the placed
   // candidates and their offsets, the minima's keep flags, the survivors'

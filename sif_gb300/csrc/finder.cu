@@ -398,6 +398,38 @@ __device__ __forceinline__ bool is_interior(R cx, R cy, R cz, R s, R box) {
          fsub(cz, s) >= 0.0f && fadd(cz, s) < box;
 }
 
+// cll_axis_index, src/structures/cell_linked_list.c:40-58 (periodic).
+template <class R>
+__device__ __forceinline__ uint32_t void_axis(R c, R inv) {
+  int32_t i = (int32_t)ffloor(fmul(c, inv));
+  i %= (int32_t)kVoidCells;
+  if (i < 0) i += kVoidCells;
+  return (uint32_t)i;
+}
+
+// Whether void j's index cell lies in the window of cells [x0, x1] x [y0, y1] x
+// [z0, z1] (taken modulo the index, as the walk above takes them).
+template <class R>
+__device__ __forceinline__ bool in_window(const VoidViewT<R>& v, R vx, R vy, R vz, int32_t x0,
+                                          int32_t x1, int32_t y0, int32_t y1, int32_t z0, int32_t z1) {
+  const uint32_t m = kVoidCells - 1;
+  return ((void_axis(vx, v.inv_cell) - (uint32_t)x0) & m) <= (uint32_t)(x1 - x0) &&
+         ((void_axis(vy, v.inv_cell) - (uint32_t)y0) & m) <= (uint32_t)(y1 - y0) &&
+         ((void_axis(vz, v.inv_cell) - (uint32_t)z0) & m) <= (uint32_t)(z1 - z0);
+}
+
+// Whether the overlap tests take the catalogue's voids one after another
+// instead of the window's cells: a rung's early voids are few and the window of
+// a large sphere many cells, each a dependent load of its range (64^3 and
+// survey boxes, whose spheres reach a quarter of the box: 650 to 1,000 cells
+// for a few dozen voids, and the pre-filter 70 to 200 us a rung). A void's
+// loads go to every lane at once and do not wait on one another. A void
+// outside the window is not tested against, as the walk over cells would not.
+__device__ __forceinline__ bool walk_voids(uint32_t n, int32_t x0, int32_t x1, int32_t y0, int32_t y1,
+                                           int32_t z0, int32_t z1) {
+  return n <= (uint32_t)(x1 - x0 + 1) * (uint32_t)(y1 - y0 + 1) * (uint32_t)(z1 - z0 + 1);
+}
+
 // sif__overlap_exact (src/finder/utils.c:850-960) over the void index.
 template <class R>
 __device__ bool overlap_exact(const VoidViewT<R>& v, R cx, R cy, R cz, R r, R f,
@@ -412,6 +444,15 @@ __device__ bool overlap_exact(const VoidViewT<R>& v, R cx, R cy, R cz, R r, R f,
   const int32_t z0 = (int32_t)ffloor(fmul(fsub(cz, s), v.inv_cell));
   const int32_t z1 = (int32_t)ffloor(fmul(fadd(cz, s), v.inv_cell));
   const bool interior = is_interior(cx, cy, cz, s, box);
+  if (walk_voids(v.n, x0, x1, y0, y1, z0, z1)) {
+    for (uint32_t j = 0; j < v.n; j++) {
+      const R vx = v.cx[j], vy = v.cy[j], vz = v.cz[j];
+      if (collide(cx, cy, cz, r, vx, vy, vz, v.r[j], f, scale, box, half, interior) &&
+          in_window(v, vx, vy, vz, x0, x1, y0, y1, z0, z1))
+        return true;
+    }
+    return false;
+  }
   for (int32_t ix = x0; ix <= x1; ix++) {
     const uint32_t wx = (uint32_t)ix & (kVoidCells - 1);
     for (int32_t iy = y0; iy <= y1; iy++) {
@@ -448,6 +489,19 @@ __device__ bool overlap_exact_warp(const VoidViewT<R>& v, R cx, R cy, R cz, R r,
   const int32_t z0 = (int32_t)ffloor(fmul(fsub(cz, s), v.inv_cell));
   const int32_t z1 = (int32_t)ffloor(fmul(fadd(cz, s), v.inv_cell));
   const bool interior = is_interior(cx, cy, cz, s, box);
+  if (walk_voids(v.n, x0, x1, y0, y1, z0, z1)) {
+    for (uint32_t j0 = 0; j0 < v.n; j0 += 32) {
+      const uint32_t j = j0 + lane;
+      bool hit = false;
+      if (j < v.n) {
+        const R vx = v.cx[j], vy = v.cy[j], vz = v.cz[j];
+        hit = collide(cx, cy, cz, r, vx, vy, vz, v.r[j], f, scale, box, half, interior) &&
+              in_window(v, vx, vy, vz, x0, x1, y0, y1, z0, z1);
+      }
+      if (__any_sync(0xffffffffu, hit)) return true;
+    }
+    return false;
+  }
   const uint32_t ny = (uint32_t)(y1 - y0 + 1), nz = (uint32_t)(z1 - z0 + 1);
   const uint32_t cells = (uint32_t)(x1 - x0 + 1) * ny * nz;
   for (uint32_t k0 = 0; k0 < cells; k0 += 32) {
@@ -640,118 +694,67 @@ __device__ __forceinline__ bool cand_masked(const uint32_t* mask, uint32_t node,
 // Pre-filter
 // ---------------------------------------------------------------------------
 
+// The survivors are appended as they are found, a warp's together (one atomic a
+// warp): nothing depends on the order they are listed in -- the commit goes by
+// their ranks -- but neighbours in the list staying near one another keeps the
+// growth's reads together. *n_surv is zeroed before.
 template <class R>
 __global__ void prefilter_kernel(const uint32_t* __restrict__ cflat, uint32_t m,
                                  const uint32_t* __restrict__ mask, VoidViewT<R> voids, RungConstsT<R> rc,
-                                 uint8_t* __restrict__ alive, bool keep_all,
-                                 const CandOffT<R>* __restrict__ coff) {
+                                 bool keep_all, const CandOffT<R>* __restrict__ coff,
+                                 uint32_t* __restrict__ surv_cand, uint32_t* __restrict__ sflat,
+                                 R* __restrict__ scx, R* __restrict__ scy, R* __restrict__ scz,
+                                 uint8_t* __restrict__ sreason, R* __restrict__ soff,
+                                 uint32_t* __restrict__ n_surv) {
   const uint32_t n = rc.grid_n;
-  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < m; k += gridDim.x * blockDim.x) {
-    const uint32_t flat = cflat[k];
-    const CandOffT<R> o = coff ? coff[k] : CandOffT<R>{R(0), R(0), R(0), R(-1.0f)};
-    uint8_t ok = 1;
-    if (keep_all) {
-      // Under displacement a void refusing a candidate now may be gone by
-      // its turn (exodus_finder.c:1873-1875): nothing is refused here.
-    } else if (cand_masked(mask, flat, o.len, rc.radius, rc)) {
-      ok = 0;
-    } else {
+  const unsigned lane = threadIdx.x & 31u;
+  for (uint32_t k0 = blockIdx.x * blockDim.x + threadIdx.x - lane; k0 < m; k0 += gridDim.x * blockDim.x) {
+    const uint32_t k = k0 + lane;
+    bool ok = k < m;
+    uint32_t flat = 0;
+    CandOffT<R> o{R(0), R(0), R(0), R(-1.0f)};
+    R cx = 0, cy = 0, cz = 0;
+    if (ok) {
+      flat = cflat[k];
+      if (coff) o = coff[k];
+      // candidate_centre (exodus_finder.c:366-388): its node, and its offset
+      // off the node where the refinement moved it.
       const uint32_t ix = flat / (n * n), iy = (flat / n) % n, iz = flat % n;
-      if (rc.proxy_pole > 0 && overlap_quick(mask, n, ix, iy, iz, (uint32_t)rc.proxy_pole)) {
-        ok = 0;
-      } else {
-        const R cx = cand_axis(ix, o.dx, rc), cy = cand_axis(iy, o.dy, rc),
-                cz = cand_axis(iz, o.dz, rc);
-        if (overlap_exact(voids, cx, cy, cz, rc.radius, rc.f, rc.scale, rc.box)) ok = 0;
-      }
+      cx = cand_axis(ix, o.dx, rc);
+      cy = cand_axis(iy, o.dy, rc);
+      cz = cand_axis(iz, o.dz, rc);
+      // Under displacement (keep_all) a void refusing a candidate now may be
+      // gone by its turn (exodus_finder.c:1873-1875): nothing is refused here.
+      if (!keep_all)
+        ok = !cand_masked(mask, flat, o.len, rc.radius, rc) &&
+             !(rc.proxy_pole > 0 && overlap_quick(mask, n, ix, iy, iz, (uint32_t)rc.proxy_pole)) &&
+             !overlap_exact(voids, cx, cy, cz, rc.radius, rc.f, rc.scale, rc.box);
     }
-    alive[k] = ok;
-  }
-}
-
-constexpr int kCompactT = 256;
-constexpr int kCompactRounds = 8;
-constexpr uint32_t kCompactChunk = kCompactT * kCompactRounds;
-
-__global__ void __launch_bounds__(kCompactT) flag_count_kernel(const uint8_t* __restrict__ flags,
-                                                               uint32_t m,
-                                                               uint32_t* __restrict__ counts) {
-  __shared__ uint32_t ws[kCompactT / 32];
-  const uint32_t base = blockIdx.x * kCompactChunk;
-  uint32_t c = 0;
-  for (int j = 0; j < kCompactRounds; j++) {
-    const uint32_t i = base + j * kCompactT + threadIdx.x;
-    c += (i < m && flags[i]) ? 1u : 0u;
-  }
-  c = __reduce_add_sync(0xffffffffu, c);
-  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = c;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    uint32_t t = 0;
-    for (int w = 0; w < kCompactT / 32; w++) t += ws[w];
-    counts[blockIdx.x] = t;
-  }
-}
-
-template <class R>
-__global__ void __launch_bounds__(kCompactT) survivor_write_kernel(
-    const uint8_t* __restrict__ flags, uint32_t m, const uint32_t* __restrict__ offsets,
-    const uint32_t* __restrict__ cflat, RungConstsT<R> rc, uint32_t* __restrict__ surv_cand,
-    uint32_t* __restrict__ sflat, R* __restrict__ scx, R* __restrict__ scy,
-    R* __restrict__ scz, const CandOffT<R>* __restrict__ coff, R* __restrict__ soff) {
-  __shared__ uint32_t wsum[kCompactT / 32];
-  const uint32_t base = blockIdx.x * kCompactChunk;
-  const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  uint32_t out = offsets[blockIdx.x];
-  const uint32_t n = rc.grid_n;
-  for (int j = 0; j < kCompactRounds; j++) {
-    const uint32_t i = base + j * kCompactT + threadIdx.x;
-    const bool p = i < m && flags[i];
-    const unsigned bal = __ballot_sync(0xffffffffu, p);
-    if (lane == 0) wsum[warp] = __popc(bal);
-    __syncthreads();
-    uint32_t before = 0, total = 0;
-    for (int w = 0; w < kCompactT / 32; w++) {
-      const uint32_t v = wsum[w];
-      before += (w < (int)warp) ? v : 0u;
-      total += v;
+    const unsigned bal = __ballot_sync(0xffffffffu, ok);
+    uint32_t at = 0;
+    if (lane == 0 && bal) at = atomicAdd(n_surv, (uint32_t)__popc(bal));
+    at = __shfl_sync(0xffffffffu, at, 0) + __popc(bal & ((1u << lane) - 1u));
+    if (ok) {
+      surv_cand[at] = k;
+      sflat[at] = flat;
+      scx[at] = cx;
+      scy[at] = cy;
+      scz[at] = cz;
+      sreason[at] = kRescaleOk;
+      if (soff) soff[at] = o.len;
     }
-    if (p) {
-      const uint32_t pos = out + before + __popc(bal & ((1u << lane) - 1u));
-      const uint32_t flat = cflat[i];
-      surv_cand[pos] = i;
-      sflat[pos] = flat;
-      // candidate_centre (exodus_finder.c:366-388): its node, and its
-      // offset off the node where the refinement moved it.
-      const CandOffT<R> o = coff ? coff[i] : CandOffT<R>{R(0), R(0), R(0), R(-1.0f)};
-      scx[pos] = cand_axis(flat / (n * n), o.dx, rc);
-      scy[pos] = cand_axis((flat / n) % n, o.dy, rc);
-      scz[pos] = cand_axis(flat % n, o.dz, rc);
-      if (soff) soff[pos] = o.len;
-    }
-    out += total;
-    __syncthreads();
   }
 }
 
 template <class R>
 void prefilter(const uint32_t* cand_flat, uint32_t m, const uint32_t* mask, VoidViewT<R> voids,
-               RungConstsT<R> rc, uint8_t* alive, uint32_t* block_counts, uint32_t* surv_cand,
-               uint32_t* surv_flat, R* scx, R* scy, R* scz, uint32_t* d_surv_count,
-               cudaStream_t st, bool keep_all, const CandOffT<R>* coff, R* soff) {
-  if (m == 0) {
-    SIFG_CUDA(cudaMemsetAsync(d_surv_count, 0, sizeof(uint32_t), st));
-    return;
-  }
-  prefilter_kernel<<<grid_for(m, 128), 128, 0, st>>>(cand_flat, m, mask, voids, rc, alive, keep_all,
-                                                      coff);
-  SIFG_LAUNCH_CHECK();
-  const uint32_t nb = (m + kCompactChunk - 1) / kCompactChunk;
-  flag_count_kernel<<<nb, kCompactT, 0, st>>>(alive, m, block_counts);
-  SIFG_LAUNCH_CHECK();
-  exclusive_scan_total(block_counts, nb, d_surv_count, st);
-  survivor_write_kernel<<<nb, kCompactT, 0, st>>>(alive, m, block_counts, cand_flat, rc,
-                                                  surv_cand, surv_flat, scx, scy, scz, coff, soff);
+               RungConstsT<R> rc, uint32_t* surv_cand, uint32_t* surv_flat, R* scx, R* scy, R* scz,
+               uint8_t* sreason, uint32_t* d_surv_count, cudaStream_t st, bool keep_all,
+               const CandOffT<R>* coff, R* soff) {
+  if (m == 0) return;
+  prefilter_kernel<<<grid_for(m, 64), 64, 0, st>>>(cand_flat, m, mask, voids, rc, keep_all, coff,
+                                                   surv_cand, surv_flat, scx, scy, scz, sreason, soff,
+                                                   d_surv_count);
   SIFG_LAUNCH_CHECK();
 }
 
@@ -1701,21 +1704,18 @@ __global__ void __launch_bounds__(kGrowT) witness_kernel(MeshViewT<R> mesh, Temp
 // saves; the catalogue is the same either way.
 static int g_witness = 0;
 void set_witness(int on) { g_witness = on; }
+bool witness_on() { return g_witness != 0; }
 
 template <class R>
 void witness(MeshViewT<R> mesh, TemplateViewT<R> tpl, RungConstsT<R> rc, SurvivorsT<R> s,
              VoidViewT<R> voids, uint32_t max_survivors, unsigned long long* traffic,
              cudaStream_t st, KernelTimer* timer, uint32_t* work) {
-  if (max_survivors == 0) return;
-  if (!g_witness) {
-    // Every survivor to be grown (kRescaleOk is 0).
-    SIFG_CUDA(cudaMemsetAsync(s.reason, 0, max_survivors, st));
-    return;
-  }
+  // Without it, every survivor to be grown: kRescaleOk, as the pre-filter left
+  // them.
+  if (max_survivors == 0 || !g_witness) return;
   // As many CTAs as the GPU keeps resident (four an SM at 64 registers),
   // taking survivors from the counter.
   const uint32_t ctas_needed = (max_survivors + kGrowWarps - 1) / kGrowWarps;
-  SIFG_CUDA(cudaMemsetAsync(work, 0, sizeof(uint32_t), st));
   if (timer) timer->begin(st);
   witness_kernel<R><<<std::min<uint32_t>(ctas_needed, 152u * 4u), kGrowT, 0, st>>>(
       mesh, tpl, rc, s, voids, traffic, work);
@@ -1740,7 +1740,6 @@ void grow(MeshViewT<R> mesh, TemplateViewT<R> tpl, RungConstsT<R> rc, SurvivorsT
   if (max_survivors == 0) return;
   // work[0] for the first launch, work[1] for the per-CTA pass after the
   // warp kernel, work[2] the warp kernel's leftovers listed in pend.
-  SIFG_CUDA(cudaMemsetAsync(work, 0, 3 * sizeof(uint32_t), st));
   const bool by_warp = g_growth_mode == 2 || (g_growth_mode == 0 && max_survivors >= kWarpGrowthMin);
   const unsigned g = max_survivors < growth_grid() ? max_survivors : growth_grid();
   if (timer) timer->begin(st);
@@ -2132,7 +2131,6 @@ void grow_weighted(MeshViewT<R> mesh, TemplateViewT<R> tpl, RungConstsT<R> rc, S
                    unsigned long long* traffic, cudaStream_t st, KernelTimer* timer, uint8_t only,
                    uint32_t* work) {
   if (max_survivors == 0) return;
-  SIFG_CUDA(cudaMemsetAsync(work, 0, sizeof(uint32_t), st));
   constexpr size_t smem = weighted_smem_bytes<R>();
   thread_local bool attr = false;  // the attribute is per thread's view of the function
   if (!attr) {
@@ -2479,7 +2477,6 @@ void grow_survey(MeshViewT<R> dm, TemplateViewT<R> dt, MeshViewT<R> rm, Template
                  long long* gwbuf, uint32_t gcap, unsigned long long* traffic, cudaStream_t st,
                  KernelTimer* timer, uint32_t* work) {
   if (max_survivors == 0) return;
-  SIFG_CUDA(cudaMemsetAsync(work, 0, sizeof(uint32_t), st));
   constexpr size_t smem = survey_smem_bytes<R>();
   thread_local bool attr = false;  // the attribute is per thread's view of the function
   if (!attr) {
@@ -3165,15 +3162,6 @@ void append_accepted(SurvivorsT<R> s, const uint32_t* rank, const uint32_t* acc,
 // Void index
 // ---------------------------------------------------------------------------
 
-// cll_axis_index, src/structures/cell_linked_list.c:40-58 (periodic).
-template <class R>
-__device__ __forceinline__ uint32_t void_axis(R c, R inv) {
-  int32_t i = (int32_t)ffloor(fmul(c, inv));
-  i %= (int32_t)kVoidCells;
-  if (i < 0) i += kVoidCells;
-  return (uint32_t)i;
-}
-
 template <class R>
 __global__ void void_count_kernel(const R* __restrict__ x, const R* __restrict__ y,
                                   const R* __restrict__ z, uint32_t n, R inv,
@@ -3781,8 +3769,8 @@ void compact_voids(R* cx, R* cy, R* cz, R* r, uint32_t* state, cudaStream_t st) 
   template void scan_compact<R>(const uint32_t*, uint64_t, const R*, const uint32_t*, R*,          \
                                 uint32_t*, cudaStream_t);                                          \
   template void prefilter<R>(const uint32_t*, uint32_t, const uint32_t*, VoidViewT<R>,             \
-                             RungConstsT<R>, uint8_t*, uint32_t*, uint32_t*, uint32_t*, R*, R*,    \
-                             R*, uint32_t*, cudaStream_t, bool, const CandOffT<R>*, R*);          \
+                             RungConstsT<R>, uint32_t*, uint32_t*, R*, R*, R*, uint8_t*,           \
+                             uint32_t*, cudaStream_t, bool, const CandOffT<R>*, R*);              \
   template uint32_t refine_candidates<R>(const R*, const R*, const uint32_t*, R, uint32_t, R,      \
                                          uint32_t, bool, R*&, uint32_t*&, R*, uint32_t*,           \
                                          CandOffT<R>*, CandOffT<R>*&, CandOffT<R>*, uint32_t*,     \

@@ -189,18 +189,18 @@ void below_write_pass(const uint32_t* counts, const float* delta, const uint32_t
                       const uint32_t* block_offsets, float* cand_delta, uint32_t* cand_flat,
                       cudaStream_t st);
 
-// Pre-filter at the rung radius (prefilter_cells, exodus_finder.c:871-944)
-// and compaction of the survivors, candidate order kept; with keep_all
+// Pre-filter at the rung radius (prefilter_cells, exodus_finder.c:871-944),
+// the survivors appended in no fixed order (outcome kRescaleOk, to be grown)
+// and counted in *d_surv_count, which the caller zeroes; with keep_all
 // (displacement) every candidate survives.
 // coff: the candidates' offsets (SIF_FINDER_REFINE_GAUSSIAN), or NULL when
 // every candidate sits on its node; soff then receives each survivor's
 // offset length (or is NULL).
 template <class R>
 void prefilter(const uint32_t* cand_flat, uint32_t m, const uint32_t* mask, VoidViewT<R> voids,
-               RungConstsT<R> rc, uint8_t* alive, uint32_t* block_counts, uint32_t* surv_cand,
-               uint32_t* surv_flat, R* scx, R* scy, R* scz, uint32_t* d_surv_count,
-               cudaStream_t st, bool keep_all = false, const CandOffT<R>* coff = nullptr,
-               R* soff = nullptr);
+               RungConstsT<R> rc, uint32_t* surv_cand, uint32_t* surv_flat, R* scx, R* scy, R* scz,
+               uint8_t* sreason, uint32_t* d_surv_count, cudaStream_t st, bool keep_all = false,
+               const CandOffT<R>* coff = nullptr, R* soff = nullptr);
 
 // SIF_FINDER_REFINE_GAUSSIAN's placing (sif__finder_scan_refined, src/finder/
 // utils.c:406-552): the m candidates (cdelta, cflat: the cells at or below
@@ -224,8 +224,9 @@ uint32_t refine_candidates(const R* fa, const R* fb, const uint32_t* mask, R thr
 // collides with a void of `voids` (the catalogue as the rung begins) is
 // refused before any growth, as the reference refuses it -- the commit would
 // refuse it at any radius it could return. Writes every survivor's outcome:
-// kRescaleWitness (radius -1) or kRescaleOk (to be grown). traffic as grow's;
-// work: a device counter (zeroed here) from which the warps take survivors.
+// kRescaleWitness (radius -1) or kRescaleOk (to be grown); switched off, it
+// does nothing (the pre-filter left them kRescaleOk). traffic as grow's;
+// work: a device counter (zeroed by the caller) from which the warps take survivors.
 template <class R>
 void witness(MeshViewT<R> mesh, TemplateViewT<R> tpl, RungConstsT<R> rc, SurvivorsT<R> s,
              VoidViewT<R> voids, uint32_t max_survivors, unsigned long long* traffic,
@@ -234,6 +235,7 @@ void witness(MeshViewT<R> mesh, TemplateViewT<R> tpl, RungConstsT<R> rc, Survivo
 // 1 (default): the witness runs; 0: every survivor is grown. The catalogue
 // does not depend on it (tests run both).
 void set_witness(int on);
+bool witness_on();
 
 // Sphere growth of every survivor, or (only != kAllSurvivors) of those whose
 // rescale outcome is `only`; with only == kAllSurvivors, survivors the
@@ -242,8 +244,8 @@ void set_witness(int on);
 constexpr uint8_t kAllSurvivors = 0xff;
 unsigned growth_grid();
 // traffic (may be NULL): two counters the kernel adds to -- particles read
-// and template cells visited. work: two device counters (zeroed here) from
-// which the warps or CTAs take survivors.
+// and template cells visited. work: three device counters (zeroed by the
+// caller) from which the warps or CTAs take survivors.
 template <class R>
 void grow(MeshViewT<R> mesh, TemplateViewT<R> tpl, RungConstsT<R> rc, SurvivorsT<R> s,
           uint32_t max_survivors, R* gbuf, uint32_t gcap, unsigned long long* traffic,
