@@ -51,13 +51,15 @@ Engine::Engine(int device) : device_(device) {
   // and takes what bandwidth the smoothing leaves.
   const int mid_prio = hi_prio < lo_prio ? hi_prio + 1 : lo_prio;
   SIFG_CUDA(cudaStreamCreateWithPriority(&st_, cudaStreamNonBlocking, hi_prio));
-  SIFG_CUDA(cudaStreamCreateWithPriority(&st_fft_, cudaStreamNonBlocking, mid_prio));
+  for (cudaStream_t& s : st_fft_)
+    SIFG_CUDA(cudaStreamCreateWithPriority(&s, cudaStreamNonBlocking, mid_prio));
   SIFG_CUDA(cudaStreamCreateWithPriority(&st_copy_, cudaStreamNonBlocking, lo_prio));
   SIFG_CUDA(cudaEventCreateWithFlags(&ev_copy_start_, cudaEventDisableTiming));
   SIFG_CUDA(cudaEventCreateWithFlags(&ev_mesh_ready_, cudaEventDisableTiming));
   SIFG_CUDA(cudaEventCreateWithFlags(&ev_cand_, cudaEventDisableTiming));
   SIFG_CUDA(cudaEventCreateWithFlags(&ev_start_, cudaEventDisableTiming));
-  for (int k = 0; k < 2; k++) {
+  SIFG_CUDA(cudaEventCreateWithFlags(&ev_forward_, cudaEventDisableTiming));
+  for (int k = 0; k < kLanes; k++) {
     SIFG_CUDA(cudaEventCreateWithFlags(&ev_smoothed_[k], cudaEventDisableTiming));
     SIFG_CUDA(cudaEventCreateWithFlags(&ev_scanned_[k], cudaEventDisableTiming));
   }
@@ -70,10 +72,13 @@ Engine::~Engine() {
   cudaFreeHost(h_rank_);
   cudaFreeHost(h_counters_);
   if (ev_cand_) cudaEventDestroy(ev_cand_);
-  for (cudaEvent_t ev : {ev_start_, ev_smoothed_[0], ev_smoothed_[1], ev_scanned_[0], ev_scanned_[1],
-                         ev_copy_start_, ev_mesh_ready_})
+  for (cudaEvent_t ev : {ev_start_, ev_forward_, ev_copy_start_, ev_mesh_ready_})
     if (ev) cudaEventDestroy(ev);
-  if (st_fft_) cudaStreamDestroy(st_fft_);
+  for (int k = 0; k < kLanes; k++) {
+    if (ev_smoothed_[k]) cudaEventDestroy(ev_smoothed_[k]);
+    if (ev_scanned_[k]) cudaEventDestroy(ev_scanned_[k]);
+    if (st_fft_[k]) cudaStreamDestroy(st_fft_[k]);
+  }
   if (st_copy_) cudaStreamDestroy(st_copy_);
   if (st_) cudaStreamDestroy(st_);
 }
@@ -518,11 +523,20 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
   std::vector<R> radii = p.radii;
   std::sort(radii.begin(), radii.end(), [](R a, R b) { return a > b; });
 
-  R* fields[2] = {grow_to<R>(field_[0], cells), grow_to<R>(field_[1], cells)};
+  // How many rungs are smoothed at once, each on a lane of its own (a stream, a
+  // field). The own transforms at 512 fill the GPU and list their cells as
+  // they go: one after another, a rung ahead. Elsewhere a rung's chain of five
+  // small launches leaves most of the GPU idle up to about 256^3 (64^3: 35 us
+  // of launches one waiting on another, 25 us of kernels on a few SMs), and
+  // rung after rung without a candidate waits for nothing else: four lanes;
+  // past that two, whose kernels fill one another's tails.
+  const bool own = !p.inject && sizeof(R) == 4 && N == 512;
+  const uint32_t lanes = own || p.inject || cells > (1ull << 24) ? 2 : kLanes;
+  R *fields[kLanes], *gfields[kLanes], *rfields[kLanes];
+  for (uint32_t k = 0; k < lanes; k++) fields[k] = grow_to<R>(field_[k], cells);
   // The refinement's own fields (the top-hat times the Gaussian), alongside.
-  R* gfields[2] = {nullptr, nullptr};
   if (gaussian)
-    for (int k = 0; k < 2; k++) gfields[k] = grow_to<R>(gfield_[k], cells);
+    for (uint32_t k = 0; k < lanes; k++) gfields[k] = grow_to<R>(gfield_[k], cells);
   // Injected fields are consumed in the order the run's transforms return
   // them: per rung the top-hat and, refined, for a rung with candidates, the
   // refinement's field (the reference runs that transform only then).
@@ -533,11 +547,10 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
   // (sif__exodus_survey_occupancy, exodus_survey.c:159-201): the nodes the
   // randoms are nearest to, closed over the window that expects enough of
   // them; and the randoms' two fields.
-  R* rfields[2] = {nullptr, nullptr};
   uint32_t* occ = nullptr;
   bool mesh_waited = false;
   if (survey) {
-    for (int k = 0; k < 2; k++) rfields[k] = grow_to<R>(rfield_[k], cells);
+    for (uint32_t k = 0; k < lanes; k++) rfields[k] = grow_to<R>(rfield_[k], cells);
     const uint64_t words = (cells + 31) / 32;
     occ = grow_to<uint32_t>(occ_, words);
     if (p.mesh_ready) {
@@ -553,51 +566,58 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
                    survey_closing_k(rmesh.n_particles, marked), st_);
   }
   SmootherT<R>& rsmoother = rsmoother_for<R>();
-  // The smoothing stream starts after everything queued on the run's stream
-  // (the density contrast among it); rung ri's field is fields[ri % 2].
+  // The smoothing streams start after everything queued on the run's stream
+  // (the density contrast among it); rung ri's lane is ri % lanes.
   SIFG_CUDA(cudaEventRecord(ev_start_, st_));
-  SIFG_CUDA(cudaStreamWaitEvent(st_fft_, ev_start_, 0));
-  for (int k = 0; k < 2; k++) SIFG_CUDA(cudaEventRecord(ev_scanned_[k], st_));
+  SIFG_CUDA(cudaStreamWaitEvent(st_fft_[0], ev_start_, 0));
+  for (uint32_t k = 0; k < lanes; k++) SIFG_CUDA(cudaEventRecord(ev_scanned_[k], st_));
   // Under the cell seeds, where the smoothing can list the cells at or below
   // the threshold as it writes them (the float form's own transform), the
   // scan is a mask filter over that list; two lists alternate with the fields.
-  BelowList below[2];
+  BelowList below[kLanes];
   bool listed = false;
   auto smooth_rung = [&](uint32_t ri) {
-    SIFG_CUDA(cudaStreamWaitEvent(st_fft_, ev_scanned_[ri % 2], 0));
-    if (tm) tm->smoothing.begin(st_fft_);
+    const uint32_t lane = ri % lanes;
+    const int at = own ? 0 : (int)lane;  // the own transforms share one stream
+    const cudaStream_t fs = st_fft_[at];
+    SIFG_CUDA(cudaStreamWaitEvent(fs, ev_scanned_[lane], 0));
+    if (tm) tm->smoothing.begin(fs);
     // With the list, the field's only other reader is SIF_FINDER_CONSUME_GRID
     // (the last rung's): the other rungs' fields are not written.
-    if (listed) below[ri % 2].field = p.consume_out && ri + 1 == radii.size();
-    smoother.smooth(kFilterTopHat, radii[ri], 0.0f, fields[ri % 2], tm ? &tm->filter : nullptr,
-                    listed ? &below[ri % 2] : nullptr);
+    if (listed) below[lane].field = p.consume_out && ri + 1 == radii.size();
+    smoother.smooth(kFilterTopHat, radii[ri], 0.0f, fields[lane], tm ? &tm->filter : nullptr,
+                    listed ? &below[lane] : nullptr, at);
     // RUNG_MINIMA_SIGMA (exodus_finder.c:1362-1365) of the rung on top of
     // the top-hat, for every rung: a rung without candidates never reads it.
     if (gaussian)
-      smoother.smooth(kFilterTopHat, radii[ri], R(0.15f) * radii[ri], gfields[ri % 2],
-                      tm ? &tm->filter : nullptr);
+      smoother.smooth(kFilterTopHat, radii[ri], R(0.15f) * radii[ri], gfields[lane],
+                      tm ? &tm->filter : nullptr, nullptr, at);
     // A survey's rung (exodus_finder.c:1729-1737): the randoms smoothed the
     // same way, and the field scanned is the data against them.
     if (survey) {
-      rsmoother.smooth(kFilterTopHat, radii[ri], 0.0f, rfields[ri % 2], nullptr);
-      survey_contrast(fields[ri % 2], (const R*)rfields[ri % 2], occ, p.survey_alpha, cells, st_fft_);
+      rsmoother.smooth(kFilterTopHat, radii[ri], 0.0f, rfields[lane], nullptr, nullptr, at);
+      survey_contrast(fields[lane], (const R*)rfields[lane], occ, p.survey_alpha, cells, fs);
     }
-    if (tm) tm->smoothing.end(st_fft_);
-    SIFG_CUDA(cudaEventRecord(ev_smoothed_[ri % 2], st_fft_));
+    if (tm) tm->smoothing.end(fs);
+    SIFG_CUDA(cudaEventRecord(ev_smoothed_[lane], fs));
   };
   // On every way out, nothing of the run is left in flight on the smoothing
-  // stream.
+  // streams.
   struct FftDrain {
-    cudaStream_t s;
-    ~FftDrain() { cudaStreamSynchronize(s); }
+    const cudaStream_t* s;
+    ~FftDrain() {
+      for (int k = 0; k < kLanes; k++) cudaStreamSynchronize(s[k]);
+    }
   } drain{st_fft_};
   const uint32_t nb_below = (uint32_t)((cells + kBelowBlock - 1) / kBelowBlock);
   if (!p.inject) {
-    smoother.setup(N, box, window_mode, st_fft_);
+    smoother.setup(N, box, window_mode, st_fft_[0]);
+    if (!own) smoother.set_lanes((int)lanes, st_fft_);
     listed = g_scan_mode == 0 && sizeof(R) == 4 && !minima && !gaussian && !survey &&
              smoother.lists_below() && cells % kBelowBlock == 0;
     if (survey) {
-      rsmoother.setup(N, box, window_mode, st_fft_);
+      rsmoother.setup(N, box, window_mode, st_fft_[0]);
+      if (!own) rsmoother.set_lanes((int)lanes, st_fft_);
       rsmoother.forward(p.random_density, nullptr);
     }
     if (listed)
@@ -608,7 +628,11 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
         below[k].flat = grow_to<uint32_t>(below_flat_[k], cells);
       }
     smoother.forward(d_delta, p.contrast_mean);
-    if (p.first_rung < radii.size()) smooth_rung(p.first_rung);
+    SIFG_CUDA(cudaEventRecord(ev_forward_, st_fft_[0]));
+    for (uint32_t k = 1; !own && k < lanes; k++)
+      SIFG_CUDA(cudaStreamWaitEvent(st_fft_[k], ev_forward_, 0));
+    for (uint32_t k = 0; k + 1 < lanes && p.first_rung + k < radii.size(); k++)
+      smooth_rung(p.first_rung + k);
   }
 
   // Loop invariants, exodus_finder.c:1629-1632.
@@ -844,28 +868,29 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
     const R radius = radii[ri];
     rs.radius = radius;
 
-    // 1. The rung's field; the next rung's smoothing queued behind this
-    //    rung's last read of the buffer it overwrites.
-    R* field = fields[ri % 2];
+    // 1. The rung's field; the smoothing of the rung `lanes` - 1 on queued
+    //    behind the last read of the buffer it overwrites.
+    const uint32_t lane = ri % lanes;
+    R* field = fields[lane];
     const cudaMemcpyKind inj_kind =
         p.inject_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     if (p.inject) {
       SIFG_CUDA(cudaMemcpyAsync(field, p.inject + inj_k++ * cells, cells * sizeof(R), inj_kind, st_));
       if (survey) {
-        R* rf = rfields[ri % 2];
+        R* rf = rfields[lane];
         SIFG_CUDA(cudaMemcpyAsync(rf, p.inject + inj_k++ * cells, cells * sizeof(R), inj_kind, st_));
         survey_contrast(field, (const R*)rf, occ, p.survey_alpha, cells, st_);
       }
     } else {
-      if (ri + 1 < radii.size()) smooth_rung(ri + 1);
-      SIFG_CUDA(cudaStreamWaitEvent(st_, ev_smoothed_[ri % 2], 0));
+      if (ri + lanes - 1 < radii.size()) smooth_rung(ri + lanes - 1);
+      SIFG_CUDA(cudaStreamWaitEvent(st_, ev_smoothed_[lane], 0));
     }
     if (tm) tm->rung.begin(st_);
 
     // 2. Candidates, in flat order.
     R* region_delta = nullptr;
     uint32_t* region_flat = nullptr;
-    const BelowList& bl = below[ri % 2];
+    const BelowList& bl = below[lane];
     rs.from_list = listed ? 1u : 0u;
     if (listed) {
       below_count_pass(bl.counts, bl.flat, nb_below, kBelowBlock, mask, blocks, h_counters_, st_);
@@ -877,9 +902,9 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
       // (the minima are found on the refinement's field, below).
       scan_fused_pass(field, mask, cells, threshold, blocks, h_counters_, region_delta, region_flat,
                       st_, N, minima && !gaussian);
-      // The field's last reader: the next rung but one may smooth into it
+      // The field's last reader: a later rung may smooth into it
       // (refined, the placing reads it again: recorded after that).
-      if (!gaussian) SIFG_CUDA(cudaEventRecord(ev_scanned_[ri % 2], st_));
+      if (!gaussian) SIFG_CUDA(cudaEventRecord(ev_scanned_[lane], st_));
     }
     // The total goes straight to pinned host memory.
     const auto t_wait = clk::now();
@@ -897,7 +922,7 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
         cdelta = grow_to<R>(cand_delta_, m);
         cflat = grow_to<uint32_t>(cand_flat_, m);
         scan_compact(blocks, cells, region_delta, region_flat, cdelta, cflat, st_);
-        R* gf = gfields[ri % 2];
+        R* gf = gfields[lane];
         if (p.inject)
           SIFG_CUDA(cudaMemcpyAsync(gf, p.inject + inj_k++ * cells, cells * sizeof(R), inj_kind, st_));
         CandOffT<R>* ocoff = nullptr;
@@ -909,7 +934,7 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
         coff = ocoff;
       }
       // Both fields' last reader was the placing.
-      SIFG_CUDA(cudaEventRecord(ev_scanned_[ri % 2], st_));
+      SIFG_CUDA(cudaEventRecord(ev_scanned_[lane], st_));
       rs.n_candidates = m;
     }
 
@@ -921,7 +946,7 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
     rs.r_search = r_search;
     if (m == 0) {
       // The list's last reader was its count pass.
-      if (listed) SIFG_CUDA(cudaEventRecord(ev_scanned_[ri % 2], st_));
+      if (listed) SIFG_CUDA(cudaEventRecord(ev_scanned_[lane], st_));
       if (tm) tm->rung.end(st_);
       rs.rung_ms = ms_since(t_rung);
       if (stats) stats->push_back(rs);
@@ -941,7 +966,7 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
         below_write_pass(bl.counts, bl.delta, bl.flat, nb_below, kBelowBlock, mask, blocks, cdelta,
                          cflat, st_);
       // The list's last reader: the next rung but one may smooth into it.
-      SIFG_CUDA(cudaEventRecord(ev_scanned_[ri % 2], st_));
+      SIFG_CUDA(cudaEventRecord(ev_scanned_[lane], st_));
     } else {
       cdelta = (R*)h_delta_;
       cflat = grow_to<uint32_t>(cand_flat_, m);
@@ -1283,7 +1308,7 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
   }
 
   if (p.consume_out) {
-    const R* last = fields[(radii.size() + 1) % 2];
+    const R* last = fields[(radii.size() + lanes - 1) % lanes];
     SIFG_CUDA(cudaMemcpyAsync(p.consume_out, last, cells * sizeof(R), cudaMemcpyDeviceToDevice, st_));
   }
   const size_t base = out.cx.size();

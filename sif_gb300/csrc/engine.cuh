@@ -187,7 +187,8 @@ class Engine {
  private:
   int device_;
   cudaStream_t st_ = 0;
-  DevBuf field_[2], mask_, cand_delta_, cand_flat_, blocks_, rank_, rank_slots_;
+  static constexpr int kLanes = Smoother::kLanes;  // rungs smoothed at once
+  DevBuf field_[kLanes], mask_, cand_delta_, cand_flat_, blocks_, rank_, rank_slots_;
   DevBuf surv_cand_, surv_flat_, scx_, scy_, scz_, sr_, sreason_, state_a_, state_b_, acc_;
   DevBuf commit_bar_;  // the cooperative commit's grid barrier and its report
   DevBuf counters_, dcount_, sgrid_start_, sgrid_ids_, sgrid_cellof_, sgrid_pack_, sgrid_rank_;
@@ -199,12 +200,12 @@ class Engine {
   // SIF_FINDER_REFINE_GAUSSIAN: the refinement's fields, the placed
   // candidates and their offsets, the minima's keep flags, the survivors'
   // offset lengths.
-  DevBuf gfield_[2], cand_delta2_, cand_flat2_, cand_off_, cand_off2_, keep_, soff_;
+  DevBuf gfield_[kLanes], cand_delta2_, cand_flat2_, cand_off_, cand_off2_, keep_, soff_;
   DevBuf tpl_, gbuf_, traffic_, region_delta_, region_flat_;
   // A survey: the randoms' smoothed fields, the footprint (and the closing's
   // other mask, the marked count), the randoms' template, the voids' observed
   // fractions.
-  DevBuf rfield_[2], occ_, occ_tmp_, occ_count_, rtpl_, foot_, shell_;
+  DevBuf rfield_[kLanes], occ_, occ_tmp_, occ_count_, rtpl_, foot_, shell_;
   static constexpr uint32_t kExtMaxLevels = 32;  // EXT_MAX_LEVELS, exodus_finder.c:244
   DevBuf ext_tpl_[kExtMaxLevels];  // the extended reach's templates, one per level
   DevBuf below_counts_[2], below_delta_[2], below_flat_[2];  // the smoothing's below-threshold lists
@@ -215,12 +216,13 @@ class Engine {
   uint32_t* h_counters_ = nullptr;
   size_t h_cap_ = 0;
   cudaEvent_t ev_cand_ = nullptr;
-  // The smoothing runs on its own, lower-priority stream into two field
-  // buffers: rung i+1's transform overlaps rung i's growth and commit.
-  cudaStream_t st_fft_ = 0, st_copy_ = 0;
+  // The smoothing runs on streams of its own, of lower priority, each lane into
+  // a field buffer of its own: the next rungs' transforms overlap one another
+  // and rung i's growth and commit.
+  cudaStream_t st_fft_[kLanes] = {}, st_copy_ = 0;
   cudaEvent_t ev_copy_start_ = nullptr, ev_mesh_ready_ = nullptr;
-  cudaEvent_t ev_start_ = nullptr, ev_smoothed_[2] = {nullptr, nullptr},
-              ev_scanned_[2] = {nullptr, nullptr};
+  cudaEvent_t ev_start_ = nullptr, ev_forward_ = nullptr, ev_smoothed_[kLanes] = {},
+              ev_scanned_[kLanes] = {};
   void ensure_host(size_t m);
 };
 

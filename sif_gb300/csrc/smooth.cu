@@ -869,6 +869,7 @@ void SmootherT<R>::setup(uint32_t n_, R box_, int window_mode_, cudaStream_t st)
       if (plan_work) SIFG_CUFFT(cufftSetWorkArea(h, area.ptr));
     }
     stream = st;
+    bound_lane = 0;
   }
   box = box_;
   window_mode = window_mode_;
@@ -895,6 +896,18 @@ void SmootherT<R>::setup(uint32_t n_, R box_, int window_mode_, cudaStream_t st)
   }
 }
 
+template <class R>
+void SmootherT<R>::set_lanes(int lanes, const cudaStream_t* streams) {
+  for (int k = 1; k < lanes; k++) {
+    Lane& l = extra[k - 1];
+    l.st = streams[k];
+    l.work.ensure((uint64_t)n * n * (n / 2 + 1) * 2 * sizeof(R));
+    if (plan_work) l.area.ensure(plan_work);
+    const uint32_t h = n >> 1;
+    l.lut.ensure(((size_t)3 * h * h + 1) * sizeof(R));
+  }
+}
+
 static void launch_forward512(const SmootherT<float>& s, const float* grid, const double* mean);
 
 template <>
@@ -912,16 +925,17 @@ void SmootherT<double>::forward(const double* grid, const double* mean) {
   SIFG_CUFFT(cufftExecD2Z(plan_r2c, (cufftDoubleReal*)grid, (cufftDoubleComplex*)spectrum.ptr));
 }
 
-static void launch_filter(const SmootherT<float>& s, int filter, float norm) {
+static void launch_filter(const SmootherT<float>& s, int filter, float norm, const DevBuf& lut,
+                          const DevBuf& work, cudaStream_t st) {
   const uint64_t modes = (uint64_t)s.n * s.n * (s.n / 2 + 1);
   const float* w = (s.window_mode && filter != kFilterNone) ? s.win.as<float>() : nullptr;
   const unsigned grd = grid_for(modes / 2 + 1, 256, 152u * 8u);
   if (modes < (1ull << 32))
-    filter_kernel<uint32_t><<<grd, 256, 0, s.stream>>>(s.spectrum.as<float4>(), s.work.as<float4>(),
-                                                       s.n, s.lut.as<float>(), w, norm);
+    filter_kernel<uint32_t><<<grd, 256, 0, st>>>(s.spectrum.as<float4>(), work.as<float4>(), s.n,
+                                                 lut.as<float>(), w, norm);
   else
-    filter_kernel<uint64_t><<<grd, 256, 0, s.stream>>>(s.spectrum.as<float4>(), s.work.as<float4>(),
-                                                       s.n, s.lut.as<float>(), w, norm);
+    filter_kernel<uint64_t><<<grd, 256, 0, st>>>(s.spectrum.as<float4>(), work.as<float4>(), s.n,
+                                                 lut.as<float>(), w, norm);
 }
 
 // The three passes of the n = 512 inverse transform, on the smoother's stream.
@@ -1040,16 +1054,17 @@ const float* SmootherT<R>::factor_table(int filter, R r, R sigma) {
   }
 }
 
-static void launch_filter(const SmootherT<double>& s, int filter, double norm) {
+static void launch_filter(const SmootherT<double>& s, int filter, double norm, const DevBuf& lut,
+                          const DevBuf& work, cudaStream_t st) {
   const uint64_t modes = (uint64_t)s.n * s.n * (s.n / 2 + 1);
   const double* w = (s.window_mode && filter != kFilterNone) ? s.win.as<double>() : nullptr;
-  filter_kernel_f64<<<grid_for(modes, 256, 152u * 8u), 256, 0, s.stream>>>(
-      s.spectrum.as<double2>(), s.work.as<double2>(), s.n, s.lut.as<double>(), w, norm);
+  filter_kernel_f64<<<grid_for(modes, 256, 152u * 8u), 256, 0, st>>>(
+      s.spectrum.as<double2>(), work.as<double2>(), s.n, lut.as<double>(), w, norm);
 }
 
 template <class R>
 void SmootherT<R>::smooth(int filter, R r, R sigma, R* out, KernelTimer* timer,
-                          const BelowList* below) {
+                          const BelowList* below, int lane) {
   const uint32_t h = n >> 1;
   const uint32_t max_k2 = 3 * h * h;
   const double factor = (double)r * 2.0 * M_PI / (double)box;
@@ -1064,17 +1079,26 @@ void SmootherT<R>::smooth(int filter, R r, R sigma, R* out, KernelTimer* timer,
     launch_inverse512(*this, filter, rf, norm, out, timer, below ? *below : BelowList{}, ftab);
     return;
   }
-  lut_kernel<R><<<grid_for((uint64_t)max_k2 + 1, 256), 256, 0, stream>>>(lut.as<R>(), max_k2, filter,
-                                                                         factor, gfactor);
+  const cudaStream_t st = lane ? extra[lane - 1].st : stream;
+  const DevBuf& lwork = lane ? extra[lane - 1].work : work;
+  const DevBuf& llut = lane ? extra[lane - 1].lut : lut;
+  if (lane != bound_lane) {
+    const DevBuf& larea = lane ? extra[lane - 1].area : area;
+    SIFG_CUFFT(cufftSetStream(plan_c2r, st));
+    if (plan_work) SIFG_CUFFT(cufftSetWorkArea(plan_c2r, larea.ptr));
+    bound_lane = lane;
+  }
+  lut_kernel<R><<<grid_for((uint64_t)max_k2 + 1, 256), 256, 0, st>>>(llut.as<R>(), max_k2, filter,
+                                                                     factor, gfactor);
   SIFG_LAUNCH_CHECK();
-  if (timer) timer->begin(stream);
-  launch_filter(*this, filter, norm);
+  if (timer) timer->begin(st);
+  launch_filter(*this, filter, norm, llut, lwork, st);
   SIFG_LAUNCH_CHECK();
-  if (timer) timer->end(stream);
+  if (timer) timer->end(st);
   if (sizeof(R) == 8)
-    SIFG_CUFFT(cufftExecZ2D(plan_c2r, (cufftDoubleComplex*)work.ptr, (cufftDoubleReal*)out));
+    SIFG_CUFFT(cufftExecZ2D(plan_c2r, (cufftDoubleComplex*)lwork.ptr, (cufftDoubleReal*)out));
   else
-    SIFG_CUFFT(cufftExecC2R(plan_c2r, (cufftComplex*)work.ptr, (cufftReal*)out));
+    SIFG_CUFFT(cufftExecC2R(plan_c2r, (cufftComplex*)lwork.ptr, (cufftReal*)out));
 }
 
 template <class R>

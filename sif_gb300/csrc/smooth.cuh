@@ -54,6 +54,18 @@ struct SmootherT {
     void* twiddles = nullptr;  // the float form's own inverse at n = 512: its tables (no plans)
   };
   size_t plan_work = 0;  // the current plans' need
+  // Further lanes, for several smoothings of the one spectrum at once: each a
+  // stream with its own transform input, work area and table (lane 0 is
+  // `stream` with work, area and lut). The inverse plan is bound to the lane it
+  // runs on next (a launch takes the stream and area it is bound to then).
+  static constexpr int kLanes = 4;
+  struct Lane {
+    cudaStream_t st = 0;
+    DevBuf work, area, lut;
+  };
+  Lane extra[kLanes - 1];
+  int bound_lane = 0;
+  void set_lanes(int lanes, const cudaStream_t* streams);  // after setup
   const void* twiddles = nullptr;
   std::vector<Plans> plans;
   // The own inverse's filter factors at n = 512, one table per smoothing
@@ -81,8 +93,9 @@ struct SmootherT {
   // on top) into out (n^3 values), asynchronously on the stream.
   // below (float form): the cells at or below below->thr listed as the
   // transform writes them, where lists_below() -- else the caller scans.
+  // lane: where it runs (set_lanes; the own transforms only on 0).
   void smooth(int filter, R r, R sigma, R* out, KernelTimer* timer,
-              const BelowList* below = nullptr);
+              const BelowList* below = nullptr, int lane = 0);
   bool lists_below() const { return sizeof(R) == 4 && twiddles != nullptr; }
   void restore(R* out);
   void release();
