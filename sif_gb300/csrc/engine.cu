@@ -59,6 +59,7 @@ Engine::Engine(int device) : device_(device) {
   SIFG_CUDA(cudaEventCreateWithFlags(&ev_cand_, cudaEventDisableTiming));
   SIFG_CUDA(cudaEventCreateWithFlags(&ev_start_, cudaEventDisableTiming));
   SIFG_CUDA(cudaEventCreateWithFlags(&ev_forward_, cudaEventDisableTiming));
+  SIFG_CUDA(cudaEventCreateWithFlags(&ev_tables_, cudaEventDisableTiming));
   for (int k = 0; k < kLanes; k++) {
     SIFG_CUDA(cudaEventCreateWithFlags(&ev_smoothed_[k], cudaEventDisableTiming));
     SIFG_CUDA(cudaEventCreateWithFlags(&ev_scanned_[k], cudaEventDisableTiming));
@@ -72,7 +73,7 @@ Engine::~Engine() {
   cudaFreeHost(h_rank_);
   cudaFreeHost(h_counters_);
   if (ev_cand_) cudaEventDestroy(ev_cand_);
-  for (cudaEvent_t ev : {ev_start_, ev_forward_, ev_copy_start_, ev_mesh_ready_})
+  for (cudaEvent_t ev : {ev_start_, ev_forward_, ev_tables_, ev_copy_start_, ev_mesh_ready_})
     if (ev) cudaEventDestroy(ev);
   for (int k = 0; k < kLanes; k++) {
     if (ev_smoothed_[k]) cudaEventDestroy(ev_smoothed_[k]);
@@ -576,6 +577,11 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
   // scan is a mask filter over that list; two lists alternate with the fields.
   BelowList below[kLanes];
   bool listed = false;
+  // The rungs' radial tables (the own transforms have theirs).
+  const R *tables = nullptr, *gtables = nullptr;
+  auto table_of = [&](const R* t, uint32_t ri) {
+    return t ? t + (ri - p.first_rung) * smoother.table_size() : nullptr;
+  };
   auto smooth_rung = [&](uint32_t ri) {
     const uint32_t lane = ri % lanes;
     const int at = own ? 0 : (int)lane;  // the own transforms share one stream
@@ -586,16 +592,17 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
     // (the last rung's): the other rungs' fields are not written.
     if (listed) below[lane].field = p.consume_out && ri + 1 == radii.size();
     smoother.smooth(kFilterTopHat, radii[ri], 0.0f, fields[lane], tm ? &tm->filter : nullptr,
-                    listed ? &below[lane] : nullptr, at);
+                    listed ? &below[lane] : nullptr, at, table_of(tables, ri));
     // RUNG_MINIMA_SIGMA (exodus_finder.c:1362-1365) of the rung on top of
     // the top-hat, for every rung: a rung without candidates never reads it.
     if (gaussian)
       smoother.smooth(kFilterTopHat, radii[ri], R(0.15f) * radii[ri], gfields[lane],
-                      tm ? &tm->filter : nullptr, nullptr, at);
+                      tm ? &tm->filter : nullptr, nullptr, at, table_of(gtables, ri));
     // A survey's rung (exodus_finder.c:1729-1737): the randoms smoothed the
     // same way, and the field scanned is the data against them.
     if (survey) {
-      rsmoother.smooth(kFilterTopHat, radii[ri], 0.0f, rfields[lane], nullptr, nullptr, at);
+      rsmoother.smooth(kFilterTopHat, radii[ri], 0.0f, rfields[lane], nullptr, nullptr, at,
+                       table_of(tables, ri));
       survey_contrast(fields[lane], (const R*)rfields[lane], occ, p.survey_alpha, cells, fs);
     }
     if (tm) tm->smoothing.end(fs);
@@ -612,7 +619,24 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
   const uint32_t nb_below = (uint32_t)((cells + kBelowBlock - 1) / kBelowBlock);
   if (!p.inject) {
     smoother.setup(N, box, window_mode, st_fft_[0]);
-    if (!own) smoother.set_lanes((int)lanes, st_fft_);
+    if (!own) {
+      smoother.set_lanes((int)lanes, st_fft_);
+      // Every rung's table at once, on a lane that waits for nothing yet (beside
+      // whatever made the contrast), where that is little work: past 128^3 the
+      // tables together hold up the forward transform for longer than each
+      // holds up its own lane (201^3 particles on 243^3: 5.45 ms against 5.03).
+      const uint32_t left =
+          N <= 128 ? (uint32_t)radii.size() - std::min<uint32_t>(p.first_rung, radii.size()) : 0;
+      const R* r0 = radii.data() + p.first_rung;
+      if (left) tables = smoother.tables(kFilterTopHat, r0, nullptr, left, tables_, st_fft_[1]);
+      if (left && gaussian) {
+        std::vector<R> sigmas(r0, r0 + left);
+        for (R& v : sigmas) v = R(0.15f) * v;
+        gtables = smoother.tables(kFilterTopHat, r0, sigmas.data(), left, gtables_, st_fft_[1]);
+      }
+      SIFG_CUDA(cudaEventRecord(ev_tables_, st_fft_[1]));
+      SIFG_CUDA(cudaStreamWaitEvent(st_fft_[0], ev_tables_, 0));
+    }
     listed = g_scan_mode == 0 && sizeof(R) == 4 && !minima && !gaussian && !survey &&
              smoother.lists_below() && cells % kBelowBlock == 0;
     if (survey) {
@@ -709,6 +733,8 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
   uint32_t* n_surv = dcount;
   uint32_t* work = dcount + 1;
   constexpr uint32_t kWork = 3;
+  uint32_t* scan_done = dcount + 8;  // the scan's finished blocks
+  SIFG_CUDA(cudaMemsetAsync(scan_done, 0, sizeof(uint32_t), st_));
   // Gathered particles and visited cells of each rung's sphere growth.
   const size_t n_rungs = radii.size();
   unsigned long long* traffic = (unsigned long long*)grow_to<uint64_t>(traffic_, 2 * n_rungs + 2);
@@ -901,7 +927,7 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
       // Refined, the candidates are every cell at or below the threshold
       // (the minima are found on the refinement's field, below).
       scan_fused_pass(field, mask, cells, threshold, blocks, h_counters_, region_delta, region_flat,
-                      st_, N, minima && !gaussian);
+                      st_, N, minima && !gaussian, scan_done);
       // The field's last reader: a later rung may smooth into it
       // (refined, the placing reads it again: recorded after that).
       if (!gaussian) SIFG_CUDA(cudaEventRecord(ev_scanned_[lane], st_));

@@ -201,6 +201,7 @@ class Engine {
   // candidates and their offsets, the minima's keep flags, the survivors'
   // offset lengths.
   DevBuf gfield_[kLanes], cand_delta2_, cand_flat2_, cand_off_, cand_off2_, keep_, soff_;
+  DevBuf tables_, gtables_;  // the rungs' radial tables (and the refinement's)
   DevBuf tpl_, gbuf_, traffic_, region_delta_, region_flat_;
   // A survey: the randoms' smoothed fields, the footprint (and the closing's
   // other mask, the marked count), the randoms' template, the voids' observed
@@ -221,8 +222,8 @@ class Engine {
   // and rung i's growth and commit.
   cudaStream_t st_fft_[kLanes] = {}, st_copy_ = 0;
   cudaEvent_t ev_copy_start_ = nullptr, ev_mesh_ready_ = nullptr;
-  cudaEvent_t ev_start_ = nullptr, ev_forward_ = nullptr, ev_smoothed_[kLanes] = {},
-              ev_scanned_[kLanes] = {};
+  cudaEvent_t ev_start_ = nullptr, ev_forward_ = nullptr, ev_tables_ = nullptr, 
+              ev_smoothed_[kLanes] = {}, ev_scanned_[kLanes] = {};
   void ensure_host(size_t m);
 };
 

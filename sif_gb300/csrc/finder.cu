@@ -108,10 +108,86 @@ __device__ __forceinline__ uint32_t quad_candidates(const R* __restrict__ f,
   return bits;
 }
 
-// Exclusive scan of one value per thread across the block; *total the sum.
-__device__ __forceinline__ uint32_t block_scan_excl(uint32_t v, uint32_t* ws, uint32_t* total) {
+// One pass over the field: each CTA writes its candidates, in flat order, to
+// the start of its own region of kScanChunk slots and its count to
+// counts[block]; the compaction then moves only the candidates. A warp takes
+// kScanRounds consecutive runs of 128 cells, all of its loads in flight at
+// once, and keeps its candidate bits (four a run) in one word; one exchange of
+// the warps' totals places their entries. With `done` set (zeroed; it is left
+// zero) the last CTA to finish scans the counts -- up to kScanTail of them: a
+// launch and its wait less -- and writes the total.
+constexpr uint32_t kScanTail = 4096;
+template <class R>
+__global__ void __launch_bounds__(kScanT) scan_regions_kernel(
+    const R* __restrict__ f, const uint32_t* __restrict__ mask, uint64_t n, R thr,
+    uint32_t* counts, R* __restrict__ rdelta, uint32_t* __restrict__ rflat, uint32_t grid_n,
+    bool minima, uint32_t* done, uint32_t* total_out) {
+  __shared__ uint32_t ws[kScanT / 32];
+  __shared__ bool last;
+  static_assert(kScanRounds == 8, "a lane's bits, four a run, fill one word");
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  uint32_t x = v;
+  const uint64_t base = (uint64_t)blockIdx.x * kScanChunk;
+  const uint64_t first = base + (uint64_t)warp * (128 * kScanRounds) + lane * 4;
+  R v[kScanRounds][4];
+  uint32_t bits = 0;
+#pragma unroll
+  for (int j = 0; j < kScanRounds; j++)
+    bits |= quad_candidates(f, mask, first + 128 * j, n, thr, v[j], grid_n, minima) << (4 * j);
+  const uint32_t mine = __reduce_add_sync(0xffffffffu, (uint32_t)__popc(bits));
+  if (lane == 0) ws[warp] = mine;
+  __syncthreads();
+  uint32_t pos = 0, total = 0;
+#pragma unroll
+  for (int w = 0; w < kScanT / 32; w++) {
+    pos += w < (int)warp ? ws[w] : 0u;
+    total += ws[w];
+  }
+  if (mine) {
+#pragma unroll
+    for (int j = 0; j < kScanRounds; j++) {
+      const uint32_t b = (bits >> (4 * j)) & 15u;
+      if (!__any_sync(0xffffffffu, b)) continue;
+      const uint32_t cnt = __popc(b);
+      uint32_t x = cnt;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
+        if (lane >= (unsigned)d) x += y;
+      }
+      uint64_t at = base + pos + x - cnt;
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        if (b & (1u << k)) {
+          rdelta[at] = v[j][k];
+          rflat[at] = (uint32_t)(first + 128 * j + k);
+          at++;
+        }
+      }
+      pos += __shfl_sync(0xffffffffu, x, 31);
+    }
+  }
+  if (threadIdx.x == 0) {
+    counts[blockIdx.x] = total;
+    last = false;
+    if (done) {
+      __threadfence();
+      last = atomicAdd(done, 1u) == gridDim.x - 1;
+    }
+  }
+  __syncthreads();
+  if (!last) return;
+  // Every block's count is written: sixteen consecutive ones a thread.
+  __threadfence();
+  constexpr int kPer = kScanTail / kScanT;
+  const uint32_t nb = gridDim.x;
+  uint32_t c[kPer], sum = 0;
+#pragma unroll
+  for (int k = 0; k < kPer; k++) {
+    const uint32_t i = threadIdx.x * kPer + k;
+    c[k] = i < nb ? __ldcg(counts + i) : 0u;
+    sum += c[k];
+  }
+  uint32_t x = sum;
 #pragma unroll
   for (int d = 1; d < 32; d <<= 1) {
     const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
@@ -119,97 +195,23 @@ __device__ __forceinline__ uint32_t block_scan_excl(uint32_t v, uint32_t* ws, ui
   }
   if (lane == 31) ws[warp] = x;
   __syncthreads();
-  uint32_t before = 0, t = 0;
+  uint32_t run = x - sum, all = 0;
 #pragma unroll
   for (int w = 0; w < kScanT / 32; w++) {
-    const uint32_t s = ws[w];
-    before += (w < (int)warp) ? s : 0u;
-    t += s;
+    run += w < (int)warp ? ws[w] : 0u;
+    all += ws[w];
   }
-  __syncthreads();
-  *total = t;
-  return before + x - v;
-}
-
-template <class R>
-__global__ void __launch_bounds__(kScanT) scan_count_kernel(const R* __restrict__ f,
-                                                            const uint32_t* __restrict__ mask,
-                                                            uint64_t n, R thr,
-                                                            uint32_t* __restrict__ counts,
-                                                            uint32_t grid_n, bool minima) {
-  __shared__ uint32_t ws[kScanT / 32];
-  const uint64_t base = (uint64_t)blockIdx.x * kScanChunk;
-  uint32_t c = 0;
 #pragma unroll
-  for (int j = 0; j < kScanRounds; j++) {
-    R v[4];
-    c += __popc(quad_candidates(f, mask, base + ((uint64_t)j * kScanT + threadIdx.x) * 4, n, thr, v,
-                                grid_n, minima));
+  for (int k = 0; k < kPer; k++) {
+    const uint32_t i = threadIdx.x * kPer + k;
+    if (i < nb) counts[i] = run;
+    run += c[k];
   }
-  c = __reduce_add_sync(0xffffffffu, c);
-  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = c;
-  __syncthreads();
   if (threadIdx.x == 0) {
-    uint32_t t = 0;
-    for (int w = 0; w < kScanT / 32; w++) t += ws[w];
-    counts[blockIdx.x] = t;
+    counts[nb] = all;
+    *done = 0;
+    *total_out = all;
   }
-}
-
-template <class R>
-__global__ void __launch_bounds__(kScanT) scan_write_kernel(
-    const R* __restrict__ f, const uint32_t* __restrict__ mask, uint64_t n, R thr,
-    const uint32_t* __restrict__ offsets, R* __restrict__ cdelta, uint32_t* __restrict__ cflat,
-    uint32_t grid_n, bool minima) {
-  __shared__ uint32_t ws[kScanT / 32];
-  const uint64_t base = (uint64_t)blockIdx.x * kScanChunk;
-  uint32_t out = offsets[blockIdx.x];
-  for (int j = 0; j < kScanRounds; j++) {
-    const uint64_t c0 = base + ((uint64_t)j * kScanT + threadIdx.x) * 4;
-    R v[4];
-    const uint32_t bits = quad_candidates(f, mask, c0, n, thr, v, grid_n, minima);
-    uint32_t total;
-    uint32_t pos = out + block_scan_excl(__popc(bits), ws, &total);
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      if (bits & (1u << k)) {
-        cdelta[pos] = v[k];
-        cflat[pos] = (uint32_t)(c0 + k);
-        pos++;
-      }
-    }
-    out += total;
-  }
-}
-
-// One pass over the field: each CTA writes its candidates, in flat order, to
-// the start of its own region of kScanChunk slots and its count to
-// counts[block]; the compaction then moves only the candidates.
-template <class R>
-__global__ void __launch_bounds__(kScanT) scan_regions_kernel(
-    const R* __restrict__ f, const uint32_t* __restrict__ mask, uint64_t n, R thr,
-    uint32_t* __restrict__ counts, R* __restrict__ rdelta, uint32_t* __restrict__ rflat,
-    uint32_t grid_n, bool minima) {
-  __shared__ uint32_t ws[kScanT / 32];
-  const uint64_t base = (uint64_t)blockIdx.x * kScanChunk;
-  uint32_t out = 0;
-  for (int j = 0; j < kScanRounds; j++) {
-    const uint64_t c0 = base + ((uint64_t)j * kScanT + threadIdx.x) * 4;
-    R v[4];
-    const uint32_t bits = quad_candidates(f, mask, c0, n, thr, v, grid_n, minima);
-    uint32_t total;
-    uint32_t pos = out + block_scan_excl(__popc(bits), ws, &total);
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      if (bits & (1u << k)) {
-        rdelta[base + pos] = v[k];
-        rflat[base + pos] = (uint32_t)(c0 + k);
-        pos++;
-      }
-    }
-    out += total;
-  }
-  if (threadIdx.x == 0) counts[blockIdx.x] = out;
 }
 
 // A warp per region: its candidates to their place in the compacted list.
@@ -301,12 +303,15 @@ void below_write_pass(const uint32_t* counts, const float* delta, const uint32_t
 template <class R>
 void scan_fused_pass(const R* field, const uint32_t* mask, uint64_t n_cells, R threshold,
                      uint32_t* block_counts, uint32_t* d_count, R* region_delta,
-                     uint32_t* region_flat, cudaStream_t st, uint32_t grid_n, bool minima) {
+                     uint32_t* region_flat, cudaStream_t st, uint32_t grid_n, bool minima,
+                     uint32_t* done) {
   const uint32_t nb = scan_blocks(n_cells);
+  const bool tail = nb <= kScanTail;
   scan_regions_kernel<R><<<nb, kScanT, 0, st>>>(field, mask, n_cells, threshold, block_counts,
-                                                region_delta, region_flat, grid_n, minima);
+                                                region_delta, region_flat, grid_n, minima,
+                                                tail ? done : nullptr, d_count);
   SIFG_LAUNCH_CHECK();
-  exclusive_scan_total(block_counts, nb, d_count, st);
+  if (!tail) exclusive_scan_total(block_counts, nb, d_count, st);
 }
 
 template <class R>
@@ -317,27 +322,6 @@ void scan_compact(const uint32_t* block_counts, uint64_t n_cells, const R* regio
   const uint32_t warps = nb < 152u * 64u ? nb : 152u * 64u;
   scan_compact_kernel<R><<<(warps + 7) / 8, 256, 0, st>>>(block_counts, nb, region_delta,
                                                            region_flat, cand_delta, cand_flat);
-  SIFG_LAUNCH_CHECK();
-}
-
-template <class R>
-void scan_count_pass(const R* field, const uint32_t* mask, uint64_t n_cells, R threshold,
-                     uint32_t* block_counts, uint32_t* d_count, cudaStream_t st, uint32_t grid_n,
-                     bool minima) {
-  const uint32_t nb = scan_blocks(n_cells);
-  scan_count_kernel<<<nb, kScanT, 0, st>>>(field, mask, n_cells, threshold, block_counts, grid_n,
-                                           minima);
-  SIFG_LAUNCH_CHECK();
-  exclusive_scan_total(block_counts, nb, d_count, st);
-}
-
-template <class R>
-void scan_write_pass(const R* field, const uint32_t* mask, uint64_t n_cells, R threshold,
-                     const uint32_t* block_counts, R* cand_delta, uint32_t* cand_flat,
-                     cudaStream_t st, uint32_t grid_n, bool minima) {
-  scan_write_kernel<<<scan_blocks(n_cells), kScanT, 0, st>>>(field, mask, n_cells, threshold,
-                                                             block_counts, cand_delta, cand_flat,
-                                                             grid_n, minima);
   SIFG_LAUNCH_CHECK();
 }
 
@@ -3760,12 +3744,8 @@ void compact_voids(R* cx, R* cy, R* cz, R* r, uint32_t* state, cudaStream_t st) 
 // The two forms: the reference's float build and its SIF_USE_DOUBLE build.
 // ---------------------------------------------------------------------------
 #define SIFG_FINDER_FORM(R)                                                                        \
-  template void scan_count_pass<R>(const R*, const uint32_t*, uint64_t, R, uint32_t*, uint32_t*,   \
-                                   cudaStream_t, uint32_t, bool);                                  \
-  template void scan_write_pass<R>(const R*, const uint32_t*, uint64_t, R, const uint32_t*, R*,    \
-                                   uint32_t*, cudaStream_t, uint32_t, bool);                       \
   template void scan_fused_pass<R>(const R*, const uint32_t*, uint64_t, R, uint32_t*, uint32_t*,   \
-                                   R*, uint32_t*, cudaStream_t, uint32_t, bool);                   \
+                                   R*, uint32_t*, cudaStream_t, uint32_t, bool, uint32_t*);        \
   template void scan_compact<R>(const uint32_t*, uint64_t, const R*, const uint32_t*, R*,          \
                                 uint32_t*, cudaStream_t);                                          \
   template void prefilter<R>(const uint32_t*, uint32_t, const uint32_t*, VoidViewT<R>,             \

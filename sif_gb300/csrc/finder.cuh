@@ -150,26 +150,18 @@ using Survivors = SurvivorsT<float>;
 // Candidate scan (src/finder/utils.c:130-213): cells with delta <= threshold
 // whose mask bit is clear, in flat order; with `minima` only those that are
 // local minima of the field (SIF_FINDER_SEEDS_MINIMA, utils.c:406-552).
-// The count pass leaves per-block offsets in `block_counts`
-// (scan_blocks(n) + 1 entries) and the total in *d_count; the write pass
-// fills the candidates. grid_n: the grid's side.
+// One pass over the field leaves each block's in a region of its own
+// (scan_region_slots(n) slots in all), the blocks' offsets in `block_counts`
+// (scan_blocks(n) + 1 entries) and the total in *d_count (device or pinned host
+// memory); scan_compact then gathers them in order. grid_n: the grid's side;
+// done: a device word, zero, left zero.
 uint32_t scan_blocks(uint64_t n_cells);
-template <class R>
-void scan_count_pass(const R* field, const uint32_t* mask, uint64_t n_cells, R threshold,
-                     uint32_t* block_counts, uint32_t* d_count, cudaStream_t st, uint32_t grid_n,
-                     bool minima);
-template <class R>
-void scan_write_pass(const R* field, const uint32_t* mask, uint64_t n_cells, R threshold,
-                     const uint32_t* block_counts, R* cand_delta, uint32_t* cand_flat,
-                     cudaStream_t st, uint32_t grid_n, bool minima);
-// The same candidates from one pass over the field: each block's go to its
-// own region (scan_region_slots(n) slots in all) with the count and offsets
-// as scan_count_pass leaves them; scan_compact then gathers them in order.
 uint64_t scan_region_slots(uint64_t n_cells);
 template <class R>
 void scan_fused_pass(const R* field, const uint32_t* mask, uint64_t n_cells, R threshold,
                      uint32_t* block_counts, uint32_t* d_count, R* region_delta,
-                     uint32_t* region_flat, cudaStream_t st, uint32_t grid_n, bool minima);
+                     uint32_t* region_flat, cudaStream_t st, uint32_t grid_n, bool minima,
+                     uint32_t* done);
 template <class R>
 void scan_compact(const uint32_t* block_counts, uint64_t n_cells, const R* region_delta,
                   const uint32_t* region_flat, R* cand_delta, uint32_t* cand_flat,
@@ -180,7 +172,7 @@ void scan_compact(const uint32_t* block_counts, uint64_t n_cells, const R* regio
 // of its region of delta and flat): the listed cells whose mask bit is
 // clear, in flat order. The count pass leaves the per-block offsets in
 // block_counts (nb + 1 entries) and the total in *d_count, as
-// scan_count_pass does; the write pass fills the candidates.
+// scan_fused_pass does; the write pass fills the candidates.
 void below_count_pass(const uint32_t* counts, const uint32_t* flat, uint32_t nb, uint32_t block,
                       const uint32_t* mask, uint32_t* block_counts, uint32_t* d_count,
                       cudaStream_t st);

@@ -753,24 +753,37 @@ static bool own_inverse(uint32_t n) { return n == 512; }
 // fft_build_filter_lut, src/math/fft.c:521-568: the radial factor by integer
 // |k|^2, computed in double.
 template <class R>
-__global__ void lut_kernel(R* __restrict__ lut, uint32_t max_k2, int filter, double factor,
-                           double gfactor) {
-  for (uint32_t k2 = blockIdx.x * blockDim.x + threadIdx.x; k2 <= max_k2;
-       k2 += gridDim.x * blockDim.x) {
-    double v;
-    if (k2 == 0) {
-      v = 1.0;
-    } else if (filter == kFilterTopHat) {
-      const double kr = factor * sqrt((double)k2);
-      v = kr > 1e-4 ? 3.0 * (sin(kr) - kr * cos(kr)) / (kr * kr * kr) : 1.0;
-    } else if (filter == kFilterGaussian) {
-      v = exp(-0.5 * factor * factor * (double)k2);
-    } else {
-      v = 1.0;
-    }
-    if (gfactor > 0.0 && k2 > 0) v *= exp(-0.5 * gfactor * gfactor * (double)k2);
-    lut[k2] = (R)v;
+__device__ __forceinline__ R lut_value(uint32_t k2, int filter, double factor, double gfactor) {
+  double v;
+  if (k2 == 0) {
+    v = 1.0;
+  } else if (filter == kFilterTopHat) {
+    const double kr = factor * sqrt((double)k2);
+    v = kr > 1e-4 ? 3.0 * (sin(kr) - kr * cos(kr)) / (kr * kr * kr) : 1.0;
+  } else if (filter == kFilterGaussian) {
+    v = exp(-0.5 * factor * factor * (double)k2);
+  } else {
+    v = 1.0;
   }
+  if (gfactor > 0.0 && k2 > 0) v *= exp(-0.5 * gfactor * gfactor * (double)k2);
+  return (R)v;
+}
+
+// One table a blockIdx.y. A small grid's tables are built together, before its
+// transform and beside its deposit: in line, each rung's smoothing waits for
+// its own (double precision runs at a sixty-fourth of the float rate here: 7 us
+// of a 64^3 smoothing's 35).
+constexpr uint32_t kLutSet = 64;
+struct LutSet {
+  double factor[kLutSet], gfactor[kLutSet];
+};
+template <class R>
+__global__ void lut_kernel(R* __restrict__ lut, uint32_t max_k2, int filter, LutSet set) {
+  const double factor = set.factor[blockIdx.y], gfactor = set.gfactor[blockIdx.y];
+  R* out = lut + (size_t)blockIdx.y * (max_k2 + 1);
+  for (uint32_t k2 = blockIdx.x * blockDim.x + threadIdx.x; k2 <= max_k2;
+       k2 += gridDim.x * blockDim.x)
+    out[k2] = lut_value<R>(k2, filter, factor, gfactor);
 }
 
 template <class R>
@@ -877,8 +890,6 @@ void SmootherT<R>::setup(uint32_t n_, R box_, int window_mode_, cudaStream_t st)
   spectrum.ensure(twiddles ? kTileWorkElems * sizeof(float2) : modes * 2 * sizeof(R));
   work.ensure(twiddles ? kTileWorkElems * sizeof(float2) : modes * 2 * sizeof(R));
   const uint32_t h = n >> 1;
-  const uint32_t max_k2 = 3 * h * h;
-  lut.ensure(((size_t)max_k2 + 1) * sizeof(R));
   win.ensure((size_t)n * sizeof(R));
   if (window_mode) {
     // fft_build_window_axis, src/math/fft.c:958-975, CIC (order 2): 1/W full,
@@ -903,9 +914,29 @@ void SmootherT<R>::set_lanes(int lanes, const cudaStream_t* streams) {
     l.st = streams[k];
     l.work.ensure((uint64_t)n * n * (n / 2 + 1) * 2 * sizeof(R));
     if (plan_work) l.area.ensure(plan_work);
-    const uint32_t h = n >> 1;
-    l.lut.ensure(((size_t)3 * h * h + 1) * sizeof(R));
   }
+}
+
+template <class R>
+const R* SmootherT<R>::tables(int filter, const R* radii, const R* sigmas, uint32_t count, DevBuf& buf,
+                              cudaStream_t st) {
+  const uint32_t h = n >> 1;
+  const uint32_t max_k2 = 3 * h * h;
+  R* out = (R*)buf.ensure((size_t)count * (max_k2 + 1) * sizeof(R));
+  for (uint32_t k0 = 0; k0 < count; k0 += kLutSet) {
+    const uint32_t nk = std::min(kLutSet, count - k0);
+    LutSet set{};
+    for (uint32_t k = 0; k < nk; k++) {
+      set.factor[k] = (double)radii[k0 + k] * 2.0 * M_PI / (double)box;
+      set.gfactor[k] = sigmas && sigmas[k0 + k] > R(0)
+                           ? (double)sigmas[k0 + k] * 2.0 * M_PI / (double)box
+                           : 0.0;
+    }
+    lut_kernel<R><<<dim3(grid_for((uint64_t)max_k2 + 1, 256), nk), 256, 0, st>>>(
+        out + (size_t)k0 * (max_k2 + 1), max_k2, filter, set);
+    SIFG_LAUNCH_CHECK();
+  }
+  return out;
 }
 
 static void launch_forward512(const SmootherT<float>& s, const float* grid, const double* mean);
@@ -925,17 +956,17 @@ void SmootherT<double>::forward(const double* grid, const double* mean) {
   SIFG_CUFFT(cufftExecD2Z(plan_r2c, (cufftDoubleReal*)grid, (cufftDoubleComplex*)spectrum.ptr));
 }
 
-static void launch_filter(const SmootherT<float>& s, int filter, float norm, const DevBuf& lut,
+static void launch_filter(const SmootherT<float>& s, int filter, float norm, const float* lut,
                           const DevBuf& work, cudaStream_t st) {
   const uint64_t modes = (uint64_t)s.n * s.n * (s.n / 2 + 1);
   const float* w = (s.window_mode && filter != kFilterNone) ? s.win.as<float>() : nullptr;
   const unsigned grd = grid_for(modes / 2 + 1, 256, 152u * 8u);
   if (modes < (1ull << 32))
     filter_kernel<uint32_t><<<grd, 256, 0, st>>>(s.spectrum.as<float4>(), work.as<float4>(), s.n,
-                                                 lut.as<float>(), w, norm);
+                                                 lut, w, norm);
   else
     filter_kernel<uint64_t><<<grd, 256, 0, st>>>(s.spectrum.as<float4>(), work.as<float4>(), s.n,
-                                                 lut.as<float>(), w, norm);
+                                                 lut, w, norm);
 }
 
 // The three passes of the n = 512 inverse transform, on the smoother's stream.
@@ -1054,19 +1085,17 @@ const float* SmootherT<R>::factor_table(int filter, R r, R sigma) {
   }
 }
 
-static void launch_filter(const SmootherT<double>& s, int filter, double norm, const DevBuf& lut,
+static void launch_filter(const SmootherT<double>& s, int filter, double norm, const double* lut,
                           const DevBuf& work, cudaStream_t st) {
   const uint64_t modes = (uint64_t)s.n * s.n * (s.n / 2 + 1);
   const double* w = (s.window_mode && filter != kFilterNone) ? s.win.as<double>() : nullptr;
   filter_kernel_f64<<<grid_for(modes, 256, 152u * 8u), 256, 0, st>>>(
-      s.spectrum.as<double2>(), work.as<double2>(), s.n, lut.as<double>(), w, norm);
+      s.spectrum.as<double2>(), work.as<double2>(), s.n, lut, w, norm);
 }
 
 template <class R>
 void SmootherT<R>::smooth(int filter, R r, R sigma, R* out, KernelTimer* timer,
-                          const BelowList* below, int lane) {
-  const uint32_t h = n >> 1;
-  const uint32_t max_k2 = 3 * h * h;
+                          const BelowList* below, int lane, const R* table) {
   const double factor = (double)r * 2.0 * M_PI / (double)box;
   const double gfactor = sigma > R(0) ? (double)sigma * 2.0 * M_PI / (double)box : 0.0;
   const R norm = (R)(1.0 / ((double)n * n * n));
@@ -1081,18 +1110,15 @@ void SmootherT<R>::smooth(int filter, R r, R sigma, R* out, KernelTimer* timer,
   }
   const cudaStream_t st = lane ? extra[lane - 1].st : stream;
   const DevBuf& lwork = lane ? extra[lane - 1].work : work;
-  const DevBuf& llut = lane ? extra[lane - 1].lut : lut;
   if (lane != bound_lane) {
     const DevBuf& larea = lane ? extra[lane - 1].area : area;
     SIFG_CUFFT(cufftSetStream(plan_c2r, st));
     if (plan_work) SIFG_CUFFT(cufftSetWorkArea(plan_c2r, larea.ptr));
     bound_lane = lane;
   }
-  lut_kernel<R><<<grid_for((uint64_t)max_k2 + 1, 256), 256, 0, st>>>(llut.as<R>(), max_k2, filter,
-                                                                     factor, gfactor);
-  SIFG_LAUNCH_CHECK();
+  if (!table) table = tables(filter, &r, &sigma, 1, lane ? extra[lane - 1].lut : lut, st);
   if (timer) timer->begin(st);
-  launch_filter(*this, filter, norm, llut, lwork, st);
+  launch_filter(*this, filter, norm, table, lwork, st);
   SIFG_LAUNCH_CHECK();
   if (timer) timer->end(st);
   if (sizeof(R) == 8)

@@ -93,9 +93,16 @@ struct SmootherT {
   // on top) into out (n^3 values), asynchronously on the stream.
   // below (float form): the cells at or below below->thr listed as the
   // transform writes them, where lists_below() -- else the caller scans.
-  // lane: where it runs (set_lanes; the own transforms only on 0).
+  // lane: where it runs (set_lanes; the own transforms only on 0). table: the
+  // smoothing's radial table where it is already made, or NULL (the own
+  // transforms take none).
   void smooth(int filter, R r, R sigma, R* out, KernelTimer* timer,
-              const BelowList* below = nullptr, int lane = 0);
+              const BelowList* below = nullptr, int lane = 0, const R* table = nullptr);
+  // The radial tables of `count` smoothings (sigmas NULL: none on top), each
+  // of table_size() values one after another in buf, built on st.
+  const R* tables(int filter, const R* radii, const R* sigmas, uint32_t count, DevBuf& buf,
+                  cudaStream_t st);
+  size_t table_size() const { return 3 * (size_t)(n >> 1) * (n >> 1) + 1; }
   bool lists_below() const { return sizeof(R) == 4 && twiddles != nullptr; }
   void restore(R* out);
   void release();
