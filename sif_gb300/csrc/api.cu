@@ -2157,7 +2157,10 @@ static int run_batch(sifg_box_job_t* jobs, uint32_t n_jobs, uint32_t n_engines) 
   if (!jobs && n_jobs) return fail(SIF_ERR_INVALID, "batch: NULL jobs");
   if (n_jobs == 0) return SIF_OK;
   n_engines = std::max(1u, std::min(n_engines, n_jobs));
-  while (g_pool.size() < n_engines) g_pool.emplace_back(new Engine(main->device()));
+  while (g_pool.size() < n_engines) {
+    g_pool.emplace_back(new Engine(main->device()));
+    g_pool.back()->in_batch = true;
+  }
   const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
   for (uint32_t k = 0; k < n_engines; k++) g_pool[k]->host_threads = (int)std::max(1u, hw / n_engines);
   std::vector<uint32_t> order(n_jobs);

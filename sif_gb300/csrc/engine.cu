@@ -64,7 +64,7 @@ Engine::Engine(int device) : device_(device) {
     SIFG_CUDA(cudaEventCreateWithFlags(&ev_smoothed_[k], cudaEventDisableTiming));
     SIFG_CUDA(cudaEventCreateWithFlags(&ev_scanned_[k], cudaEventDisableTiming));
   }
-  SIFG_CUDA(cudaMallocHost(&h_counters_, 2 * kCommitCounters * sizeof(uint32_t)));
+  SIFG_CUDA(cudaMallocHost(&h_counters_, (2 * kCommitCounters + kLanes) * sizeof(uint32_t)));
 }
 
 Engine::~Engine() {
@@ -530,9 +530,11 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
   // small launches leaves most of the GPU idle up to about 256^3 (64^3: 35 us
   // of launches one waiting on another, 25 us of kernels on a few SMs), and
   // rung after rung without a candidate waits for nothing else: four lanes;
-  // past that two, whose kernels fill one another's tails.
+  // past that two, whose kernels fill one another's tails. An engine of a batch
+  // has the other engines for that: one stream.
   const bool own = !p.inject && sizeof(R) == 4 && N == 512;
-  const uint32_t lanes = own || p.inject || cells > (1ull << 24) ? 2 : kLanes;
+  const bool one_stream = own || in_batch;
+  const uint32_t lanes = one_stream || p.inject || cells > (1ull << 24) ? 2 : kLanes;
   R *fields[kLanes], *gfields[kLanes], *rfields[kLanes];
   for (uint32_t k = 0; k < lanes; k++) fields[k] = grow_to<R>(field_[k], cells);
   // The refinement's own fields (the top-hat times the Gaussian), alongside.
@@ -544,6 +546,9 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
   uint64_t inj_k = 0;
   uint32_t* mask = grow_to<uint32_t>(mask_, (cells + 31) / 32);
   SIFG_CUDA(cudaMemsetAsync(mask, 0, ((cells + 31) / 32) * sizeof(uint32_t), st_));
+  uint32_t* dcount = grow_to<uint32_t>(dcount_, 16);
+  uint32_t* scan_done = dcount + 8;  // each lane's scan's finished blocks
+  SIFG_CUDA(cudaMemsetAsync(scan_done, 0, kLanes * sizeof(uint32_t), st_));
   // A survey's footprint, before any field is scanned
   // (sif__exodus_survey_occupancy, exodus_survey.c:159-201): the nodes the
   // randoms are nearest to, closed over the window that expects enough of
@@ -577,6 +582,26 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
   // scan is a mask filter over that list; two lists alternate with the fields.
   BelowList below[kLanes];
   bool listed = false;
+  // A lane's scan buffers (the list's passes use lane 0's block counts).
+  const uint32_t nb_below = (uint32_t)((cells + kBelowBlock - 1) / kBelowBlock);
+  uint32_t* blocks[kLanes] = {};
+  R* region_delta[kLanes] = {};
+  uint32_t* region_flat[kLanes] = {};
+  auto scan_buffers = [&](uint32_t lane) {
+    blocks[lane] = grow_to<uint32_t>(blocks_[lane],
+                                     std::max<size_t>(std::max(scan_blocks(cells), nb_below) + 1, 1024));
+    if (listed) return;
+    region_delta[lane] = grow_to<R>(region_delta_[lane], scan_region_slots(cells));
+    region_flat[lane] = grow_to<uint32_t>(region_flat_[lane], scan_region_slots(cells));
+  };
+  // Until the first void is accepted no cell is masked, and a rung's candidates
+  // do not wait for the rung before: its scan follows its smoothing on its lane,
+  // and a rung found empty costs the run's stream nothing. (Most of a ladder's
+  // upper rungs are: 15 of 19 at 64^3, each a scan and a wait of 15 us before.)
+  // A scan made ahead is dropped if a void is accepted meanwhile. Only a scan
+  // that shares no scratch with the run's stream can be.
+  bool mask_empty = p.n_prior == 0, ahead[kLanes] = {};
+  uint32_t* const h_ahead = h_counters_ + 2 * kCommitCounters;  // each lane's total
   // The rungs' radial tables (the own transforms have theirs).
   const R *tables = nullptr, *gtables = nullptr;
   auto table_of = [&](const R* t, uint32_t ri) {
@@ -584,7 +609,7 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
   };
   auto smooth_rung = [&](uint32_t ri) {
     const uint32_t lane = ri % lanes;
-    const int at = own ? 0 : (int)lane;  // the own transforms share one stream
+    const int at = one_stream ? 0 : (int)lane;
     const cudaStream_t fs = st_fft_[at];
     SIFG_CUDA(cudaStreamWaitEvent(fs, ev_scanned_[lane], 0));
     if (tm) tm->smoothing.begin(fs);
@@ -606,6 +631,12 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
       survey_contrast(fields[lane], (const R*)rfields[lane], occ, p.survey_alpha, cells, fs);
     }
     if (tm) tm->smoothing.end(fs);
+    ahead[lane] = mask_empty && !listed && !gaussian && scan_is_one_launch(cells);
+    if (ahead[lane]) {
+      scan_buffers(lane);
+      scan_fused_pass(fields[lane], mask, cells, threshold, blocks[lane], h_ahead + lane,
+                      region_delta[lane], region_flat[lane], fs, N, minima, scan_done + lane);
+    }
     SIFG_CUDA(cudaEventRecord(ev_smoothed_[lane], fs));
   };
   // On every way out, nothing of the run is left in flight on the smoothing
@@ -616,11 +647,10 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
       for (int k = 0; k < kLanes; k++) cudaStreamSynchronize(s[k]);
     }
   } drain{st_fft_};
-  const uint32_t nb_below = (uint32_t)((cells + kBelowBlock - 1) / kBelowBlock);
   if (!p.inject) {
     smoother.setup(N, box, window_mode, st_fft_[0]);
     if (!own) {
-      smoother.set_lanes((int)lanes, st_fft_);
+      if (!one_stream) smoother.set_lanes((int)lanes, st_fft_);
       // Every rung's table at once, on a lane that waits for nothing yet (beside
       // whatever made the contrast), where that is little work: past 128^3 the
       // tables together hold up the forward transform for longer than each
@@ -641,7 +671,7 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
              smoother.lists_below() && cells % kBelowBlock == 0;
     if (survey) {
       rsmoother.setup(N, box, window_mode, st_fft_[0]);
-      if (!own) rsmoother.set_lanes((int)lanes, st_fft_);
+      if (!one_stream) rsmoother.set_lanes((int)lanes, st_fft_);
       rsmoother.forward(p.random_density, nullptr);
     }
     if (listed)
@@ -653,7 +683,7 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
       }
     smoother.forward(d_delta, p.contrast_mean);
     SIFG_CUDA(cudaEventRecord(ev_forward_, st_fft_[0]));
-    for (uint32_t k = 1; !own && k < lanes; k++)
+    for (uint32_t k = 1; !one_stream && k < lanes; k++)
       SIFG_CUDA(cudaStreamWaitEvent(st_fft_[k], ev_forward_, 0));
     for (uint32_t k = 0; k + 1 < lanes && p.first_rung + k < radii.size(); k++)
       smooth_rung(p.first_rung + k);
@@ -727,22 +757,16 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
                      vids_.as<uint32_t>(), vcell_.as<uint32_t>(), st_);
   }
   R* gbuf = grow_to<R>(gbuf_, (size_t)growth_grid() * kGrowCap);
-  uint32_t* dcount = grow_to<uint32_t>(dcount_, 16);
   // The survivors' count and the growth and witness kernels' work counters
   // (the survivors' queue), zeroed together.
   uint32_t* n_surv = dcount;
   uint32_t* work = dcount + 1;
   constexpr uint32_t kWork = 3;
-  uint32_t* scan_done = dcount + 8;  // the scan's finished blocks
-  SIFG_CUDA(cudaMemsetAsync(scan_done, 0, sizeof(uint32_t), st_));
   // Gathered particles and visited cells of each rung's sphere growth.
   const size_t n_rungs = radii.size();
   unsigned long long* traffic = (unsigned long long*)grow_to<uint64_t>(traffic_, 2 * n_rungs + 2);
   SIFG_CUDA(cudaMemsetAsync(traffic, 0, (2 * n_rungs + 2) * sizeof(uint64_t), st_));
   uint32_t* counters = grow_to<uint32_t>(counters_, kCommitCounters);
-  const uint32_t nb_scan = scan_blocks(cells);
-  uint32_t* blocks = grow_to<uint32_t>(
-      blocks_, (size_t)std::max<uint64_t>(std::max<uint64_t>(nb_scan, nb_below) + 1, 1024));
 
   MeshViewT<R> mv{mesh.x,          mesh.y,          mesh.z,
                   mesh.offsets,    (int32_t)mesh.n_cells, mesh.box_length,
@@ -909,34 +933,43 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
       }
     } else {
       if (ri + lanes - 1 < radii.size()) smooth_rung(ri + lanes - 1);
-      SIFG_CUDA(cudaStreamWaitEvent(st_, ev_smoothed_[lane], 0));
     }
+    // Whether the rung's scan was made with its smoothing, and still stands;
+    // with no candidate the run's stream does not hear of the rung.
+    const bool scanned = !p.inject && ahead[lane] && mask_empty;
+    uint32_t m = 0;
+    if (scanned) {
+      const auto t_wait = clk::now();
+      SIFG_CUDA(cudaEventSynchronize(ev_smoothed_[lane]));
+      rs.count_wait_ms = ms_since(t_wait);
+      m = ((volatile uint32_t*)h_ahead)[lane];
+    }
+    if (!p.inject && !(scanned && m == 0)) SIFG_CUDA(cudaStreamWaitEvent(st_, ev_smoothed_[lane], 0));
     if (tm) tm->rung.begin(st_);
 
     // 2. Candidates, in flat order.
-    R* region_delta = nullptr;
-    uint32_t* region_flat = nullptr;
     const BelowList& bl = below[lane];
     rs.from_list = listed ? 1u : 0u;
-    if (listed) {
-      below_count_pass(bl.counts, bl.flat, nb_below, kBelowBlock, mask, blocks, h_counters_, st_);
-    } else {
-      const uint64_t slots = scan_region_slots(cells);
-      region_delta = grow_to<R>(region_delta_, slots);
-      region_flat = grow_to<uint32_t>(region_flat_, slots);
-      // Refined, the candidates are every cell at or below the threshold
-      // (the minima are found on the refinement's field, below).
-      scan_fused_pass(field, mask, cells, threshold, blocks, h_counters_, region_delta, region_flat,
-                      st_, N, minima && !gaussian, scan_done);
-      // The field's last reader: a later rung may smooth into it
-      // (refined, the placing reads it again: recorded after that).
-      if (!gaussian) SIFG_CUDA(cudaEventRecord(ev_scanned_[lane], st_));
+    if (!scanned) {
+      scan_buffers(lane);
+      if (listed) {
+        below_count_pass(bl.counts, bl.flat, nb_below, kBelowBlock, mask, blocks[lane], h_counters_,
+                         st_);
+      } else {
+        // Refined, the candidates are every cell at or below the threshold
+        // (the minima are found on the refinement's field, below).
+        scan_fused_pass(field, mask, cells, threshold, blocks[lane], h_counters_, region_delta[lane],
+                        region_flat[lane], st_, N, minima && !gaussian, scan_done + lane);
+        // The field's last reader: a later rung may smooth into it
+        // (refined, the placing reads it again: recorded after that).
+        if (!gaussian) SIFG_CUDA(cudaEventRecord(ev_scanned_[lane], st_));
+      }
+      // The total goes straight to pinned host memory.
+      const auto t_wait = clk::now();
+      SIFG_CUDA(cudaStreamSynchronize(st_));
+      rs.count_wait_ms = ms_since(t_wait);
+      m = h_counters_[0];
     }
-    // The total goes straight to pinned host memory.
-    const auto t_wait = clk::now();
-    SIFG_CUDA(cudaStreamSynchronize(st_));
-    rs.count_wait_ms = ms_since(t_wait);
-    uint32_t m = h_counters_[0];
     rs.n_candidates = m;
     R* cdelta = nullptr;
     uint32_t* cflat = nullptr;
@@ -947,7 +980,7 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
         // one, or the smoothing's.
         cdelta = grow_to<R>(cand_delta_, m);
         cflat = grow_to<uint32_t>(cand_flat_, m);
-        scan_compact(blocks, cells, region_delta, region_flat, cdelta, cflat, st_);
+        scan_compact(blocks[lane], cells, region_delta[lane], region_flat[lane], cdelta, cflat, st_);
         R* gf = gfields[lane];
         if (p.inject)
           SIFG_CUDA(cudaMemcpyAsync(gf, p.inject + inj_k++ * cells, cells * sizeof(R), inj_kind, st_));
@@ -989,14 +1022,16 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
       cdelta = (R*)h_delta_;
       cflat = grow_to<uint32_t>(cand_flat_, m);
       if constexpr (sizeof(R) == 4)
-        below_write_pass(bl.counts, bl.delta, bl.flat, nb_below, kBelowBlock, mask, blocks, cdelta,
-                         cflat, st_);
+        below_write_pass(bl.counts, bl.delta, bl.flat, nb_below, kBelowBlock, mask, blocks[lane],
+                         cdelta, cflat, st_);
       // The list's last reader: the next rung but one may smooth into it.
       SIFG_CUDA(cudaEventRecord(ev_scanned_[lane], st_));
     } else {
       cdelta = (R*)h_delta_;
       cflat = grow_to<uint32_t>(cand_flat_, m);
-      scan_compact(blocks, cells, region_delta, region_flat, cdelta, cflat, st_);
+      scan_compact(blocks[lane], cells, region_delta[lane], region_flat[lane], cdelta, cflat, st_);
+      // Made ahead, the lane's next scan waits for this one's entries to be read.
+      if (scanned) SIFG_CUDA(cudaEventRecord(ev_scanned_[lane], st_));
     }
     SIFG_CUDA(cudaEventRecord(ev_cand_, st_));
 
@@ -1120,10 +1155,10 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
     if (small) {
       if (ng < 3) ng = 1;
       if (ng > 16) ng = 16;
-      // Room for every survivor; a catalogue that moved takes its index anew.
-      const void* was = vids_.ptr;
+      // Room for every survivor; an index that had to grow is built anew.
+      const size_t had = vids_.bytes;
       ensure_cat(n_voids + m);
-      if (vids_.ptr != was)
+      if (vids_.bytes != had)
         build_void_index(cat_x_.as<R>(), cat_y_.as<R>(), cat_z_.as<R>(), n_voids, box, vstart,
                          vids_.as<uint32_t>(), vcell_.as<uint32_t>(), st_);
       vv = void_view();
@@ -1215,6 +1250,7 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
         return kErrInvalid;
       }
       const uint32_t n_acc = h_counters_[1], n_removed = h_counters_[2];
+      if (n_acc) mask_empty = false;
       rs.n_mismatched = h_counters_[6];
       std::memcpy(&max_r, &h_counters_[4], sizeof(R));
       if (n_removed) {
@@ -1254,6 +1290,7 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
       rs.n_witness = h_counters_[8];
       rs.n_mismatched = h_counters_[9];
       if (h_counters_[0]) {
+        mask_empty = false;
         R rmax;
         std::memcpy(&rmax, sizeof(R) == 4 ? (void*)&h_counters_[3] : (void*)&h_counters_[6], sizeof(R));
         if (rmax > max_r) max_r = rmax;
@@ -1317,6 +1354,7 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
     rs.n_witness = h_counters_[8];
     rs.n_mismatched = h_counters_[9];
     if (n_acc) {
+      mask_empty = false;
       R rmax;
       std::memcpy(&rmax, sizeof(R) == 4 ? (void*)&h_counters_[3] : (void*)&h_counters_[6], sizeof(R));
       if (rmax > max_r) max_r = rmax;

@@ -183,12 +183,14 @@ class Engine {
   template <class R>
   SmootherT<R>& rsmoother_for();
   int host_threads = 0;
+  // One of a batch's engines: it smooths on one lane (the others fill the GPU).
+  bool in_batch = false;
 
  private:
   int device_;
   cudaStream_t st_ = 0;
   static constexpr int kLanes = Smoother::kLanes;  // rungs smoothed at once
-  DevBuf field_[kLanes], mask_, cand_delta_, cand_flat_, blocks_, rank_, rank_slots_;
+  DevBuf field_[kLanes], mask_, cand_delta_, cand_flat_, blocks_[kLanes], rank_, rank_slots_;
   DevBuf surv_cand_, surv_flat_, scx_, scy_, scz_, sr_, sreason_, state_a_, state_b_, acc_;
   DevBuf commit_bar_;  // the cooperative commit's grid barrier and its report
   DevBuf counters_, dcount_, sgrid_start_, sgrid_ids_, sgrid_cellof_, sgrid_pack_, sgrid_rank_;
@@ -202,7 +204,7 @@ class Engine {
   // offset lengths.
   DevBuf gfield_[kLanes], cand_delta2_, cand_flat2_, cand_off_, cand_off2_, keep_, soff_;
   DevBuf tables_, gtables_;  // the rungs' radial tables (and the refinement's)
-  DevBuf tpl_, gbuf_, traffic_, region_delta_, region_flat_;
+  DevBuf tpl_, gbuf_, traffic_, region_delta_[kLanes], region_flat_[kLanes];
   // A survey: the randoms' smoothed fields, the footprint (and the closing's
   // other mask, the marked count), the randoms' template, the voids' observed
   // fractions.

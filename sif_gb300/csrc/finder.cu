@@ -231,6 +231,8 @@ __global__ void scan_compact_kernel(const uint32_t* __restrict__ offsets, uint32
   }
 }
 
+bool scan_is_one_launch(uint64_t n_cells) { return scan_blocks(n_cells) <= kScanTail; }
+
 uint64_t scan_region_slots(uint64_t n_cells) { return (uint64_t)scan_blocks(n_cells) * kScanChunk; }
 
 // The candidates from a below-threshold list made by the smoothing (blocks
@@ -306,7 +308,7 @@ void scan_fused_pass(const R* field, const uint32_t* mask, uint64_t n_cells, R t
                      uint32_t* region_flat, cudaStream_t st, uint32_t grid_n, bool minima,
                      uint32_t* done) {
   const uint32_t nb = scan_blocks(n_cells);
-  const bool tail = nb <= kScanTail;
+  const bool tail = scan_is_one_launch(n_cells);
   scan_regions_kernel<R><<<nb, kScanT, 0, st>>>(field, mask, n_cells, threshold, block_counts,
                                                 region_delta, region_flat, grid_n, minima,
                                                 tail ? done : nullptr, d_count);

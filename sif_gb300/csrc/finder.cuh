@@ -157,6 +157,7 @@ using Survivors = SurvivorsT<float>;
 // done: a device word, zero, left zero.
 uint32_t scan_blocks(uint64_t n_cells);
 uint64_t scan_region_slots(uint64_t n_cells);
+bool scan_is_one_launch(uint64_t n_cells);  // its counts scanned by its own last block
 template <class R>
 void scan_fused_pass(const R* field, const uint32_t* mask, uint64_t n_cells, R threshold,
                      uint32_t* block_counts, uint32_t* d_count, R* region_delta,

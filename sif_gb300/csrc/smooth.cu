@@ -36,100 +36,52 @@ namespace sifg {
     if (r_ != CUFFT_SUCCESS) throw ::sifg::CudaError{cudaErrorUnknown, #call};  \
   } while (0)
 
-__device__ __forceinline__ float filter_factor(uint32_t ix, uint32_t iy, uint32_t iz, uint32_t n,
-                                               const float* __restrict__ lut,
-                                               const float* __restrict__ win, float norm) {
-  const uint32_t h = n >> 1;
-  const int32_t kx = ix > h ? (int32_t)ix - (int32_t)n : (int32_t)ix;
-  const int32_t ky = iy > h ? (int32_t)iy - (int32_t)n : (int32_t)iy;
-  const uint32_t k2 = (uint32_t)(kx * kx + ky * ky) + iz * iz;
-  float s = __ldg(lut + k2) * norm;
-  if (win) s = s * __ldg(win + ix) * __ldg(win + iy) * __ldg(win + iz);
-  return s;
-}
+// The factor is even in kx and ky, so a thread finds it once, at (|kx|, |ky|,
+// kz), and applies it to the up to four modes that share it: the table by
+// |k|^2 is a gather whose lanes fall in as many cache lines, and with a gather
+// a mode it was what the kernel waited on. (256^3: 33 us a pass of 135 MB with
+// a gather a mode, 105 in double, where four products a mode cost more than
+// the modes' own two.) Product by product the factor is the one a mode alone
+// would have found.
+template <class R>
+struct Mode;
+template <>
+struct Mode<float> {
+  using T = float2;
+};
+template <>
+struct Mode<double> {
+  using T = double2;
+};
 
-// Two modes per 16-byte load and store (an odd grid's last mode on its own),
-// four loads in flight per thread before any is used: the kernel is bound by
-// the latency of its loads. Index is 32-bit whenever the count allows.
-template <class Index>
-__device__ __forceinline__ float4 filter_pair(float4 v, Index j, uint32_t n, uint32_t zd,
-                                              const float* __restrict__ lut,
-                                              const float* __restrict__ win, float norm) {
-  const Index i = 2 * j;
-  const Index row = i / zd;
-  const uint32_t iz = (uint32_t)(i - row * zd);
-  const uint32_t iy = (uint32_t)(row % n), ix = (uint32_t)(row / n);
-  const float s0 = filter_factor(ix, iy, iz, n, lut, win, norm);
-  float s1;
-  if (iz + 1 < zd) {
-    s1 = filter_factor(ix, iy, iz + 1, n, lut, win, norm);
-  } else {
-    const uint32_t iy1 = iy + 1 == n ? 0u : iy + 1;
-    s1 = filter_factor(iy1 == 0 ? ix + 1 : ix, iy1, 0, n, lut, win, norm);
-  }
-  return make_float4(v.x * s0, v.y * s0, v.z * s1, v.w * s1);
-}
-
-constexpr int kFilterUnroll = 4;
-
-template <class Index>
-__global__ void __launch_bounds__(256) filter_kernel(const float4* __restrict__ spec,
-                                                     float4* __restrict__ out, uint32_t n,
-                                                     const float* __restrict__ lut,
-                                                     const float* __restrict__ win, float norm) {
-  const uint32_t zd = n / 2 + 1;
-  const Index pairs = (Index)n * n * zd / 2;
-  const Index stride = (Index)gridDim.x * blockDim.x;
-  for (Index j0 = (Index)blockIdx.x * blockDim.x + threadIdx.x; j0 < pairs;
-       j0 += kFilterUnroll * stride) {
-    float4 v[kFilterUnroll];
+template <class R>
+__global__ void __launch_bounds__(256) filter_kernel(const typename Mode<R>::T* __restrict__ spec,
+                                                     typename Mode<R>::T* __restrict__ out, uint32_t n,
+                                                     const R* __restrict__ lut,
+                                                     const R* __restrict__ win, R norm) {
+  using M = typename Mode<R>::T;
+  const uint32_t zd = n / 2 + 1, half = n / 2 + 1;  // |k| from 0 to n / 2 on every axis
+  const uint32_t ix = blockIdx.y, jx = ix == 0 || 2 * ix == n ? ix : n - ix;
+  const R wx = win ? __ldg(win + ix) : R(1);
+  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < half * zd; t += gridDim.x * blockDim.x) {
+    const uint32_t iy = t / zd, iz = t - iy * zd;
+    const uint32_t jy = iy == 0 || 2 * iy == n ? iy : n - iy;
+    const size_t at[4] = {(size_t)(ix * n + iy) * zd + iz, (size_t)(ix * n + jy) * zd + iz,
+                          (size_t)(jx * n + iy) * zd + iz, (size_t)(jx * n + jy) * zd + iz};
+    const bool on[4] = {true, jy != iy, jx != ix, jx != ix && jy != iy};
+    M v[4];
 #pragma unroll
-    for (int u = 0; u < kFilterUnroll; u++) {
-      const Index j = j0 + u * stride;
-      if (j < pairs) v[u] = __ldg(spec + j);
-    }
+    for (int k = 0; k < 4; k++)
+      if (on[k]) v[k] = __ldg(spec + at[k]);
+    R s = __ldg(lut + (ix * ix + iy * iy + iz * iz)) * norm;
+    if (win) s = s * wx * __ldg(win + iy) * __ldg(win + iz);
 #pragma unroll
-    for (int u = 0; u < kFilterUnroll; u++) {
-      const Index j = j0 + u * stride;
-      if (j < pairs) out[j] = filter_pair(v[u], j, n, zd, lut, win, norm);
-    }
-  }
-  const Index total = (Index)n * n * zd;
-  if ((total & 1) && blockIdx.x == 0 && threadIdx.x == 0) {
-    const float s = filter_factor(n - 1, n - 1, zd - 1, n, lut, win, norm);
-    const float2 v = ((const float2*)spec)[total - 1];
-    ((float2*)out)[total - 1] = make_float2(v.x * s, v.y * s);
-  }
-}
-
-// The FP64 form's filter: one mode per 16-byte load, four in flight.
-__global__ void __launch_bounds__(256) filter_kernel_f64(const double2* __restrict__ spec,
-                                                         double2* __restrict__ out, uint32_t n,
-                                                         const double* __restrict__ lut,
-                                                         const double* __restrict__ win,
-                                                         double norm) {
-  const uint32_t zd = n / 2 + 1, h = n >> 1;
-  const uint64_t total = (uint64_t)n * n * zd;
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < total;
-       i0 += kFilterUnroll * stride) {
-    double2 v[kFilterUnroll];
-#pragma unroll
-    for (int u = 0; u < kFilterUnroll; u++)
-      if (i0 + u * stride < total) v[u] = __ldg(spec + i0 + u * stride);
-#pragma unroll
-    for (int u = 0; u < kFilterUnroll; u++) {
-      const uint64_t i = i0 + u * stride;
-      if (i >= total) continue;
-      const uint64_t row = i / zd;
-      const uint32_t iz = (uint32_t)(i - row * zd);
-      const uint32_t iy = (uint32_t)(row % n), ix = (uint32_t)(row / n);
-      const int32_t kx = ix > h ? (int32_t)ix - (int32_t)n : (int32_t)ix;
-      const int32_t ky = iy > h ? (int32_t)iy - (int32_t)n : (int32_t)iy;
-      const uint32_t k2 = (uint32_t)(kx * kx + ky * ky) + iz * iz;
-      double s = __ldg(lut + k2) * norm;
-      if (win) s = s * __ldg(win + ix) * __ldg(win + iy) * __ldg(win + iz);
-      out[i] = make_double2(v[u].x * s, v[u].y * s);
+    for (int k = 0; k < 4; k++) {
+      if (!on[k]) continue;
+      M o;
+      o.x = v[k].x * s;
+      o.y = v[k].y * s;
+      out[at[k]] = o;
     }
   }
 }
@@ -795,6 +747,8 @@ template <class R>
 static void destroy_plans(typename SmootherT<R>::Plans& p) {
   if (p.r2c) cufftDestroy(p.r2c);
   if (p.c2r) cufftDestroy(p.c2r);
+  for (cufftHandle h : p.lane)
+    if (h) cufftDestroy(h);
   if (p.twiddles) cudaFree(p.twiddles);
 }
 
@@ -882,7 +836,6 @@ void SmootherT<R>::setup(uint32_t n_, R box_, int window_mode_, cudaStream_t st)
       if (plan_work) SIFG_CUFFT(cufftSetWorkArea(h, area.ptr));
     }
     stream = st;
-    bound_lane = 0;
   }
   box = box_;
   window_mode = window_mode_;
@@ -909,11 +862,17 @@ void SmootherT<R>::setup(uint32_t n_, R box_, int window_mode_, cudaStream_t st)
 
 template <class R>
 void SmootherT<R>::set_lanes(int lanes, const cudaStream_t* streams) {
+  auto it = std::find_if(plans.begin(), plans.end(), [&](const Plans& p) { return p.n == n; });
   for (int k = 1; k < lanes; k++) {
     Lane& l = extra[k - 1];
+    size_t need = plan_work;
+    if (!it->lane[k - 1]) it->lane[k - 1] = make_plan(n, sizeof(R) == 8 ? CUFFT_Z2D : CUFFT_C2R, &need);
+    if (need > it->work) it->work = need;
     l.st = streams[k];
+    l.c2r = it->lane[k - 1];
     l.work.ensure((uint64_t)n * n * (n / 2 + 1) * 2 * sizeof(R));
-    if (plan_work) l.area.ensure(plan_work);
+    SIFG_CUFFT(cufftSetStream(l.c2r, l.st));
+    if (it->work) SIFG_CUFFT(cufftSetWorkArea(l.c2r, l.area.ensure(it->work)));
   }
 }
 
@@ -956,17 +915,14 @@ void SmootherT<double>::forward(const double* grid, const double* mean) {
   SIFG_CUFFT(cufftExecD2Z(plan_r2c, (cufftDoubleReal*)grid, (cufftDoubleComplex*)spectrum.ptr));
 }
 
-static void launch_filter(const SmootherT<float>& s, int filter, float norm, const float* lut,
-                          const DevBuf& work, cudaStream_t st) {
-  const uint64_t modes = (uint64_t)s.n * s.n * (s.n / 2 + 1);
-  const float* w = (s.window_mode && filter != kFilterNone) ? s.win.as<float>() : nullptr;
-  const unsigned grd = grid_for(modes / 2 + 1, 256, 152u * 8u);
-  if (modes < (1ull << 32))
-    filter_kernel<uint32_t><<<grd, 256, 0, st>>>(s.spectrum.as<float4>(), work.as<float4>(), s.n,
-                                                 lut, w, norm);
-  else
-    filter_kernel<uint64_t><<<grd, 256, 0, st>>>(s.spectrum.as<float4>(), work.as<float4>(), s.n,
-                                                 lut, w, norm);
+template <class R>
+static void launch_filter(const SmootherT<R>& s, int filter, R norm, const R* lut, const DevBuf& work,
+                          cudaStream_t st) {
+  using M = typename Mode<R>::T;
+  const R* w = (s.window_mode && filter != kFilterNone) ? s.win.template as<R>() : nullptr;
+  const uint32_t half = s.n / 2 + 1;
+  filter_kernel<R><<<dim3(grid_for((uint64_t)half * half, 256), half), 256, 0, st>>>(
+      s.spectrum.template as<M>(), work.as<M>(), s.n, lut, w, norm);
 }
 
 // The three passes of the n = 512 inverse transform, on the smoother's stream.
@@ -1085,14 +1041,6 @@ const float* SmootherT<R>::factor_table(int filter, R r, R sigma) {
   }
 }
 
-static void launch_filter(const SmootherT<double>& s, int filter, double norm, const double* lut,
-                          const DevBuf& work, cudaStream_t st) {
-  const uint64_t modes = (uint64_t)s.n * s.n * (s.n / 2 + 1);
-  const double* w = (s.window_mode && filter != kFilterNone) ? s.win.as<double>() : nullptr;
-  filter_kernel_f64<<<grid_for(modes, 256, 152u * 8u), 256, 0, st>>>(
-      s.spectrum.as<double2>(), work.as<double2>(), s.n, lut, w, norm);
-}
-
 template <class R>
 void SmootherT<R>::smooth(int filter, R r, R sigma, R* out, KernelTimer* timer,
                           const BelowList* below, int lane, const R* table) {
@@ -1110,21 +1058,16 @@ void SmootherT<R>::smooth(int filter, R r, R sigma, R* out, KernelTimer* timer,
   }
   const cudaStream_t st = lane ? extra[lane - 1].st : stream;
   const DevBuf& lwork = lane ? extra[lane - 1].work : work;
-  if (lane != bound_lane) {
-    const DevBuf& larea = lane ? extra[lane - 1].area : area;
-    SIFG_CUFFT(cufftSetStream(plan_c2r, st));
-    if (plan_work) SIFG_CUFFT(cufftSetWorkArea(plan_c2r, larea.ptr));
-    bound_lane = lane;
-  }
+  const cufftHandle plan = lane ? extra[lane - 1].c2r : plan_c2r;
   if (!table) table = tables(filter, &r, &sigma, 1, lane ? extra[lane - 1].lut : lut, st);
   if (timer) timer->begin(st);
   launch_filter(*this, filter, norm, table, lwork, st);
   SIFG_LAUNCH_CHECK();
   if (timer) timer->end(st);
   if (sizeof(R) == 8)
-    SIFG_CUFFT(cufftExecZ2D(plan_c2r, (cufftDoubleComplex*)lwork.ptr, (cufftDoubleReal*)out));
+    SIFG_CUFFT(cufftExecZ2D(plan, (cufftDoubleComplex*)lwork.ptr, (cufftDoubleReal*)out));
   else
-    SIFG_CUFFT(cufftExecC2R(plan_c2r, (cufftComplex*)lwork.ptr, (cufftReal*)out));
+    SIFG_CUFFT(cufftExecC2R(plan, (cufftComplex*)lwork.ptr, (cufftReal*)out));
 }
 
 template <class R>

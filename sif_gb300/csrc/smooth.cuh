@@ -44,6 +44,7 @@ struct SmootherT {
   // time. A plan made with its own area would allocate it, and destroying
   // it free it, a device-wide wait that stalls every other engine.
   DevBuf area;
+  static constexpr int kLanes = 4;  // smoothings at once, at most
   // Plans by grid size, kept between runs: at most kPlanCache sizes, oldest
   // out; a batch of boxes of many sizes keeps them all.
   static constexpr int kPlanCache = 64;
@@ -52,19 +53,18 @@ struct SmootherT {
     cufftHandle r2c, c2r;
     size_t work = 0;           // bytes of work area the two need
     void* twiddles = nullptr;  // the float form's own inverse at n = 512: its tables (no plans)
+    cufftHandle lane[kLanes - 1] = {};  // the further lanes' inverses, made when first wanted
   };
   size_t plan_work = 0;  // the current plans' need
   // Further lanes, for several smoothings of the one spectrum at once: each a
-  // stream with its own transform input, work area and table (lane 0 is
-  // `stream` with work, area and lut). The inverse plan is bound to the lane it
-  // runs on next (a launch takes the stream and area it is bound to then).
-  static constexpr int kLanes = 4;
+  // stream with its own inverse plan, transform input, work area and table
+  // (lane 0 is `stream` with plan_c2r, work, area and lut).
   struct Lane {
     cudaStream_t st = 0;
+    cufftHandle c2r = 0;
     DevBuf work, area, lut;
   };
   Lane extra[kLanes - 1];
-  int bound_lane = 0;
   void set_lanes(int lanes, const cudaStream_t* streams);  // after setup
   const void* twiddles = nullptr;
   std::vector<Plans> plans;
