@@ -758,6 +758,13 @@ void prefilter(const uint32_t* cand_flat, uint32_t m, const uint32_t* mask, Void
 // exactly: the same distances, the same bin_of, the same classification.
 constexpr int kGrowT = 256;
 constexpr int kGrowWarps = kGrowT / 32;
+// The survey growth's CTA: its tables of 2,048 bins let two CTAs an SM in
+// whatever their size, and two of 512 threads keep the SM's registers full.
+// Survey 96^3, data and randoms on their own meshes: 10.2 to 9.6 ms a
+// search. The other per-CTA kernels stay at 256, four an SM: wider CTAs gave
+// nothing where survivors are few and cost the weighted 150^3 search 13%
+// where they are not (more threads at each barrier and sort step).
+constexpr int kSurveyT = 512;
 constexpr uint32_t kMaxBins = 2048;
 constexpr uint32_t kSmemBuf = 2048;
 constexpr int kWalkUnroll = 4;  // particle loads in flight per lane
@@ -799,7 +806,7 @@ __device__ __forceinline__ unsigned long long block_sum_u64(unsigned long long v
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
   __syncthreads();
   unsigned long long t = 0;
-  for (int w = 0; w < kGrowWarps; w++) t += red[w];
+  for (unsigned w = 0; w < blockDim.x >> 5; w++) t += red[w];
   __syncthreads();
   return t;
 }
@@ -814,13 +821,13 @@ __device__ __forceinline__ void block_sum2_u64(unsigned long long& a, unsigned l
   __syncthreads();
   if ((threadIdx.x & 31) == 0) {
     red[threadIdx.x >> 5] = a;
-    red[kGrowWarps + (threadIdx.x >> 5)] = b;
+    red[(blockDim.x + threadIdx.x) >> 5] = b;
   }
   __syncthreads();
   unsigned long long ta = 0, tb = 0;
-  for (int w = 0; w < kGrowWarps; w++) {
+  for (unsigned w = 0; w < blockDim.x >> 5; w++) {
     ta += red[w];
-    tb += red[kGrowWarps + w];
+    tb += red[(blockDim.x >> 5) + w];
   }
   __syncthreads();
   a = ta;
@@ -870,7 +877,7 @@ __device__ __forceinline__ int block_max_int(int v, int* red) {
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
   __syncthreads();
   int t = red[0];
-  for (int w = 1; w < kGrowWarps; w++) t = max(t, red[w]);
+  for (unsigned w = 1; w < blockDim.x >> 5; w++) t = max(t, red[w]);
   __syncthreads();
   return t;
 }
@@ -887,7 +894,7 @@ template <class R>
 __device__ void bitonic_sort(R* buf, uint32_t p) {
   for (uint32_t k = 2; k <= p; k <<= 1) {
     for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-      for (uint32_t i = threadIdx.x; i < p; i += kGrowT) {
+      for (uint32_t i = threadIdx.x; i < p; i += blockDim.x) {
         const uint32_t l = i ^ j;
         if (l > i) {
           const R a = buf[i], b = buf[l];
@@ -918,7 +925,7 @@ __device__ __forceinline__ void walk_cells(const MeshViewT<R>& mesh, const Templ
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   // A CTA's warps share the template's chunks; a warp on its own takes all.
   const uint32_t first = whole_warp ? 0u : warp * 32;
-  const uint32_t step = whole_warp ? 32u : kGrowWarps * 32;
+  const uint32_t step = whole_warp ? 32u : blockDim.x;
   for (uint32_t c0 = first; c0 < tpl.count; c0 += step) {
     const uint32_t i = c0 + lane;
     CellRange<R> c{0, 0, 0.f, 0.f, 0.f, 0};
@@ -1817,7 +1824,7 @@ template <class R>
 __device__ void bitonic_sort_pairs(R* key, long long* val, uint32_t p) {
   for (uint32_t k = 2; k <= p; k <<= 1) {
     for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-      for (uint32_t i = threadIdx.x; i < p; i += kGrowT) {
+      for (uint32_t i = threadIdx.x; i < p; i += blockDim.x) {
         const uint32_t l = i ^ j;
         if (l > i) {
           const R a = key[i], b = key[l];
@@ -1839,21 +1846,18 @@ __device__ void bitonic_sort_pairs(R* key, long long* val, uint32_t p) {
 // v[k] = v[k] + v[k + 1] + ... + v[p - 1], in place, by the block: a
 // contiguous chunk per thread, the chunks' totals combined by warp 0.
 __device__ void suffix_sums(long long* v, uint32_t p, long long* tsum) {
-  static_assert(kGrowT == 256, "warp 0 combines 8 chunk totals per lane");
   const unsigned lane = threadIdx.x & 31u;
-  const uint32_t per = (p + kGrowT - 1) / kGrowT;
+  const uint32_t per = (p + blockDim.x - 1) / blockDim.x;
   const uint32_t a = min(p, threadIdx.x * per), e = min(p, a + per);
   long long t = 0;
   for (uint32_t k = a; k < e; k++) t += v[k];
   tsum[threadIdx.x] = t;
   __syncthreads();
   if (threadIdx.x < 32) {
-    long long loc[8], ls = 0;
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-      loc[j] = tsum[threadIdx.x * 8 + j];
-      ls += loc[j];
-    }
+    const int share = blockDim.x >> 5;  // chunk totals a lane combines
+    long long* mine = tsum + threadIdx.x * share;
+    long long ls = 0;
+    for (int j = 0; j < share; j++) ls += mine[j];
     long long incl = ls;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
@@ -1861,10 +1865,10 @@ __device__ void suffix_sums(long long* v, uint32_t p, long long* tsum) {
       if (lane + d < 32) incl += y;
     }
     long long after = incl - ls;
-#pragma unroll
-    for (int j = 7; j >= 0; j--) {
-      tsum[threadIdx.x * 8 + j] = after;
-      after += loc[j];
+    for (int j = share - 1; j >= 0; j--) {
+      const long long own = mine[j];
+      mine[j] = after;
+      after += own;
     }
   }
   __syncthreads();
@@ -1876,24 +1880,28 @@ __device__ void suffix_sums(long long* v, uint32_t p, long long* tsum) {
   __syncthreads();
 }
 
+// A rung's bins only, not the most there can be: 60 KB a CTA with 2,048 of them
+// let three CTAs an SM in where the registers allow four of 256 threads.
+// Weighted 150^3 search: 5.2 to 5.1 ms.
 template <class R>
-constexpr size_t weighted_smem_bytes() {
-  return (2 * (size_t)kMaxBins + kWBuf) * sizeof(long long) + 2 * (size_t)kMaxBins * sizeof(uint32_t) +
+constexpr size_t weighted_smem_bytes(uint32_t nb) {
+  return (2 * (size_t)nb + kWBuf) * sizeof(long long) + 2 * (size_t)nb * sizeof(uint32_t) +
          kWBuf * sizeof(R);
 }
 
 template <class R>
-__global__ void __launch_bounds__(kGrowT) growth_weighted_kernel(
+__global__ void __launch_bounds__(kGrowT, 4) growth_weighted_kernel(
     MeshViewT<R> mesh, TemplateViewT<R> tpl, RungConstsT<R> rc, SurvivorsT<R> sv,
     R* __restrict__ gbuf, long long* __restrict__ gwbuf, uint32_t gcap,
     unsigned long long* __restrict__ traffic, uint8_t only, uint32_t* work) {
   extern __shared__ __align__(16) unsigned char wsm[];
+  const uint32_t nbs = (rc.nb + 1) & ~1u;    // bins of each table, even for alignment
   long long* bw = (long long*)wsm;           // weight per bin
-  long long* belw = bw + kMaxBins;           // weight inside bin b's lower edge
-  long long* pwv = belw + kMaxBins;          // a window's weights (then their suffix sums)
+  long long* belw = bw + nbs;                // weight inside bin b's lower edge
+  long long* pwv = belw + nbs;               // a window's weights (then their suffix sums)
   uint32_t* bn = (uint32_t*)(pwv + kWBuf);   // tracers per bin (sizes the windows)
-  uint32_t* beln = bn + kMaxBins;            // tracers in the bins below b
-  R* pd2 = (R*)(beln + kMaxBins);            // a window's distances
+  uint32_t* beln = bn + nbs;                 // tracers in the bins below b
+  R* pd2 = (R*)(beln + nbs);                 // a window's distances
   __shared__ unsigned long long red64[2 * kGrowWarps];
   __shared__ long long tsum[kGrowT];
   __shared__ int redi[kGrowWarps];
@@ -2117,11 +2125,12 @@ void grow_weighted(MeshViewT<R> mesh, TemplateViewT<R> tpl, RungConstsT<R> rc, S
                    unsigned long long* traffic, cudaStream_t st, KernelTimer* timer, uint8_t only,
                    uint32_t* work) {
   if (max_survivors == 0) return;
-  constexpr size_t smem = weighted_smem_bytes<R>();
+  const size_t smem = weighted_smem_bytes<R>((rc.nb + 1) & ~1u);
   thread_local bool attr = false;  // the attribute is per thread's view of the function
   if (!attr) {
     SIFG_CUDA(cudaFuncSetAttribute(growth_weighted_kernel<R>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)weighted_smem_bytes<R>(kMaxBins)));
     attr = true;
   }
   const unsigned g = max_survivors < growth_grid() ? max_survivors : growth_grid();
@@ -2169,7 +2178,7 @@ __device__ __forceinline__ long long cell_wt(const MeshViewT<R>& m, uint32_t fla
 }
 
 template <class R>
-__global__ void __launch_bounds__(kGrowT) growth_survey_kernel(
+__global__ void __launch_bounds__(kSurveyT, 2) growth_survey_kernel(
     MeshViewT<R> dm, TemplateViewT<R> dt, MeshViewT<R> rm, TemplateViewT<R> rt, RungConstsT<R> rc,
     R K, SurvivorsT<R> sv, R* __restrict__ gbuf, long long* __restrict__ gwbuf, uint32_t gcap,
     unsigned long long* __restrict__ traffic, uint32_t* work) {
@@ -2182,9 +2191,9 @@ __global__ void __launch_bounds__(kGrowT) growth_survey_kernel(
   uint32_t* bn = (uint32_t*)(pwv + kWBuf);  // data tracers per bin (sizes the windows)
   uint32_t* beln = bn + kMaxBins;           // data tracers in the bins below b
   R* pd2 = (R*)(beln + kMaxBins);           // a window's distances
-  __shared__ unsigned long long red64[2 * kGrowWarps];
-  __shared__ long long tsum[kGrowT];
-  __shared__ int redi[kGrowWarps];
+  __shared__ unsigned long long red64[2 * kSurveyT / 32];
+  __shared__ long long tsum[kSurveyT];
+  __shared__ int redi[kSurveyT / 32];
   __shared__ uint32_t collected;
   __shared__ uint32_t s_item;
 
@@ -2256,7 +2265,7 @@ __global__ void __launch_bounds__(kGrowT) growth_survey_kernel(
           nb = (uint32_t)want;
       }
       const R inv_w = fdiv((R)nb, span), bin_w = fdiv(span, (R)nb);
-      for (uint32_t b = threadIdx.x; b < nb; b += kGrowT) {
+      for (uint32_t b = threadIdx.x; b < nb; b += kSurveyT) {
         dbin[b] = 0;
         rbin[b] = 0;
         bn[b] = 0;
@@ -2352,7 +2361,7 @@ __global__ void __launch_bounds__(kGrowT) growth_survey_kernel(
         reason = kRescaleBelowRung;
         while (cursor >= 0) {
           int best = -1;
-          for (int32_t b = threadIdx.x; b <= cursor; b += kGrowT) {
+          for (int32_t b = threadIdx.x; b <= cursor; b += kSurveyT) {
             if (!(dbin[b] > 0)) continue;
             const R d_in_min = wreal<R>(dbel[b], dinv);
             const R r_in_max = wreal<R>(rbel[b] + rbin[b], rinv);
@@ -2406,7 +2415,7 @@ __global__ void __launch_bounds__(kGrowT) growth_survey_kernel(
           const uint32_t m = collected < cap ? collected : cap;
           uint32_t p2 = 1;
           while (p2 < m) p2 <<= 1;
-          for (uint32_t i = m + threadIdx.x; i < p2; i += kGrowT) {
+          for (uint32_t i = m + threadIdx.x; i < p2; i += kSurveyT) {
             kb[i] = real_inf<R>();
             vb[i] = 0;
           }
@@ -2419,7 +2428,7 @@ __global__ void __launch_bounds__(kGrowT) growth_survey_kernel(
           // randoms up to it.
           const long long d_top = dbel[b_hi] + dbin[b_hi];
           int found = -1;
-          for (uint32_t k = threadIdx.x; k < m; k += kGrowT) {
+          for (uint32_t k = threadIdx.x; k < m; k += kSurveyT) {
             const R d2 = kb[k];
             if (d2 == R(0)) continue;
             const uint32_t bi = bin_of(d2, rc2, inv_w, nb);
@@ -2472,7 +2481,7 @@ void grow_survey(MeshViewT<R> dm, TemplateViewT<R> dt, MeshViewT<R> rm, Template
   }
   const unsigned g = max_survivors < growth_grid() ? max_survivors : growth_grid();
   if (timer) timer->begin(st);
-  growth_survey_kernel<R><<<g, kGrowT, smem, st>>>(dm, dt, rm, rt, rc, K, s, gbuf, gwbuf, gcap,
+  growth_survey_kernel<R><<<g, kSurveyT, smem, st>>>(dm, dt, rm, rt, rc, K, s, gbuf, gwbuf, gcap,
                                                   traffic, work);
   SIFG_LAUNCH_CHECK();
   if (timer) timer->end(st);
@@ -3486,7 +3495,7 @@ __device__ void paint_cta(R cx, R cy, R cz, R r, uint32_t* mask, const RungConst
   const int32_t cr = (int32_t)fmul(r, inv) + 1;
   const int32_t ci = (int32_t)fmul(cx, inv), cj = (int32_t)fmul(cy, inv), ck = (int32_t)fmul(cz, inv);
   const int32_t side = 2 * cr + 1;
-  for (int32_t q = threadIdx.x; q < side * side; q += blockDim.x) {
+  for (int32_t q = threadIdx.x; q < side * side; q += kSurveyT) {
     const int32_t gx = ci + q / side - cr, gy = cj + q % side - cr;
     R ddx = fabs_(fsub(fmul((R)gx, rc.cell), cx));
     ddx = ddx > half ? fsub(rc.gbox, ddx) : ddx;
@@ -3684,7 +3693,7 @@ __global__ void __launch_bounds__(1024) compact_voids_kernel(R* cx, R* cy, R* cz
   const uint32_t n = state[kDispVoids];
   if (threadIdx.x == 0) base = 0;
   __syncthreads();
-  for (uint32_t c0 = 0; c0 < n; c0 += blockDim.x) {
+  for (uint32_t c0 = 0; c0 < n; c0 += kSurveyT) {
     const uint32_t i = c0 + threadIdx.x;
     R v[4] = {0, 0, 0, 0};
     bool keep = false;
