@@ -3495,7 +3495,7 @@ __device__ void paint_cta(R cx, R cy, R cz, R r, uint32_t* mask, const RungConst
   const int32_t cr = (int32_t)fmul(r, inv) + 1;
   const int32_t ci = (int32_t)fmul(cx, inv), cj = (int32_t)fmul(cy, inv), ck = (int32_t)fmul(cz, inv);
   const int32_t side = 2 * cr + 1;
-  for (int32_t q = threadIdx.x; q < side * side; q += kSurveyT) {
+  for (int32_t q = threadIdx.x; q < side * side; q += blockDim.x) {
     const int32_t gx = ci + q / side - cr, gy = cj + q % side - cr;
     R ddx = fabs_(fsub(fmul((R)gx, rc.cell), cx));
     ddx = ddx > half ? fsub(rc.gbox, ddx) : ddx;
@@ -3693,7 +3693,7 @@ __global__ void __launch_bounds__(1024) compact_voids_kernel(R* cx, R* cy, R* cz
   const uint32_t n = state[kDispVoids];
   if (threadIdx.x == 0) base = 0;
   __syncthreads();
-  for (uint32_t c0 = 0; c0 < n; c0 += kSurveyT) {
+  for (uint32_t c0 = 0; c0 < n; c0 += blockDim.x) {
     const uint32_t i = c0 + threadIdx.x;
     R v[4] = {0, 0, 0, 0};
     bool keep = false;
