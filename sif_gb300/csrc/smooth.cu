@@ -1,7 +1,7 @@
 // The per-rung smoothing: cuFFT R2C of the density contrast once, then per
 // radius one fused filter kernel and a cuFFT C2R -- or, for the float form on
-// a 512^3 grid, three passes of its own that fuse the filter into the first
-// (below).
+// a 512^3 grid (below) and the FP64 form on 128^3 and 256^3 (fft64.cu), three
+// passes of its own that fuse the filter into the first.
 //
 // Replaces sif__fft_grid_forward, fft_build_filter_lut,
 // sif__fft_apply_filter_smoothed and sif__fft_grid_backward
@@ -791,7 +791,13 @@ void SmootherT<R>::setup(uint32_t n_, R box_, int window_mode_, cudaStream_t st)
         plans.erase(plans.begin());
       }
       Plans p{n_, 0, 0};
-      if (!dbl && own_inverse(n_)) {
+      if (dbl && fft64_takes(n_)) {
+        const std::vector<double> t = fft64_tables(n_);
+        SIFG_CUDA(cudaMalloc(&p.twiddles, t.size() * sizeof(double)));
+        SIFG_CUDA(cudaMemcpyAsync(p.twiddles, t.data(), t.size() * sizeof(double),
+                                  cudaMemcpyHostToDevice, st));
+        SIFG_CUDA(cudaStreamSynchronize(st));
+      } else if (!dbl && own_inverse(n_)) {
         // The tables of the three-pass inverse, computed in double.
         std::vector<float2> tw(kTw512);
         auto root = [](double num, double den) {
@@ -840,8 +846,8 @@ void SmootherT<R>::setup(uint32_t n_, R box_, int window_mode_, cudaStream_t st)
   box = box_;
   window_mode = window_mode_;
   const uint64_t modes = (uint64_t)n * n * (n / 2 + 1);
-  spectrum.ensure(twiddles ? kTileWorkElems * sizeof(float2) : modes * 2 * sizeof(R));
-  work.ensure(twiddles ? kTileWorkElems * sizeof(float2) : modes * 2 * sizeof(R));
+  spectrum.ensure(twiddles && !dbl ? kTileWorkElems * sizeof(float2) : modes * 2 * sizeof(R));
+  work.ensure(twiddles && !dbl ? kTileWorkElems * sizeof(float2) : modes * 2 * sizeof(R));
   const uint32_t h = n >> 1;
   win.ensure((size_t)n * sizeof(R));
   if (window_mode) {
@@ -866,11 +872,12 @@ void SmootherT<R>::set_lanes(int lanes, const cudaStream_t* streams) {
   for (int k = 1; k < lanes; k++) {
     Lane& l = extra[k - 1];
     size_t need = plan_work;
+    l.st = streams[k];
+    l.work.ensure((uint64_t)n * n * (n / 2 + 1) * 2 * sizeof(R));
+    if (twiddles) continue;  // no plans
     if (!it->lane[k - 1]) it->lane[k - 1] = make_plan(n, sizeof(R) == 8 ? CUFFT_Z2D : CUFFT_C2R, &need);
     if (need > it->work) it->work = need;
-    l.st = streams[k];
     l.c2r = it->lane[k - 1];
-    l.work.ensure((uint64_t)n * n * (n / 2 + 1) * 2 * sizeof(R));
     SIFG_CUFFT(cufftSetStream(l.c2r, l.st));
     if (it->work) SIFG_CUFFT(cufftSetWorkArea(l.c2r, l.area.ensure(it->work)));
   }
@@ -911,6 +918,10 @@ void SmootherT<float>::forward(const float* grid, const double* mean) {
 }
 template <>
 void SmootherT<double>::forward(const double* grid, const double* mean) {
+  if (twiddles) {
+    fft64_forward(n, grid, mean, spectrum.as<double2>(), (const double*)twiddles, stream);
+    return;
+  }
   if (mean) apply_contrast(const_cast<double*>(grid), (uint64_t)n * n * n, mean, stream);
   SIFG_CUFFT(cufftExecD2Z(plan_r2c, (cufftDoubleReal*)grid, (cufftDoubleComplex*)spectrum.ptr));
 }
@@ -1047,7 +1058,7 @@ void SmootherT<R>::smooth(int filter, R r, R sigma, R* out, KernelTimer* timer,
   const double factor = (double)r * 2.0 * M_PI / (double)box;
   const double gfactor = sigma > R(0) ? (double)sigma * 2.0 * M_PI / (double)box : 0.0;
   const R norm = (R)(1.0 / ((double)n * n * n));
-  if (twiddles) {
+  if (sizeof(R) == 4 && twiddles) {
     // The own inverse reads the smoothing's factor table (built on first use)
     // or evaluates the radial factor as it applies it.
     const RadialFilter rf = radial_filter_of(filter, factor, gfactor);
@@ -1060,6 +1071,14 @@ void SmootherT<R>::smooth(int filter, R r, R sigma, R* out, KernelTimer* timer,
   const DevBuf& lwork = lane ? extra[lane - 1].work : work;
   const cufftHandle plan = lane ? extra[lane - 1].c2r : plan_c2r;
   if (!table) table = tables(filter, &r, &sigma, 1, lane ? extra[lane - 1].lut : lut, st);
+  if constexpr (sizeof(R) == 8) {
+    if (twiddles) {
+      const double* w = window_mode && filter != kFilterNone ? win.template as<double>() : nullptr;
+      fft64_inverse(n, spectrum.template as<double2>(), lwork.as<double2>(), out, table, w, norm,
+                    (const double*)twiddles, st, timer);
+      return;
+    }
+  }
   if (timer) timer->begin(st);
   launch_filter(*this, filter, norm, table, lwork, st);
   SIFG_LAUNCH_CHECK();

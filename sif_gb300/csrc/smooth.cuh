@@ -38,7 +38,7 @@ struct SmootherT {
   R box = 0;
   int window_mode = 1;
   cudaStream_t stream = 0;
-  cufftHandle plan_r2c = 0, plan_c2r = 0;  // the plans for n (unset on the own path at 512)
+  cufftHandle plan_r2c = 0, plan_c2r = 0;  // the plans for n (unset where the transforms are our own)
   DevBuf spectrum, work, lut, win;
   // The plans' work area, one for all of them: they run on `stream`, one at a
   // time. A plan made with its own area would allocate it, and destroying
@@ -52,7 +52,7 @@ struct SmootherT {
     uint32_t n;
     cufftHandle r2c, c2r;
     size_t work = 0;           // bytes of work area the two need
-    void* twiddles = nullptr;  // the float form's own inverse at n = 512: its tables (no plans)
+    void* twiddles = nullptr;  // the own transforms' tables (no plans)
     cufftHandle lane[kLanes - 1] = {};  // the further lanes' inverses, made when first wanted
   };
   size_t plan_work = 0;  // the current plans' need
@@ -93,9 +93,9 @@ struct SmootherT {
   // on top) into out (n^3 values), asynchronously on the stream.
   // below (float form): the cells at or below below->thr listed as the
   // transform writes them, where lists_below() -- else the caller scans.
-  // lane: where it runs (set_lanes; the own transforms only on 0). table: the
-  // smoothing's radial table where it is already made, or NULL (the own
-  // transforms take none).
+  // lane: where it runs (set_lanes; the float form's own transforms only on
+  // 0). table: the smoothing's radial table where it is already made, or NULL
+  // (the float form's own transforms take none).
   void smooth(int filter, R r, R sigma, R* out, KernelTimer* timer,
               const BelowList* below = nullptr, int lane = 0, const R* table = nullptr);
   // The radial tables of `count` smoothings (sigmas NULL: none on top), each
@@ -109,6 +109,18 @@ struct SmootherT {
   ~SmootherT();
 };
 using Smoother = SmootherT<float>;
+
+// The FP64 form's own transforms (fft64.cu): the sizes they take, their tables
+// (for the device), the forward of a grid (with mean set, of its contrast) and
+// the inverse of the filtered spectrum through `work`, an n^2 (n / 2 + 1) buffer
+// like the spectrum's; `timer` covers the pass that filters.
+bool fft64_takes(uint32_t n);
+std::vector<double> fft64_tables(uint32_t n);
+void fft64_forward(uint32_t n, const double* grid, const double* mean, double2* spec,
+                   const double* tab, cudaStream_t st);
+void fft64_inverse(uint32_t n, const double2* spec, double2* work, double* out, const double* lut,
+                   const double* win, double norm, const double* tab, cudaStream_t st,
+                   KernelTimer* timer);
 
 // 1 (default): the own inverse at 512 reads per-smoothing factor tables; 0:
 // it evaluates the factors as it applies them. The same bits either way.
