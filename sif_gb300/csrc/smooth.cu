@@ -197,17 +197,7 @@ __device__ __forceinline__ void dft_inv(float2 (&v)[16]) {
   }
 }
 
-// A column of 512 in shared memory: element i at col_slot(i), columns
-// kColStride slots apart (odd). The stage-to-stage exchange uses rows of
-// kColSpan slots. With these, every shared access of the transform, and the
-// 16-column row loads and stores, is free of bank conflicts.
-__host__ __device__ constexpr int col_slot(int i) { return i + (i >> 4) + 8 * (i >> 8); }
 constexpr int kColCols = 16;
-constexpr int kColWarps = 8;  // each warp transforms kColCols / kColWarps columns
-constexpr int kColSpan = 34;
-constexpr int kColStride = 551;
-static_assert(kColStride > col_slot(511) && kColStride >= 16 * kColSpan && (kColStride & 1),
-              "column layout");
 
 // Twiddle tables of the n = 512 transform, one device block:
 //   [0, 512):    W512^(j k), at k * 32 + j (j < 32, k < 16), the column pass
@@ -313,118 +303,25 @@ __device__ __forceinline__ float radial_factor(uint32_t k2, const RadialFilter& 
 
 constexpr RadialFilter kNoFilter{-1, 0.0f, 0.0f, 0.0f, 0.0f};  // a pass that applies no filter
 
-struct ColumnFilter {
-  bool on;
-  RadialFilter rf;
-  const float* win;
-  float norm, wy, wz;
-  uint32_t q;  // ky'^2 + kz^2
-  const float* tab;  // the column's factors by |kx| (257), or NULL: evaluate them
-};
-
-// The factor table of a smoothing at n = 512: entry ((|ky| * 257 + kz) * 257
-// + |kx|) holds the factor the filter pass applies to mode (kx, ky, kz) --
+// The factor table of a smoothing at n = 512: entry ((|ky| * 257 + |kx|) * 257
+// + kz) holds the factor the filter pass applies to mode (kx, ky, kz) --
 // radial_factor(k^2) * norm, then the window's three factors, in the order
-// and with the values ifft512_column computes them, so the table changes no
-// bit of the transform.
+// and with the values the pass computes them without the table, so the table
+// changes no bit of the transform. kz runs fastest: the pass's lanes hold
+// neighbouring kz.
 constexpr uint32_t kFactorSide = 257;
 __global__ void factor_table_kernel(float* __restrict__ tab, RadialFilter rf,
                                     const float* __restrict__ win, float norm) {
   constexpr uint64_t total = (uint64_t)kFactorSide * kFactorSide * kFactorSide;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t kx = (uint32_t)(i % kFactorSide);
-    const uint32_t kz = (uint32_t)((i / kFactorSide) % kFactorSide);
+    const uint32_t kz = (uint32_t)(i % kFactorSide);
+    const uint32_t kx = (uint32_t)((i / kFactorSide) % kFactorSide);
     const uint32_t ky = (uint32_t)(i / ((uint64_t)kFactorSide * kFactorSide));
     float v = radial_factor(kx * kx + (ky * ky + kz * kz), rf) * norm;
     if (win) v = v * __ldg(win + kx) * __ldg(win + ky) * __ldg(win + kz);
     tab[i] = v;
   }
-}
-
-// One warp's inverse DFT of the 512 values in `col`, in place; with a filter
-// (f.on) each value is first scaled by its filter factor.
-// With `forward` the forward DFT instead (e^{-2 pi i jk/512}), as the
-// conjugate of the inverse DFT of the conjugate.
-__device__ __forceinline__ void ifft512_column(float2* col, const float2* __restrict__ tw,
-                                               unsigned lane, const ColumnFilter& f,
-                                               bool forward) {
-  float2 v[16];
-#pragma unroll
-  for (int r = 0; r < 16; r++) {
-    v[r] = col[col_slot((int)lane + 32 * r)];
-    if (forward) v[r].y = -v[r].y;
-  }
-  if (f.on) {
-    // The factor is even in kx (the window table is built from |k|): a lane
-    // finds it for its kx < 256 and takes kx > 256 from the lane holding
-    // 512 - kx, half the evaluations. Lane 0 holds both kx = 32 r and
-    // 512 - 32 r itself, and alone finds kx = 256.
-    float lo[8];
-    float nyq = 0.f;
-    if (f.tab) {
-#pragma unroll
-      for (int r = 0; r < 8; r++) lo[r] = __ldg(f.tab + lane + 32u * r);
-      if (lane == 0) nyq = __ldg(f.tab + 256);
-    } else {
-#pragma unroll
-      for (int r = 0; r < 8; r++) {
-        const uint32_t kx = lane + 32u * r;
-        lo[r] = radial_factor(kx * kx + f.q, f.rf) * f.norm;
-        if (f.win) lo[r] = lo[r] * __ldg(f.win + kx) * f.wy * f.wz;
-      }
-      if (lane == 0) {
-        nyq = radial_factor(256u * 256u + f.q, f.rf) * f.norm;
-        if (f.win) nyq = nyq * __ldg(f.win + 256) * f.wy * f.wz;
-      }
-    }
-    const unsigned partner = (32u - lane) & 31u;
-#pragma unroll
-    for (int r = 0; r < 16; r++) {
-      float s;
-      if (r < 8) {
-        s = lo[r];
-      } else {
-        s = __shfl_sync(0xffffffffu, lo[15 - r], partner);
-        if (lane == 0) s = r == 8 ? nyq : lo[(16 - r) & 7];
-      }
-      v[r] = make_float2(v[r].x * s, v[r].y * s);
-    }
-  }
-  dft_inv(v);
-#pragma unroll
-  for (int k = 1; k < 16; k++) v[k] = cmul(v[k], __ldg(tw + k * 32 + lane));
-  __syncwarp();
-#pragma unroll
-  for (int k = 0; k < 16; k++) col[kColSpan * k + lane] = v[k];
-  __syncwarp();
-  const unsigned k1 = lane >> 1, q = lane & 1u;
-#pragma unroll
-  for (int m = 0; m < 16; m++) v[m] = col[kColSpan * k1 + q + 2 * m];
-  dft_inv(v);  // E_q[k], k < 16
-  // The radix-2 step between the pair: X[k1 + 16 k] = E_0[k] + W32^k E_1[k],
-  // X[k1 + 16 (k + 16)] = E_0[k] - W32^k E_1[k]. Lane q = 0 finishes k < 8,
-  // lane q = 1 k >= 8; each sends the half of its E it does not keep, and
-  // W32^(8 + i) = i W32^i leaves one twiddle per register for both lanes.
-#pragma unroll
-  for (int i = 0; i < 8; i++) {
-    const float2 send = q ? v[i] : v[8 + i];
-    const float2 got = make_float2(__shfl_xor_sync(0xffffffffu, send.x, 1),
-                                   __shfl_xor_sync(0xffffffffu, send.y, 1));
-    const float2 a = q ? got : v[i];          // E_0[8 q + i]
-    const float2 b = q ? cmul_i(v[8 + i]) : got;  // E_1[8 q + i] (times i for q = 1)
-    const float2 t = i == 0 ? b : cmul(b, kW32[i]);
-    v[i] = cadd(a, t);
-    v[8 + i] = csub(a, t);
-  }
-  __syncwarp();
-#pragma unroll
-  for (int i = 0; i < 8; i++) {
-    const int x = (int)k1 + 16 * (8 * (int)q + i);
-    col[col_slot(x)] = forward ? make_float2(v[i].x, -v[i].y) : v[i];
-    col[col_slot(x + 256)] = forward ? make_float2(v[8 + i].x, -v[8 + i].y) : v[8 + i];
-  }
-  __syncwarp();
 }
 
 // The work buffer between the passes holds the half spectrum in tiles of 16
@@ -435,65 +332,107 @@ __device__ __forceinline__ void ifft512_column(float2* col, const float2* __rest
 constexpr uint32_t kKzBlocks = 17;
 constexpr size_t kTileWorkElems = (size_t)512 * kKzBlocks * 512 * 16;
 
-// Where passes (1) and (2) find their columns: line `blockIdx.y`, kz block
-// `blockIdx.x`; element a of the block's column c at
-// line * line + kb * kblock + a * elem + c.
+// Where passes (1) and (2) find their columns: element a of column kz of a
+// line at line * line + kz / 16 * kblock + a * elem + kz % 16.
 struct ColumnLayout {
   uint32_t line, kblock, elem;
 };
 
-// Passes (1) and (2): the inverse FFT along one axis of 16 neighbouring kz
-// columns of one line. The tile arrives by asynchronous copies; pass (1)
-// (rf.kind >= 0) reads the spectrum (line = ky, kx along the column), scales each
-// mode by its filter factor as the transform first reads it, and writes the
-// tiles; pass (2) (line = x, ky along the column) works on the tiles in
-// place. Columns past kz = 256 (in the last CTA of a line) are neither read,
-// transformed nor written.
-__global__ void __launch_bounds__(32 * kColWarps, 3)
+// Passes (1) and (2), and the forward's ky and kx: the FFT along one axis of 16
+// columns, 32 threads a column and 16 values a thread, neighbouring lanes on
+// neighbouring kz. A thread loads its stride-32 values straight into registers
+// and stores its results straight out, 128 contiguous bytes a half-warp either
+// way; shared memory is crossed once, between the two 16-point stages, and the
+// last radix-2 step goes between lanes 16 apart. A CTA takes one line's block of
+// 16 kz; the columns of kz = 256, one a line, are taken 16 lines at a time by the
+// last CTAs.
+//
+// Memory bounds it: 1.1 GB a pass at 512^3, 166 us at the measured copy rate.
+// (With the tile staged through shared memory both ways, six crossings where
+// this has two, and a warp a column: 215 us, 259 with the filter.)
+//
+// The filter (kColTable, kColEvaluate) scales each mode as it is read: by its
+// entry in the smoothing's table, or by the factor evaluated. The forward DFT
+// (e^{-2 pi i jk/512}) is the conjugate of the inverse DFT of the conjugate.
+enum ColMode { kColInverse, kColForward, kColTable, kColEvaluate };
+constexpr unsigned kColCtas = 512 * 16 + 512 / kColCols;
+constexpr size_t kColBytes = (size_t)512 * kColCols * sizeof(float2);
+
+template <ColMode kMode>
+__global__ void __launch_bounds__(32 * kColCols, 2)
     colfft512_kernel(const float2* src, float2* dst, ColumnLayout in, ColumnLayout out,
-                     RadialFilter rf, const float* __restrict__ win, float norm,
-                     const float2* __restrict__ tw, bool forward,
-                     const float* __restrict__ ftab = nullptr) {
-  extern __shared__ float2 cols[];  // kColCols columns of kColStride slots
-  constexpr uint32_t zd = 257;
-  constexpr uint32_t kRowStep = 32 * kColWarps / kColCols;  // rows a pass of the CTA covers
-  const uint32_t kb = blockIdx.x, kz0 = kb * kColCols, line = blockIdx.y;
-  const uint32_t c = threadIdx.x % kColCols, row0 = threadIdx.x / kColCols;
-  const bool live = kz0 + c < zd;
-  if (live) {
-    const float2* p = src + (size_t)line * in.line + (size_t)kb * in.kblock + c +
-                      (size_t)row0 * in.elem;
-    const size_t step = (size_t)kRowStep * in.elem;
-#pragma unroll 8
-    for (uint32_t i = 0; i < 512 / kRowStep; i++, p += step)
-      cp_async8(cols + c * kColStride + col_slot((int)(row0 + kRowStep * i)), p);
+                     const float2* __restrict__ tw, RadialFilter rf, const float* __restrict__ win,
+                     float norm, const float* __restrict__ ftab) {
+  extern __shared__ float2 ex[];  // element e of column c at e * kColCols + c
+  const uint32_t c = threadIdx.x % kColCols, j = threadIdx.x / kColCols;
+  const bool last = blockIdx.x >= 512 * 16;
+  const uint32_t line = last ? (blockIdx.x - 512 * 16) * kColCols + c : blockIdx.x / 16;
+  const uint32_t kb = last ? 16 : blockIdx.x % 16, kz = last ? 256 : kb * 16 + c;
+  float2 v[16];
+  {
+    const float2* p = src + (size_t)line * in.line + kb * in.kblock + (kz & 15u) + (size_t)j * in.elem;
+    const size_t step = (size_t)32 * in.elem;
+#pragma unroll
+    for (int r = 0; r < 16; r++) v[r] = p[r * step];
   }
-  cp_async_wait_all();
-  __syncthreads();
-  const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-#pragma unroll 1
-  for (uint32_t w = warp; w < kColCols && kz0 + w < zd; w += kColWarps) {
-    ColumnFilter f{};
-    if (rf.kind >= 0) {
-      const uint32_t kz = kz0 + w;
-      const int32_t ks = line > 256 ? (int32_t)line - 512 : (int32_t)line;
-      const uint32_t aky = (uint32_t)(ks < 0 ? -ks : ks);
-      f = ColumnFilter{true, rf, win, norm, win ? __ldg(win + line) : 1.f,
-                       win ? __ldg(win + kz) : 1.f, (uint32_t)(ks * ks) + kz * kz,
-                       ftab ? ftab + ((size_t)aky * kFactorSide + kz) * kFactorSide : nullptr};
+  if constexpr (kMode == kColForward) {
+#pragma unroll
+    for (int r = 0; r < 16; r++) v[r].y = -v[r].y;
+  }
+  if constexpr (kMode == kColTable || kMode == kColEvaluate) {
+    const uint32_t aky = line > 256 ? 512 - line : line;
+    const uint32_t q = aky * aky + kz * kz;
+    const float* t = ftab + (size_t)aky * (kFactorSide * kFactorSide) + kz;
+    const float wy = win ? __ldg(win + line) : 1.f, wz = win ? __ldg(win + kz) : 1.f;
+#pragma unroll
+    for (int r = 0; r < 16; r++) {
+      const uint32_t kx = j + 32u * r, a = kx > 256 ? 512 - kx : kx;
+      float s;
+      if constexpr (kMode == kColTable) {
+        s = __ldg(t + a * kFactorSide);
+      } else {
+        s = radial_factor(a * a + q, rf) * norm;
+        if (win) s = s * __ldg(win + a) * wy * wz;
+      }
+      // Rounded as a product: fused into the transform's first sums it would
+      // be other bits than a mode scaled and stored.
+      v[r] = make_float2(__fmul_rn(v[r].x, s), __fmul_rn(v[r].y, s));
     }
-    ifft512_column(cols + w * kColStride, tw, lane, f, forward);
   }
+  dft_inv(v);
+#pragma unroll
+  for (int k = 1; k < 16; k++) v[k] = cmul(v[k], __ldg(tw + k * 32 + j));
+#pragma unroll
+  for (int k = 0; k < 16; k++) ex[(k * 32 + j) * kColCols + c] = v[k];
   __syncthreads();
-  if (live) {
-    float2* p = dst + (size_t)line * out.line + (size_t)kb * out.kblock + c +
-                (size_t)row0 * out.elem;
-    const size_t step = (size_t)kRowStep * out.elem;
-#pragma unroll 8
-    for (uint32_t i = 0; i < 512 / kRowStep; i++, p += step)
-      *p = cols[c * kColStride + col_slot((int)(row0 + kRowStep * i))];
+  const uint32_t k1 = j >> 1, q = j & 1u;
+#pragma unroll
+  for (int m = 0; m < 16; m++) v[m] = ex[(k1 * 32 + q + 2 * m) * kColCols + c];
+  dft_inv(v);  // E_q[k], k < 16
+  // The radix-2 step between the two threads: X[k1 + 16 k] = E_0[k] + W32^k
+  // E_1[k], X[k1 + 16 (k + 16)] = E_0[k] - W32^k E_1[k]. q = 0 finishes k < 8,
+  // q = 1 k >= 8; each sends the half of its E it does not keep, and
+  // W32^(8 + i) = i W32^i leaves one twiddle per register for both.
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    const float2 send = q ? v[i] : v[8 + i];
+    const float2 got = make_float2(__shfl_xor_sync(0xffffffffu, send.x, kColCols),
+                                   __shfl_xor_sync(0xffffffffu, send.y, kColCols));
+    const float2 a = q ? got : v[i];              // E_0[8 q + i]
+    const float2 b = q ? cmul_i(v[8 + i]) : got;  // E_1[8 q + i] (times i for q = 1)
+    const float2 t = i == 0 ? b : cmul(b, kW32[i]);
+    v[i] = cadd(a, t);
+    v[8 + i] = csub(a, t);
+  }
+  float2* p = dst + (size_t)line * out.line + kb * out.kblock + (kz & 15u) +
+              (size_t)(k1 + 128 * q) * out.elem;
+#pragma unroll
+  for (int i = 0; i < 16; i++) {
+    const float2 o = kMode == kColForward ? make_float2(v[i].x, -v[i].y) : v[i];
+    p[(size_t)(i < 8 ? 16 * i : 256 + 16 * (i - 8)) * out.elem] = o;
   }
 }
+static_assert(2 * kColCols == 32, "a column's thread pairs lie in one warp");
 
 // Pass (3): 16 rows of 257 modes per CTA, a half-warp per row. With Z the
 // row's modes (the imaginary parts of Z[0] and Z[256] taken as zero, as a
@@ -944,13 +883,19 @@ static void launch_filter(const SmootherT<R>& s, int filter, R norm, const R* lu
 constexpr ColumnLayout kTilesByLine{kKzBlocks * 512 * kColCols, 512 * kColCols, kColCols};
 constexpr ColumnLayout kTilesByRow{kColCols, 512 * kColCols, kKzBlocks * 512 * kColCols};
 
-static void set_column_smem() {
-  thread_local bool attr = false;  // set once per thread
+template <ColMode kMode>
+static void launch_columns(const SmootherT<float>& s, const DevBuf& src, const DevBuf& dst,
+                           ColumnLayout in, ColumnLayout out, const RadialFilter& rf = kNoFilter,
+                           const float* win = nullptr, float norm = 1.f, const float* ftab = nullptr) {
+  thread_local bool attr = false;  // the attribute is per thread's view of the function
   if (!attr) {
-    SIFG_CUDA(cudaFuncSetAttribute(colfft512_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)(kColCols * kColStride * sizeof(float2))));
+    SIFG_CUDA(cudaFuncSetAttribute(colfft512_kernel<kMode>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)kColBytes));
     attr = true;
   }
+  colfft512_kernel<kMode><<<kColCtas, 32 * kColCols, kColBytes, s.stream>>>(
+      src.as<float2>(), dst.as<float2>(), in, out, (const float2*)s.twiddles, rf, win, norm, ftab);
+  SIFG_LAUNCH_CHECK();
 }
 
 // The float form's forward transform at n = 512: the R2C along z into the
@@ -958,20 +903,11 @@ static void set_column_smem() {
 // spectrum's tiles.
 static void launch_forward512(const SmootherT<float>& s, const float* grid, const double* mean) {
   constexpr uint32_t N = 512;
-  set_column_smem();
-  const size_t smem = (size_t)kColCols * kColStride * sizeof(float2);
-  const float2* tw = (const float2*)s.twiddles;
   r2c512_rows_kernel<<<N * N / kRowsPerCta, 16 * kRowsPerCta, 0, s.stream>>>(
-      grid, s.work.as<float2>(), tw, mean);
+      grid, s.work.as<float2>(), (const float2*)s.twiddles, mean);
   SIFG_LAUNCH_CHECK();
-  colfft512_kernel<<<dim3(kKzBlocks, N), 32 * kColWarps, smem, s.stream>>>(
-      s.work.as<float2>(), s.work.as<float2>(), kTilesByLine, kTilesByLine, kNoFilter, nullptr, 1.f,
-      tw, true);
-  SIFG_LAUNCH_CHECK();
-  colfft512_kernel<<<dim3(kKzBlocks, N), 32 * kColWarps, smem, s.stream>>>(
-      s.work.as<float2>(), s.spectrum.as<float2>(), kTilesByRow, kTilesByLine, kNoFilter, nullptr,
-      1.f, tw, true);
-  SIFG_LAUNCH_CHECK();
+  launch_columns<kColForward>(s, s.work, s.work, kTilesByLine, kTilesByLine);
+  launch_columns<kColForward>(s, s.work, s.spectrum, kTilesByRow, kTilesByLine);
 }
 
 // The timer, begun by the caller, ends after pass (1): the filter's kernel.
@@ -981,21 +917,14 @@ static void launch_inverse512(const SmootherT<float>& s, int filter, const Radia
                               const float* ftab) {
   constexpr uint32_t N = 512;
   const float* w = (s.window_mode && filter != kFilterNone) ? s.win.as<float>() : nullptr;
-  const size_t smem = (size_t)kColCols * kColStride * sizeof(float2);
-  set_column_smem();
-  const float2* tw = (const float2*)s.twiddles;
-  const dim3 grid(kKzBlocks, N);
-  colfft512_kernel<<<grid, 32 * kColWarps, smem, s.stream>>>(
-      s.spectrum.as<float2>(), s.work.as<float2>(), kTilesByLine, kTilesByRow, rf, w,
-      norm, tw, false, ftab);
-  SIFG_LAUNCH_CHECK();
+  if (ftab)
+    launch_columns<kColTable>(s, s.spectrum, s.work, kTilesByLine, kTilesByRow, rf, w, norm, ftab);
+  else
+    launch_columns<kColEvaluate>(s, s.spectrum, s.work, kTilesByLine, kTilesByRow, rf, w, norm);
   if (timer) timer->end(s.stream);
-  colfft512_kernel<<<grid, 32 * kColWarps, smem, s.stream>>>(
-      s.work.as<float2>(), s.work.as<float2>(), kTilesByLine, kTilesByLine, kNoFilter, nullptr, 1.f,
-      tw, false);
-  SIFG_LAUNCH_CHECK();
-  c2r512_rows_kernel<<<N * N / kRowsPerCta, 16 * kRowsPerCta, 0, s.stream>>>(s.work.as<float2>(),
-                                                                           out, tw, below);
+  launch_columns<kColInverse>(s, s.work, s.work, kTilesByLine, kTilesByLine);
+  c2r512_rows_kernel<<<N * N / kRowsPerCta, 16 * kRowsPerCta, 0, s.stream>>>(
+      s.work.as<float2>(), out, (const float2*)s.twiddles, below);
   SIFG_LAUNCH_CHECK();
 }
 static void launch_inverse512(const SmootherT<double>&, int, const RadialFilter&, double, double*,
