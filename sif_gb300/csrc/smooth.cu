@@ -92,10 +92,10 @@ __global__ void __launch_bounds__(256) filter_kernel(const typename Mode<R>::T* 
 //   (1) filter + inverse FFT along kx (spectrum -> work),
 //   (2) inverse FFT along ky (work, in place),
 //   (3) C2R along kz (work -> the real grid).
-// A 512-point transform belongs to one warp, 16 values per lane: a 16-point
-// DFT in registers over the lane's stride-32 values, a twiddle, an exchange
+// A 512-point transform belongs to 32 threads, 16 values each: a 16-point DFT
+// in registers over the thread's stride-32 values, a twiddle, an exchange
 // through shared memory, a second 16-point DFT and a radix-2 step between
-// lane pairs by shuffles (512 = 16 x 32, 32 = 16 x 2). Passes (1) and (2)
+// pairs of lanes by shuffles (512 = 16 x 32, 32 = 16 x 2). Passes (1) and (2)
 // give a CTA 16 neighbouring kz columns of one line (128 contiguous bytes
 // per row of the line); pass (3) gives each 257-mode kz row to a half-warp
 // as a 256-point complex transform of the packed even and odd samples.
@@ -108,22 +108,6 @@ __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
 __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
 __device__ __forceinline__ float2 cmul_i(float2 a) { return make_float2(-a.y, a.x); }  // a * i
-
-// Asynchronous global -> shared copies (LDGSTS): a CTA's whole tile is in
-// flight at once, with no registers held for it.
-__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(
-                   (uint32_t)__cvta_generic_to_shared(smem)),
-               "l"(gmem)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(
-                   (uint32_t)__cvta_generic_to_shared(smem)),
-               "l"(gmem)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 // e^{+2 pi i k/32}, k < 16, rounded to float.
 __constant__ float2 kW32[16] = {
@@ -434,95 +418,105 @@ __global__ void __launch_bounds__(32 * kColCols, 2)
 }
 static_assert(2 * kColCols == 32, "a column's thread pairs lie in one warp");
 
-// Pass (3): 16 rows of 257 modes per CTA, a half-warp per row. With Z the
-// row's modes (the imaginary parts of Z[0] and Z[256] taken as zero, as a
-// C2R does), c[k] = Fe[k] + i Fo[k] for k < 256, Fe = Z[k] + conj Z[256-k],
-// Fo = (Z[k] - conj Z[256-k]) W512^k, and its 256-point inverse DFT y gives
-// the real samples x[2m] = Re y[m], x[2m+1] = Im y[m]. The CTA's 16 rows
-// (x, y0 .. y0 + 15) come from the tiles in 16 contiguous 2 KB blocks (kz <
-// 256, by 16-byte asynchronous copies) and one mode each for kz = 256; a row
-// has kRowSlots slots in shared memory (even, for the 16-byte copies); the
-// stage exchange swizzles slots (k1, j) -> 16 k1 + (j ^ k1) within the row.
+// Pass (3) and the forward's first: 16 rows per CTA, a half-warp a row, as a
+// 256-point complex transform of the packed even and odd samples. A lane loads
+// its values straight into registers and stores its results straight out, 128
+// contiguous bytes a half-warp; shared memory is crossed once, between the two
+// 16-point stages (slot 16 k1 + (j ^ k1) of the row), and the partner mode 256 -
+// k comes by shuffle from the lane that holds it: value r of lane j is k = j +
+// 16 r, so its partner is value 15 - r of lane 16 - j, and lane 0's its own
+// value 16 - r.
 //
-// With `below` set the pass also lists, in flat order, the cells it writes
-// whose value is at most below.thr: the CTA's 8192 cells are one contiguous
-// flat range, and their entries go to the start of the CTA's own region of
-// 8192 slots, their number to below.counts[CTA] (the candidate scan's
-// threshold test, from the values in hand).
+// Memory bounds both: 1.1 GB each at 512^3, 166 us at the measured copy rate.
+// (With the rows staged through shared memory both ways shared memory bound
+// them: 187 us the inverse, 205 the forward.)
 constexpr int kRowsPerCta = 16;
-constexpr uint32_t kRowSlots = 258;
 static_assert(kRowsPerCta * 512 == kBelowBlock, "a CTA's cells are one below-list block");
-__global__ void __launch_bounds__(16 * kRowsPerCta, 4)
-    c2r512_rows_kernel(const float2* __restrict__ work, float* __restrict__ out,
-                       const float2* __restrict__ tw, BelowList below) {
-  __shared__ __align__(16) float2 buf[kRowsPerCta * kRowSlots];
-  const uint32_t x = blockIdx.x / (512 / kRowsPerCta);
-  const uint32_t y0 = (blockIdx.x % (512 / kRowsPerCta)) * kRowsPerCta;
-  const float2* tiles = work + ((size_t)x * kKzBlocks * 512 + y0) * 16;  // kz block 0
-  constexpr size_t kBlock = (size_t)512 * 16;                            // one kz block further
-  for (uint32_t f = threadIdx.x; f < 16 * kRowsPerCta * 8; f += blockDim.x) {
-    const uint32_t kb = f / (kRowsPerCta * 8), e = f % (kRowsPerCta * 8);
-    const uint32_t r = e / 8, jj = e % 8;
-    cp_async16(buf + r * kRowSlots + 16 * kb + 2 * jj,
-               reinterpret_cast<const float4*>(tiles + kb * kBlock) + e);
-  }
-  if (threadIdx.x < kRowsPerCta)
-    cp_async8(buf + threadIdx.x * kRowSlots + 256, tiles + 16 * kBlock + threadIdx.x * 16);
-  cp_async_wait_all();
-  __syncthreads();
-  const unsigned j = threadIdx.x & 15u;
-  float2* row = buf + (threadIdx.x >> 4) * kRowSlots;
-  const float2* twb = tw + 512;
-  const float2* wpre = tw + 768;
-  float2 v[16];
-#pragma unroll
-  for (int r = 0; r < 16; r++) {
-    const unsigned k = j + 16u * r;
-    float2 z = row[k], zc = row[256 - k];
-    if (r == 0 && j == 0) z.y = zc.y = 0.f;
-    zc.y = -zc.y;
-    const float2 fe = cadd(z, zc), fo = cmul(csub(z, zc), __ldg(wpre + k));
-    v[r] = make_float2(fe.x - fo.y, fe.y + fo.x);
-  }
+
+// The 256-point inverse DFT of a row, value r of lane j at j + 16 r before and
+// after.
+__device__ __forceinline__ void row256(float2 (&v)[16], float2* row, unsigned j,
+                                       const float2* __restrict__ twb) {
   dft_inv(v);
 #pragma unroll
   for (int k = 1; k < 16; k++) v[k] = cmul(v[k], __ldg(twb + k * 16 + j));
-  __syncwarp();
 #pragma unroll
   for (int k = 0; k < 16; k++) row[16 * k + (j ^ k)] = v[k];
   __syncwarp();
 #pragma unroll
   for (int m = 0; m < 16; m++) v[m] = row[16 * j + (m ^ j)];
   dft_inv(v);
-  __syncwarp();
+}
+
+// The partner of each value; `own0` is what lane 0's value 0 takes.
+__device__ __forceinline__ void partners(const float2 (&z)[16], float2 own0, unsigned j,
+                                         float2 (&m)[16]) {
 #pragma unroll
-  for (int k = 0; k < 16; k++) row[j + 16 * k] = v[k];
-  __syncthreads();
-  float2* dst = reinterpret_cast<float2*>(out + ((size_t)x * 512 + y0) * 512);
-  if (!below.counts) {
-    for (uint32_t f = threadIdx.x; f < kRowsPerCta * 256; f += blockDim.x)
-      dst[f] = buf[(f >> 8) * kRowSlots + (f & 255u)];
-    return;
+  for (int r = 0; r < 16; r++) {
+    m[r] = make_float2(__shfl_sync(0xffffffffu, z[15 - r].x, (16 - (int)j) & 15, 16),
+                       __shfl_sync(0xffffffffu, z[15 - r].y, (16 - (int)j) & 15, 16));
+    if (j == 0) m[r] = r == 0 ? own0 : z[(16 - r) & 15];
   }
-  // Each warp takes 512 consecutive pairs (two rows), 32 at a time: it writes
-  // them out and keeps its lanes' threshold bits (two per pair) in `bits`;
-  // the warps' totals place each warp's entries, and a second walk over the
-  // pairs with set bits writes the entries in flat order.
+}
+
+// Pass (3). With Z the row's modes (the imaginary parts of Z[0] and Z[256]
+// taken as zero, as a C2R does), c[k] = Fe[k] + i Fo[k] for k < 256, Fe = Z[k] +
+// conj Z[256-k], Fo = (Z[k] - conj Z[256-k]) W512^k, and its inverse DFT y gives
+// the real samples x[2m] = Re y[m], x[2m+1] = Im y[m].
+//
+// With `below` set the pass also lists, in flat order, the cells it writes
+// whose value is at most below.thr: the CTA's 8192 cells are one contiguous
+// flat range, and their entries go to the start of the CTA's own region of
+// 8192 slots, their number to below.counts[CTA] (the candidate scan's
+// threshold test, from the values in hand).
+__global__ void __launch_bounds__(16 * kRowsPerCta, 3)
+    c2r512_rows_kernel(const float2* __restrict__ work, float* __restrict__ out,
+                       const float2* __restrict__ tw, BelowList below) {
+  __shared__ float2 buf[kRowsPerCta * 256];
+  const uint32_t x = blockIdx.x / (512 / kRowsPerCta);
+  const uint32_t y0 = (blockIdx.x % (512 / kRowsPerCta)) * kRowsPerCta;
+  const unsigned j = threadIdx.x & 15u, ry = threadIdx.x >> 4;
+  // The row's kz block 0; a kz block further is 512 rows of 16 on.
+  const float2* p = work + ((size_t)x * kKzBlocks * 512 + y0 + ry) * 16 + j;
+  constexpr size_t kBlock = (size_t)512 * 16;
+  float2 v[16];
+  {
+    float2 z[16], zc[16], last = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int r = 0; r < 16; r++) z[r] = __ldg(p + r * kBlock);
+    if (j == 0) {
+      last = __ldg(p + 16 * kBlock);
+      z[0].y = last.y = 0.f;
+    }
+    partners(z, last, j, zc);
+    const float2* wpre = tw + 768;
+#pragma unroll
+    for (int r = 0; r < 16; r++) {
+      const float2 c = make_float2(zc[r].x, -zc[r].y);
+      const float2 fe = cadd(z[r], c), fo = cmul(csub(z[r], c), __ldg(wpre + j + 16u * r));
+      v[r] = make_float2(fe.x - fo.y, fe.y + fo.x);
+    }
+  }
+  row256(v, buf + ry * 256, j, tw + 512);
+  float2* dst = reinterpret_cast<float2*>(out + ((size_t)x * 512 + y0 + ry) * 512) + j;
+  if (!below.counts || below.field) {
+#pragma unroll
+    for (int k = 0; k < 16; k++) dst[16 * k] = v[k];
+  }
+  if (!below.counts) return;
+  // Each lane's threshold bits, two a pair; the warps' totals place each
+  // warp's entries (two rows, one after the other), each step of 16 pairs of
+  // a row in lane order.
   constexpr uint32_t kWarps = 16 * kRowsPerCta / 32;
-  constexpr uint32_t kWarpPairs = kRowsPerCta * 256 / kWarps;
-  static_assert(kWarpPairs == 32 * 16, "16 pairs a lane, two bits each in one word");
   __shared__ uint32_t ws[kWarps];
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  const uint32_t base = warp * kWarpPairs;
   uint32_t bits = 0;
 #pragma unroll
-  for (int i = 0; i < 16; i++) {
-    const uint32_t f = base + 32u * i + lane;
-    const float2 v = buf[(f >> 8) * kRowSlots + (f & 255u)];
-    if (below.field) dst[f] = v;
-    bits |= ((v.x <= below.thr ? 1u : 0u) | (v.y <= below.thr ? 2u : 0u)) << (2 * i);
-  }
-  const uint32_t n_warp = __reduce_add_sync(0xffffffffu, (unsigned)__popc(bits));
+  for (int k = 0; k < 16; k++)
+    bits |= ((v[k].x <= below.thr ? 1u : 0u) | (v[k].y <= below.thr ? 2u : 0u)) << (2 * k);
+  const uint32_t n_mine = (uint32_t)__popc(bits);
+  const uint32_t n_warp = __reduce_add_sync(0xffffffffu, n_mine);
+  const uint32_t n_first = __reduce_add_sync(0xffffffffu, lane < 16 ? n_mine : 0u);
   if (lane == 0) ws[warp] = n_warp;
   __syncthreads();
   uint32_t pos = 0, total = 0;
@@ -533,110 +527,79 @@ __global__ void __launch_bounds__(16 * kRowsPerCta, 4)
   }
   if (threadIdx.x == 0) below.counts[blockIdx.x] = total;
   if (n_warp == 0) return;
-  const uint32_t cell0 = (x * 512 + y0) * 512;
+  const uint32_t row_lanes = lane < 16 ? 0xffffu : 0xffff0000u;
+  const uint32_t lower = row_lanes & ((1u << lane) - 1u);
+  if (lane >= 16) pos += n_first;
+  const uint32_t cell0 = ((x * 512 + y0 + ry) * 512) + 2 * j;
   const size_t region = (size_t)blockIdx.x * (kRowsPerCta * 512);
-  const uint32_t lower = (1u << lane) - 1u;
 #pragma unroll
-  for (int i = 0; i < 16; i++) {
-    const uint32_t b = (bits >> (2 * i)) & 3u;
+  for (int k = 0; k < 16; k++) {
+    const uint32_t b = (bits >> (2 * k)) & 3u;
     const uint32_t mx = __ballot_sync(0xffffffffu, b & 1u), my = __ballot_sync(0xffffffffu, b & 2u);
     if ((mx | my) == 0u) continue;
-    if (b) {
-      const uint32_t f = base + 32u * i + lane;
-      const float2 v = buf[(f >> 8) * kRowSlots + (f & 255u)];
-      uint32_t p = pos + __popc(mx & lower) + __popc(my & lower);
-      if (b & 1u) {
-        below.delta[region + p] = v.x;
-        below.flat[region + p] = cell0 + 2 * f;
-        p++;
-      }
-      if (b & 2u) {
-        below.delta[region + p] = v.y;
-        below.flat[region + p] = cell0 + 2 * f + 1;
-      }
+    uint32_t at = pos + __popc(mx & lower) + __popc(my & lower);
+    if (b & 1u) {
+      below.delta[region + at] = v[k].x;
+      below.flat[region + at] = cell0 + 32 * k;
+      at++;
     }
-    pos += __popc(mx) + __popc(my);
+    if (b & 2u) {
+      below.delta[region + at] = v[k].y;
+      below.flat[region + at] = cell0 + 32 * k + 1;
+    }
+    pos += __popc(mx & row_lanes) + __popc(my & row_lanes);
   }
 }
 
-// The forward transform's first pass, the R2C along z: 16 rows of 512 reals
-// per CTA (one contiguous 32 KB block), a half-warp per row. The row read
-// as 256 complex values c[m] = x[2m] + i x[2m+1] is transformed forward (the
-// conjugate of the inverse of the conjugate); then, with C[-k] taken mod 256,
-// E[k] = (C[k] + conj C[-k]) / 2, O[k] = (C[k] - conj C[-k]) / 2i and
-// X[k] = E[k] + W512^-k O[k] for k < 256, X[256] = E[0] - O[0]. The 257 modes
-// go to the tiles (16 rows by 16 kz, 2 KB blocks).
-__global__ void __launch_bounds__(16 * kRowsPerCta, 4)
+// The forward transform's first pass, the R2C along z. The row read as 256
+// complex values c[m] = x[2m] + i x[2m+1] is transformed forward (the conjugate
+// of the inverse of the conjugate); then, with C[-k] taken mod 256, E[k] = (C[k]
+// + conj C[-k]) / 2, O[k] = (C[k] - conj C[-k]) / 2i and X[k] = E[k] + W512^-k
+// O[k] for k < 256, X[256] = E[0] - O[0]. The 257 modes go to the tiles.
+__global__ void __launch_bounds__(16 * kRowsPerCta, 3)
     r2c512_rows_kernel(const float* __restrict__ grid, float2* __restrict__ work,
                        const float2* __restrict__ tw, const double* __restrict__ mean) {
-  __shared__ __align__(16) float2 buf[kRowsPerCta * kRowSlots];
+  __shared__ float2 buf[kRowsPerCta * 256];
   const uint32_t x = blockIdx.x / (512 / kRowsPerCta);
   const uint32_t y0 = (blockIdx.x % (512 / kRowsPerCta)) * kRowsPerCta;
-  const float4* src = reinterpret_cast<const float4*>(grid + ((size_t)x * 512 + y0) * 512);
-  for (uint32_t f = threadIdx.x; f < kRowsPerCta * 128; f += blockDim.x)
-    cp_async16(buf + (f >> 7) * kRowSlots + 2 * (f & 127u), src + f);
+  const unsigned j = threadIdx.x & 15u, ry = threadIdx.x >> 4;
+  const float2* src = reinterpret_cast<const float2*>(grid + ((size_t)x * 512 + y0 + ry) * 512) + j;
+  float2 v[16];
+#pragma unroll
+  for (int r = 0; r < 16; r++) v[r] = __ldg(src + 16 * r);
   // With the mean, the rows are the density: its contrast, as the contrast
   // kernel computes it (inv rounded from the double 1 / mean), the double
-  // division done once for the CTA while its copies land.
-  __shared__ float inv_s;
-  if (mean && threadIdx.x == 0) inv_s = (float)(1.0 / __ldg(mean));
-  cp_async_wait_all();
-  __syncthreads();
-  const unsigned j = threadIdx.x & 15u;
-  float2* row = buf + (threadIdx.x >> 4) * kRowSlots;
-  const float2* twb = tw + 512;
+  // division done once for the CTA while its loads land.
+  if (mean) {
+    __shared__ float inv_s;
+    if (threadIdx.x == 0) inv_s = (float)(1.0 / __ldg(mean));
+    __syncthreads();
+    const float inv = inv_s;
+#pragma unroll
+    for (int r = 0; r < 16; r++)
+      v[r] = make_float2(__fsub_rn(__fmul_rn(v[r].x, inv), 1.0f),
+                         __fsub_rn(__fmul_rn(v[r].y, inv), 1.0f));
+  }
+#pragma unroll
+  for (int r = 0; r < 16; r++) v[r].y = -v[r].y;
+  row256(v, buf + ry * 256, j, tw + 512);
+#pragma unroll
+  for (int r = 0; r < 16; r++) v[r].y = -v[r].y;  // C
+  float2 m[16];
+  partners(v, v[0], j, m);
   const float2* wpre = tw + 768;
-  float2 v[16];
-  const float inv = mean ? inv_s : 0.f;
-#pragma unroll
-  for (int r = 0; r < 16; r++) {
-    v[r] = row[j + 16u * r];
-    if (mean) v[r] = make_float2(__fsub_rn(__fmul_rn(v[r].x, inv), 1.0f),
-                                 __fsub_rn(__fmul_rn(v[r].y, inv), 1.0f));
-    v[r].y = -v[r].y;
-  }
-  dft_inv(v);
-#pragma unroll
-  for (int k = 1; k < 16; k++) v[k] = cmul(v[k], __ldg(twb + k * 16 + j));
-  __syncwarp();
-#pragma unroll
-  for (int k = 0; k < 16; k++) row[16 * k + (j ^ k)] = v[k];
-  __syncwarp();
-#pragma unroll
-  for (int m = 0; m < 16; m++) v[m] = row[16 * j + (m ^ j)];
-  dft_inv(v);
-  __syncwarp();
-#pragma unroll
-  for (int k = 0; k < 16; k++) row[j + 16 * k] = make_float2(v[k].x, -v[k].y);  // C
-  __syncwarp();
-  float2 out[16];
-  float2 nyq = make_float2(0.f, 0.f);
-#pragma unroll
-  for (int r = 0; r < 16; r++) {
-    const unsigned k = j + 16u * r;
-    const float2 c = row[k], m = row[(256u - k) & 255u];
-    const float2 e = make_float2(0.5f * (c.x + m.x), 0.5f * (c.y - m.y));  // (C + conj C[-k]) / 2
-    const float2 d = make_float2(c.x - m.x, c.y + m.y);                    // C - conj C[-k]
-    const float2 o = make_float2(0.5f * d.y, -0.5f * d.x);                 // d / 2i
-    const float2 w = __ldg(wpre + k);
-    out[r] = cadd(e, cmul(o, make_float2(w.x, -w.y)));
-    if (r == 0 && j == 0) nyq = make_float2(e.x - o.x, e.y - o.y);
-  }
-  __syncwarp();
-#pragma unroll
-  for (int r = 0; r < 16; r++) row[j + 16u * r] = out[r];
-  if (j == 0) row[256] = nyq;
-  __syncthreads();
-  float2* tiles = work + ((size_t)x * kKzBlocks * 512 + y0) * 16;
+  float2* p = work + ((size_t)x * kKzBlocks * 512 + y0 + ry) * 16 + j;
   constexpr size_t kBlock = (size_t)512 * 16;
-  for (uint32_t f = threadIdx.x; f < 16 * kRowsPerCta * 8; f += blockDim.x) {
-    const uint32_t kb = f / (kRowsPerCta * 8), e = f % (kRowsPerCta * 8);
-    const uint32_t r = e / 8, jj = e % 8;
-    reinterpret_cast<float4*>(tiles + kb * kBlock)[e] =
-        *reinterpret_cast<const float4*>(buf + r * kRowSlots + 16 * kb + 2 * jj);
+#pragma unroll
+  for (int r = 0; r < 16; r++) {
+    const float2 c = v[r];
+    const float2 e = make_float2(0.5f * (c.x + m[r].x), 0.5f * (c.y - m[r].y));  // (C + conj C[-k]) / 2
+    const float2 d = make_float2(c.x - m[r].x, c.y + m[r].y);                    // C - conj C[-k]
+    const float2 o = make_float2(0.5f * d.y, -0.5f * d.x);                       // d / 2i
+    const float2 w = __ldg(wpre + j + 16u * r);
+    p[r * kBlock] = cadd(e, cmul(o, make_float2(w.x, -w.y)));
+    if (r == 0 && j == 0) p[16 * kBlock] = make_float2(e.x - o.x, e.y - o.y);
   }
-  if (threadIdx.x < kRowsPerCta)
-    tiles[16 * kBlock + threadIdx.x * 16] = buf[threadIdx.x * kRowSlots + 256];
 }
 
 static bool own_inverse(uint32_t n) { return n == 512; }
