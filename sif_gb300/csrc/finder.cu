@@ -80,40 +80,18 @@ __device__ bool is_minimum(const R* __restrict__ f, uint32_t n, uint64_t i) {
   return true;
 }
 
-// The candidate bits of cells c0..c0+3 (bit j for c0 + j), and their depths.
-// With `minima` (SIF_FINDER_SEEDS_MINIMA, no refinement) a cell must also be
-// a local minimum of the field (sif__finder_scan_refined with minima_only,
-// utils.c:406-552); grid_n is the grid's side.
-template <class R>
-__device__ __forceinline__ uint32_t quad_candidates(const R* __restrict__ f,
-                                                    const uint32_t* __restrict__ mask,
-                                                    uint64_t c0, uint64_t n, R thr, R* v,
-                                                    uint32_t grid_n, bool minima) {
-  if (c0 + 3 < n) {
-    load4(f, c0, v);
-  } else {
-    for (int k = 0; k < 4; k++) v[k] = c0 + k < n ? f[c0 + k] : R(1);
-  }
-  if (c0 >= n) return 0u;
-  const uint32_t m = __ldg(mask + (c0 >> 5)) >> (c0 & 31);
-  uint32_t bits = 0;
-#pragma unroll
-  for (int k = 0; k < 4; k++)
-    bits |= (v[k] <= thr && !(m & (1u << k)) && c0 + k < n) ? (1u << k) : 0u;
-  if (minima)
-    for (uint32_t b = bits; b; b &= b - 1) {
-      const int k = __ffs(b) - 1;
-      if (!is_minimum(f, grid_n, c0 + k)) bits &= ~(1u << k);
-    }
-  return bits;
-}
-
 // One pass over the field: each CTA writes its candidates, in flat order, to
 // the start of its own region of kScanChunk slots and its count to
 // counts[block]; the compaction then moves only the candidates. A warp takes
 // kScanRounds consecutive runs of 128 cells, all of its loads in flight at
 // once, and keeps its candidate bits (four a run) in one word; one exchange of
-// the warps' totals places their entries. With `done` set (zeroed; it is left
+// the warps' totals places their entries. Only cells at or below the threshold
+// look up the mask and, with `minima` (SIF_FINDER_SEEDS_MINIMA, no refinement:
+// a candidate is also a local minimum of the field,
+// sif__finder_scan_refined with minima_only, utils.c:406-552; grid_n is the
+// grid's side), their neighbours -- after every load of the field is issued:
+// between them, either held each load back for the one before (256^3: 37 us
+// against 19). With `done` set (zeroed; it is left
 // zero) the last CTA to finish scans the counts -- up to kScanTail of them: a
 // launch and its wait less -- and writes the total.
 constexpr uint32_t kScanTail = 4096;
@@ -130,9 +108,28 @@ __global__ void __launch_bounds__(kScanT) scan_regions_kernel(
   const uint64_t first = base + (uint64_t)warp * (128 * kScanRounds) + lane * 4;
   R v[kScanRounds][4];
   uint32_t bits = 0;
+  if (base + kScanChunk <= n) {
 #pragma unroll
-  for (int j = 0; j < kScanRounds; j++)
-    bits |= quad_candidates(f, mask, first + 128 * j, n, thr, v[j], grid_n, minima) << (4 * j);
+    for (int j = 0; j < kScanRounds; j++) load4(f, first + 128 * j, v[j]);
+#pragma unroll
+    for (int j = 0; j < kScanRounds; j++)
+#pragma unroll
+      for (int k = 0; k < 4; k++) bits |= v[j][k] <= thr ? 1u << (4 * j + k) : 0u;
+  } else {
+#pragma unroll
+    for (int j = 0; j < kScanRounds; j++)
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const uint64_t c = first + 128 * j + k;
+        v[j][k] = c < n ? __ldg(f + c) : R(0);
+        bits |= c < n && v[j][k] <= thr ? 1u << (4 * j + k) : 0u;
+      }
+  }
+  for (uint32_t b = bits; b; b &= b - 1) {
+    const int at = __ffs(b) - 1;
+    const uint64_t c = first + 128 * (at >> 2) + (at & 3);
+    if (mask_get(mask, c) || (minima && !is_minimum(f, grid_n, c))) bits &= ~(1u << at);
+  }
   const uint32_t mine = __reduce_add_sync(0xffffffffu, (uint32_t)__popc(bits));
   if (lane == 0) ws[warp] = mine;
   __syncthreads();
