@@ -765,6 +765,14 @@ constexpr int kSurveyT = 512;
 constexpr uint32_t kMaxBins = 2048;
 constexpr uint32_t kSmemBuf = 2048;
 constexpr int kWalkUnroll = 4;  // particle loads in flight per lane
+// A survivor's first window is rc.window bins, where the answer mostly lies;
+// a further one takes the bins below it too, to kMoreParticles of them. A
+// window costs a walk of the template, a sort and some ten barriers whatever it
+// holds, and a sparse sphere's 64 bins of a few particles each took up to eight
+// of them one after another. (No case above was
+// slower or faster by more than its runs differ; a survivor without a crossing
+// takes 2 windows of 400 particles where it took 8.)
+constexpr uint32_t kMoreParticles = 1024;
 
 unsigned growth_grid() { return 152u * 4u; }
 
@@ -920,11 +928,18 @@ __device__ __forceinline__ void walk_cells(const MeshViewT<R>& mesh, const Templ
                                            Each each, unsigned long long& visited,
                                            unsigned long long& read, bool whole_warp = false) {
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  // A CTA's warps share the template's chunks; a warp on its own takes all.
-  const uint32_t first = whole_warp ? 0u : warp * 32;
+  // A CTA's warps share the template's chunks of 32 cells; a warp on its own
+  // takes all. Where the chunks do not go round twice the warps take every so
+  // many cells each instead: of a small sphere's 200 cells seven warps would
+  // have 32 each and the others none, and a cell can hold hundreds of particles
+  // (survey 96^3: 380 randoms). Larger templates keep to chunks, whose reads of
+  // the template are coalesced.
   const uint32_t step = whole_warp ? 32u : blockDim.x;
+  const bool dealt = !whole_warp && tpl.count <= 2 * step;
+  const uint32_t first = whole_warp ? 0u : dealt ? warp : warp * 32;
+  const uint32_t each_lane = dealt ? blockDim.x >> 5 : 1u;
   for (uint32_t c0 = first; c0 < tpl.count; c0 += step) {
-    const uint32_t i = c0 + lane;
+    const uint32_t i = c0 + lane * each_lane;
     CellRange<R> c{0, 0, 0.f, 0.f, 0.f, 0};
     uint8_t type = 0;
     bool need = false;
@@ -998,7 +1013,7 @@ __device__ __forceinline__ void walk_cells(const MeshViewT<R>& mesh, const Templ
         const R qz = __shfl_sync(0xffffffffu, c.ez, own[u]);
         const uint8_t t = (uint8_t)__shfl_sync(0xffffffffu, (int)type, own[u]);
         if (pp[u] != 0xffffffffu)
-          each(t, dist2(px[u], py[u], pz[u], qx, qy, qz), pp[u], c0 + (uint32_t)own[u]);
+          each(t, dist2(px[u], py[u], pz[u], qx, qy, qz), pp[u], c0 + (uint32_t)own[u] * each_lane);
       }
     }
   }
@@ -1137,6 +1152,7 @@ __global__ void __launch_bounds__(kGrowT, 4) growth_kernel(MeshViewT<R> mesh, Te
         //    test does not rule out, resolved with the bins below it.
         int32_t cursor = (int32_t)rc.nb - 1;
         reason = kRescaleBelowRung;
+        bool more = false;
         while (cursor >= 0) {
           int best = -1;
           for (int32_t b = threadIdx.x; b <= cursor; b += kGrowT) {
@@ -1152,6 +1168,8 @@ __global__ void __launch_bounds__(kGrowT, 4) growth_kernel(MeshViewT<R> mesh, Te
           if (b_lo < 0) b_lo = 0;
           const uint32_t top = below[b_hi] + bins[b_hi];
           while (b_lo < b_hi && top - below[b_lo] > kSmemBuf) b_lo++;
+          while (more && b_lo > 0 && top - below[b_lo - 1] <= kMoreParticles) b_lo--;
+          more = true;
           const uint32_t want = top - below[b_lo];
           R* buf = sbuf;
           uint32_t cap = kSmemBuf;
@@ -1799,6 +1817,7 @@ void grow(MeshViewT<R> mesh, TemplateViewT<R> tpl, RungConstsT<R> rc, SurvivorsT
 // would, whose enclosed weight does not depend on the order).
 // ---------------------------------------------------------------------------
 constexpr uint32_t kWBuf = 1024;  // a window's pairs held in shared memory
+static_assert(kMoreParticles <= kWBuf && kMoreParticles <= kSmemBuf, "a widened window fits");
 
 template <class R>
 __device__ __forceinline__ long long wfix(R w, R scale) {
@@ -2018,6 +2037,7 @@ __global__ void __launch_bounds__(kGrowT, 4) growth_weighted_kernel(
         //    not rule out, resolved with the bins below it.
         int32_t cursor = (int32_t)rc.nb - 1;
         reason = kRescaleBelowRung;
+        bool more = false;
         while (cursor >= 0) {
           int best = -1;
           for (int32_t b = threadIdx.x; b <= cursor; b += kGrowT) {
@@ -2033,6 +2053,8 @@ __global__ void __launch_bounds__(kGrowT, 4) growth_weighted_kernel(
           if (b_lo < 0) b_lo = 0;
           const uint32_t top_n = beln[b_hi] + bn[b_hi];
           while (b_lo < b_hi && top_n - beln[b_lo] > kWBuf) b_lo++;
+          while (more && b_lo > 0 && top_n - beln[b_lo - 1] <= kMoreParticles) b_lo--;
+          more = true;
           const uint32_t want = top_n - beln[b_lo];
           R* kb = pd2;
           long long* vb = pwv;
@@ -2356,6 +2378,7 @@ __global__ void __launch_bounds__(kSurveyT, 2) growth_survey_kernel(
         //    its window resolved.
         int32_t cursor = (int32_t)nb - 1;
         reason = kRescaleBelowRung;
+        bool more = false;
         while (cursor >= 0) {
           int best = -1;
           for (int32_t b = threadIdx.x; b <= cursor; b += kSurveyT) {
@@ -2372,6 +2395,8 @@ __global__ void __launch_bounds__(kSurveyT, 2) growth_survey_kernel(
           if (b_lo < 0) b_lo = 0;
           const uint32_t top_n = beln[b_hi] + bn[b_hi];
           while (b_lo < b_hi && top_n - beln[b_lo] > kWBuf) b_lo++;
+          while (more && b_lo > 0 && top_n - beln[b_lo - 1] <= kMoreParticles) b_lo--;
+          more = true;
           const uint32_t want = top_n - beln[b_lo];
           R* kb = pd2;
           long long* vb = pwv;
