@@ -756,22 +756,21 @@ void prefilter(const uint32_t* cand_flat, uint32_t m, const uint32_t* mask, Void
 constexpr int kGrowT = 256;
 constexpr int kGrowWarps = kGrowT / 32;
 // The survey growth's CTA: its tables of 2,048 bins let two CTAs an SM in
-// whatever their size, and two of 512 threads keep the SM's registers full.
-// Survey 96^3, data and randoms on their own meshes: 10.2 to 9.6 ms a
-// search. The other per-CTA kernels stay at 256, four an SM: wider CTAs gave
-// nothing where survivors are few and cost the weighted 150^3 search 13%
-// where they are not (more threads at each barrier and sort step).
-constexpr int kSurveyT = 512;
+// whatever their size, and two of 512 threads keep the SM's registers full; up
+// to a survivor an SM, one of 1,024 shortens the survivor's own walks of two
+// meshes. Survey 96^3: 10.2 ms a search with 256 threads, 9.6 with 512 (8.1
+// with the cells dealt), 7.8. The other per-CTA kernels stay at 256, four an
+// SM: wider ones gave nothing where survivors are few and cost the weighted
+// 150^3 search 13% where they are not (more threads at each barrier and sort).
+constexpr int kSurveyT = 512, kSurveyMaxT = 1024;
 constexpr uint32_t kMaxBins = 2048;
 constexpr uint32_t kSmemBuf = 2048;
 constexpr int kWalkUnroll = 4;  // particle loads in flight per lane
 // A survivor's first window is rc.window bins, where the answer mostly lies;
 // a further one takes the bins below it too, to kMoreParticles of them. A
 // window costs a walk of the template, a sort and some ten barriers whatever it
-// holds, and a sparse sphere's 64 bins of a few particles each took up to eight
-// of them one after another. (No case above was
-// slower or faster by more than its runs differ; a survivor without a crossing
-// takes 2 windows of 400 particles where it took 8.)
+// holds, and a sparse sphere without a crossing took eight for its 64 bins of a
+// few particles each (two now; no search measured either way beyond its noise).
 constexpr uint32_t kMoreParticles = 1024;
 
 unsigned growth_grid() { return 152u * 4u; }
@@ -2197,7 +2196,7 @@ __device__ __forceinline__ long long cell_wt(const MeshViewT<R>& m, uint32_t fla
 }
 
 template <class R>
-__global__ void __launch_bounds__(kSurveyT, 2) growth_survey_kernel(
+__global__ void __launch_bounds__(kSurveyMaxT, 1) growth_survey_kernel(
     MeshViewT<R> dm, TemplateViewT<R> dt, MeshViewT<R> rm, TemplateViewT<R> rt, RungConstsT<R> rc,
     R K, SurvivorsT<R> sv, R* __restrict__ gbuf, long long* __restrict__ gwbuf, uint32_t gcap,
     unsigned long long* __restrict__ traffic, uint32_t* work) {
@@ -2210,9 +2209,9 @@ __global__ void __launch_bounds__(kSurveyT, 2) growth_survey_kernel(
   uint32_t* bn = (uint32_t*)(pwv + kWBuf);  // data tracers per bin (sizes the windows)
   uint32_t* beln = bn + kMaxBins;           // data tracers in the bins below b
   R* pd2 = (R*)(beln + kMaxBins);           // a window's distances
-  __shared__ unsigned long long red64[2 * kSurveyT / 32];
-  __shared__ long long tsum[kSurveyT];
-  __shared__ int redi[kSurveyT / 32];
+  __shared__ unsigned long long red64[2 * kSurveyMaxT / 32];
+  __shared__ long long tsum[kSurveyMaxT];
+  __shared__ int redi[kSurveyMaxT / 32];
   __shared__ uint32_t collected;
   __shared__ uint32_t s_item;
 
@@ -2284,7 +2283,7 @@ __global__ void __launch_bounds__(kSurveyT, 2) growth_survey_kernel(
           nb = (uint32_t)want;
       }
       const R inv_w = fdiv((R)nb, span), bin_w = fdiv(span, (R)nb);
-      for (uint32_t b = threadIdx.x; b < nb; b += kSurveyT) {
+      for (uint32_t b = threadIdx.x; b < nb; b += blockDim.x) {
         dbin[b] = 0;
         rbin[b] = 0;
         bn[b] = 0;
@@ -2381,7 +2380,7 @@ __global__ void __launch_bounds__(kSurveyT, 2) growth_survey_kernel(
         bool more = false;
         while (cursor >= 0) {
           int best = -1;
-          for (int32_t b = threadIdx.x; b <= cursor; b += kSurveyT) {
+          for (int32_t b = threadIdx.x; b <= cursor; b += blockDim.x) {
             if (!(dbin[b] > 0)) continue;
             const R d_in_min = wreal<R>(dbel[b], dinv);
             const R r_in_max = wreal<R>(rbel[b] + rbin[b], rinv);
@@ -2437,7 +2436,7 @@ __global__ void __launch_bounds__(kSurveyT, 2) growth_survey_kernel(
           const uint32_t m = collected < cap ? collected : cap;
           uint32_t p2 = 1;
           while (p2 < m) p2 <<= 1;
-          for (uint32_t i = m + threadIdx.x; i < p2; i += kSurveyT) {
+          for (uint32_t i = m + threadIdx.x; i < p2; i += blockDim.x) {
             kb[i] = real_inf<R>();
             vb[i] = 0;
           }
@@ -2450,7 +2449,7 @@ __global__ void __launch_bounds__(kSurveyT, 2) growth_survey_kernel(
           // randoms up to it.
           const long long d_top = dbel[b_hi] + dbin[b_hi];
           int found = -1;
-          for (uint32_t k = threadIdx.x; k < m; k += kSurveyT) {
+          for (uint32_t k = threadIdx.x; k < m; k += blockDim.x) {
             const R d2 = kb[k];
             if (d2 == R(0)) continue;
             const uint32_t bi = bin_of(d2, rc2, inv_w, nb);
@@ -2503,7 +2502,7 @@ void grow_survey(MeshViewT<R> dm, TemplateViewT<R> dt, MeshViewT<R> rm, Template
   }
   const unsigned g = max_survivors < growth_grid() ? max_survivors : growth_grid();
   if (timer) timer->begin(st);
-  growth_survey_kernel<R><<<g, kSurveyT, smem, st>>>(dm, dt, rm, rt, rc, K, s, gbuf, gwbuf, gcap,
+  growth_survey_kernel<R><<<g, max_survivors <= 152u ? kSurveyMaxT : kSurveyT, smem, st>>>(dm, dt, rm, rt, rc, K, s, gbuf, gwbuf, gcap,
                                                   traffic, work);
   SIFG_LAUNCH_CHECK();
   if (timer) timer->end(st);
