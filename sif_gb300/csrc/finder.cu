@@ -405,59 +405,16 @@ __device__ __forceinline__ bool in_window(const VoidViewT<R>& v, R vx, R vy, R v
 // instead of the window's cells: a rung's early voids are few and the window of
 // a large sphere many cells, each a dependent load of its range (64^3 and
 // survey boxes, whose spheres reach a quarter of the box: 650 to 1,000 cells
-// for a few dozen voids, and the pre-filter 70 to 200 us a rung). A void's
-// loads go to every lane at once and do not wait on one another. A void
+// for a few dozen voids, and the pre-filter 70 to 200 us a rung). A void
 // outside the window is not tested against, as the walk over cells would not.
 __device__ __forceinline__ bool walk_voids(uint32_t n, int32_t x0, int32_t x1, int32_t y0, int32_t y1,
                                            int32_t z0, int32_t z1) {
   return n <= (uint32_t)(x1 - x0 + 1) * (uint32_t)(y1 - y0 + 1) * (uint32_t)(z1 - z0 + 1);
 }
 
-// sif__overlap_exact (src/finder/utils.c:850-960) over the void index.
-template <class R>
-__device__ bool overlap_exact(const VoidViewT<R>& v, R cx, R cy, R cz, R r, R f,
-                              R scale, R box) {
-  if (v.n == 0) return false;
-  const R half = fmul(box, R(0.5f));
-  const R s = search_radius(r, v.max_r, f, scale);
-  const int32_t x0 = (int32_t)ffloor(fmul(fsub(cx, s), v.inv_cell));
-  const int32_t x1 = (int32_t)ffloor(fmul(fadd(cx, s), v.inv_cell));
-  const int32_t y0 = (int32_t)ffloor(fmul(fsub(cy, s), v.inv_cell));
-  const int32_t y1 = (int32_t)ffloor(fmul(fadd(cy, s), v.inv_cell));
-  const int32_t z0 = (int32_t)ffloor(fmul(fsub(cz, s), v.inv_cell));
-  const int32_t z1 = (int32_t)ffloor(fmul(fadd(cz, s), v.inv_cell));
-  const bool interior = is_interior(cx, cy, cz, s, box);
-  if (walk_voids(v.n, x0, x1, y0, y1, z0, z1)) {
-    for (uint32_t j = 0; j < v.n; j++) {
-      const R vx = v.cx[j], vy = v.cy[j], vz = v.cz[j];
-      if (collide(cx, cy, cz, r, vx, vy, vz, v.r[j], f, scale, box, half, interior) &&
-          in_window(v, vx, vy, vz, x0, x1, y0, y1, z0, z1))
-        return true;
-    }
-    return false;
-  }
-  for (int32_t ix = x0; ix <= x1; ix++) {
-    const uint32_t wx = (uint32_t)ix & (kVoidCells - 1);
-    for (int32_t iy = y0; iy <= y1; iy++) {
-      const uint32_t wy = (uint32_t)iy & (kVoidCells - 1);
-      for (int32_t iz = z0; iz <= z1; iz++) {
-        const uint32_t wz = (uint32_t)iz & (kVoidCells - 1);
-        const uint32_t c = (wx * kVoidCells + wy) * kVoidCells + wz;
-        for (uint32_t k = v.start[c]; k < v.start[c + 1]; k++) {
-          const uint32_t j = v.ids[k];
-          if (collide(cx, cy, cz, r, v.cx[j], v.cy[j], v.cz[j], v.r[j], f, scale, box, half,
-                      interior))
-            return true;
-        }
-      }
-    }
-  }
-  return false;
-}
-
-// overlap_exact by a warp: the same cells and the same pair tests, the
-// lanes taking the cells 32 at a time (a thread alone walks them one load
-// after another). Every lane returns the answer.
+// sif__overlap_exact (src/finder/utils.c:850-960) over the void index, by a
+// warp: the lanes take the cells (or the voids) 32 at a time, where a thread
+// alone walks them one load after another. Every lane returns the answer.
 template <class R>
 __device__ bool overlap_exact_warp(const VoidViewT<R>& v, R cx, R cy, R cz, R r, R f, R scale,
                                    R box) {
@@ -677,23 +634,33 @@ __device__ __forceinline__ bool cand_masked(const uint32_t* mask, uint32_t node,
 // Pre-filter
 // ---------------------------------------------------------------------------
 
+// `per` candidates a warp (a power of two up to 32): a lane each for the mask
+// and the poles, then the warp together for the exact overlap of each that is
+// left, whose walk of the void index -- hundreds of cells about a large sphere,
+// each a dependent load -- is what the test waits on. One a warp while the
+// candidates leave the GPU room, 32 where there are many. (A thread a candidate
+// took 54 us a rung of a weighted 150^3 search and up to 116; now 8, at most 11.)
+//
 // The survivors are appended as they are found, a warp's together (one atomic a
 // warp): nothing depends on the order they are listed in -- the commit goes by
 // their ranks -- but neighbours in the list staying near one another keeps the
 // growth's reads together. *n_surv is zeroed before.
+constexpr int kPrefilterT = 128;
 template <class R>
-__global__ void prefilter_kernel(const uint32_t* __restrict__ cflat, uint32_t m,
-                                 const uint32_t* __restrict__ mask, VoidViewT<R> voids, RungConstsT<R> rc,
-                                 bool keep_all, const CandOffT<R>* __restrict__ coff,
-                                 uint32_t* __restrict__ surv_cand, uint32_t* __restrict__ sflat,
-                                 R* __restrict__ scx, R* __restrict__ scy, R* __restrict__ scz,
-                                 uint8_t* __restrict__ sreason, R* __restrict__ soff,
-                                 uint32_t* __restrict__ n_surv) {
+__global__ void __launch_bounds__(kPrefilterT)
+    prefilter_kernel(const uint32_t* __restrict__ cflat, uint32_t m, uint32_t per,
+                     const uint32_t* __restrict__ mask, VoidViewT<R> voids, RungConstsT<R> rc,
+                     bool keep_all, const CandOffT<R>* __restrict__ coff,
+                     uint32_t* __restrict__ surv_cand, uint32_t* __restrict__ sflat,
+                     R* __restrict__ scx, R* __restrict__ scy, R* __restrict__ scz,
+                     uint8_t* __restrict__ sreason, R* __restrict__ soff, uint32_t* __restrict__ n_surv) {
   const uint32_t n = rc.grid_n;
   const unsigned lane = threadIdx.x & 31u;
-  for (uint32_t k0 = blockIdx.x * blockDim.x + threadIdx.x - lane; k0 < m; k0 += gridDim.x * blockDim.x) {
-    const uint32_t k = k0 + lane;
-    bool ok = k < m;
+  const uint32_t warps = gridDim.x * (kPrefilterT / 32);
+  const uint32_t w0 = blockIdx.x * (kPrefilterT / 32) + (threadIdx.x >> 5);
+  for (uint64_t k0 = (uint64_t)w0 * per; k0 < m; k0 += (uint64_t)warps * per) {
+    const uint32_t k = (uint32_t)k0 + lane;
+    bool ok = lane < per && k0 + lane < m;
     uint32_t flat = 0;
     CandOffT<R> o{R(0), R(0), R(0), R(-1.0f)};
     R cx = 0, cy = 0, cz = 0;
@@ -710,14 +677,20 @@ __global__ void prefilter_kernel(const uint32_t* __restrict__ cflat, uint32_t m,
       // gone by its turn (exodus_finder.c:1873-1875): nothing is refused here.
       if (!keep_all)
         ok = !cand_masked(mask, flat, o.len, rc.radius, rc) &&
-             !(rc.proxy_pole > 0 && overlap_quick(mask, n, ix, iy, iz, (uint32_t)rc.proxy_pole)) &&
-             !overlap_exact(voids, cx, cy, cz, rc.radius, rc.f, rc.scale, rc.box);
+             !(rc.proxy_pole > 0 && overlap_quick(mask, n, ix, iy, iz, (uint32_t)rc.proxy_pole));
     }
-    const unsigned bal = __ballot_sync(0xffffffffu, ok);
+    unsigned bal = __ballot_sync(0xffffffffu, ok);
+    if (!keep_all)
+      for (unsigned left = bal; left; left &= left - 1) {
+        const int q = __ffs(left) - 1;
+        if (overlap_exact_warp(voids, __shfl_sync(0xffffffffu, cx, q), __shfl_sync(0xffffffffu, cy, q),
+                               __shfl_sync(0xffffffffu, cz, q), rc.radius, rc.f, rc.scale, rc.box))
+          bal &= ~(1u << q);
+      }
     uint32_t at = 0;
     if (lane == 0 && bal) at = atomicAdd(n_surv, (uint32_t)__popc(bal));
     at = __shfl_sync(0xffffffffu, at, 0) + __popc(bal & ((1u << lane) - 1u));
-    if (ok) {
+    if (bal >> lane & 1u) {
       surv_cand[at] = k;
       sflat[at] = flat;
       scx[at] = cx;
@@ -735,9 +708,11 @@ void prefilter(const uint32_t* cand_flat, uint32_t m, const uint32_t* mask, Void
                uint8_t* sreason, uint32_t* d_surv_count, cudaStream_t st, bool keep_all,
                const CandOffT<R>* coff, R* soff) {
   if (m == 0) return;
-  prefilter_kernel<<<grid_for(m, 64), 64, 0, st>>>(cand_flat, m, mask, voids, rc, keep_all, coff,
-                                                   surv_cand, surv_flat, scx, scy, scz, sreason, soff,
-                                                   d_surv_count);
+  uint32_t per = 1;
+  while (per < 32 && m > 152u * 64u * per) per *= 2;  // a warp each while all fit at once
+  prefilter_kernel<<<grid_for((m + per - 1) / per * 32ull, kPrefilterT), kPrefilterT, 0, st>>>(
+      cand_flat, m, per, mask, voids, rc, keep_all, coff, surv_cand, surv_flat, scx, scy, scz, sreason,
+      soff, d_surv_count);
   SIFG_LAUNCH_CHECK();
 }
 
