@@ -346,12 +346,16 @@ template <ColMode kMode>
 __global__ void __launch_bounds__(32 * kColCols, 2)
     colfft512_kernel(const float2* src, float2* dst, ColumnLayout in, ColumnLayout out,
                      const float2* __restrict__ tw, RadialFilter rf, const float* __restrict__ win,
-                     float norm, const float* __restrict__ ftab) {
+                     float norm, const float* __restrict__ ftab, bool backwards) {
   extern __shared__ float2 ex[];  // element e of column c at e * kColCols + c
   const uint32_t c = threadIdx.x % kColCols, j = threadIdx.x / kColCols;
-  const bool last = blockIdx.x >= 512 * 16;
-  const uint32_t line = last ? (blockIdx.x - 512 * 16) * kColCols + c : blockIdx.x / 16;
-  const uint32_t kb = last ? 16 : blockIdx.x % 16, kz = last ? 256 : kb * 16 + c;
+  // From the end backwards where the pass before went forwards within the same
+  // planes: its last ones are still in L2 (the forward's ky after its rows: 186
+  // to 174 us; the inverse's rows turned round after its ky 172 to 161).
+  const uint32_t b = backwards ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
+  const bool last = b >= 512 * 16;
+  const uint32_t line = last ? (b - 512 * 16) * kColCols + c : b / 16;
+  const uint32_t kb = last ? 16 : b % 16, kz = last ? 256 : kb * 16 + c;
   float2 v[16];
   {
     const float2* p = src + (size_t)line * in.line + kb * in.kblock + (kz & 15u) + (size_t)j * in.elem;
@@ -473,8 +477,11 @@ __global__ void __launch_bounds__(16 * kRowsPerCta, 3)
     c2r512_rows_kernel(const float2* __restrict__ work, float* __restrict__ out,
                        const float2* __restrict__ tw, BelowList below) {
   __shared__ float2 buf[kRowsPerCta * 256];
-  const uint32_t x = blockIdx.x / (512 / kRowsPerCta);
-  const uint32_t y0 = (blockIdx.x % (512 / kRowsPerCta)) * kRowsPerCta;
+  // From the end backwards: the pass along ky, just before, left the last planes
+  // it wrote in L2.
+  const uint32_t block = gridDim.x - 1 - blockIdx.x;
+  const uint32_t x = block / (512 / kRowsPerCta);
+  const uint32_t y0 = (block % (512 / kRowsPerCta)) * kRowsPerCta;
   const unsigned j = threadIdx.x & 15u, ry = threadIdx.x >> 4;
   // The row's kz block 0; a kz block further is 512 rows of 16 on.
   const float2* p = work + ((size_t)x * kKzBlocks * 512 + y0 + ry) * 16 + j;
@@ -525,13 +532,13 @@ __global__ void __launch_bounds__(16 * kRowsPerCta, 3)
     pos += w < warp ? ws[w] : 0u;
     total += ws[w];
   }
-  if (threadIdx.x == 0) below.counts[blockIdx.x] = total;
+  if (threadIdx.x == 0) below.counts[block] = total;
   if (n_warp == 0) return;
   const uint32_t row_lanes = lane < 16 ? 0xffffu : 0xffff0000u;
   const uint32_t lower = row_lanes & ((1u << lane) - 1u);
   if (lane >= 16) pos += n_first;
   const uint32_t cell0 = ((x * 512 + y0 + ry) * 512) + 2 * j;
-  const size_t region = (size_t)blockIdx.x * (kRowsPerCta * 512);
+  const size_t region = (size_t)block * (kRowsPerCta * 512);
 #pragma unroll
   for (int k = 0; k < 16; k++) {
     const uint32_t b = (bits >> (2 * k)) & 3u;
@@ -849,7 +856,8 @@ constexpr ColumnLayout kTilesByRow{kColCols, 512 * kColCols, kKzBlocks * 512 * k
 template <ColMode kMode>
 static void launch_columns(const SmootherT<float>& s, const DevBuf& src, const DevBuf& dst,
                            ColumnLayout in, ColumnLayout out, const RadialFilter& rf = kNoFilter,
-                           const float* win = nullptr, float norm = 1.f, const float* ftab = nullptr) {
+                           const float* win = nullptr, float norm = 1.f, const float* ftab = nullptr,
+                           bool backwards = false) {
   thread_local bool attr = false;  // the attribute is per thread's view of the function
   if (!attr) {
     SIFG_CUDA(cudaFuncSetAttribute(colfft512_kernel<kMode>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -857,7 +865,8 @@ static void launch_columns(const SmootherT<float>& s, const DevBuf& src, const D
     attr = true;
   }
   colfft512_kernel<kMode><<<kColCtas, 32 * kColCols, kColBytes, s.stream>>>(
-      src.as<float2>(), dst.as<float2>(), in, out, (const float2*)s.twiddles, rf, win, norm, ftab);
+      src.as<float2>(), dst.as<float2>(), in, out, (const float2*)s.twiddles, rf, win, norm, ftab,
+      backwards);
   SIFG_LAUNCH_CHECK();
 }
 
@@ -869,7 +878,8 @@ static void launch_forward512(const SmootherT<float>& s, const float* grid, cons
   r2c512_rows_kernel<<<N * N / kRowsPerCta, 16 * kRowsPerCta, 0, s.stream>>>(
       grid, s.work.as<float2>(), (const float2*)s.twiddles, mean);
   SIFG_LAUNCH_CHECK();
-  launch_columns<kColForward>(s, s.work, s.work, kTilesByLine, kTilesByLine);
+  launch_columns<kColForward>(s, s.work, s.work, kTilesByLine, kTilesByLine, kNoFilter, nullptr, 1.f,
+                              nullptr, true);
   launch_columns<kColForward>(s, s.work, s.spectrum, kTilesByRow, kTilesByLine);
 }
 
