@@ -116,7 +116,7 @@ __global__ void box_check_kernel(const R* __restrict__ x, const R* __restrict__ 
        i += (uint64_t)gridDim.x * blockDim.x) {
     const R v[3] = {x[i], y[i], z[i]};
     bool ok = true;
-    for (int a = 0; a < 3; a++) ok = ok && v[a] >= lo && v[a] <= hi;  // false for NaN
+    for (int a = 0; a < 3; a++) ok = ok && within(v[a], lo, hi);  // false for NaN
     bad += ok ? 0u : 1u;
   }
   for (int d = 16; d > 0; d >>= 1) bad += __shfl_down_sync(0xffffffffu, bad, d);

@@ -80,6 +80,32 @@ __device__ bool is_minimum(const R* __restrict__ f, uint32_t n, uint64_t i) {
   return true;
 }
 
+// v <= thr: a double's by its bits (see in_box), which fold to integers in
+// order of value; below -infinity lie the negative NaNs, above infinity the
+// others. A thread's 32 compares took the FP64 pipe 29 us a 256^3 field.
+__device__ __forceinline__ long long ordered(double v) {
+  const long long b = __double_as_longlong(v);
+  return b ^ ((b >> 63) & 0x7fffffffffffffffll);
+}
+struct AtMost64 {
+  static constexpr long long kLowest = (long long)0x800fffffffffffffull;  // ordered(-infinity)
+  unsigned long long reach;  // from -infinity's place to thr's
+  bool any;
+  __device__ __forceinline__ explicit AtMost64(double thr)
+      : reach((unsigned long long)ordered(thr == 0.0 ? 0.0 : thr) - (unsigned long long)kLowest),
+          any(thr == thr) {}
+  __device__ __forceinline__ bool operator()(double v) const {
+    return any && (unsigned long long)ordered(v) - (unsigned long long)kLowest <= reach;
+  }
+};
+struct AtMost32 {
+  float thr;
+  __device__ __forceinline__ explicit AtMost32(float t) : thr(t) {}
+  __device__ __forceinline__ bool operator()(float v) const { return v <= thr; }
+};
+template <class R>
+using AtMost = std::conditional_t<sizeof(R) == 8, AtMost64, AtMost32>;
+
 // One pass over the field: each CTA writes its candidates, in flat order, to
 // the start of its own region of kScanChunk slots and its count to
 // counts[block]; the compaction then moves only the candidates. A warp takes
@@ -108,13 +134,14 @@ __global__ void __launch_bounds__(kScanT) scan_regions_kernel(
   const uint64_t first = base + (uint64_t)warp * (128 * kScanRounds) + lane * 4;
   R v[kScanRounds][4];
   uint32_t bits = 0;
+  const AtMost<R> at_most(thr);
   if (base + kScanChunk <= n) {
 #pragma unroll
     for (int j = 0; j < kScanRounds; j++) load4(f, first + 128 * j, v[j]);
 #pragma unroll
     for (int j = 0; j < kScanRounds; j++)
 #pragma unroll
-      for (int k = 0; k < 4; k++) bits |= v[j][k] <= thr ? 1u << (4 * j + k) : 0u;
+      for (int k = 0; k < 4; k++) bits |= at_most(v[j][k]) ? 1u << (4 * j + k) : 0u;
   } else {
 #pragma unroll
     for (int j = 0; j < kScanRounds; j++)
@@ -122,7 +149,7 @@ __global__ void __launch_bounds__(kScanT) scan_regions_kernel(
       for (int k = 0; k < 4; k++) {
         const uint64_t c = first + 128 * j + k;
         v[j][k] = c < n ? __ldg(f + c) : R(0);
-        bits |= c < n && v[j][k] <= thr ? 1u << (4 * j + k) : 0u;
+        bits |= c < n && at_most(v[j][k]) ? 1u << (4 * j + k) : 0u;
       }
   }
   for (uint32_t b = bits; b; b &= b - 1) {

@@ -45,10 +45,10 @@ template <class R>
 __device__ __forceinline__ uint32_t mesh_cell(R& x, R& y, R& z, const MeshGeom<R>& g) {
   const int32_t hi = (int32_t)g.n - 1;
   int32_t ix, iy, iz;
-  if (x >= R(0) && x < g.box && y >= R(0) && y < g.box && z >= R(0) && z < g.box) {
-    ix = (int32_t)fmul(x, g.inv_l);
-    iy = (int32_t)fmul(y, g.inv_l);
-    iz = (int32_t)fmul(z, g.inv_l);
+  if (in_box(x, g.box) && in_box(y, g.box) && in_box(z, g.box)) {
+    ix = (int32_t)whole_part(fmul(x, g.inv_l));
+    iy = (int32_t)whole_part(fmul(y, g.inv_l));
+    iz = (int32_t)whole_part(fmul(z, g.inv_l));
   } else {
     x = box_fold(x, g.box);
     y = box_fold(y, g.box);
@@ -92,9 +92,7 @@ __global__ void __launch_bounds__(kMeshT) cell_count_kernel(
       uint32_t c = 0xffffffffu;
       if (base + u * kMeshT + threadIdx.x < n) {
         if (outside)
-          bad += px[u] >= lo && px[u] <= hi && py[u] >= lo && py[u] <= hi && pz[u] >= lo && pz[u] <= hi
-                     ? 0u
-                     : 1u;
+          bad += within(px[u], lo, hi) && within(py[u], lo, hi) && within(pz[u], lo, hi) ? 0u : 1u;
         c = mesh_cell(px[u], py[u], pz[u], g);
       }
       const unsigned peers = __match_any_sync(0xffffffffu, c);
