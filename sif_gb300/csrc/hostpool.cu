@@ -22,7 +22,7 @@ namespace sifg {
 
 namespace {
 
-constexpr size_t kPoolBlocks = 8;
+constexpr size_t kPoolBlocks = 32;
 constexpr size_t kPoolBytes = 24ull << 30;
 
 struct Block {
