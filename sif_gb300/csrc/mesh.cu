@@ -257,7 +257,7 @@ __device__ __forceinline__ void canon_cell(const MeshRec<R>* __restrict__ tmp, u
 // `more` (more[0] counts them) for cell_canon_large_kernel, which takes four
 // times the registers.
 template <class R>
-__global__ void __launch_bounds__(kCanonT) cell_canon_kernel(
+__global__ void __launch_bounds__(kCanonT, 4) cell_canon_kernel(
     const MeshRec<R>* __restrict__ tmp, const uint32_t* __restrict__ offsets,
     uint32_t n_cells_total, R* __restrict__ ox, R* __restrict__ oy, R* __restrict__ oz,
     uint32_t* __restrict__ orig, uint32_t* __restrict__ more, uint32_t span) {
