@@ -2,10 +2,11 @@
 // (src/finder/exodus_finder.c:1585-2492) for a periodic box, unweighted,
 // seeds (every cell, or the local minima) on their nodes.
 //
-// Per rung, on one stream:
-//   smooth (filter + C2R)  ->  candidate count  ->  [host: M]  ->  candidate
-//   write  ->  copy to the host  ->  pre-filter  ->  sphere growth of every
-//   survivor  ->  commit rounds  ->  append in rank order  ->  void index.
+// Per rung:
+//   smooth (filter + C2R) and, until a void is accepted, scan, on the rung's
+//   lane  ->  [host: M]  ->  candidate write (depths straight to the host)  ->
+//   pre-filter  ->  sphere growth of every survivor  ->  commit rounds,
+//   append in rank order and void index (one launch up to 4,096 candidates).
 // While the GPU runs the pre-filter and the sphere growth, the host replays
 // the reference's quicksort over the candidates (the depth order, ties
 // included, is part of what the reference's catalogue is) and uploads each

@@ -3,7 +3,7 @@
 // passes each (kx, ky as columns of the half spectrum, kz as rows).
 //
 // What bounds them is the FP64 pipe: two fused multiply-adds a clock an SM,
-// 580 G/s for the GPU, against some 40 us of memory traffic a pass at 256^3.
+// 630 G/s for the GPU, against some 40 us of memory traffic a pass at 256^3.
 // A pass takes its count of FP64 instructions over that rate and everything
 // else -- the shared memory exchanges, the integer work of quarter turns, the
 // filter's gathers -- runs beside it. So the transforms are laid out to need
@@ -22,7 +22,7 @@
 // A 16-point transform is 148 instructions, 178 with its twiddles; a
 // 256-point column 5,216 (a fused radix-16 with whole complex products:
 // 6,200), a row of 256 reals 2,900. 256^3, at the pipe's rate and measured: the
-// pass that filters 342 and 350 us, the other columns 298 and 317, the rows 326
+// pass that filters 315 and 350 us, the other columns 274 and 317, the rows 300
 // and 361; cuFFT's three passes and the filter kernel took 1,870 a smoothing
 // (here 1,030). Against the identity the error is 4.8e-16 rms, 5.6e-16 before.
 //

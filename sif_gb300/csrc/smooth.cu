@@ -354,7 +354,11 @@ __global__ void __launch_bounds__(32 * kColCols, 2)
   // to 174 us; the inverse's rows turned round after its ky 172 to 161).
   const uint32_t b = backwards ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
   const bool last = b >= 512 * 16;
-  const uint32_t line = last ? (b - 512 * 16) * kColCols + c : b / 16;
+  // The filter's lines in the order 0, 1, 511, 2, 510, ...: ky and -ky share the
+  // table's entries, which are still in L2 for the second (read from memory
+  // twice 712 MB a pass, 234 us; kPairNow).
+  uint32_t line = last ? (b - 512 * 16) * kColCols + c : b / 16;
+  if (kMode == kColTable && !last) line = (line & 1u) ? (line + 1) / 2 : (512 - line / 2) & 511u;
   const uint32_t kb = last ? 16 : b % 16, kz = last ? 256 : kb * 16 + c;
   float2 v[16];
   {
