@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(32 * kColCols, 2)
   const bool last = b >= 512 * 16;
   // The filter's lines in the order 0, 1, 511, 2, 510, ...: ky and -ky share the
   // table's entries, which are still in L2 for the second (read from memory
-  // twice 712 MB a pass, 234 us; kPairNow).
+  // twice, 712 MB a pass and 234 us; 650 and 221).
   uint32_t line = last ? (b - 512 * 16) * kColCols + c : b / 16;
   if (kMode == kColTable && !last) line = (line & 1u) ? (line + 1) / 2 : (512 - line / 2) & 511u;
   const uint32_t kb = last ? 16 : b % 16, kz = last ? 256 : kb * 16 + c;
