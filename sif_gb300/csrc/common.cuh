@@ -131,11 +131,14 @@ __device__ __forceinline__ bool within(double v, double lo, double hi) {
   return (unsigned long long)__double_as_longlong(v) <= (unsigned long long)__double_as_longlong(hi) ||
          (v >= lo && v <= hi);
 }
-// The whole part of 0 <= u < 2^31.
+// The whole part of 0 <= u < 2^31; 2^32 - 1 for infinity and 0 for NaN, which a
+// coordinate over a cell length too small for a reciprocal gives: the callers
+// clamp what they index with, as an unsigned number.
 __device__ __forceinline__ uint32_t whole_part(float u) { return (uint32_t)u; }
 __device__ __forceinline__ uint32_t whole_part(double u) {
   const uint32_t hi = (uint32_t)__double2hiint(u) & 0x7fffffffu, lo = (uint32_t)__double2loint(u);
   const int e = (int)(hi >> 20) - 1023;
+  if (e == 1024) return (hi & 0xfffffu) | lo ? 0u : 0xffffffffu;
   return e < 0 ? 0u : (0x80000000u | hi << 11 | lo >> 21) >> (31 - e);
 }
 

@@ -40,24 +40,26 @@ static_assert(sizeof(MeshRec<double>) == 32, "double records are 32 bytes");
 
 // A particle's cell, its coordinates folded into the box on the way. Nearly
 // every coordinate is in [0, box), where the fold and the clamp at zero do
-// nothing; any that is not (NaN among them) takes all three through them.
+// nothing; any that is not (NaN among them) takes all three through them. The
+// clamp into the mesh holds for what an infinite 1 / cell_length makes of a
+// coordinate too (a box below about n / FLT_MAX a side).
 template <class R>
 __device__ __forceinline__ uint32_t mesh_cell(R& x, R& y, R& z, const MeshGeom<R>& g) {
-  const int32_t hi = (int32_t)g.n - 1;
-  int32_t ix, iy, iz;
+  const uint32_t hi = g.n - 1;
+  uint32_t ix, iy, iz;
   if (in_box(x, g.box) && in_box(y, g.box) && in_box(z, g.box)) {
-    ix = (int32_t)whole_part(fmul(x, g.inv_l));
-    iy = (int32_t)whole_part(fmul(y, g.inv_l));
-    iz = (int32_t)whole_part(fmul(z, g.inv_l));
+    ix = whole_part(fmul(x, g.inv_l));
+    iy = whole_part(fmul(y, g.inv_l));
+    iz = whole_part(fmul(z, g.inv_l));
   } else {
     x = box_fold(x, g.box);
     y = box_fold(y, g.box);
     z = box_fold(z, g.box);
-    ix = max((int32_t)fmul(x, g.inv_l), 0);
-    iy = max((int32_t)fmul(y, g.inv_l), 0);
-    iz = max((int32_t)fmul(z, g.inv_l), 0);
+    ix = (uint32_t)max((int32_t)fmul(x, g.inv_l), 0);
+    iy = (uint32_t)max((int32_t)fmul(y, g.inv_l), 0);
+    iz = (uint32_t)max((int32_t)fmul(z, g.inv_l), 0);
   }
-  return ((uint32_t)min(ix, hi) * g.n + (uint32_t)min(iy, hi)) * g.n + (uint32_t)min(iz, hi);
+  return (min(ix, hi) * g.n + min(iy, hi)) * g.n + min(iz, hi);
 }
 
 // The passes over the particles wait on their loads and on the atomics that
