@@ -358,15 +358,55 @@ struct TilePlace {
   }
 };
 
+// One particle's corners added into a tile's words.
+__device__ __forceinline__ void add_particle(const float4& r, uint32_t* acc) {
+  constexpr float qscale = (float)kWhole;
+  const float wx0 = fsub(1.0f, r.x), wy0 = fsub(1.0f, r.y), wz0 = fsub(1.0f, r.z);
+  const float w00 = fmul(wx0, wy0), w01 = fmul(wx0, r.y);
+  const float w10 = fmul(r.x, wy0), w11 = fmul(r.x, r.y);
+  const float w[8] = {fmul(w00, wz0), fmul(w00, r.z), fmul(w01, wz0), fmul(w01, r.z),
+                      fmul(w10, wz0), fmul(w10, r.z), fmul(w11, wz0), fmul(w11, r.z)};
+  uint32_t* cell = acc + tile_cell(__float_as_uint(r.w));
+  uint32_t sum = 0, big = 0;
+  float wbig = w[0];
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    const uint32_t q = __float_as_uint(__fmaf_rn(w[k], qscale, 8388608.0f)) - 0x4b000000u;
+    atomicAdd(cell + corner_offset(k), q);
+    sum += q;
+    if (k > 0 && w[k] > wbig) {  // the first largest, as corner_quanta finds it
+      wbig = w[k];
+      big = corner_offset(k);
+    }
+  }
+  atomicAdd(cell + big, (uint32_t)kWhole - sum);
+}
+
+// A node of a tile, at (a, b, c) of it: straight to the grid where no other
+// tile touches it, else to its face buffer; nothing where it lies past the grid.
+__device__ __forceinline__ void put_node(const TilePlace& t, const CicGeom& g, uint32_t a, uint32_t b,
+                                         uint32_t c, unsigned long long v, float qinv, float inv_cell_vol,
+                                         float* __restrict__ grid, const FaceBufs& faces) {
+  if (a > t.ex || b > t.ey || c > t.ez) return;
+  const uint32_t gx = t.ox + a == g.n ? 0u : t.ox + a;
+  const uint32_t gy = t.oy + b == g.n ? 0u : t.oy + b;
+  const uint32_t gz = t.oz + c == g.n ? 0u : t.oz + c;
+  if (a >= 1 && a < t.ex && b >= 1 && b < t.ey && c >= 1 && c < t.ez)
+    grid[((uint64_t)gx * g.n + gy) * g.n + gz] =
+        fmul(fmul(__ll2float_rn((long long)v), qinv), inv_cell_vol);
+  else if (v != 0ull)
+    atomicAdd(face_slot(faces, gx, gy, gz, g), v);
+}
+
 // The unweighted deposit, one CTA a tile at a time: the tile's sums as one
 // 32-bit word a cell, one shared atomic a corner. The word's wraps are not
 // watched add by add: every quantum is non-negative (the weights are, and the
 // remainder of a few quanta goes to a corner of at least 2^21), so the words
 // of a tile sum to its particles times 2^24 exactly when none of them wrapped,
 // and each wrap takes 2^32 from that sum. A tile whose sum falls short (a cell
-// of 256 particles or more, in an unweighted count) is left to
-// tile_deposit_wide_kernel, through `redo` (redo[0] counts them), as is one
-// with so many particles that one of its cells must have wrapped.
+// of 256 particles or more) is left to tile_dense_kernel, through `redo`
+// (redo[0] counts them), as is one of more than `dense` particles, which all but
+// surely has such a cell.
 // (Two words a cell, as the wide kernel keeps, cost a second atomic a corner:
 // the 512^3 deposit 1.57 ms in 39 KB of shared memory a CTA, 1.23 with one.)
 //
@@ -382,43 +422,23 @@ struct TilePlace {
 // half of the kernel).
 __global__ void __launch_bounds__(kDepositT, 6) tile_deposit_kernel(
     const float4* __restrict__ rec, const uint32_t* __restrict__ offsets, CicGeom g,
-    float inv_cell_vol, float* __restrict__ grid, FaceBufs faces, uint32_t* __restrict__ redo) {
+    float inv_cell_vol, float* __restrict__ grid, FaceBufs faces, uint32_t dense,
+    uint32_t* __restrict__ redo) {
   __shared__ uint32_t acc[kTileWords];
   __shared__ unsigned long long wsum[kDepositT / 32];
   const uint32_t n_tiles = g.nt * g.nt * g.nt;
-  constexpr float qscale = (float)kWhole, qinv = 1.0f / (float)kWhole;
+  constexpr float qinv = 1.0f / (float)kWhole;
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   // Cleared once; each flush leaves the cells it reads cleared for the next tile.
   for (int i = threadIdx.x; i < kTileWords; i += kDepositT) acc[i] = 0u;
   __syncthreads();
   for (uint32_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
     const uint32_t s = offsets[tile], e = offsets[tile + 1];
-    if (e - s >= 256u * kTileWords) {  // a cell must pass 256 particles
+    if (e - s > dense) {
       if (threadIdx.x == 0) redo[1 + atomicAdd(redo, 1u)] = tile;
       continue;
     }
-    for (uint32_t p = s + threadIdx.x; p < e; p += kDepositT) {
-      const float4 r = __ldg(rec + p);
-      const float wx0 = fsub(1.0f, r.x), wy0 = fsub(1.0f, r.y), wz0 = fsub(1.0f, r.z);
-      const float w00 = fmul(wx0, wy0), w01 = fmul(wx0, r.y);
-      const float w10 = fmul(r.x, wy0), w11 = fmul(r.x, r.y);
-      const float w[8] = {fmul(w00, wz0), fmul(w00, r.z), fmul(w01, wz0), fmul(w01, r.z),
-                          fmul(w10, wz0), fmul(w10, r.z), fmul(w11, wz0), fmul(w11, r.z)};
-      uint32_t* cell = acc + tile_cell(__float_as_uint(r.w));
-      uint32_t sum = 0, big = 0;
-      float wbig = w[0];
-#pragma unroll
-      for (int k = 0; k < 8; k++) {
-        const uint32_t q = __float_as_uint(__fmaf_rn(w[k], qscale, 8388608.0f)) - 0x4b000000u;
-        atomicAdd(cell + corner_offset(k), q);
-        sum += q;
-        if (k > 0 && w[k] > wbig) {  // the first largest, as corner_quanta finds it
-          wbig = w[k];
-          big = corner_offset(k);
-        }
-      }
-      atomicAdd(cell + big, (uint32_t)kWhole - sum);
-    }
+    for (uint32_t p = s + threadIdx.x; p < e; p += kDepositT) add_particle(__ldg(rec + p), acc);
     __syncthreads();
     unsigned long long sum = 0;
     for (int i = threadIdx.x; i < kTileWords; i += kDepositT) sum += acc[i];
@@ -482,9 +502,91 @@ __global__ void __launch_bounds__(kDepositT, 6) tile_deposit_kernel(
   }
 }
 
-// The deposit of any sums: weighted particles, and the tiles the kernel above
-// lists in `redo` (NULL: every tile). Two 32-bit words a cell: a 32-bit
-// shared atomic add is one instruction, a 64-bit one a compare-and-swap loop
+// The tiles with a cell of 256 particles or more, listed by the kernel above:
+// each cell's sum from two passes over the tile's particles in the one word a
+// cell, the quanta modulo 2^32 and then the quanta over 2^12. A word of up to
+// kDensePart particles' quanta over 2^12 does not wrap, and times 2^12 falls
+// short of their sum by less than 2^12 a particle: the sum is the one number
+// within 2^32 from there up with those low 32 bits. A tile of more particles
+// takes that many at a time. Most tiles of a clustered snapshot come here, and
+// the kernel ends with its densest: kDenseUnroll records in flight a thread.
+//
+// (Two words a cell in one pass over the particles, one CTA an SM as so few
+// were expected: half of 16.7 M particles in haloes, on 200^3, 2.37 ms a
+// deposit, now 1.61; every tile that way from the first, 1.98. In the kernel
+// above, which has the first pass's words: 0.110 to 0.117 ms for 16.7 M uniform
+// particles' tiles, none of them dense.)
+constexpr uint32_t kDensePart = (1u << 20) - 1;
+constexpr int kDenseUnroll = 4;
+template <class Each>
+__device__ __forceinline__ void each_record(const float4* __restrict__ rec, uint32_t s, uint32_t e, Each each) {
+  for (uint32_t p = s + threadIdx.x; p < e; p += kDenseUnroll * kDepositT) {
+    float4 r[kDenseUnroll];
+#pragma unroll
+    for (int u = 0; u < kDenseUnroll; u++)
+      if (p + u * kDepositT < e) r[u] = __ldg(rec + p + u * kDepositT);
+#pragma unroll
+    for (int u = 0; u < kDenseUnroll; u++)
+      if (p + u * kDepositT < e) each(r[u]);
+  }
+}
+
+__global__ void __launch_bounds__(kDepositT) tile_dense_kernel(
+    const float4* __restrict__ rec, const uint32_t* __restrict__ offsets, CicGeom g,
+    float inv_cell_vol, float* __restrict__ grid, FaceBufs faces, const uint32_t* __restrict__ redo) {
+  __shared__ uint32_t acc[kTileWords];
+  constexpr int kPer = (kTileWords + kDepositT - 1) / kDepositT;  // words a thread
+  const uint32_t n_items = redo[0];
+  if (blockIdx.x >= n_items) return;
+  for (int i = threadIdx.x; i < kTileWords; i += kDepositT) acc[i] = 0u;
+  __syncthreads();
+  for (uint32_t item = blockIdx.x; item < n_items; item += gridDim.x) {
+    const uint32_t tile = redo[1 + item], s = offsets[tile], e = offsets[tile + 1];
+    unsigned long long v[kPer] = {};
+    for (uint32_t p0 = s, p1; p0 < e; p0 = p1) {
+      p1 = p0 + min(kDensePart, e - p0);
+      each_record(rec, p0, p1, [&](const float4& r) { add_particle(r, acc); });
+      __syncthreads();
+      uint32_t lo[kPer];
+#pragma unroll
+      for (int j = 0; j < kPer; j++) {
+        const uint32_t i = threadIdx.x + j * kDepositT;
+        if (i >= kTileWords) break;
+        lo[j] = acc[i];
+        acc[i] = 0u;
+      }
+      __syncthreads();
+      each_record(rec, p0, p1, [&](const float4& r) {
+        uint32_t q[8];
+        corner_quanta(r.x, r.y, fsub(1.0f, r.z), r.z, (float)kWhole, kWhole, q);
+        uint32_t* cell = acc + tile_cell(__float_as_uint(r.w));
+#pragma unroll
+        for (int k = 0; k < 8; k++) atomicAdd(cell + corner_offset(k), q[k] >> 12);
+      });
+      __syncthreads();
+#pragma unroll
+      for (int j = 0; j < kPer; j++) {
+        const uint32_t i = threadIdx.x + j * kDepositT;
+        if (i >= kTileWords) break;
+        const unsigned long long least = (unsigned long long)acc[i] << 12;
+        v[j] += least + (uint32_t)(lo[j] - (uint32_t)least);
+        acc[i] = 0u;
+      }
+      __syncthreads();
+    }
+    const TilePlace t(tile, g);
+#pragma unroll
+    for (int j = 0; j < kPer; j++) {
+      const uint32_t i = threadIdx.x + j * kDepositT;
+      if (i >= kTileWords) break;
+      put_node(t, g, i / (TS * TS), i / TS % TS, i % TS, v[j], 1.0f / (float)kWhole, inv_cell_vol, grid,
+               faces);
+    }
+  }
+}
+
+// The weighted deposit. Two 32-bit words a cell: a 32-bit shared atomic add is
+// one instruction, a 64-bit one a compare-and-swap loop
 // (measured: the 512^3 deposit with one 64-bit add per corner took 3.4 ms,
 // against 1.7). A tile with fewer than 2^16 particles adds each quantum's low
 // 16 bits to the first word and its high bits (arithmetic shift) to the
@@ -496,40 +598,28 @@ __global__ void __launch_bounds__(kDepositT, 6) tile_deposit_kernel(
 __global__ void __launch_bounds__(kDepositT) tile_deposit_wide_kernel(
     const float4* __restrict__ rec, const uint32_t* __restrict__ offsets, CicGeom g,
     float inv_cell_vol, float* __restrict__ grid, FaceBufs faces,
-    const float* __restrict__ wrec, const unsigned* __restrict__ wmax,
-    const uint32_t* __restrict__ redo) {
+    const float* __restrict__ wrec, const unsigned* __restrict__ wmax) {
   extern __shared__ uint32_t acc_lo[];  // TS^3 words, then TS^3 carries
   uint32_t* acc_hi = acc_lo + kTileWords;
-  const uint32_t n_items = redo ? redo[0] : g.nt * g.nt * g.nt;
-  if (blockIdx.x >= n_items) return;
-  // The quantum: 2^-24 of a particle, or of the largest weight's binade.
-  float qscale = (float)kWhole, qinv = 1.0f / (float)kWhole;
-  if (wrec) {
-    const int e = weight_scale_exp(wmax);
-    qscale = __uint_as_float((uint32_t)(127 + e) << 23);
-    qinv = __uint_as_float((uint32_t)(127 - e) << 23);
-  }
+  const uint32_t n_tiles = g.nt * g.nt * g.nt;
+  // The quantum: 2^-24 of the largest weight's binade.
+  const int we = weight_scale_exp(wmax);
+  const float qscale = __uint_as_float((uint32_t)(127 + we) << 23);
+  const float qinv = __uint_as_float((uint32_t)(127 - we) << 23);
   // Cleared once; each flush leaves the cells it reads cleared for the next tile.
   for (int i = threadIdx.x; i < 2 * kTileWords; i += kDepositT) acc_lo[i] = 0u;
   __syncthreads();
-  for (uint32_t item = blockIdx.x; item < n_items; item += gridDim.x) {
-    const uint32_t tile = redo ? redo[1 + item] : item;
+  for (uint32_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
     const uint32_t s = offsets[tile], e = offsets[tile + 1];
     const bool split = e - s < (1u << 16);
     for (uint32_t p = s + threadIdx.x; p < e; p += kDepositT) {
       const float4 r = __ldg(rec + p);
-      float wz0 = fsub(1.0f, r.z), wz1 = r.z;
-      int whole = kWhole;
-      if (wrec) {
-        // A non-finite weight is added afterwards, outside the sums.
-        float pw = __ldg(wrec + p);
-        if ((__float_as_uint(pw) & 0x7fffffffu) >= 0x7f800000u) pw = 0.0f;
-        wz0 = fmul(pw, wz0);
-        wz1 = fmul(pw, wz1);
-        whole = __float2int_rn(fmul(pw, qscale));  // the particle's own quantised weight
-      }
+      // A non-finite weight is added afterwards, outside the sums.
+      float pw = __ldg(wrec + p);
+      if ((__float_as_uint(pw) & 0x7fffffffu) >= 0x7f800000u) pw = 0.0f;
       uint32_t q[8];
-      corner_quanta(r.x, r.y, wz0, wz1, qscale, whole, q);
+      corner_quanta(r.x, r.y, fmul(pw, fsub(1.0f, r.z)), fmul(pw, r.z), qscale,
+                    __float2int_rn(fmul(pw, qscale)), q);  // summing to the weight's own quanta
       const uint32_t cell = tile_cell(__float_as_uint(r.w));
       // One shared atomic per word and corner. (Reducing lanes bound for the
       // same cell first with __reduce_add_sync over each lane group's own mask
@@ -556,25 +646,14 @@ __global__ void __launch_bounds__(kDepositT) tile_deposit_wide_kernel(
       }
     }
     __syncthreads();
-    // Nodes 1 .. e-1 of the tile on every axis are touched by no other tile
-    // and go straight to the grid; the rest are shared with a neighbour.
     const TilePlace t(tile, g);
     for (int i = threadIdx.x; i < kTileWords; i += kDepositT) {
-      const uint32_t a = i / (TS * TS), b = (i / TS) % TS, c = i % TS;
-      if (a > t.ex || b > t.ey || c > t.ez) continue;
       const unsigned long long v =
           split ? (unsigned long long)((long long)(int)acc_hi[i] * 65536ll + (long long)acc_lo[i])
                 : ((unsigned long long)acc_hi[i] << 32) | acc_lo[i];
       acc_lo[i] = 0u;
       acc_hi[i] = 0u;
-      const uint32_t gx = t.ox + a == g.n ? 0u : t.ox + a;
-      const uint32_t gy = t.oy + b == g.n ? 0u : t.oy + b;
-      const uint32_t gz = t.oz + c == g.n ? 0u : t.oz + c;
-      if (a >= 1 && a < t.ex && b >= 1 && b < t.ey && c >= 1 && c < t.ez)
-        grid[((uint64_t)gx * g.n + gy) * g.n + gz] =
-            fmul(fmul(__ll2float_rn((long long)v), qinv), inv_cell_vol);
-      else if (v != 0ull)
-        atomicAdd(face_slot(faces, gx, gy, gz, g), v);
+      put_node(t, g, i / (TS * TS), i / TS % TS, i % TS, v, qinv, inv_cell_vol, grid, faces);
     }
     __syncthreads();
   }
@@ -1059,18 +1138,22 @@ void cic_deposit(const float* x, const float* y, const float* z, uint64_t n_part
   auto grid_of = [&](unsigned per_sm) { return (unsigned)std::min<uint64_t>(b.tiles, 152u * per_sm); };
   if (timer) timer->begin(st);
   if (w) {
-    tile_deposit_wide_kernel<<<grid_of(5), kDepositT, smem, st>>>(b.rec, b.counts, g, inv_cell_vol,
-                                                                  grid, b.faces, b.wrec, b.wmax, nullptr);
+    tile_deposit_wide_kernel<<<grid_of(5), kDepositT, smem, st>>>(b.rec, b.counts, g, inv_cell_vol, grid,
+                                                                  b.faces, b.wrec, b.wmax);
     SIFG_LAUNCH_CHECK();
   } else {
-    // The scatter's cursors are free: the list of tiles to do again.
+    // The scatter's cursors are free: the list of tiles to do again. A tile of
+    // eight particles a node and four times the box's mean is taken for one of
+    // them unseen: it would be found to be one after a pass of its own.
     uint32_t* redo = b.cursor;
+    const uint64_t dense = std::min<uint64_t>(
+        std::max<uint64_t>(4 * n_particles / b.tiles, 8u * TB * TB * TB), kDensePart);
     SIFG_CUDA(cudaMemsetAsync(redo, 0, sizeof(uint32_t), st));
-    tile_deposit_kernel<<<grid_of(6), kDepositT, 0, st>>>(b.rec, b.counts, g, inv_cell_vol, grid,
-                                                          b.faces, redo);
+    tile_deposit_kernel<<<grid_of(6), kDepositT, 0, st>>>(b.rec, b.counts, g, inv_cell_vol, grid, b.faces,
+                                                          (uint32_t)dense, redo);
     SIFG_LAUNCH_CHECK();
-    tile_deposit_wide_kernel<<<grid_of(1), kDepositT, smem, st>>>(
-        b.rec, b.counts, g, inv_cell_vol, grid, b.faces, nullptr, nullptr, redo);
+    tile_dense_kernel<<<grid_of(4), kDepositT, 0, st>>>(b.rec, b.counts, g, inv_cell_vol, grid, b.faces,
+                                                        redo);
     SIFG_LAUNCH_CHECK();
   }
   if (timer) timer->end(st);
