@@ -59,3 +59,27 @@ def test_runs_of_cells(dev, counts):
     pos = [((c + rng.uniform(0.05, 0.95, len(cell))) * side).astype(np.float32)
            for c in (cell // 64, cell // 8 % 8, cell % 8)]
     _check(dev, pos, n_cells)
+
+
+# Neighbours of a few entries each, taken by a warp together up to 32 of them;
+# empty cells among them; and cells past what the warp holds between.
+@pytest.mark.parametrize("counts", [[1] * 512, [0, 1, 2] * 170, [4] * 8 + [0] * 100 + [16, 16, 1] * 60,
+                                    [31, 1, 32, 0, 33, 1, 0, 0, 31, 2] * 50, [0] * 31 + [32] + [0] * 480])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_neighbours_taken_together(dev, counts, dtype):
+    n_cells = 70  # enough for 32 neighbours a warp
+    rng = np.random.default_rng(len(counts))
+    cell = np.repeat(np.arange(len(counts)) + 7000, counts)
+    cell = cell[rng.permutation(len(cell))]
+    side = BOX / n_cells
+    pos = [((c + rng.uniform(0.05, 0.95, len(cell))) * side).astype(dtype)
+           for c in (cell // 4900, cell // 70 % 70, cell % 70)]
+    _check(dev, pos, n_cells)
+
+
+# The passes over the particles one and four a thread, about where they change.
+@pytest.mark.parametrize("n", [(1 << 17) - 1, 1 << 17, (1 << 17) + 1])
+@pytest.mark.parametrize("n_cells", [9, 100])
+def test_few_and_many_particles(dev, n, n_cells):
+    rng = np.random.default_rng(n)
+    _check(dev, [(rng.uniform(0, BOX, n) * 0.999999).astype(np.float32) for _ in range(3)], n_cells)
