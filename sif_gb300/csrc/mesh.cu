@@ -63,25 +63,28 @@ __device__ __forceinline__ uint32_t mesh_cell(R& x, R& y, R& z, const MeshGeom<R
 }
 
 // The passes over the particles wait on their loads and on the atomics that
-// hand out slots: kMeshUnroll particles a thread in flight. (One at a time,
-// the scatter of 64.5 M particles into 117^3 cells spent 87% of its stalls on
-// them.)
+// hand out slots: kMeshUnroll particles a thread in flight, U in the kernels.
+// (One at a time, the scatter of 64.5 M particles into 117^3 cells spent 87% of
+// its stalls on them.) One a thread up to kMeshFew particles, which do not fill
+// the SMs: four in a row are the longer way there. A mesh of 10,000 particles
+// 21.0 to 18.9 us past its count, of 120,000 26.1 to 24.8, of 250,000 the same.
 constexpr int kMeshT = 256;
 constexpr int kMeshUnroll = 4;
+constexpr uint64_t kMeshFew = 1u << 17;
 
 // With `outside` set, also counts the particles outside [lo, hi] on any axis
 // (NaN included): the box check, from the same reads.
-template <class R>
+template <class R, int U>
 __global__ void __launch_bounds__(kMeshT) cell_count_kernel(
     const R* __restrict__ x, const R* __restrict__ y, const R* __restrict__ z, uint64_t n,
     MeshGeom<R> g, uint32_t* __restrict__ counts, R lo, R hi,
     unsigned long long* __restrict__ outside) {
-  const uint64_t stride = (uint64_t)gridDim.x * kMeshT * kMeshUnroll;
+  const uint64_t stride = (uint64_t)gridDim.x * kMeshT * U;
   uint32_t bad = 0;
-  for (uint64_t base = (uint64_t)blockIdx.x * kMeshT * kMeshUnroll; base < n; base += stride) {
-    R px[kMeshUnroll], py[kMeshUnroll], pz[kMeshUnroll];
+  for (uint64_t base = (uint64_t)blockIdx.x * kMeshT * U; base < n; base += stride) {
+    R px[U], py[U], pz[U];
 #pragma unroll
-    for (int u = 0; u < kMeshUnroll; u++) {
+    for (int u = 0; u < U; u++) {
       const uint64_t p = base + u * kMeshT + threadIdx.x;
       if (p < n) {
         px[u] = x[p];
@@ -90,7 +93,7 @@ __global__ void __launch_bounds__(kMeshT) cell_count_kernel(
       }
     }
 #pragma unroll
-    for (int u = 0; u < kMeshUnroll; u++) {
+    for (int u = 0; u < U; u++) {
       uint32_t c = 0xffffffffu;
       if (base + u * kMeshT + threadIdx.x < n) {
         if (outside)
@@ -140,17 +143,17 @@ struct ToArrays {
   }
 };
 
-template <class R, class To>
+template <class R, int U, class To>
 __global__ void __launch_bounds__(kMeshT) cell_scatter_kernel(
     const R* __restrict__ x, const R* __restrict__ y, const R* __restrict__ z, uint64_t n,
     MeshGeom<R> g, uint32_t* __restrict__ cursor, To to) {
-  const uint64_t stride = (uint64_t)gridDim.x * kMeshT * kMeshUnroll;
+  const uint64_t stride = (uint64_t)gridDim.x * kMeshT * U;
   const unsigned lane = threadIdx.x & 31u;
-  for (uint64_t base = (uint64_t)blockIdx.x * kMeshT * kMeshUnroll; base < n; base += stride) {
-    R px[kMeshUnroll], py[kMeshUnroll], pz[kMeshUnroll];
-    uint32_t slot[kMeshUnroll], peers[kMeshUnroll];
+  for (uint64_t base = (uint64_t)blockIdx.x * kMeshT * U; base < n; base += stride) {
+    R px[U], py[U], pz[U];
+    uint32_t slot[U], peers[U];
 #pragma unroll
-    for (int u = 0; u < kMeshUnroll; u++) {
+    for (int u = 0; u < U; u++) {
       const uint64_t p = base + u * kMeshT + threadIdx.x;
       if (p < n) {
         px[u] = x[p];
@@ -159,7 +162,7 @@ __global__ void __launch_bounds__(kMeshT) cell_scatter_kernel(
       }
     }
 #pragma unroll
-    for (int u = 0; u < kMeshUnroll; u++) {
+    for (int u = 0; u < U; u++) {
       const bool valid = base + u * kMeshT + threadIdx.x < n;
       const uint32_t c = valid ? mesh_cell(px[u], py[u], pz[u], g) : 0xffffffffu;
       peers[u] = __match_any_sync(0xffffffffu, c);
@@ -167,7 +170,7 @@ __global__ void __launch_bounds__(kMeshT) cell_scatter_kernel(
         slot[u] = atomicAdd(cursor + c, (uint32_t)__popc(peers[u]));
     }
 #pragma unroll
-    for (int u = 0; u < kMeshUnroll; u++) {
+    for (int u = 0; u < U; u++) {
       const uint64_t p = base + u * kMeshT + threadIdx.x;
       const uint32_t s = __shfl_sync(0xffffffffu, slot[u], __ffs(peers[u]) - 1) +
                          __popc(peers[u] & ((1u << lane) - 1u));
@@ -288,14 +291,16 @@ __device__ __forceinline__ void canon_few(const MeshRec<R>* __restrict__ tmp, ui
 
 // Cells of up to kCanonSort entries, a warp each, or as many neighbours together
 // as hold 32 entries between them (a cell at a time 1 M particles in 100^3 cells
-// took 0.275 ms a call, now 0.148); the larger ones are listed in `more` (more[0] counts them) for
+// took 0.275 ms a call, now 0.148); the larger ones are listed in `more` (*n_more counts them) for
 // cell_canon_large_kernel, which takes four times the registers.
 template <class R>
 __global__ void __launch_bounds__(kCanonT, 4) cell_canon_kernel(
     const MeshRec<R>* __restrict__ tmp, const uint32_t* __restrict__ offsets,
     uint32_t n_cells_total, R* __restrict__ ox, R* __restrict__ oy, R* __restrict__ oz,
-    uint32_t* __restrict__ orig, uint32_t* __restrict__ more, uint32_t span) {
+    uint32_t* __restrict__ orig, uint32_t* __restrict__ more, uint32_t* __restrict__ n_more,
+    uint32_t span) {
   __shared__ uint32_t keys[kCanonT / 32 * kCanonSort];
+  cudaTriggerProgrammaticLaunchCompletion();
   const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
   uint32_t* wk = keys + warp * kCanonSort;
   const uint32_t warps = gridDim.x * (kCanonT / 32);
@@ -325,7 +330,7 @@ __global__ void __launch_bounds__(kCanonT, 4) cell_canon_kernel(
       } else if (cnt <= kCanonSort) {
         canon_cell<8>(tmp, s, e, wk, ox, oy, oz, orig);
       } else if (lane == 0) {
-        more[1 + atomicAdd(more, 1u)] = c0 + k;
+        more[atomicAdd(n_more, 1u)] = c0 + k;
       }
       k = k2;
     }
@@ -338,21 +343,22 @@ __global__ void __launch_bounds__(kCanonT, 4) cell_canon_kernel(
 template <class R>
 __global__ void __launch_bounds__(kCanonT) cell_canon_large_kernel(
     const MeshRec<R>* __restrict__ tmp, const uint32_t* __restrict__ offsets,
-    const uint32_t* __restrict__ more, R* __restrict__ ox, R* __restrict__ oy, R* __restrict__ oz,
-    uint32_t* __restrict__ orig) {
+    const uint32_t* __restrict__ more, const uint32_t* __restrict__ n_more, R* __restrict__ ox,
+    R* __restrict__ oy, R* __restrict__ oz, uint32_t* __restrict__ orig) {
   __shared__ uint32_t keys[kCanonT / 32 * kCanonLarge];
-  const uint32_t n = more[0];
+  cudaGridDependencySynchronize();
+  const uint32_t n = *n_more;
   const unsigned warp = threadIdx.x >> 5;
   uint32_t* wk = keys + warp * kCanonLarge;
   for (uint32_t i = blockIdx.x * (kCanonT / 32) + warp; i < n; i += gridDim.x * (kCanonT / 32)) {
-    const uint32_t s = offsets[more[1 + i]], e = offsets[more[1 + i] + 1];
+    const uint32_t s = offsets[more[i]], e = offsets[more[i] + 1];
     if (e - s <= kCanonLarge / 2)
       canon_cell<16>(tmp, s, e, wk, ox, oy, oz, orig);
     else if (e - s <= kCanonLarge)
       canon_cell<32>(tmp, s, e, wk, ox, oy, oz, orig);
   }
   for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
-    const uint32_t s = offsets[more[1 + i]], e = offsets[more[1 + i] + 1];
+    const uint32_t s = offsets[more[i]], e = offsets[more[i] + 1];
     if (e - s <= kCanonLarge) continue;
     for (uint32_t p0 = s; p0 < e; p0 += kCanonT) {
       const uint32_t p = p0 + threadIdx.x;
@@ -374,7 +380,7 @@ __global__ void __launch_bounds__(kCanonT) cell_canon_large_kernel(
 
 size_t mesh_scratch_bytes(uint64_t n_particles, uint32_t n_cells) {
   const uint64_t cells = (uint64_t)n_cells * n_cells * n_cells;
-  return n_particles * sizeof(MeshRec<float>) + (cells + 1) * sizeof(uint32_t) + 1024;
+  return n_particles * sizeof(MeshRec<float>) + (cells + 2) * sizeof(uint32_t) + 1024;
 }
 
 template <class R>
@@ -382,8 +388,13 @@ static MeshGeom<R> mesh_geom(const DeviceMeshT<R>& m) {
   return MeshGeom<R>{m.n_cells, m.box_length, R(1.0f) / m.cell_length};
 }
 
+// cells + 1 counts, then starts and cursors; then how many cells are large.
 static uint32_t* mesh_cursor(void* scratch, uint64_t n_particles, size_t record) {
   return (uint32_t*)((char*)scratch + ((n_particles * record + 255) & ~(size_t)255));
+}
+
+static unsigned mesh_grid(uint64_t n) {
+  return grid_for(n, kMeshT * (n <= kMeshFew ? 1 : kMeshUnroll), 152u * 8u);
 }
 
 template <class R>
@@ -391,8 +402,9 @@ void mesh_count(const R* x, const R* y, const R* z, uint64_t n_particles, const 
                 void* scratch, cudaStream_t st, const R* bounds, unsigned long long* outside) {
   const uint64_t cells = (uint64_t)m.n_cells * m.n_cells * m.n_cells;
   uint32_t* cursor = mesh_cursor(scratch, n_particles, sizeof(MeshRec<R>));
-  SIFG_CUDA(cudaMemsetAsync(cursor, 0, (cells + 1) * sizeof(uint32_t), st));
-  cell_count_kernel<R><<<grid_for(n_particles, kMeshT * kMeshUnroll, 152u * 8u), kMeshT, 0, st>>>(
+  SIFG_CUDA(cudaMemsetAsync(cursor, 0, (cells + 2) * sizeof(uint32_t), st));
+  (n_particles <= kMeshFew ? cell_count_kernel<R, 1> : cell_count_kernel<R, kMeshUnroll>)<<<
+      mesh_grid(n_particles), kMeshT, 0, st>>>(
       x, y, z, n_particles, mesh_geom(m), cursor, bounds ? bounds[0] : R(0), bounds ? bounds[1] : R(0),
       bounds ? outside : nullptr);
   SIFG_LAUNCH_CHECK();
@@ -406,35 +418,48 @@ void mesh_build(const R* x, const R* y, const R* z, uint64_t n_particles, Device
   const uint64_t cells = (uint64_t)m.n_cells * m.n_cells * m.n_cells;
   MeshRec<R>* tmp = (MeshRec<R>*)scratch;
   uint32_t* cursor = mesh_cursor(scratch, n_particles, sizeof(MeshRec<R>));
-  const unsigned grd = grid_for(n_particles, kMeshT * kMeshUnroll, 152u * 8u);
   if (timer) timer->begin(st);
   if (!counted) mesh_count(x, y, z, n_particles, m, scratch, st, (const R*)nullptr, nullptr);
   exclusive_scan_u32(cursor, (uint32_t)(cells + 1), st, scan_sums);
   SIFG_CUDA(cudaMemcpyAsync(m.offsets, cursor, (cells + 1) * sizeof(uint32_t),
                             cudaMemcpyDeviceToDevice, st));
+  auto scatter = [&](auto to) {
+    (n_particles <= kMeshFew ? cell_scatter_kernel<R, 1, decltype(to)>
+                             : cell_scatter_kernel<R, kMeshUnroll, decltype(to)>)<<<
+        mesh_grid(n_particles), kMeshT, 0, st>>>(x, y, z, n_particles, g, cursor, to);
+    SIFG_LAUNCH_CHECK();
+  };
   if (!canonical) {
     if constexpr (sizeof(R) == 4)
-      cell_scatter_kernel<R><<<grd, kMeshT, 0, st>>>(x, y, z, n_particles, g, cursor, ToXyzw{m.xyzw});
+      scatter(ToXyzw{m.xyzw});
     else
-      cell_scatter_kernel<R><<<grd, kMeshT, 0, st>>>(x, y, z, n_particles, g, cursor,
-                                                     ToArrays<R>{m.x, m.y, m.z});
-    SIFG_LAUNCH_CHECK();
+      scatter(ToArrays<R>{m.x, m.y, m.z});
     if (timer) timer->end(st);
     m.n_particles = n_particles;
     return;
   }
-  cell_scatter_kernel<R><<<grd, kMeshT, 0, st>>>(x, y, z, n_particles, g, cursor, ToRecord<R>{tmp});
-  SIFG_LAUNCH_CHECK();
+  scatter(ToRecord<R>{tmp});
   // The scatter's cursors are free: the list of the large cells.
-  uint32_t* more = cursor;
-  SIFG_CUDA(cudaMemsetAsync(more, 0, sizeof(uint32_t), st));
+  uint32_t *more = cursor, *n_more = cursor + cells + 1;
   // As many neighbours a warp as still leave every SM its warps.
   const uint32_t span = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(cells / (152u * 64u), 1), 32);
   cell_canon_kernel<R><<<grid_for(cells, kCanonT / 32 * span, 152u * 8u), kCanonT, 0, st>>>(
-      tmp, m.offsets, (uint32_t)cells, m.x, m.y, m.z, m.orig, more, span);
+      tmp, m.offsets, (uint32_t)cells, m.x, m.y, m.z, m.orig, more, n_more, span);
   SIFG_LAUNCH_CHECK();
-  cell_canon_large_kernel<R><<<(unsigned)std::min<uint64_t>(cells, 152u * 2u), kCanonT, 0, st>>>(
-      tmp, m.offsets, more, m.x, m.y, m.z, m.orig);
+  // Mostly with nothing to do: launched beside the kernel above, whose end it
+  // waits for, so that its launch does not come after (10,000 particles: 3 us).
+  cudaLaunchAttribute beside{};
+  beside.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  beside.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t large{};
+  large.gridDim = (unsigned)std::min<uint64_t>(cells, 152u * 2u);
+  large.blockDim = kCanonT;
+  large.stream = st;
+  large.attrs = &beside;
+  large.numAttrs = 1;
+  SIFG_CUDA(cudaLaunchKernelEx(&large, cell_canon_large_kernel<R>, (const MeshRec<R>*)tmp,
+                               (const uint32_t*)m.offsets, (const uint32_t*)more,
+                               (const uint32_t*)n_more, m.x, m.y, m.z, m.orig));
   SIFG_LAUNCH_CHECK();
   if (timer) timer->end(st);
   m.n_particles = n_particles;
