@@ -180,7 +180,6 @@ template <class R>
 static int count_cells(const R* dx, const R* dy, const R* dz, uint64_t n, const DeviceMeshT<R>& m,
                        void* scratch, cudaStream_t st, DevBuf& flag) {
   unsigned long long* d = (unsigned long long*)flag.ensure(16);
-  SIFG_CUDA(cudaMemsetAsync(d, 0, 16, st));
   R bounds[2];
   box_bounds(m.box_length, &bounds[0], &bounds[1]);
   mesh_count(dx, dy, dz, n, m, scratch, st, (const R*)bounds, d);

@@ -403,6 +403,7 @@ void mesh_count(const R* x, const R* y, const R* z, uint64_t n_particles, const 
   const uint64_t cells = (uint64_t)m.n_cells * m.n_cells * m.n_cells;
   uint32_t* cursor = mesh_cursor(scratch, n_particles, sizeof(MeshRec<R>));
   SIFG_CUDA(cudaMemsetAsync(cursor, 0, (cells + 2) * sizeof(uint32_t), st));
+  if (bounds) SIFG_CUDA(cudaMemsetAsync(outside, 0, sizeof(*outside), st));
   (n_particles <= kMeshFew ? cell_count_kernel<R, 1> : cell_count_kernel<R, kMeshUnroll>)<<<
       mesh_grid(n_particles), kMeshT, 0, st>>>(
       x, y, z, n_particles, mesh_geom(m), cursor, bounds ? bounds[0] : R(0), bounds ? bounds[1] : R(0),
