@@ -531,11 +531,27 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
   // small launches leaves most of the GPU idle up to about 256^3 (64^3: 35 us
   // of launches one waiting on another, 25 us of kernels on a few SMs), and
   // rung after rung without a candidate waits for nothing else: four lanes;
-  // past that two, whose kernels fill one another's tails. An engine of a batch
-  // has the other engines for that: one stream.
+  // past that two, whose kernels fill one another's tails (a search at 300^3
+  // 7.14 to 6.68 ms, 384^3 12.8 to 12.5, 500^3 28.1 to 27.7; FP64 at 300^3 105.2
+  // to 103.7, 512^3 328 to 327). A second lane holds another transform input and
+  // work area, 8 or 16 bytes a cell: past 2^28 cells, where it gives nothing (640^3
+  // 56.0 either way, 768^3 111.3 to 110.5), and where the GPU has no room for
+  // twice the lanes' buffers, one stream and two fields do. An engine of a batch
+  // has the other engines to fill the GPU: one stream.
   const bool own = !p.inject && sizeof(R) == 4 && N == 512;
-  const bool one_stream = own || in_batch;
-  const uint32_t lanes = one_stream || p.inject || cells > (1ull << 24) ? 2 : kLanes;
+  const bool lane_scans = !gaussian && !p.inject && scan_is_one_launch(cells);
+  bool one_stream = own || in_batch || p.inject || cells > (1ull << 28);
+  uint32_t lanes = one_stream || cells > (1ull << 24) ? 2 : kLanes;
+  if (!one_stream && field_[lanes - 1].bytes < cells * sizeof(R)) {
+    const size_t values = (1 + (gaussian ? 1 : 0) + (survey ? 1 : 0)) * sizeof(R);
+    const size_t transform = (survey ? 4 : 2) * sizeof(R), lists = lane_scans ? sizeof(R) + 4 : 0;
+    size_t free_bytes = 0, all = 0;
+    SIFG_CUDA(cudaMemGetInfo(&free_bytes, &all));
+    if (free_bytes / 2 < cells * lanes * (values + transform + lists)) {
+      one_stream = true;
+      lanes = 2;
+    }
+  }
   R *fields[kLanes], *gfields[kLanes], *rfields[kLanes];
   for (uint32_t k = 0; k < lanes; k++) fields[k] = grow_to<R>(field_[k], cells);
   // The refinement's own fields (the top-hat times the Gaussian), alongside.
@@ -583,17 +599,19 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
   // scan is a mask filter over that list; two lists alternate with the fields.
   BelowList below[kLanes];
   bool listed = false;
-  // A lane's scan buffers (the list's passes use lane 0's block counts).
+  // A lane's scan buffers; lane 0's do where every scan is the run's stream's,
+  // one after another.
   const uint32_t nb_below = (uint32_t)((cells + kBelowBlock - 1) / kBelowBlock);
   uint32_t* blocks[kLanes] = {};
   R* region_delta[kLanes] = {};
   uint32_t* region_flat[kLanes] = {};
   auto scan_buffers = [&](uint32_t lane) {
-    blocks[lane] = grow_to<uint32_t>(blocks_[lane],
+    const uint32_t k = lane_scans && !listed ? lane : 0;
+    blocks[lane] = grow_to<uint32_t>(blocks_[k],
                                      std::max<size_t>(std::max(scan_blocks(cells), nb_below) + 1, 1024));
     if (listed) return;
-    region_delta[lane] = grow_to<R>(region_delta_[lane], scan_region_slots(cells));
-    region_flat[lane] = grow_to<uint32_t>(region_flat_[lane], scan_region_slots(cells));
+    region_delta[lane] = grow_to<R>(region_delta_[k], scan_region_slots(cells));
+    region_flat[lane] = grow_to<uint32_t>(region_flat_[k], scan_region_slots(cells));
   };
   // Until the first void is accepted no cell is masked, and a rung's candidates
   // do not wait for the rung before: its scan follows its smoothing on its lane,
@@ -632,7 +650,7 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
       survey_contrast(fields[lane], (const R*)rfields[lane], occ, p.survey_alpha, cells, fs);
     }
     if (tm) tm->smoothing.end(fs);
-    ahead[lane] = mask_empty && !listed && !gaussian && scan_is_one_launch(cells);
+    ahead[lane] = mask_empty && lane_scans && !listed;
     if (ahead[lane]) {
       scan_buffers(lane);
       scan_fused_pass(fields[lane], mask, cells, threshold, blocks[lane], h_ahead + lane,
