@@ -536,12 +536,17 @@ int Engine::exodus(const R* d_delta, const DeviceMeshT<R>& mesh, const RunParams
   // to 103.7, 512^3 328 to 327). A second lane holds another transform input and
   // work area, 8 or 16 bytes a cell: past 2^28 cells, where it gives nothing (640^3
   // 56.0 either way, 768^3 111.3 to 110.5), and where the GPU has no room for
-  // twice the lanes' buffers, one stream and two fields do. An engine of a batch
-  // has the other engines to fill the GPU: one stream.
+  // twice the lanes' buffers, one stream and two fields do. So they do for an
+  // engine of a batch, which has the other engines to fill the GPU, and for a
+  // size's first search, whose next ones make a lane each (the first searches at
+  // 128^3 2.8, 2.4, 2.8, 2.8, then 1.9 ms; with every lane made by the first, 4.8
+  // and then 1.9).
   const bool own = !p.inject && sizeof(R) == 4 && N == 512;
   const bool lane_scans = !gaussian && !p.inject && scan_is_one_launch(cells);
-  bool one_stream = own || in_batch || p.inject || cells > (1ull << 28);
-  uint32_t lanes = one_stream || cells > (1ull << 24) ? 2 : kLanes;
+  const uint32_t made = survey ? std::min(smoother.lanes_for(N), rsmoother_for<R>().lanes_for(N))
+                               : smoother.lanes_for(N);
+  bool one_stream = own || in_batch || p.inject || cells > (1ull << 28) || made < 2;
+  uint32_t lanes = one_stream || cells > (1ull << 24) ? 2 : made;
   if (!one_stream && field_[lanes - 1].bytes < cells * sizeof(R)) {
     const size_t values = (1 + (gaussian ? 1 : 0) + (survey ? 1 : 0)) * sizeof(R);
     const size_t transform = (survey ? 4 : 2) * sizeof(R), lists = lane_scans ? sizeof(R) + 4 : 0;

@@ -780,6 +780,15 @@ void SmootherT<R>::setup(uint32_t n_, R box_, int window_mode_, cudaStream_t st)
 }
 
 template <class R>
+uint32_t SmootherT<R>::lanes_for(uint32_t n_) const {
+  if (sizeof(R) == 8 && fft64_takes(n_)) return kLanes;  // no plans
+  for (const Plans& p : plans)
+    if (p.n == n_) return std::min<uint32_t>(kLanes, 2 + (uint32_t)std::count_if(p.lane, p.lane + kLanes - 1,
+                                                                               [](cufftHandle h) { return h != 0; }));
+  return 1;
+}
+
+template <class R>
 void SmootherT<R>::set_lanes(int lanes, const cudaStream_t* streams) {
   auto it = std::find_if(plans.begin(), plans.end(), [&](const Plans& p) { return p.n == n; });
   for (int k = 1; k < lanes; k++) {

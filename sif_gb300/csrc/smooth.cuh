@@ -66,6 +66,10 @@ struct SmootherT {
   };
   Lane extra[kLanes - 1];
   void set_lanes(int lanes, const cudaStream_t* streams);  // after setup
+  // The lanes a search at n takes, 1 for `stream` alone: those whose plans are
+  // made and one more. A plan and a lane's buffers take most of a millisecond,
+  // which one search does not gain, so each of a size's first makes one.
+  uint32_t lanes_for(uint32_t n) const;
   const void* twiddles = nullptr;
   std::vector<Plans> plans;
   // The own inverse's filter factors at n = 512, one table per smoothing

@@ -24,7 +24,9 @@ def test_lanes_find_what_the_fields_hold(gpu_lib, n, dtype):
     device.density_contrast(grid)
     mesh = device.chain_mesh(*xs, MESH, BOX)
     radii = np.array([30.0, 22.0, 16.0, 12.0, 10.0], dtype)
-    got = device.exodus(grid, n, BOX, mesh, MESH, radii, -0.75)
+    # A size's first search takes one stream, the ones after it a lane more each.
+    got = [device.exodus(grid, n, BOX, mesh, MESH, radii, -0.75) for _ in range(4)]
     fields = torch.cat([device.smooth(grid, n, BOX, float(r)) for r in radii])
     want = device.exodus(grid, n, BOX, mesh, MESH, radii, -0.75, inject=fields)
-    assert len(want[0]) > 5 and same_catalogue(got, want), (len(got[0]), len(want[0]))
+    assert len(want[0]) > 5
+    assert [same_catalogue(c, want) for c in got] == [True] * 4, [len(c[0]) for c in (*got, want)]
