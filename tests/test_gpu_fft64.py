@@ -67,3 +67,38 @@ def test_fp64_transforms_from_an_odd_double(dev, n):
     got = dev.smooth(delta, n, BOX, 1e-7, window="none")
     rms = float((got - delta).pow(2).mean().sqrt())
     assert rms <= _bar(n) / 2, rms
+
+
+@pytest.mark.parametrize("n", [128, 256])
+def test_fp64_transforms_lose_no_bits(dev, n):
+    """White noise there and back: a value's rounding at a level is a random
+    step of rms 2^-53 of the values at most (a rotation, a butterfly and the
+    constant between them, each uniform within half a unit), so the steps of 2
+    * 3 log2(n) levels and four more of the packing add up as their root."""
+    import torch
+
+    delta = torch.from_numpy(_noise(n)).cuda()
+    got = dev.smooth(delta, n, BOX, 1e-7, window="none")
+    rms = float((got - delta).pow(2).mean().sqrt() / delta.pow(2).mean().sqrt())
+    assert rms <= np.sqrt(2 * 3 * np.log2(n) + 4) * 2.0 ** -53, rms
+
+
+# One wave each, at the modes where the rows' packing and the columns' filter
+# change form, through a Gaussian: the wave times its factor, to what every
+# level's two units give when all of them go one way.
+@pytest.mark.parametrize("n", [128, 256])
+def test_fp64_transforms_of_single_waves(dev, n):
+    import torch
+
+    h = n // 2
+    i = torch.arange(n, dtype=torch.int64, device="cuda")
+    for kx, ky, kz in [(0, 0, 1), (0, 0, n // 8), (1, 0, n // 8 + 1), (0, 3, n // 4), (5, h, n // 4 - 1),
+                       (0, 0, h), (h, h, h), (h, 0, 0), (0, h, 0), (n - 1, 2, 0), (h - 1, h + 1, 3 * n // 8),
+                       (7, n - 7, h - 1)]:
+        turn = (kx * i[:, None, None] + ky * i[None, :, None] + kz * i[None, None, :]) % n
+        wave = torch.cos(2 * np.pi / n * turn.double()).reshape(-1)
+        got = dev.smooth(wave, n, BOX, RADIUS / 8, filter="gaussian", window="none")
+        k = [min(v, n - v) for v in (kx, ky, kz)]
+        factor = np.exp(-0.5 * (RADIUS / 8 * 2 * np.pi / BOX) ** 2 * sum(v * v for v in k))
+        err = float((got - factor * wave).abs().max())
+        assert err <= _bar(n) / 2, (kx, ky, kz, err)
