@@ -11,7 +11,8 @@
 //
 //   A rotation by an angle of at most pi/4 is cos (1 + i tan): the two fused
 //   multiply-adds of (1 + i tan) are applied and the cos is carried as the
-//   element's scale. A butterfly of two elements of scales a and b takes
+//   element's scale (as Linzer and Feig, 1993, and Goedecker, 1997, lay out
+//   transforms for fused multiply-adds). A butterfly of two elements of scales a and b takes
 //   x +- (b / a) y, four fused multiply-adds as four additions would have
 //   been, and leaves scale a. Quarter turns, which bring every angle within
 //   pi/4, are exchanges of parts and signs and no arithmetic. Decimation in
@@ -457,7 +458,7 @@ constexpr size_t column_bytes(bool filter) {
 
 template <int N>
 void set_smem() {
-  thread_local bool attr = false;  // the attribute is per thread's view of the function
+  thread_local bool attr = false;  // set once a thread: one device a process
   if (attr) return;
   SIFG_CUDA(cudaFuncSetAttribute(columns64_kernel<N, kFilterPass>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)column_bytes<N>(true)));

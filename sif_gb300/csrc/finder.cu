@@ -418,7 +418,7 @@ __device__ __forceinline__ uint32_t void_axis(R c, R inv) {
 }
 
 // Whether void j's index cell lies in the window of cells [x0, x1] x [y0, y1] x
-// [z0, z1] (taken modulo the index, as the walk above takes them).
+// [z0, z1] (taken modulo the index, as the walk over cells takes them).
 template <class R>
 __device__ __forceinline__ bool in_window(const VoidViewT<R>& v, R vx, R vy, R vz, int32_t x0,
                                           int32_t x1, int32_t y0, int32_t y1, int32_t z0, int32_t z1) {
@@ -1768,7 +1768,7 @@ void grow(MeshViewT<R> mesh, TemplateViewT<R> tpl, RungConstsT<R> rc, SurvivorsT
     if (g_shell_list >= 0)
       shell_cap = std::min<uint32_t>(kShellListMax, ((uint32_t)g_shell_list + 31u) & ~31u);
     const size_t smem = warp_slice_bytes<R>(nb_stride, shell_cap) * kGrowWarps;
-    thread_local size_t attr_bytes = 0;  // the attribute is per thread's view of the function
+    thread_local size_t attr_bytes = 0;  // set once a thread: one device a process
     if (smem > attr_bytes) {
       SIFG_CUDA(cudaFuncSetAttribute(growth_warp_kernel<R>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -2146,7 +2146,7 @@ void grow_weighted(MeshViewT<R> mesh, TemplateViewT<R> tpl, RungConstsT<R> rc, S
                    uint32_t* work) {
   if (max_survivors == 0) return;
   const size_t smem = weighted_smem_bytes<R>((rc.nb + 1) & ~1u);
-  thread_local bool attr = false;  // the attribute is per thread's view of the function
+  thread_local bool attr = false;  // set once a thread: one device a process
   if (!attr) {
     SIFG_CUDA(cudaFuncSetAttribute(growth_weighted_kernel<R>,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2496,7 +2496,7 @@ void grow_survey(MeshViewT<R> dm, TemplateViewT<R> dt, MeshViewT<R> rm, Template
                  KernelTimer* timer, uint32_t* work) {
   if (max_survivors == 0) return;
   constexpr size_t smem = survey_smem_bytes<R>();
-  thread_local bool attr = false;  // the attribute is per thread's view of the function
+  thread_local bool attr = false;  // set once a thread: one device a process
   if (!attr) {
     SIFG_CUDA(cudaFuncSetAttribute(growth_survey_kernel<R>,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -2504,8 +2504,8 @@ void grow_survey(MeshViewT<R> dm, TemplateViewT<R> dt, MeshViewT<R> rm, Template
   }
   const unsigned g = max_survivors < growth_grid() ? max_survivors : growth_grid();
   if (timer) timer->begin(st);
-  growth_survey_kernel<R><<<g, max_survivors <= 152u ? kSurveyMaxT : kSurveyT, smem, st>>>(dm, dt, rm, rt, rc, K, s, gbuf, gwbuf, gcap,
-                                                  traffic, work);
+  growth_survey_kernel<R><<<g, max_survivors <= 152u ? kSurveyMaxT : kSurveyT, smem, st>>>(
+      dm, dt, rm, rt, rc, K, s, gbuf, gwbuf, gcap, traffic, work);
   SIFG_LAUNCH_CHECK();
   if (timer) timer->end(st);
 }
@@ -3221,9 +3221,14 @@ void build_void_index(const R* cx, const R* cy, const R* cz, uint32_t n, R box,
 // scanned and filled from the counts commit_init left, the rounds, the
 // accepted voids appended in rank order, and the void index rebuilt, the
 // outcome written straight to pinned host memory. Eight blocks (the portable
-// cluster) hold 2,048 threads, so this is for up to kSmallSurvivors; past that
-// the rounds want the whole GPU. (201^3 particles on 243^3, rungs of 5 to 2,351
-// candidates: see the rule at commit_small.)
+// cluster) hold 2,048 threads, so this is for up to kSmallSurvivors candidates;
+// past that the rounds want the whole GPU. Whole rungs of float searches, this
+// against the chain: up to 1,000 candidates 1.2 to 1.5 times as fast (174 us
+// for 258 at 499), at 2,400 to 2,700 1.06 to 1.2, at 3,717 1.09 (404 for 441). The
+// FP64 form gains the same up to 1,000 and is even or up to a tenth behind
+// between 1,400 and 3,800, its tests on eight SMs' FP64 pipes: whole searches
+// the same within 1% with the line at 1,024 (128^3 20.1 for 20.2 ms, 256^3 47.0
+// for 46.6), so one line for both.
 constexpr int kSmallT = 256;
 constexpr int kSmallCtas = 8;
 constexpr uint32_t kVoidIndexCells = kVoidCells * kVoidCells * kVoidCells;
@@ -3413,8 +3418,8 @@ bool commit_is_small(uint32_t max_survivors) {
 //
 // The chain of survivors bounds it. One thread walking the window's cells (up to
 // thousands, each a dependent load, for some hundred voids) and a sphere painted
-// at a time, the kernel took 2.7 ms of
-// the excursion-peak 256^3 search, 7.9 ms in all; now 0.3 of 4.5.
+// at a time, the kernel took 2.7 ms of the excursion-peak 256^3 search, 7.9 ms
+// in all; now 0.3 of 4.5.
 
 // The void index as linked chains: head per cell of the 32^3 index, next per
 // void, -1 ends a chain.
@@ -3590,9 +3595,10 @@ __device__ __forceinline__ bool conflict(const VoidListT<R>& vl, uint32_t j, R c
 }
 
 // Whether survivor i is accepted against the catalogue as it stands (0: no, 1:
-// yes, 2: yes, displacing voids), by a warp: the rescaling succeeded; the node's mask bit; the poles and the exact overlap
-// at the rung radius (sif__overlap_exact, src/finder/utils.c:850-960); then at
-// the rescaled radius (find_conflicts) no void it collides with is as large.
+// yes, 2: yes, displacing voids), by a warp: the rescaling succeeded; the node's
+// mask bit; the poles and the exact overlap at the rung radius
+// (sif__overlap_exact, src/finder/utils.c:850-960); then at the rescaled radius
+// (find_conflicts) no void it collides with is as large.
 template <class R>
 __device__ uint32_t displace_test(const SurvivorsT<R>& sv, uint32_t i, const VoidListT<R>& vl, uint32_t n,
                               R max_r, const uint32_t* mask, const RungConstsT<R>& rc) {

@@ -225,7 +225,7 @@ void witness(MeshViewT<R> mesh, TemplateViewT<R> tpl, RungConstsT<R> rc, Survivo
              VoidViewT<R> voids, uint32_t max_survivors, unsigned long long* traffic,
              cudaStream_t st, KernelTimer* timer, uint32_t* work);
 
-// 1 (default): the witness runs; 0: every survivor is grown. The catalogue
+// 0 (default): every survivor is grown; 1: the witness runs. The catalogue
 // does not depend on it (tests run both).
 void set_witness(int on);
 bool witness_on();

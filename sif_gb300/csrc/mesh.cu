@@ -10,9 +10,11 @@
 //   2. exclusive scan, copied to the cell offsets;
 //   3. cell_scatter: (source index, x, y, z) into each cell's range, in the
 //      order the atomics hand out slots;
-//   4. cell_canon:  per entry, its rank among its cell's source indices (a
-//      count over the cell's keys in shared memory), and the entry written
-//      to that rank -- the canonical order, which no atomic race can change.
+//   4. cell_canon:  per entry, its rank among its cell's source indices, and
+//      the entry written to that rank -- the canonical order, which no atomic
+//      race can change. The rank by a warp's sort of the cell's keys (up to
+//      1,024 of them; neighbouring cells of a few entries together) or, in a
+//      larger cell, by a CTA's count of the smaller ones.
 #include <cuda_runtime.h>
 
 #include <algorithm>

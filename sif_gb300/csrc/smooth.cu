@@ -871,7 +871,7 @@ static void launch_columns(const SmootherT<float>& s, const DevBuf& src, const D
                            ColumnLayout in, ColumnLayout out, const RadialFilter& rf = kNoFilter,
                            const float* win = nullptr, float norm = 1.f, const float* ftab = nullptr,
                            bool backwards = false) {
-  thread_local bool attr = false;  // the attribute is per thread's view of the function
+  thread_local bool attr = false;  // set once a thread: one device a process
   if (!attr) {
     SIFG_CUDA(cudaFuncSetAttribute(colfft512_kernel<kMode>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)kColBytes));
