@@ -70,7 +70,6 @@ Engine::Engine(int device) : device_(device) {
 
 Engine::~Engine() {
   cudaFreeHost(h_delta_);
-  cudaFreeHost(h_flat_);
   cudaFreeHost(h_rank_);
   cudaFreeHost(h_counters_);
   if (ev_cand_) cudaEventDestroy(ev_cand_);
@@ -88,11 +87,9 @@ Engine::~Engine() {
 void Engine::ensure_host(size_t m) {
   if (m <= h_cap_) return;
   cudaFreeHost(h_delta_);
-  cudaFreeHost(h_flat_);
   cudaFreeHost(h_rank_);
   const size_t cap = m + m / 4 + 1024;
   SIFG_CUDA(cudaMallocHost(&h_delta_, cap * sizeof(double)));
-  SIFG_CUDA(cudaMallocHost(&h_flat_, cap * sizeof(uint32_t)));
   SIFG_CUDA(cudaMallocHost(&h_rank_, cap * sizeof(uint32_t)));
   h_cap_ = cap;
 }

@@ -214,7 +214,6 @@ class Engine {
   DevBuf below_counts_[2], below_delta_[2], below_flat_[2];  // the smoothing's below-threshold lists
   std::vector<uint8_t> h_tpl_;  // the packed template, staged for its upload
   void* h_delta_ = nullptr;  // candidate depths, float or double
-  uint32_t* h_flat_ = nullptr;
   uint32_t* h_rank_ = nullptr;
   uint32_t* h_counters_ = nullptr;
   size_t h_cap_ = 0;
@@ -224,7 +223,7 @@ class Engine {
   // and rung i's growth and commit.
   cudaStream_t st_fft_[kLanes] = {}, st_copy_ = 0;
   cudaEvent_t ev_copy_start_ = nullptr, ev_mesh_ready_ = nullptr;
-  cudaEvent_t ev_start_ = nullptr, ev_forward_ = nullptr, ev_tables_ = nullptr, 
+  cudaEvent_t ev_start_ = nullptr, ev_forward_ = nullptr, ev_tables_ = nullptr,
               ev_smoothed_[kLanes] = {}, ev_scanned_[kLanes] = {};
   void ensure_host(size_t m);
 };
