@@ -314,10 +314,14 @@ __global__ void __launch_bounds__(kCanonT, 4) cell_canon_kernel(
     const uint32_t first = lane < nc ? offsets[c0 + lane] : 0u;
     const uint32_t next = __shfl_down_sync(0xffffffffu, first, 1);
     const uint32_t end = lane + 1 == nc ? offsets[c0 + nc] : next;  // of lane's cell
+    // Past a half warp's entries a cell no two share a warp, and looking for
+    // some costs 64.5 M particles in 117^3 cells 1% of the call.
+    const bool few = __shfl_sync(0xffffffffu, end, nc - 1) - __shfl_sync(0xffffffffu, first, 0) <= 16u * nc;
     for (uint32_t k = 0; k < nc;) {
       const uint32_t s = __shfl_sync(0xffffffffu, first, k);
       // The cells from the k-th whose entries fit in the warp.
-      const uint32_t fit = __popc(__ballot_sync(0xffffffffu, lane >= k && lane < nc && end - s <= 32u));
+      uint32_t fit = 0;
+      if (few) fit = __popc(__ballot_sync(0xffffffffu, lane >= k && lane < nc && end - s <= 32u));
       const uint32_t k2 = k + max(fit, 1u);
       const uint32_t e = __shfl_sync(0xffffffffu, end, k2 - 1), cnt = e - s;
       if (cnt == 0) {
