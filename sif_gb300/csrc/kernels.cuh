@@ -166,12 +166,10 @@ size_t mesh_scratch_bytes(uint64_t n_particles, uint32_t n_cells);
 // mesh_count is the build's first pass on its own, for a caller that checks
 // the positions before anything of the mesh is written (bounds, outside: as
 // cic_count's): it counts into the scratch, and a build with `counted` set
-// goes on from there. timer: a span of the pass (a build's own span has it when
-// the build makes it).
+// goes on from there.
 template <class R>
 void mesh_count(const R* x, const R* y, const R* z, uint64_t n_particles, const DeviceMeshT<R>& m,
-                void* scratch, cudaStream_t st, const R* bounds, unsigned long long* outside,
-                KernelTimer* timer = nullptr);
+                void* scratch, cudaStream_t st, const R* bounds, unsigned long long* outside);
 template <class R>
 void mesh_build(const R* x, const R* y, const R* z, uint64_t n_particles, DeviceMeshT<R>& m,
                 void* scratch, cudaStream_t st, KernelTimer* timer, uint32_t* scan_sums = nullptr,

@@ -405,19 +405,16 @@ static unsigned mesh_grid(uint64_t n) {
 
 template <class R>
 void mesh_count(const R* x, const R* y, const R* z, uint64_t n_particles, const DeviceMeshT<R>& m,
-                void* scratch, cudaStream_t st, const R* bounds, unsigned long long* outside,
-                KernelTimer* timer) {
+                void* scratch, cudaStream_t st, const R* bounds, unsigned long long* outside) {
   const uint64_t cells = (uint64_t)m.n_cells * m.n_cells * m.n_cells;
   uint32_t* cursor = mesh_cursor(scratch, n_particles, sizeof(MeshRec<R>));
   SIFG_CUDA(cudaMemsetAsync(cursor, 0, (cells + 2) * sizeof(uint32_t), st));
   if (bounds) SIFG_CUDA(cudaMemsetAsync(outside, 0, sizeof(*outside), st));
-  if (timer) timer->begin(st);
   (n_particles <= kMeshFew ? cell_count_kernel<R, 1> : cell_count_kernel<R, kMeshUnroll>)<<<
       mesh_grid(n_particles), kMeshT, 0, st>>>(
       x, y, z, n_particles, mesh_geom(m), cursor, bounds ? bounds[0] : R(0), bounds ? bounds[1] : R(0),
       bounds ? outside : nullptr);
   SIFG_LAUNCH_CHECK();
-  if (timer) timer->end(st);
 }
 
 template <class R>
@@ -553,9 +550,9 @@ template void mesh_build<double>(const double*, const double*, const double*, ui
                                  uint32_t*, bool, bool);
 template void mesh_count<float>(const float*, const float*, const float*, uint64_t,
                                 const DeviceMeshT<float>&, void*, cudaStream_t, const float*,
-                                unsigned long long*, KernelTimer*);
+                                unsigned long long*);
 template void mesh_count<double>(const double*, const double*, const double*, uint64_t,
                                  const DeviceMeshT<double>&, void*, cudaStream_t, const double*,
-                                 unsigned long long*, KernelTimer*);
+                                 unsigned long long*);
 
 }  // namespace sifg
